@@ -5,6 +5,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <unordered_map>
 #include <utility>
 
@@ -51,6 +52,40 @@ int current_device_once(const void *key, int (*init)(void *arg, int *value), voi
   if (int rc = check_cuda(cudaGetDevice(&device), "cudaGetDevice"))
     return rc;
   return per_device_once(key, device, init, arg, value);
+}
+
+int resident_blocks(const void *kernel, int threads, size_t dynamic_smem, int *blocks) {
+  struct Key {
+    const void *kernel;
+    int device, threads;
+    size_t smem;
+    bool operator<(const Key &o) const {
+      return std::tie(kernel, device, threads, smem) < std::tie(o.kernel, o.device, o.threads, o.smem);
+    }
+  };
+  static std::map<Key, int> known;
+  static std::map<std::pair<const void *, int>, size_t> opted_in; // the limit is per function: it only grows
+  Key key{kernel, 0, threads, dynamic_smem};
+  if (int rc = check_cuda(cudaGetDevice(&key.device), "cudaGetDevice"))
+    return rc;
+  std::lock_guard<std::mutex> lock(g_once_mutex);
+  const auto it = known.find(key);
+  if (it != known.end()) {
+    *blocks = it->second;
+    return kOk;
+  }
+  size_t &limit = opted_in[{kernel, key.device}];
+  if (dynamic_smem > 48 * 1024 && dynamic_smem > limit) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic_smem),
+                            "cudaFuncSetAttribute(dynamic shared memory)"))
+      return rc;
+    limit = dynamic_smem;
+  }
+  int n = 0;
+  if (int rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, dynamic_smem), "occupancy"))
+    return rc;
+  known[key] = *blocks = n < 1 ? 1 : n;
+  return kOk;
 }
 
 void set_last_error(const std::string &text) { g_last_error = text; }

@@ -35,6 +35,11 @@ int sm_count();
 int per_device_once(const void *key, int device, int (*init)(void *arg, int *value), void *arg, int *value);
 int current_device_once(const void *key, int (*init)(void *arg, int *value), void *arg, int *value);
 
+// Blocks of `kernel` that are resident at once on one SM of the current device with this block size
+// and dynamic shared memory; opts the kernel in to that much shared memory the first time. The
+// answer is a property of the device and is looked up once per (kernel, device, block, bytes).
+int resident_blocks(const void *kernel, int threads, size_t dynamic_smem, int *blocks);
+
 // Device-side status words written by kernels whose bounded waits ran out. Index 0 is a
 // sticky flag, 1..3 describe where (kernel id, role, iteration).
 struct DeviceStatus {

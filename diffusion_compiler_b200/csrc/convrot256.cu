@@ -1,0 +1,595 @@
+// QuantizeInt8Rows for sm_100a, the 256-wide ConvRot variants: orthogonal block rotation fused with
+// per-row absmax INT8 quantisation. Semantics follow the reference opcode bit for bit (reference
+// src/runtime/cpu_executor.cpp:124-307; generated GPU kernel src/compiler/compiler.cpp:635-845).
+// bf16 is read once from HBM, codes and scales are written once.
+//
+// A 256-wide group is the Kronecker product H4 (x) H4 (x) H4 (x) H4, applied as four radix-4 stages with
+// strides 1, 4, 16, 64 in exactly the reference's fp32 association order ((x0+x1)+x2)-x3 etc. The
+// reference multiplies every stage by 0.5; a multiplication by a power of two commutes with fp32
+// rounding, so the kernel skips it and carries values scaled by 16, folding the factor into the
+// divisor. Results are bit-identical unless an intermediate leaves the normal fp32 range.
+//
+// Layout. A warp works on 4 groups (1024 columns) at a time; each thread owns 16 consecutive elements of
+// two neighbouring groups as 16 packed fp32x2 registers (lane 0 of the pair = first group, lane 1 =
+// second group), so every butterfly is one packed add/sub for two groups. Stages 0-1 run on the
+// thread's own 16 elements; a 16x16 transpose through shared memory (XOR-swizzled, conflict-free)
+// gives the thread the 16 elements of stride 16, on which stages 2-3 run.
+//
+// What bounds it: the SM's arithmetic and its issue slots, not HBM (3 bytes per element against about 16
+// thread instructions, 5 of them packed additions that take two clocks each). A warp therefore takes
+// up to three such blocks of its row (NIT) before it needs the row's scale: the scale arithmetic, the
+// reductions and the loop overhead are paid once per 96 elements of a thread instead of once per 32, and
+// a row of up to 3072 columns needs no barrier at all. Between rotation and quantisation the bf16
+// variants keep the values as packed bf16 (their result is defined on the rounded values), half the
+// registers of fp32. The one-block form instead fits 64 registers, so that 32 warps per SM hide the
+// load latency without a prefetch. Measured against the one-block form with 80 registers and fp32
+// values that came before: 33272 x 3072 93.4 -> 86.9 us, 33272 x 8192 249 -> 226 us, 9216 x 12288 (signed)
+// 124 -> 111 us, 9216 x 3072 30.2 -> 28.8 us; the scale search of the weight form 12288 x 3072 454 -> 78 us
+// (all lanes evaluate samples, doubles only where the square needs them), with input equalisation
+// 478 -> 118 us; with RmsNormModulate in front 33272 x 3072 262 -> 145 us (packed arithmetic, 24 warps
+// instead of 16). Staging the input with bulk copies through shared memory instead of registers gave
+// nothing (30.0 us and 93.7 us for the first and third shape): loads are not what it waits for.
+#include "quant_common.cuh"
+
+namespace difb200 {
+namespace {
+
+// Shared memory per warp: 4 groups x 256 fp32 (two swizzled 16x32-word transposes), reused for the
+// code bytes and the sampled elements of the scale search.
+constexpr int kWarpBytes = 4096;
+
+enum Extra { kPlain = 0, kPack = 1, kNorm = 2 };
+
+// 32 bytes of one thread: one 256-bit load where every run starts on 32 bytes, else two of 128 bits.
+__device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, uint4 &b) {
+  if (wide) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(src));
+  } else {
+    a = __ldg(src);
+    b = __ldg(src + 1);
+  }
+}
+
+template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB)
+convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_per_cta) {
+  static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
+  extern __shared__ __align__(128) uint32_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = warp / warps_per_row;         // which row of this CTA's batch
+  const int wrow = warp - slot * warps_per_row;  // warp index inside the row
+  const int h = lane >> 4, a = lane & 15;
+  const int total_warps = blockDim.x >> 5;
+  const uint32_t smem_addr = smem_u32(smem);
+  const uint32_t warp_addr = smem_addr + warp * kWarpBytes;
+  float *red = reinterpret_cast<float *>(smem + total_warps * (kWarpBytes / 4)); // [2][2][total_warps]
+  const float clip = p.clip_device ? __ldg(p.clip_device) : p.clip;
+  constexpr float kCarry = 16.0f; // the values carried through the rotation are scaled by 2^stages
+  const uint32_t columns = p.columns;
+  const uint32_t col_warp = (uint32_t)wrow * (NIT * 1024u);
+  const uint32_t col0 = col_warp + 512u * h + 16u * a; // this thread's run in the first group of block 0
+
+  // Transpose addressing (per half-warp area of 2048 bytes; rows of 128 bytes = 16 pairs):
+  // thread a writes its 8 chunks of 2 pairs at chunk position c ^ (a & 7), and reads pair a of
+  // every row j from chunk position (a >> 1) ^ (j & 7).
+  const uint32_t half_addr = warp_addr + h * 2048u;
+  const uint32_t wr_addr = half_addr + 128u * a + ((a & 7u) << 4);                // ^ (c << 4)
+  const uint32_t rd_addr = half_addr + ((uint32_t)(a >> 1) << 4) + 8u * (a & 1u); // ^ ((j&7)<<4), + 128 j
+  // Code bytes of one block are staged at index(col) = col + 64 * (col >> 9): a 64-byte skew per 512
+  // columns, so that the two half-warps hit different banks; blocks are 1152 bytes apart.
+  const uint32_t code_a = warp_addr + 512u * h + a + 64u * h, code_b = code_a + 256u;
+  const uint32_t copy_addr = warp_addr + 16u * lane;
+  const uint32_t copy_col = col_warp + 16u * lane;
+
+  // Sign flips of this thread's columns as XOR masks on the packed bf16 pairs (bits 15 and 31 of
+  // word i: elements 2i and 2i+1), kept in shared memory: per block four 16-byte vectors per thread
+  // (two per group), vector q of all threads contiguous.
+  const uint32_t mask_step = blockDim.x * 16u;
+  const uint32_t mask_addr = smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u) + 64u + threadIdx.x * 16u;
+  if (SIGNED) {
+#pragma unroll 1
+    for (int q = 0; q < 4 * NIT; ++q) {
+      const uint32_t c = col0 + (uint32_t)(q >> 2) * 1024u + (uint32_t)((q >> 1) & 1) * 256u + 8u * (q & 1);
+      uint32_t m[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        m[i] = (sign_bit(c + 2 * i) << 15) | (sign_bit(c + 2 * i + 1) << 31);
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(mask_addr + q * mask_step), "r"(m[0]), "r"(m[1]),
+                   "r"(m[2]), "r"(m[3])
+                   : "memory");
+    }
+  }
+  // Weight packing: may the fast quotient be used for every entry of this thread's columns?
+  bool equalise_fast = true;
+  if (EXTRA == kPack && p.equalise) {
+#pragma unroll 1
+    for (int q = 0; q < 32 * NIT; ++q) {
+      const uint32_t c = col0 + (uint32_t)(q >> 5) * 1024u + (uint32_t)((q >> 4) & 1) * 256u + (q & 15);
+      if (c < columns) {
+        const float e = fabsf(bf16_bits_to_f32(__ldg(p.equalise + c)));
+        equalise_fast = equalise_fast && e > 1.0e-9f && e < 1.0e9f;
+      }
+    }
+  }
+
+  // The 64 bytes of a thread's two runs in block `it` of a row. Widths of concatenated inputs are
+  // multiples of 16, so a run never straddles two of them.
+  auto run_of = [&](uint64_t row, uint32_t c) {
+    if (p.part_count == 1)
+      return reinterpret_cast<const uint4 *>(p.part[0] + row * columns + c);
+    uint32_t i = 0;
+    while (c >= p.width[i])
+      c -= p.width[i++];
+    return reinterpret_cast<const uint4 *>(p.part[i] + row * p.width[i] + c);
+  };
+  auto fetch = [&](uint64_t row, int it, uint4 (&v)[4]) {
+    v[0] = v[1] = v[2] = v[3] = make_uint4(0, 0, 0, 0);
+    const uint32_t c = col0 + 1024u * it;
+    if (row < p.rows) {
+      if (c < columns)
+        load_run(run_of(row, c), p.wide != 0, v[0], v[1]);
+      if (c + 256u < columns)
+        load_run(run_of(row, c + 256u), p.wide != 0, v[2], v[3]);
+    }
+  };
+  auto row_barrier = [&]() { // the warps of one row only; rows in flight do not wait for each other
+    if (NIT == 1 || warps_per_row > 1)
+      asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(warps_per_row * 32) : "memory");
+  };
+
+  const uint64_t row_step = (uint64_t)gridDim.x * rows_per_cta;
+  uint64_t row = (uint64_t)blockIdx.x * rows_per_cta + slot;
+  uint4 next[4];
+  if (PREFETCH)
+    fetch(row, 0, next);
+  uint32_t parity = 0;
+  for (; row < p.rows; row += row_step, parity ^= 1u) {
+    uint64_t PF[F32 ? 16 : 1];        // rotated values of the fp32 variants
+    uint32_t V[F32 ? 1 : 16 * NIT];   // rotated values of the bf16 variants, as bf16 pairs
+    float m = 0.0f;
+    float mean = 0.0f, inv = 0.0f;
+    if (EXTRA == kNorm) {
+      const float2 st = __ldg(p.norm_stats + row);
+      mean = st.x;
+      inv = st.y;
+    }
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) {
+      uint64_t P[16];
+      {
+        if (!PREFETCH)
+          fetch(row, it, next);
+        uint32_t wa[8] = {next[0].x, next[0].y, next[0].z, next[0].w, next[1].x, next[1].y, next[1].z, next[1].w};
+        uint32_t wb[8] = {next[2].x, next[2].y, next[2].z, next[2].w, next[3].x, next[3].y, next[3].z, next[3].w};
+        // software pipeline: the next block is requested before this one is processed
+        if (PREFETCH) {
+          if (it + 1 < NIT)
+            fetch(row, it + 1, next);
+          else
+            fetch(row + row_step, 0, next);
+        }
+        const uint32_t c = col0 + 1024u * it;
+        const bool act_a = c < columns, act_b = c + 256u < columns;
+        if (EXTRA == kNorm) {
+          // The norm in front (reference cpu_executor.cpp:1241-1264 RmsNormModulate, :1108-1148
+          // LayerNormModulate): the words are replaced by the bf16 result the unfused op would have
+          // stored, rounding for rounding, two groups per packed operation.
+          const uint64_t at = (row / p.norm_rows_per_mod) * (uint64_t)columns + c;
+          const bool layer = p.norm_bias != nullptr, weighted = p.norm_weight != nullptr;
+          auto product = [&](uint64_t u, uint64_t v) { return fma2(u, v, p.minus_zero2); };
+          const uint64_t inv2 = pack2(inv, inv), mean2 = pack2(mean, mean), one2 = pack2(1.0f, 1.0f);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+            auto pick = [&](const uint16_t *base, uint64_t index, bool active, const uint4 &other) {
+              return active ? __ldg(reinterpret_cast<const uint4 *>(base + index) + half) : other;
+            };
+            const uint4 sa4 = pick(p.norm_scale, at, act_a, zero), sb4 = pick(p.norm_scale, at + 256u, act_b, zero);
+            const uint4 ha4 = pick(p.norm_shift, at, act_a, zero), hb4 = pick(p.norm_shift, at + 256u, act_b, zero);
+            const uint4 ga4 = pick(p.norm_weight, c, act_a && weighted, one),
+                        gb4 = pick(p.norm_weight, c + 256u, act_b && weighted, one);
+            const uint4 ba4 = pick(p.norm_bias, c, act_a && layer, zero),
+                        bb4 = pick(p.norm_bias, c + 256u, act_b && layer, zero);
+            const uint32_t sa[4] = {sa4.x, sa4.y, sa4.z, sa4.w}, sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+            const uint32_t ha[4] = {ha4.x, ha4.y, ha4.z, ha4.w}, hb[4] = {hb4.x, hb4.y, hb4.z, hb4.w};
+            const uint32_t ga[4] = {ga4.x, ga4.y, ga4.z, ga4.w}, gb[4] = {gb4.x, gb4.y, gb4.z, gb4.w};
+            const uint32_t ba[4] = {ba4.x, ba4.y, ba4.z, ba4.w}, bb[4] = {bb4.x, bb4.y, bb4.z, bb4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                auto pair_of = [&](uint32_t wa_, uint32_t wb_) {
+                  return k ? pack2(__uint_as_float(wa_ & 0xffff0000u), __uint_as_float(wb_ & 0xffff0000u))
+                           : pack2(__uint_as_float(wa_ << 16), __uint_as_float(wb_ << 16));
+                };
+                const uint64_t x2 = pair_of(wa[4 * half + i], wb[4 * half + i]);
+                const uint64_t s2 = pair_of(sa[i], sb[i]), h2 = pair_of(ha[i], hb[i]), g2 = pair_of(ga[i], gb[i]);
+                uint64_t y2;
+                if (layer) { // intermediate bf16 roundings of the reference's LayerNormModulate
+                  const uint64_t b2 = pair_of(ba[i], bb[i]);
+                  const uint64_t n2 = round_bf16_2(add2(product(product(sub2(x2, mean2), inv2), g2), b2));
+                  y2 = add2(round_bf16_2(product(n2, round_bf16_2(add2(one2, s2)))), h2);
+                } else {
+                  const uint64_t n2 = product(product(x2, inv2), g2);
+                  y2 = add2(product(n2, add2(one2, s2)), h2);
+                }
+                P[8 * half + 2 * i + k] = y2;
+              }
+            }
+          }
+          // the bf16 result, and the sign flips of the signed variants on it
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            P[e] = round_bf16_2(P[e]);
+          if (SIGNED) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const uint4 ma4 = lds128(mask_addr + (4 * it + q) * mask_step), mb4 = lds128(mask_addr + (4 * it + 2 + q) * mask_step);
+              const uint32_t ma[4] = {ma4.x, ma4.y, ma4.z, ma4.w}, mb[4] = {mb4.x, mb4.y, mb4.z, mb4.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                P[8 * q + 2 * i] ^= ((uint64_t)(mb[i] << 16) << 32) | (uint64_t)(ma[i] << 16);
+                P[8 * q + 2 * i + 1] ^= ((uint64_t)(mb[i] & 0xffff0000u) << 32) | (uint64_t)(ma[i] & 0xffff0000u);
+              }
+            }
+          }
+        } else {
+          if (SIGNED) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const uint4 ma4 = lds128(mask_addr + (4 * it + q) * mask_step), mb4 = lds128(mask_addr + (4 * it + 2 + q) * mask_step);
+              const uint32_t ma[4] = {ma4.x, ma4.y, ma4.z, ma4.w}, mb[4] = {mb4.x, mb4.y, mb4.z, mb4.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                wa[4 * q + i] ^= ma[i];
+                wb[4 * q + i] ^= mb[i];
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            P[2 * i] = pack2(__uint_as_float(wa[i] << 16), __uint_as_float(wb[i] << 16));
+            P[2 * i + 1] = pack2(__uint_as_float(wa[i] & 0xffff0000u), __uint_as_float(wb[i] & 0xffff0000u));
+          }
+          if (EXTRA == kPack && p.equalise) {
+            // weight rows with input equalisation: w / e in fp32 before anything else (reference
+            // tools/difflux2sample.cpp:3005-3014; the sign flip commutes with the division).
+            // One Markstein step from the approximate reciprocal: the quotient of two 8-bit
+            // significands is never within 2^-33 of a rounding boundary of fp32, far outside the
+            // 2^-44 error of fma(r, y, q).
+            const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
+            const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + c);
+            const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z,
+                                 act_b ? __ldg(ep + 33) : z};
+            const uint32_t ea[8] = {e4[0].x, e4[0].y, e4[0].z, e4[0].w, e4[1].x, e4[1].y, e4[1].z, e4[1].w};
+            const uint32_t eb[8] = {e4[2].x, e4[2].y, e4[2].z, e4[2].w, e4[3].x, e4[3].y, e4[3].z, e4[3].w};
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float e0 = __uint_as_float((i & 1) ? (ea[i >> 1] & 0xffff0000u) : (ea[i >> 1] << 16));
+              const float e1 = __uint_as_float((i & 1) ? (eb[i >> 1] & 0xffff0000u) : (eb[i >> 1] << 16));
+              if (equalise_fast) {
+                float y0, y1;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(e0));
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(e1));
+                const uint64_t y2 = pack2(y0, y1), q2 = mul2(P[i], y2);
+                P[i] = fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2);
+              } else {
+                float w0, w1;
+                unpack2(P[i], w0, w1);
+                P[i] = pack2(__fdiv_rn(w0, e0), __fdiv_rn(w1, e1));
+              }
+            }
+          }
+        }
+      }
+      // stage 0 (stride 1) and stage 1 (stride 4)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        bfly(P[4 * q], P[4 * q + 1], P[4 * q + 2], P[4 * q + 3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        bfly(P[q], P[q + 4], P[q + 8], P[q + 12]);
+      // 16x16 transpose of pairs through shared memory.
+      {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          float x0, x1, x2, x3;
+          unpack2(P[2 * c], x0, x1);
+          unpack2(P[2 * c + 1], x2, x3);
+          sts128(wr_addr ^ (uint32_t)(c << 4), x0, x1, x2, x3);
+        }
+        __syncwarp();
+#define DIFB200_READ_PAIR(J) P[J] = lds64<(J) * 128>(rd_addr ^ (uint32_t)(((J) & 7) << 4));
+        DIFB200_READ_PAIR(0) DIFB200_READ_PAIR(1) DIFB200_READ_PAIR(2) DIFB200_READ_PAIR(3)
+        DIFB200_READ_PAIR(4) DIFB200_READ_PAIR(5) DIFB200_READ_PAIR(6) DIFB200_READ_PAIR(7)
+        DIFB200_READ_PAIR(8) DIFB200_READ_PAIR(9) DIFB200_READ_PAIR(10) DIFB200_READ_PAIR(11)
+        DIFB200_READ_PAIR(12) DIFB200_READ_PAIR(13) DIFB200_READ_PAIR(14) DIFB200_READ_PAIR(15)
+#undef DIFB200_READ_PAIR
+        __syncwarp();
+      }
+      // Now P[j] = element 16*j + a of both groups. stage 2 (stride 16), stage 3 (stride 64).
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        bfly(P[4 * q], P[4 * q + 1], P[4 * q + 2], P[4 * q + 3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        bfly(P[q], P[q + 4], P[q + 8], P[q + 12]);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        m = absmax2(m, P[j]);
+        if (F32)
+          PF[F32 ? j : 0] = P[j];
+        else
+          V[F32 ? 0 : 16 * it + j] = pack_bf16_pair(P[j]);
+      }
+    }
+
+    // Row maximum: thread -> warp (the bits of a non-negative float order like integers) -> row.
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    float *redp = red + parity * 2 * total_warps;
+    if (NIT == 1 || warps_per_row > 1) {
+      if (lane == 0)
+        redp[warp] = m;
+      row_barrier();
+      m = 0.0f;
+      for (int w = 0; w < warps_per_row; ++w)
+        m = fmaxf(m, redp[slot * warps_per_row + w]);
+    }
+    const float maximum = m * (1.0f / kCarry);
+    float scale = row_scale(maximum, clip);
+    if (EXTRA == kPack && p.mse) {
+      // The scale is the one of seven clipped candidates with the lowest squared error over every
+      // fourth rotated element, the offline packer's rule (reference tools/difflux2sample.cpp:
+      // 1225-1259). Those elements sit in the lanes with a % 4 == 0; they go through shared memory
+      // so that all 32 lanes take an equal share. The reference evaluates in double: value and candidate have 8 significant bits and the code 8,
+      // so value - code * candidate is exact in fp32 (15 bits at the granularity of either term)
+      // and only its square and the sum need double. The sum's order differs from the reference's
+      // sequential one, which matters only for candidates that tie to 1e-15.
+      constexpr float factors[7] = {1.0f, 0.96f, 0.92f, 0.88f, 0.84f, 0.80f, 0.76f};
+      const int samples = F32 ? 16 : 16 * NIT; // pairs per sampled lane
+      if ((a & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < (F32 ? 16 : 16 * NIT); ++i)
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(warp_addr + 4u * (uint32_t)((lane >> 2) * samples + i)),
+                       "r"(F32 ? pack_bf16_pair(PF[F32 ? i : 0]) : V[F32 ? 0 : i])
+                       : "memory");
+      }
+      __syncwarp();
+      float candidate[7], reciprocal[7];
+      double e[7];
+#pragma unroll
+      for (int f = 0; f < 7; ++f) {
+        candidate[f] = round_bf16(row_scale(maximum, factors[f])) * kCarry;
+        reciprocal[f] = __frcp_rn(candidate[f]);
+        e[f] = 0.0;
+      }
+#pragma unroll 1
+      for (int i = lane; i < 8 * samples; i += 32) {
+        uint32_t pair;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(pair) : "r"(warp_addr + 4u * i) : "memory");
+        const float v0 = __uint_as_float(pair << 16), v1 = __uint_as_float(pair & 0xffff0000u);
+#pragma unroll
+        for (int f = 0; f < 7; ++f) {
+          const uint32_t q = pack_bf16_pair(__fmul_rn(v0, reciprocal[f]), __fmul_rn(v1, reciprocal[f]));
+          // nearest-even integer by the magic constant 1.5 * 2^23 (|q| < 2^9)
+          const float n0 = __fadd_rn(fminf(fmaxf(__uint_as_float(q << 16), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
+          const float n1 =
+              __fadd_rn(fminf(fmaxf(__uint_as_float(q & 0xffff0000u), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
+          const double d0 = (double)__fmaf_rn(-n0, candidate[f], v0), d1 = (double)__fmaf_rn(-n1, candidate[f], v1);
+          e[f] = fma(d0, d0, e[f]); // the square is exact in double: one rounding, as multiply then add
+          e[f] = fma(d1, d1, e[f]);
+        }
+      }
+      double *errors = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(smem) +
+                                                  (size_t)total_warps * (kWarpBytes + 16) + 64 +
+                                                  (SIGNED ? (size_t)total_warps * 32 * 64 * NIT : 0));
+#pragma unroll
+      for (int f = 0; f < 7; ++f) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          e[f] = __dadd_rn(e[f], __shfl_xor_sync(0xffffffffu, e[f], o));
+        if (warps_per_row > 1 && lane == 0)
+          errors[f * total_warps + warp] = e[f];
+      }
+      if (warps_per_row > 1) {
+        row_barrier();
+#pragma unroll
+        for (int f = 0; f < 7; ++f) {
+          e[f] = 0.0;
+          for (int w = 0; w < warps_per_row; ++w)
+            e[f] = __dadd_rn(e[f], errors[f * total_warps + slot * warps_per_row + w]);
+        }
+        row_barrier(); // the error slots are reused by the next row
+      }
+      double best = e[0];
+      float chosen = candidate[0];
+#pragma unroll
+      for (int f = 1; f < 7; ++f)
+        if (e[f] < best) {
+          best = e[f];
+          chosen = candidate[f];
+        }
+      scale = maximum == 0.0f ? 1.0e-30f : chosen * (1.0f / kCarry);
+      __syncwarp(); // the samples are read before the codes overwrite them
+    }
+    const float scale_bf16 = round_bf16(scale);
+    const float stored = ((SIGNED || (EXTRA == kPack && p.mse)) && !F32) ? scale_bf16 : scale;
+    const float divisor = (F32 ? scale : scale_bf16) * kCarry;
+    const float recip = __frcp_rn(divisor);
+    const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
+    if (wrow == 0 && lane == 0)
+      p.scales[row] = stored;
+
+    auto code_pair = [&](int i, int &c0, int &c1) { // codes of pair i (block i / 16, element 16 (i % 16) + a)
+      if (F32) {
+        float q0, q1;
+        unpack2(div2_exact(PF[F32 ? i : 0], y2, nb2), q0, q1);
+        c0 = max(sat_s8(q0), -127);
+        c1 = max(sat_s8(q1), -127);
+      } else {
+        codes_of(pack_bf16_pair(div2_bf16(unpack_bf16_pair(V[F32 ? 0 : i]), y2)), c0, c1);
+      }
+    };
+    auto flush_codes = [&](int8_t *dst) { // every lane copies 2 x 16 bytes of each block's 1024 columns
+      __syncwarp();
+#pragma unroll
+      for (int part = 0; part < 2 * NIT; ++part) {
+        const uint32_t col = copy_col + part * 512u;
+        if (col < columns)
+          *reinterpret_cast<uint4 *>(dst + row * columns + col) = lds128(copy_addr + part * 576u);
+      }
+      __syncwarp();
+    };
+#define DIFB200_STAGE(J)                     \
+  {                                          \
+    int ca, cb;                              \
+    emit(16 * it + (J), ca, cb);             \
+    sts8<16 * (J)>(code_a + 1152u * it, ca); \
+    sts8<16 * (J)>(code_b + 1152u * it, cb); \
+  }
+#define DIFB200_STAGE_ALL                                                                                     \
+  _Pragma("unroll") for (int it = 0; it < NIT; ++it) {                                                        \
+    DIFB200_STAGE(0) DIFB200_STAGE(1) DIFB200_STAGE(2) DIFB200_STAGE(3) DIFB200_STAGE(4) DIFB200_STAGE(5)     \
+    DIFB200_STAGE(6) DIFB200_STAGE(7) DIFB200_STAGE(8) DIFB200_STAGE(9) DIFB200_STAGE(10) DIFB200_STAGE(11)   \
+    DIFB200_STAGE(12) DIFB200_STAGE(13) DIFB200_STAGE(14) DIFB200_STAGE(15)                                   \
+  }
+    float rm = 0.0f;
+    // Residual of an element (reference cpu_executor.cpp:262-305): r = fma(-code, stored, value).
+    auto residual_pair = [&](int i, int c0, int c1, float &r0, float &r1) {
+      float x0, x1;
+      unpack2(F32 ? PF[F32 ? i : 0] : unpack_bf16_pair(V[F32 ? 0 : i]), x0, x1);
+      r0 = __fmaf_rn(-(float)c0, stored, x0 * (1.0f / kCarry));
+      r1 = __fmaf_rn(-(float)c1, stored, x1 * (1.0f / kCarry));
+    };
+    {
+      auto emit = [&](int i, int &c0, int &c1) {
+        code_pair(i, c0, c1);
+        if (RESIDUAL) {
+          float r0, r1;
+          residual_pair(i, c0, c1, r0, r1);
+          asm("max.f32 %0, %0, %1, %2;" : "+f"(rm) : "f"(fabsf(r0)), "f"(fabsf(r1)));
+        }
+      };
+      DIFB200_STAGE_ALL
+    }
+    flush_codes(p.codes);
+
+    if (RESIDUAL) {
+      rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
+      if (lane == 0)
+        redp[total_warps + warp] = rm;
+      row_barrier();
+      rm = 0.0f;
+      for (int w = 0; w < warps_per_row; ++w)
+        rm = fmaxf(rm, redp[total_warps + slot * warps_per_row + w]);
+      const float rscale = row_scale(rm, 1.0f);
+      const float rscale_bf16 = round_bf16(rscale);
+      if (wrow == 0 && lane == 0)
+        p.rscales[row] = (SIGNED && !F32) ? rscale_bf16 : rscale;
+      const float rdivisor = F32 ? rscale : rscale_bf16, rrecip = __frcp_rn(rdivisor);
+      const uint64_t ry2 = pack2(rrecip, rrecip), rnb2 = pack2(-rdivisor, -rdivisor);
+      auto emit = [&](int i, int &c0, int &c1) {
+        int f0, f1;
+        float r0, r1;
+        code_pair(i, f0, f1);
+        residual_pair(i, f0, f1, r0, r1);
+        if (F32) {
+          float q0, q1;
+          unpack2(div2_exact(pack2(r0, r1), ry2, rnb2), q0, q1);
+          c0 = max(sat_s8(q0), -127);
+          c1 = max(sat_s8(q1), -127);
+        } else {
+          codes_of(pack_bf16_pair(div2_bf16(round_bf16_2(pack2(r0, r1)), ry2)), c0, c1);
+        }
+      };
+      DIFB200_STAGE_ALL
+      flush_codes(p.rcodes);
+    }
+#undef DIFB200_STAGE_ALL
+#undef DIFB200_STAGE
+  }
+}
+
+template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB>
+int launch_form(const QuantParams &p, cudaStream_t stream) {
+  const uint32_t groups = p.columns >> 8;
+  const int warps_per_row = (int)((groups + 4u * NIT - 1u) / (4u * NIT));
+  if (warps_per_row > MAXT / 32)
+    return fail(kUnsupported, "QuantizeInt8Rows: ConvRot width above 16384 is not supported");
+  constexpr int kWarps = MAXT / 32 < 8 ? MAXT / 32 : 8;
+  int rows_per_cta = kWarps / warps_per_row;
+  rows_per_cta = rows_per_cta < 1 ? 1 : rows_per_cta;
+  if ((uint64_t)rows_per_cta > p.rows)
+    rows_per_cta = (int)p.rows;
+  const int warps = warps_per_row * rows_per_cta, threads = warps * 32;
+  // per warp: transpose / staging area; row maxima; for the signed variants 16 XOR masks per thread and block
+  const size_t smem = (size_t)warps * kWarpBytes + (size_t)warps * 4 * sizeof(float) + 64 +
+                      (SIGNED ? (size_t)warps * 32 * 64 * NIT : 0) + (EXTRA == kPack ? (size_t)warps * 7 * sizeof(double) : 0);
+  auto kernel = convrot256_kernel<SIGNED, F32, RESIDUAL, EXTRA, NIT, PREFETCH, MAXT, MINB>;
+  int resident = 1;
+  if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), threads, smem, &resident))
+    return rc;
+  const uint64_t batches = (p.rows + rows_per_cta - 1) / rows_per_cta;
+  uint64_t grid = (uint64_t)sm_count() * resident; // persistent: as many CTAs as are resident at once
+  grid = grid > batches ? batches : grid;
+  kernel<<<(unsigned)grid, threads, smem, stream>>>(p, warps_per_row, rows_per_cta);
+  return launched(cudaGetLastError(), "convrot256_kernel launch");
+}
+
+// One block of 1024 columns per warp: the fp32 and residual forms, narrow rows, and calls of few rows.
+template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
+int launch_single(const QuantParams &p, cudaStream_t stream) {
+  if (((p.columns >> 8) + 3u) / 4u > 8u)
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
+  if constexpr (EXTRA == kNorm)
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream); // 24 warps, three tensors in flight
+  else if constexpr (EXTRA != kPlain || (RESIDUAL && !F32))
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
+  else // 64 registers and 32 warps per SM hide the load latency without a prefetch
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, RESIDUAL ? 3 : 4>(p, stream);
+}
+
+template <bool SIGNED>
+int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
+  const bool pack = p.mse || p.equalise, norm = p.norm_scale != nullptr;
+  if ((pack || norm) && p.rcodes)
+    return fail(kUnsupported, "QuantizeInt8Rows: weight packing (MSE scale, input equalisation) exists for "
+                              "the 256-wide variants without residual outputs");
+  if (f32) {
+    if (pack)
+      return launch_single<SIGNED, true, false, kPack>(p, stream);
+    if (norm)
+      return launch_single<SIGNED, true, false, kNorm>(p, stream);
+    return p.rcodes ? launch_single<SIGNED, true, true, kPlain>(p, stream)
+                    : launch_single<SIGNED, true, false, kPlain>(p, stream);
+  }
+  if (p.rcodes)
+    return launch_single<SIGNED, false, true, kPlain>(p, stream);
+  if (norm)
+    return launch_single<SIGNED, false, false, kNorm>(p, stream);
+  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, so calls
+  // whose rows fill the machine less than once with one block per warp keep that form, and so do
+  // rows of up to 8 blocks that three do not divide (8192 columns: 34.3 us against 41.5 us for 4159
+  // rows, the last warp would idle on a third of its slots). Wider rows take three in any case:
+  // one block per warp would make CTAs of up to 16 warps that meet at one barrier (4608 x 15360: 92 us
+  // against 73 us).
+  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+  const bool few = p.rows * blocks <= (uint64_t)sm_count() * 24u;
+  const bool three = (blocks % 3u == 0 || blocks > 8u) && !few;
+  if (pack)
+    return few || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
+                               : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
+  return three ? launch_form<SIGNED, false, false, kPlain, 3, true, 256, 2>(p, stream)
+               : launch_single<SIGNED, false, false, kPlain>(p, stream);
+}
+
+} // namespace
+
+int launch_convrot256(const QuantParams &p, int implementation, cudaStream_t stream) {
+  const bool is_signed = implementation == 3 || implementation == 6, f32 = implementation >= 5;
+  return is_signed ? launch_variant<true>(p, f32, stream) : launch_variant<false>(p, f32, stream);
+}
+
+} // namespace difb200

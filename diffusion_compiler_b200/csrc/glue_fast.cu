@@ -160,6 +160,39 @@ k_row_stats_sequential(const uint4 *x, float2 *stats, uint64_t rows, uint32_t co
   }
 }
 
+// The statistics as parallel sums, one warp per row.
+__global__ void __launch_bounds__(256)
+k_row_stats_parallel(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols, float eps, int layer) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t cols8 = cols >> 3;
+  for (uint64_t r = warp; r < rows; r += (uint64_t)gridDim.x * (blockDim.x >> 5)) {
+    float mean = 0.0f, sum = 0.0f;
+    if (layer) {
+      for (uint32_t c = lane; c < cols8; c += 32) {
+        float f[8];
+        unpack8(__ldg(x + r * cols8 + c), f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          mean += f[e];
+      }
+      mean = __fdiv_rn(warp_sum(mean), (float)cols);
+    }
+    for (uint32_t c = lane; c < cols8; c += 32) {
+      float f[8];
+      unpack8(__ldg(x + r * cols8 + c), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float d = __fsub_rn(f[e], mean);
+        sum = __fmaf_rn(d, d, sum);
+      }
+    }
+    sum = warp_sum(sum);
+    if (lane == 0)
+      stats[r] = make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps))));
+  }
+}
+
 // ---- RmsNormModulate, explicit scale / shift (cpu_executor.cpp:1241-1264) ----
 // One warp per row; lane l owns the 8-element groups l, l + 32, ... CHUNKS > 0: the row has
 // CHUNKS * 256 columns and stays in registers; CHUNKS == 0: any multiple of 256, read twice.
@@ -501,6 +534,22 @@ bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps
   *rc = done("k_row_stats_sequential");
   *stats = area;
   return true;
+}
+
+int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats, cudaStream_t s) {
+  int rc = 0;
+  if (row_stats_sequential(x, rows, cols, eps, layer, stats, s, &rc))
+    return rc;
+  float2 *area = static_cast<float2 *>(device_scratch(rows * sizeof(float2)));
+  if (!area)
+    return fail(kOutOfMemory, "cannot allocate the row statistics scratch");
+  uint64_t blocks = (rows + 7) / 8;
+  const uint64_t cap = (uint64_t)sm_count() * 8;
+  blocks = blocks > cap ? cap : blocks;
+  k_row_stats_parallel<<<(unsigned)blocks, 256, 0, s>>>(static_cast<const uint4 *>(x), area, rows, (uint32_t)cols, eps,
+                                                        layer ? 1 : 0);
+  *stats = area;
+  return done("k_row_stats_parallel");
 }
 
 bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const void *b, void *o, uint32_t dt,

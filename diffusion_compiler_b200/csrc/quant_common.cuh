@@ -1,0 +1,164 @@
+// Shared by the QuantizeInt8Rows kernels: parameters, the radix-4 butterfly, exact divisions.
+#pragma once
+
+#include "common.cuh"
+
+namespace difb200 {
+
+constexpr int kMaxParts = 8;
+
+struct QuantParams {
+  const uint16_t *part[kMaxParts];
+  uint32_t width[kMaxParts];
+  uint32_t part_count;
+  uint32_t wide;  // every part starts on 32 bytes
+  uint32_t columns;
+  uint64_t rows;
+  float clip;
+  const float *clip_device;
+  int8_t *codes;
+  float *scales;
+  int8_t *rcodes;
+  float *rscales;
+  uint32_t mse;   // weight rows: choose the row scale by the offline packer's MSE search
+  const uint16_t *equalise; // weight rows: bf16 [columns], every element is divided by its entry first
+  // RmsNormModulate in front of the quantiser (explicit scale / shift layout), all bf16:
+  const uint16_t *norm_weight; // [columns] or nullptr
+  const uint16_t *norm_scale;  // [rows, columns]; nullptr = no prologue
+  const uint16_t *norm_shift;  // [rows, columns]
+  const uint16_t *norm_bias;   // [columns]: LayerNormModulate (mean removed, weight and bias); nullptr = RMS
+  uint64_t norm_rows_per_mod;  // rows that share one row of scale / shift
+  const float2 *norm_stats;    // per row (mean, inverse deviation)
+  // Two fp32 -0, added to products of the norm. The assembler contracts mul.rn.f32x2 followed by add.rn.f32x2
+  // into one fused operation (seen as single codes off by one), and an fma with a constant -0 as well; with
+  // a -0 it cannot see, the product keeps its own rounding (x + -0 = x for every x, signed zeros included).
+  uint64_t minus_zero2;
+};
+
+// The 256-wide variants (2, 3, 5, 6), with or without residual outputs, weight packing or a norm in front.
+int launch_convrot256(const QuantParams &p, int implementation, cudaStream_t stream);
+
+#ifdef __CUDACC__
+
+// Fixed Rademacher diagonal of the signed variants (reference cpu_executor.cpp:183-189).
+__device__ __forceinline__ uint32_t sign_bit(uint32_t column) {
+  uint32_t hash = column + 0x9e3779b9u;
+  hash = (hash ^ (hash >> 16)) * 0x7feb352du;
+  hash = (hash ^ (hash >> 15)) * 0x846ca68bu;
+  hash ^= hash >> 16;
+  return hash & 1u;
+}
+
+// One radix-4 butterfly on packed pairs, without the reference's exact factor 0.5.
+__device__ __forceinline__ void bfly(uint64_t &x0, uint64_t &x1, uint64_t &x2, uint64_t &x3) {
+  const uint64_t s = add2(x0, x1);
+  const uint64_t t = sub2(x0, x1);
+  const uint64_t y0 = sub2(add2(s, x2), x3);
+  const uint64_t y1 = add2(sub2(s, x2), x3);
+  const uint64_t y2 = add2(add2(t, x2), x3);
+  // the reference forms (x1 - x0) + x2: x1 - x0 = -t exactly, and (-t) + x2 = x2 - t
+  const uint64_t y3 = add2(sub2(x2, t), x3);
+  x0 = y0;
+  x1 = y1;
+  x2 = y2;
+  x3 = y3;
+}
+
+__device__ __forceinline__ float absmax2(float m, uint64_t v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(lo)), "f"(fabsf(hi))); // one three-input maximum
+  return m;
+}
+
+// Correctly rounded fp32 quotient a/b from y = RN(1/b): two Markstein refinements.
+__device__ __forceinline__ uint64_t div2_exact(uint64_t a, uint64_t y, uint64_t negb) {
+  uint64_t q = mul2(a, y);
+  uint64_t r = fma2(negb, q, a);
+  q = fma2(r, y, q);
+  r = fma2(negb, q, a);
+  return fma2(r, y, q);
+}
+// bf16(a / b) for bf16 values a and b (8 significant bits each, integers V and S in [128, 255]
+// times powers of two) needs no refinement at all: a rounding boundary of the quotient is M / 2^k
+// with M odd in [257, 511], and |V / S - M / 2^k| = |2^k V - M S| / (S 2^k) is either 0 -- which
+// would need the odd M > 255 to divide V <= 255, impossible -- or at least 2^-17 of the quotient,
+// while a * RN(1 / b) is within 2^-23 of it. So the plain product rounds to the same bf16 value
+// as the IEEE quotient, ties cannot occur, and a zero numerator gives zero.
+__device__ __forceinline__ uint64_t div2_bf16(uint64_t a, uint64_t y) { return mul2(a, y); }
+
+__device__ __forceinline__ uint32_t pack_bf16_pair(float lo, float hi) {
+  uint32_t packed;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
+  return packed;
+}
+__device__ __forceinline__ uint32_t pack_bf16_pair(uint64_t v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  return pack_bf16_pair(lo, hi);
+}
+__device__ __forceinline__ uint64_t unpack_bf16_pair(uint32_t packed) {
+  return pack2(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u));
+}
+__device__ __forceinline__ uint64_t round_bf16_2(uint64_t v) { return unpack_bf16_pair(pack_bf16_pair(v)); }
+
+__device__ __forceinline__ int sat_s8(float v) {
+  int r;
+  asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(r) : "f"(v));
+  return r;
+}
+
+// INT8 codes of a packed pair of bf16 quotients: round to nearest even, saturate.
+__device__ __forceinline__ void codes_of(uint32_t q, int &c0, int &c1) {
+  c0 = sat_s8(__uint_as_float(q << 16));
+  c1 = sat_s8(__uint_as_float(q & 0xffff0000u));
+}
+
+// max * clip / 127 as the reference rounds it (IEEE product, IEEE quotient, then the guard): one
+// Markstein step from RN(1/127) gives the correctly rounded quotient for every fp32 mantissa
+// (checked exhaustively), and below 2^-90, where the residual could underflow, the guard decides.
+__device__ __forceinline__ float row_scale(float maximum, float clip) {
+  constexpr float kInv127 = 1.0f / 127.0f;
+  const float a = __fmul_rn(maximum, clip);
+  float q = __fmul_rn(a, kInv127);
+  q = __fmaf_rn(__fmaf_rn(-127.0f, q, a), kInv127, q);
+  if (!(a < 3.0e38f)) // inf and NaN as the plain division treats them
+    q = a / 127.0f;
+  return fmaxf(q, 1.0e-30f);
+}
+
+// ---- shared-memory access through 32-bit shared addresses (cheap address arithmetic) ----
+__device__ __forceinline__ void sts128(uint32_t addr, float x, float y, float z, float w) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(w)
+               : "memory");
+}
+template <int OFF>
+__device__ __forceinline__ uint64_t lds64(uint32_t addr) {
+  uint64_t v;
+  asm volatile("ld.shared.b64 %0, [%1+%2];" : "=l"(v) : "r"(addr), "n"(OFF) : "memory");
+  return v;
+}
+template <int OFF>
+__device__ __forceinline__ void sts8(uint32_t addr, int v) {
+  asm volatile("st.shared.u8 [%0+%1], %2;" ::"r"(addr), "n"(OFF), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t addr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ float lds32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+#endif // __CUDACC__
+
+} // namespace difb200

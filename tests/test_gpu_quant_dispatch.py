@@ -1,0 +1,88 @@
+"""The forms of the 256-wide ConvRot quantiser at the edges of their dispatch: one or three blocks of 1024
+columns per warp, partial blocks, several warps per row, rows that only start on 16 bytes, and the
+norm prologue. Codes and scales are whole numbers and exact fp32 values: every bit must agree."""
+import numpy as np
+import pytest
+
+import oracle_bridge as ob
+from helpers import activations, bf16_normal, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits_equal(want, got):
+    got = got.cpu().numpy().reshape(want.shape)
+    return np.array_equal(want.view(np.uint8), got.view(np.uint8))
+
+
+@pytest.mark.parametrize("impl,rows,widths,clip,residual", [
+    (2, 1200, [3072], 1.0, False),        # three blocks per warp, more rows than resident warps
+    (3, 1190, [3072], 0.97, False),       # the same with sign masks and clipped codes
+    (2, 1301, [2816], 1.0, False),        # the row's last block holds three of four groups
+    (2, 800, [3072, 12288], 1.0, False),  # five warps per row, two inputs
+    (2, 3, [3072, 12288], 1.0, False),    # the same width with few rows: one block per warp
+    (2, 330, [10496], 1.0, False),        # eleven blocks: the last warp has an empty one
+    (2, 500, [8192], 1.0, False),         # eight blocks: one per warp although the rows are many
+    (5, 130, [8192], 1.0, False),         # fp32 division
+    (6, 40, [256], 1.0, True),            # the narrowest row, residual pair
+    (2, 7, [16384], 1.0, True),           # the widest row, residual pair
+    (4, 5, [16384], 1.0, False),          # 4096-wide rotation at its widest
+])
+def test_forms_bit_exact(impl, rows, widths, clip, residual):
+    import torch
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(rows + sum(widths))
+    x = activations(rng, rows, sum(widths))
+    x[rows // 2] = 0
+    cuts = np.cumsum([0] + widths)
+    parts = [np.ascontiguousarray(x[:, cuts[i]:cuts[i + 1]]) for i in range(len(widths))]
+    want = ob.orc().quantize_int8_rows(parts, impl, clip, residual)
+    for shift in (0, 8):  # 8 elements: parts that start on 16 bytes and not on 32
+        tensors = []
+        for p in parts:
+            room = torch.empty(p.size + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(p.shape)
+            tensors.append(room.copy_(to_torch_bf16(p)))
+        got = ops.quantize_int8_rows(tensors, impl, clip, residual=residual)
+        for name, w, g in zip(("codes", "scales", "rcodes", "rscales"), want, got):
+            assert _bits_equal(w, g), (name, shift)
+
+
+@pytest.mark.parametrize("N,K,impl", [(1300, 3072, 2), (450, 8192, 3), (9, 8192, 2), (20, 10496, 5)])
+def test_packing_forms_bit_exact(N, K, impl):
+    import torch
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(N)
+    w = ob.f32_to_bf16((rng.standard_normal((N, K)) * 0.02).astype(np.float32))
+    w[N // 2] = 0
+    eq = ob.orc().weight_equalization(w)
+    for vector in (None, eq):
+        want_codes, want_scales = ob.orc().quantize_weight_rows(w, impl, mse=True, equalise=vector)
+        codes, scales = ops.quantize_weight_rows(to_torch_bf16(w), impl, mse_scale=True,
+                                                 input_scale=None if vector is None else to_torch_bf16(vector))
+        assert _bits_equal(want_scales, scales) and _bits_equal(want_codes, codes)
+
+
+@pytest.mark.parametrize("rows,K", [(5, 3072), (1201, 3072), (33, 2816), (17, 12288), (70, 256)])
+@pytest.mark.parametrize("impl", [2, 3, 5])
+def test_norm_prologue_equals_the_two_ops(rows, K, impl):
+    """RmsNormModulate / LayerNormModulate in front of the quantiser give the bits of the separate ops
+    (the contraction of a product and a sum, or a lost rounding, shows as codes off by one)."""
+    import ctypes as C
+
+    import torch
+    from diffusion_compiler_b200 import _lib, ops
+    rng = np.random.default_rng(rows * 7 + K)
+    t = lambda *shape, std=1.0: to_torch_bf16(bf16_normal(rng, shape, std))  # noqa: E731
+    x, w, b, s, h = t(rows, K), t(K), t(K, std=0.1), t(rows, K, std=0.3), t(rows, K, std=0.3)
+    p = lambda v: C.c_void_p(v.data_ptr())  # noqa: E731
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    normed = torch.empty_like(x)
+    _lib.check(_lib.lib().difb200_rms_norm_modulate(p(x), p(w), p(s), p(h), p(normed), 2, rows, K, 1e-5, stream))
+    want = ops.quantize_int8_rows([normed], impl)
+    got = ops.rms_norm_modulate_quant(x, w, s, h, 1e-5, impl)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+    _lib.check(_lib.lib().difb200_layer_norm_modulate(p(x), p(w), p(b), p(s), p(h), p(normed), 2, rows, K, rows, 1e-6,
+                                                      stream))
+    want = ops.quantize_int8_rows([normed], impl)
+    got = ops.layer_norm_modulate_quant(x, w, b, s, h, 1e-6, impl)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
