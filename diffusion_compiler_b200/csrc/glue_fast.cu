@@ -9,6 +9,7 @@
 #include "common.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace difb200 {
 namespace glue {
@@ -84,76 +85,116 @@ k_swiglu_bf16(const uint4 *x, uint4 *o, uint64_t rows, uint64_t width8, uint64_t
 // norm amplifies such a flip across its 256-wide group. So the statistic is computed here in the
 // reference's order: one lane per row walks its row sequentially. A warp owns 32 rows and moves them
 // through shared memory 64 columns at a time (asynchronous 16-byte copies in coalesced 128-byte
-// runs, rows 9 x 16 bytes apart so that lanes read their own rows without bank conflicts), four
-// chunks deep: the memory latency of a chunk hides under the chains of the three before it.
+// runs, rows 9 x 16 bytes apart so that lanes read their own rows without bank conflicts), four or eight
+// chunks deep: a chunk takes a warp about 0.17 us, so seven in flight cover the HBM latency even with
+// one or two warps on an SM.
 // Squares of bf16 values are exact in fp32, so the
 // fused multiply-add equals the reference's multiply followed by add; the deviations of the layer
-// form are not, and get the two roundings.
+// form are not, and get the two roundings. The mixed-precision adds and fused multiply-adds take the bf16
+// operand as it is, so an element of the chain is one instruction (the layer form's second pass: three)
+// and the kernel is bound by that chain -- cols dependent operations of about four clocks -- for few
+// rows and by HBM for many.
 constexpr int kStatCols = 64, kStatPitch = 9; // uint4 per row in shared memory (8 + 1 pad)
-constexpr int kStatStages = 4, kStatWarps = 2;  // chunks in flight per warp (hides the HBM latency), warps per CTA
+constexpr int kStatWarps = 2;                 // warps per CTA
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
   // 16 bytes global -> shared, asynchronously; zero-filled when the row does not exist
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-template <bool LAYER>
+// acc after the two bf16 elements of a word, low half first. KIND 0: acc + x; 1: acc + x * x (exact
+// square, one rounding); 2: acc + (x - mean)^2 with the roundings of subtract, multiply and add.
+template <int KIND>
+__device__ __forceinline__ float accumulate_word(uint32_t word, float mean, float acc) {
+  if (KIND == 0) {
+    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; add.rn.f32.bf16 %0, lo, %0; add.rn.f32.bf16 %0, hi, %0; }"
+        : "+f"(acc) : "r"(word));
+  } else if (KIND == 1) {
+    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; fma.rn.f32.bf16 %0, lo, lo, %0; fma.rn.f32.bf16 %0, hi, hi, %0; }"
+        : "+f"(acc) : "r"(word));
+  } else {
+    float d0, d1;
+    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; sub.rn.f32.bf16 %0, lo, %3; sub.rn.f32.bf16 %1, hi, %3; }"
+        : "=f"(d0), "=f"(d1) : "r"(word), "f"(mean));
+    acc = __fadd_rn(acc, __fmul_rn(d0, d0));
+    acc = __fadd_rn(acc, __fmul_rn(d1, d1));
+  }
+  return acc;
+}
+
+template <bool LAYER, int STAGES>
 __global__ void __launch_bounds__(32 * kStatWarps)
 k_row_stats_sequential(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols, float eps) {
-  __shared__ uint4 tile[kStatWarps][kStatStages][32 * kStatPitch];
+  extern __shared__ uint4 stat_smem[];
+  auto tile = reinterpret_cast<uint4 (*)[STAGES][32 * kStatPitch]>(stat_smem); // [kStatWarps]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t cols8 = cols >> 3, chunks = cols / kStatCols;
   for (uint64_t row0 = ((uint64_t)blockIdx.x * kStatWarps + warp) * 32; row0 < rows;
        row0 += (uint64_t)gridDim.x * kStatWarps * 32) {
     const uint64_t row = row0 + lane;
     // lane l copies, for j = 0..7, the 16 bytes (row0 + 4 j + l / 8, chunk column l % 8) of a chunk
-    auto issue = [&](uint32_t chunk) {
-      if (chunk < chunks) {
-        uint4 *stage = tile[warp][chunk % kStatStages];
+    const uint4 *src = x + (row0 + (lane >> 3)) * cols8 + (lane & 7);
+    const uint32_t slot = smem_u32(&tile[warp][0][(lane >> 3) * kStatPitch + (lane & 7)]);
+    auto issue = [&](uint32_t chunk) { // no branch: past the last chunk the copies only zero-fill
+      const uint32_t dst = slot + (chunk % STAGES) * (uint32_t)sizeof(tile[0][0]);
+      const uint4 *from = src + chunk * (kStatCols / 8);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint64_t r = row0 + 4 * j + (lane >> 3);
-          const bool valid = r < rows;
-          cp_async16(smem_u32(stage + (4 * j + (lane >> 3)) * kStatPitch + (lane & 7)),
-                     x + (valid ? r : 0) * cols8 + chunk * (kStatCols / 8) + (lane & 7), valid);
-        }
+      for (int j = 0; j < 8; ++j) {
+        const bool valid = chunk < chunks && row0 + 4 * j + (lane >> 3) < rows;
+        cp_async16(dst + 64u * j * kStatPitch, valid ? from + 4ull * j * cols8 : x, valid);
       }
-      asm volatile("cp.async.commit_group;" ::: "memory"); // one group per chunk slot, also when empty
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto read = [&](uint32_t chunk, uint4 (&v)[8]) {
+      const uint4 *stage = tile[warp][chunk % STAGES] + lane * kStatPitch;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        v[c] = stage[c];
     };
     float mean = 0.0f, acc = 0.0f;
-#pragma unroll 1
-    for (int pass = LAYER ? 0 : 1; pass < 2; ++pass) {
-      acc = 0.0f;
-      __syncwarp();
-      for (uint32_t c = 0; c < (uint32_t)kStatStages - 1; ++c)
-        issue(c);
-#pragma unroll 1
-      for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
-        issue(chunk + kStatStages - 1);              // its stage was read during chunk - 1
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStatStages - 1) : "memory");
-        __syncwarp();                                // every lane's copies of this chunk have landed
-        const uint4 *stage = tile[warp][chunk % kStatStages];
+    auto pass = [&](auto kind) {
+      auto chain = [&](const uint4 (&v)[8]) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          float f[8];
-          unpack8(stage[lane * kStatPitch + c], f);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (pass == 0) {
-              acc = __fadd_rn(acc, f[e]);
-            } else if (LAYER) {
-              const float d = __fsub_rn(f[e], mean);
-              acc = __fadd_rn(acc, __fmul_rn(d, d));
-            } else {
-              acc = __fmaf_rn(f[e], f[e], acc);
-            }
-          }
+          acc = accumulate_word<decltype(kind)::value>(v[c].x, mean, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].y, mean, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].z, mean, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].w, mean, acc);
         }
-        __syncwarp();                                // before a later copy overwrites this stage
+      };
+      // The chunk after the one being summed is already in registers, and the requests sit between the
+      // dependent sums, so that nothing but the chain itself takes time.
+      auto advance = [&](uint32_t chunk, const uint4 (&v)[8], uint4 (&next)[8]) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 3) : "memory");
+        __syncwarp();                 // chunk + 1 has landed for every lane, chunk - 1 has been summed by all
+        issue(chunk + STAGES - 1);    // into the stage of chunk - 1
+        read(chunk + 1, next);
+        chain(v);
+      };
+      acc = 0.0f;
+      __syncwarp();
+      for (uint32_t c = 0; c < (uint32_t)STAGES - 1; ++c)
+        issue(c);
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+      __syncwarp();
+      uint4 a[8], b[8];
+      read(0, a);
+      uint32_t chunk = 0;
+#pragma unroll 1
+      for (; chunk + 1 < chunks; chunk += 2) {
+        advance(chunk, a, b);
+        advance(chunk + 1, b, a);
       }
+      if (chunk < chunks)
+        chain(a);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (pass == 0)
-        mean = __fdiv_rn(acc, (float)cols);
+    };
+    if (LAYER) {
+      pass(std::integral_constant<int, 0>{});
+      mean = __fdiv_rn(acc, (float)cols);
+      pass(std::integral_constant<int, 2>{});
+    } else {
+      pass(std::integral_constant<int, 1>{});
     }
     if (row < rows)
       stats[row] = make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(acc, (float)cols), eps))));
@@ -522,15 +563,20 @@ bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps
     *rc = fail(kOutOfMemory, "cannot allocate the row statistics scratch");
     return true;
   }
-  uint64_t blocks = (rows + 32 * kStatWarps - 1) / (32 * kStatWarps);
-  const uint64_t cap = (uint64_t)sm_count() * 6; // 37 KB of shared memory per CTA: six resident per SM
+  // Eight chunks in flight where a few warps per SM have to cover the latency alone, four where the rows
+  // give an SM more than six warps (33272 x 3072: one wave of resident CTAs instead of two).
+  const uint64_t warps = (rows + 31) / 32;
+  const bool deep = warps <= (uint64_t)sm_count() * 6;
+  auto kernel = deep ? (layer ? k_row_stats_sequential<true, 8> : k_row_stats_sequential<false, 8>)
+                     : (layer ? k_row_stats_sequential<true, 4> : k_row_stats_sequential<false, 4>);
+  const size_t smem = sizeof(uint4) * kStatWarps * (deep ? 8 : 4) * 32 * kStatPitch;
+  int resident = 1;
+  if ((*rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * kStatWarps, smem, &resident)))
+    return true;
+  uint64_t blocks = (warps + kStatWarps - 1) / kStatWarps;
+  const uint64_t cap = (uint64_t)sm_count() * resident;
   blocks = blocks > cap ? cap : blocks;
-  if (layer)
-    k_row_stats_sequential<true><<<(unsigned)blocks, 32 * kStatWarps, 0, s>>>(static_cast<const uint4 *>(x), area,
-                                                                              rows, (uint32_t)cols, eps);
-  else
-    k_row_stats_sequential<false><<<(unsigned)blocks, 32 * kStatWarps, 0, s>>>(static_cast<const uint4 *>(x), area,
-                                                                               rows, (uint32_t)cols, eps);
+  kernel<<<(unsigned)blocks, 32 * kStatWarps, smem, s>>>(static_cast<const uint4 *>(x), area, rows, (uint32_t)cols, eps);
   *rc = done("k_row_stats_sequential");
   *stats = area;
   return true;
