@@ -45,6 +45,7 @@
 #include "common.cuh"
 #include "ops.h"
 #include "ptx.cuh"
+#include "quant_common.cuh"
 
 #include <mutex>
 
@@ -85,6 +86,16 @@ __device__ __forceinline__ void report(DeviceStatus *status, uint32_t role, uint
   }
 }
 
+// The entry of one key: (ks', -C ks') and the key's contribution to its tile's bound, from the key scale
+// and the sum of squares of its codes.
+__device__ __forceinline__ void key_entry(float ks, int n2, float &k22, float &bias, float &bound) {
+  uint32_t bits = __float_as_uint(ks);
+  bits = (bits + 1u + ((bits >> 2) & 1u)) & ~3u; // nearest-even to 22 significant bits
+  k22 = __uint_as_float(bits);
+  bias = -12582912.0f * k22;
+  bound = __fmul_rn(__fsqrt_rn((float)n2), k22);
+}
+
 // Builds the per-key table [B,KV,S_pad] of (ks', -C * ks') with C = 1.5 * 2^23: the key scales of
 // the [B,S,KV] row order re-laid contiguous along keys, stored per key pair as
 // (ks'_j, ks'_j+1, bias_j, bias_j+1) so that one 16-byte load feeds one packed fma. The softmax
@@ -108,10 +119,6 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
   const uint32_t j = tile * kTile + threadIdx.x;
   float k22 = 0.0f, bias = -INFINITY, bound = 0.0f;
   if (j < S && (key_valid == nullptr || key_valid[(uint64_t)b * S + j] != 0)) {
-    uint32_t bits = __float_as_uint(ks[((uint64_t)b * S + j) * KV + kvh]);
-    bits = (bits + 1u + ((bits >> 2) & 1u)) & ~3u; // nearest-even to 22 significant bits
-    k22 = __uint_as_float(bits);
-    bias = -12582912.0f * k22;
     const uint4 *row = reinterpret_cast<const uint4 *>(k8 + (((uint64_t)b * S + j) * KV + kvh) * kTile);
     int n2 = 0;
 #pragma unroll
@@ -122,7 +129,7 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
       n2 = __dp4a((int)w.z, (int)w.z, n2);
       n2 = __dp4a((int)w.w, (int)w.w, n2);
     }
-    bound = __fmul_rn(__fsqrt_rn((float)n2), k22);
+    key_entry(ks[((uint64_t)b * S + j) * KV + kvh], n2, k22, bias, bound);
   }
   float *t = table + (((uint64_t)b * KV + kvh) * S_pad + (j & ~1u)) * 2u + (j & 1u);
   t[0] = k22;
@@ -137,6 +144,121 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
   if (threadIdx.x == 0)
     tile_bound[((uint64_t)b * KV + kvh) * tiles + tile] =
         fmaxf(fmaxf(warp_max[0], warp_max[1]), fmaxf(warp_max[2], warp_max[3]));
+}
+
+// QuantizeInt8Rows(Direct, clip 1) of 128-wide bf16 rows for the attention's operands, and the key table
+// from the same pass: the codes, row scales and (for keys) the table entries and tile bounds that the
+// quantiser and key_table_kernel would give one after the other, bit for bit. 8 lanes hold a row
+// (16 elements each), so every access is a full 32-byte sector; HBM-bound (3 bytes per element). The first
+// `key_blocks` CTAs each take the 128 keys of one (batch, kv head, tile), the others 128 query rows each.
+// Replaces two thread-per-row quantiser launches (uncoalesced: 2.4 TB/s) and the table's own pass over the
+// codes: B2 S4608 H24 72 + 9 us before.
+struct OperandParams {
+  const uint4 *q, *k;
+  int8_t *q8, *k8;
+  float *qs, *ks;
+  const uint8_t *key_valid;
+  float *table, *tile_bound;
+  uint64_t q_rows;
+  uint32_t S, KV, S_pad, key_blocks;
+};
+__global__ void __launch_bounds__(256)
+attention_operands_kernel(const OperandParams p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
+  // codes of this lane's 16 elements of a row, the row's scale and sum of squared codes (in every lane)
+  auto quantise = [&](const uint4 *row, bool valid, uint4 &codes, float &scale) {
+    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+    if (valid) {
+      lo = __ldg(row + 2 * part);
+      hi = __ldg(row + 2 * part + 1);
+    }
+    const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint64_t v[8];
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] = unpack_bf16_pair(w[i]);
+      m = absmax2(m, v[i]);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    scale = row_scale(m, 1.0f);
+    const float recip = __frcp_rn(scale);
+    const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-scale, -scale);
+    uint32_t out[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float f[4];
+      unpack2(div2_exact(v[2 * i], y2, nb2), f[0], f[1]);
+      unpack2(div2_exact(v[2 * i + 1], y2, nb2), f[2], f[3]);
+      uint32_t c[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        c[e] = (uint32_t)max(sat_s8(f[e]), -127);
+      out[i] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
+    }
+    codes = make_uint4(out[0], out[1], out[2], out[3]);
+  };
+  if (blockIdx.x < p.key_blocks) {
+    const uint32_t tiles = p.S_pad / kTile, tile = blockIdx.x % tiles, kvh = (blockIdx.x / tiles) % p.KV,
+                   b = blockIdx.x / (tiles * p.KV);
+    float most = 0.0f;
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+      const uint32_t j = tile * kTile + step * 32u + warp * 4u + (lane >> 3);
+      const bool exists = j < p.S;
+      const uint64_t row = ((uint64_t)b * p.S + (exists ? j : 0)) * p.KV + kvh;
+      uint4 codes;
+      float scale;
+      quantise(p.k + row * 16, exists, codes, scale);
+      int n2 = __dp4a((int)codes.x, (int)codes.x, 0);
+      n2 = __dp4a((int)codes.y, (int)codes.y, n2);
+      n2 = __dp4a((int)codes.z, (int)codes.z, n2);
+      n2 = __dp4a((int)codes.w, (int)codes.w, n2);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+        n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+      float k22 = 0.0f, bias = -INFINITY, bound = 0.0f;
+      if (exists) {
+        reinterpret_cast<uint4 *>(p.k8 + row * kTile)[part] = codes;
+        if (part == 0)
+          p.ks[row] = scale;
+        if (p.key_valid == nullptr || p.key_valid[(uint64_t)b * p.S + j] != 0)
+          key_entry(scale, n2, k22, bias, bound);
+      }
+      most = fmaxf(most, bound);
+      if (part == 0) {
+        float *t = p.table + (((uint64_t)b * p.KV + kvh) * p.S_pad + (j & ~1u)) * 2u + (j & 1u);
+        t[0] = k22;
+        t[2] = bias;
+      }
+    }
+    __shared__ float warp_max[8];
+    most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most))); // non-negative
+    if (lane == 0)
+      warp_max[warp] = most;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w)
+        most = fmaxf(most, warp_max[w]);
+      p.tile_bound[((uint64_t)b * p.KV + kvh) * tiles + tile] = most;
+    }
+  } else {
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+      const uint64_t row = (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * 32u + warp * 4u + (lane >> 3);
+      const bool exists = row < p.q_rows;
+      uint4 codes;
+      float scale;
+      quantise(p.q + (exists ? row : 0) * 16, exists, codes, scale);
+      if (exists) {
+        reinterpret_cast<uint4 *>(p.q8 + row * kTile)[part] = codes;
+        if (part == 0)
+          p.qs[row] = scale;
+      }
+    }
+  }
 }
 
 __device__ __forceinline__ float ex2(float x) {
@@ -621,7 +743,7 @@ size_t attention_int8_state_bytes(uint64_t B, uint64_t Sq, uint64_t H) {
 int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const float *ks, const void *v_bf16,
                    const uint8_t *key_valid, uint64_t B, uint64_t Sq, uint64_t S, uint64_t H, uint64_t KV,
                    uint64_t D, float scale, void *scratch, size_t scratch_bytes, void *out_bf16,
-                   cudaStream_t stream, const AttentionChunk *chunk) {
+                   cudaStream_t stream, const AttentionChunk *chunk, const AttentionSource *source) {
   // S is the number of key/value tokens from here on; Sq the number of query tokens.
   if (!q8 || !qs || !k8 || !ks || !v_bf16 || !out_bf16 || !scratch)
     return fail(kInvalidArgument, "Attention(INT8): null pointer");
@@ -695,7 +817,33 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
 
   float2 *table = static_cast<float2 *>(scratch);
   float *tile_bound = reinterpret_cast<float *>(table + B * KV * s_pad);
-  {
+  // q / k still in bf16: one launch quantises them and, with k, also builds the key table
+  if (source && (source->q || source->k)) {
+    if (chunk || (reinterpret_cast<uintptr_t>(source->q) | reinterpret_cast<uintptr_t>(source->k)) & 15)
+      return fail(kUnsupported, "Attention(INT8): pointers must be 16-byte aligned");
+    OperandParams o{};
+    o.q = static_cast<const uint4 *>(source->q);
+    o.k = static_cast<const uint4 *>(source->k);
+    o.q8 = const_cast<int8_t *>(q8);
+    o.k8 = const_cast<int8_t *>(k8);
+    o.qs = const_cast<float *>(qs);
+    o.ks = const_cast<float *>(ks);
+    o.key_valid = key_valid;
+    o.table = reinterpret_cast<float *>(table);
+    o.tile_bound = tile_bound;
+    o.q_rows = source->q ? B * Sq * H : 0;
+    o.S = (uint32_t)S;
+    o.KV = (uint32_t)KV;
+    o.S_pad = s_pad;
+    const uint64_t key_blocks = source->k ? B * KV * all_tiles : 0, blocks = key_blocks + (o.q_rows + 127) / 128;
+    if (blocks > 0x7fffffffull)
+      return fail(kUnsupported, "Attention(INT8): problem too large");
+    o.key_blocks = (uint32_t)key_blocks;
+    attention_operands_kernel<<<(unsigned)blocks, 256, 0, stream>>>(o);
+    if (int rc = launched(cudaGetLastError(), "attention_operands_kernel launch"))
+      return rc;
+  }
+  if (!(source && source->k)) {
     const uint64_t blocks = B * KV * (count[0] + count[1]);
     if (blocks > 0x7fffffffull)
       return fail(kUnsupported, "Attention(INT8): problem too large");

@@ -63,16 +63,9 @@ int attention_bf16_via_int8(const void *q, const void *k, const void *v, const u
   if (!scratch || scratch_bytes < attention_scratch_bytes(B, S, H, KV))
     return fail(kInvalidArgument, "Attention(INT8): scratch buffer too small");
   const AttentionScratch l = attention_scratch_layout(scratch, B, S, H, KV);
-  const void *qp[1] = {q}, *kp[1] = {k};
-  const uint64_t w[1] = {128};
-  if (q)
-    if (int rc = quantize_int8_rows(qp, w, 1, B * S * H, 1, 1.0f, nullptr, l.q8, l.qs, nullptr, nullptr, stream))
-      return rc;
-  if (k)
-    if (int rc = quantize_int8_rows(kp, w, 1, B * S * KV, 1, 1.0f, nullptr, l.k8, l.ks, nullptr, nullptr, stream))
-      return rc;
+  const AttentionSource source{q, k};
   return attention_int8(l.q8, l.qs, l.k8, l.ks, v, key_valid, B, S, S, H, KV, D, scale, l.rest,
-                        attention_int8_scratch_bytes(B, S, KV), out_bf16, stream);
+                        attention_int8_scratch_bytes(B, S, KV), out_bf16, stream, nullptr, &source);
 }
 
 } // namespace difb200

@@ -53,10 +53,15 @@ struct AttentionChunk {
   void *state; // attention_int8_state_bytes(B, Sq, H) bytes, 16-byte aligned
 };
 size_t attention_int8_state_bytes(uint64_t B, uint64_t Sq, uint64_t H);
+// q and / or k as bf16 tensors: attention_int8 then writes their codes and scales to its q8 / qs / k8 / ks first.
+struct AttentionSource {
+  const void *q, *k;
+};
 int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const float *ks, const void *v_bf16,
                    const uint8_t *key_valid, uint64_t B, uint64_t Sq, uint64_t Sk, uint64_t H, uint64_t KV,
                    uint64_t D, float scale, void *scratch, size_t scratch_bytes, void *out_bf16,
-                   cudaStream_t stream, const AttentionChunk *chunk = nullptr);
+                   cudaStream_t stream, const AttentionChunk *chunk = nullptr,
+                   const AttentionSource *source = nullptr);
 
 // DiffIR Attention on bf16 q/k/v in its INT8 lowering: Direct quantisation of q and k per
 // token-head, then attention_int8. Scratch holds the codes, scales and the key table.
