@@ -6,20 +6,25 @@
 //
 // Structure: persistent CTAs, one per SM. Both operands are K-major INT8, brought in by TMA as
 // 128-byte-swizzled [rows x 128 B] boxes into a shared-memory ring. One thread issues
-// tcgen05.mma kind::i8 into one of two 256-column INT32 accumulators in tensor memory, so the
+// tcgen05.mma kind::i8 into one of two BN-column INT32 accumulators in tensor memory, so the
 // epilogue of tile i overlaps the MMAs of tile i+1. Warp roles: 0 = TMA producer, 1 = TMEM owner
 // + MMA issuer, 2..9 = epilogue: two warps per TMEM lane quarter (warp_id % 4), one for each
-// 128-column half of the tile (four epilogue warps could not keep up with the K = 3072 main
+// column half of the tile (four epilogue warps could not keep up with the K = 3072 main
 // loop once bias and GELU are fused in).
 //
-// Two forms of the same kernel (template parameter CTAS):
-//   CTAS = 1: 128x256 tile per CTA, cta_group::1, 4 stages of 48 KB.
-//   CTAS = 2: a CTA pair (cluster of 2) computes a 256x256 tile with cta_group::2 MMAs: each CTA
-//             stages its 128 rows of A and only its 128 rows (half) of the B tile, 5 stages of
-//             32 KB. This halves the B bytes every SM moves through shared memory per MAC -- at
-//             8192 INT8 MACs/clk/SM the 128x256 single-CTA tile needs 48 KB written plus 48 KB read
-//             per 512 clocks, which is what bounds the CTAS = 1 form. The leader CTA (cluster rank
-//             0) issues the MMAs; both CTAs load, and both run the epilogue on their own 128 rows.
+// Forms of the same kernel (template parameters CTAS and BN, the tile's columns; choose_form has the rule):
+//   CTAS = 1: 128 x BN tile per CTA, cta_group::1, 4 stages of 48 KB (BN 256) or 5 of 32 KB (BN 128). A tile
+//             may be split over the k-blocks: the CTAs of a cluster each sum their share, then every CTA
+//             finishes the 32-column chunks it owns (chunk % split) from its own accumulator and the others'
+//             partial sums, which arrive in its freed stage ring through distributed shared memory. INT32
+//             sums are exact, so the bits do not depend on the split.
+//   CTAS = 2: a CTA pair (cluster of 2) computes a 256 x BN tile with cta_group::2 MMAs: each CTA
+//             stages its 128 rows of A and only its BN / 2 rows (half) of the B tile, 5 stages of
+//             32 KB (BN 256) or 7 of 24 KB (BN 128). This halves the B bytes every SM moves through
+//             shared memory per MAC -- at 8192 INT8 MACs/clk/SM the 128x256 single-CTA tile needs
+//             48 KB written plus 48 KB read per 512 clocks, which is what bounds the CTAS = 1 form.
+//             The leader CTA (cluster rank 0) issues the MMAs; both CTAs load, and both run the
+//             epilogue on their own 128 rows.
 //             TMA loads never use multicast. The bytes of both CTAs are counted on the leader's
 //             mbarrier (the peer issues the cta_group::2 form of the load, whose completion may
 //             target the peer CTA's barrier); the leader releases stages and publishes
@@ -30,6 +35,7 @@
 #include "common.cuh"
 #include "ptx.cuh"
 
+#include <cstdio>
 #include <cstdlib>
 #include <mutex>
 
@@ -74,32 +80,33 @@ int encode_tensor_map(CUtensorMap *out, CUtensorMapDataType type, uint32_t rank,
 
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 128; // per-CTA rows, tile columns, BK in bytes == INT8 elements
+constexpr int kBM = 128, kBK = 128; // per-CTA rows, BK in bytes == INT8 elements
 constexpr int kUmmaK = 32;
 constexpr uint32_t kABytes = kBM * kBK;
 constexpr int kThreads = 320;
 constexpr int kEpilogueWarps = 8;
-template <int CTAS>
+template <int CTAS, int BN>
 struct Cfg {
-  static constexpr int kStages = CTAS == 2 ? 5 : 4;
-  // staging boxes per epilogue warp (two let a TMA store drain while the next box is filled;
-  // the single-CTA form has room for one)
-  static constexpr uint32_t kBoxes = CTAS == 2 ? 2 : 1;
-  static constexpr uint32_t kStagingBytes = 8 /*epilogue warps*/ * kBoxes * 32 * 64;
-  static constexpr uint32_t kBRows = kBN / CTAS;                 // rows of the B tile this CTA stages
+  static constexpr uint32_t kBRows = BN / CTAS;                  // rows of the B tile this CTA stages
   static constexpr uint32_t kBBytes = kBRows * kBK;
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = kStageBytes <= 24 * 1024 ? 7 : kStageBytes <= 32 * 1024 ? 5 : 4; // 160-192 KB
+  // staging boxes per epilogue warp (two let a TMA store drain while the next box is filled;
+  // the 128x256 form has room for one)
+  static constexpr uint32_t kBoxes = kStageBytes <= 32 * 1024 ? 2 : 1;
+  static constexpr uint32_t kStagingBytes = kEpilogueWarps * kBoxes * 32 * 64;
+  static constexpr uint32_t kScaleBytes = kEpilogueWarps * BN * 4; // per warp: scales and biases of its BN / 2 columns
   static constexpr uint32_t kTileM = kBM * CTAS;                 // rows of the (pair's) output tile
+  static constexpr uint32_t kTmemCols = 2 * BN;                  // two accumulators
 };
-constexpr uint32_t kTmemCols = 512;
-// Epilogue staging: per epilogue warp two [32 rows x 32 bf16] boxes (64-byte rows, 64B TMA
-// swizzle); plus, per epilogue warp, 256 column scales and 256 biases (fp32) of the tile.
+// Epilogue staging: per epilogue warp one or two [32 rows x 32 bf16] boxes (64-byte rows, 64B TMA swizzle).
 constexpr uint32_t kStoreBoxBytes = 32 * 64;
-constexpr uint32_t kScaleBytes = kEpilogueWarps * 2 * (kBN / 2) * 4; // per warp: scales and biases of its 128 columns
-template <int CTAS>
+// Split form: a partial [32 rows x 32 columns] of INT32 on its way to the CTA that finishes it.
+constexpr uint32_t kPartialBytes = 32 * 32 * 4;
+template <int CTAS, int BN>
 constexpr size_t smem_bytes() {
-  return 1024 /*alignment slack*/ + (size_t)Cfg<CTAS>::kStages * Cfg<CTAS>::kStageBytes + Cfg<CTAS>::kStagingBytes +
-         kScaleBytes + 256;
+  return 1024 /*alignment slack*/ + (size_t)Cfg<CTAS, BN>::kStages * Cfg<CTAS, BN>::kStageBytes +
+         Cfg<CTAS, BN>::kStagingBytes + Cfg<CTAS, BN>::kScaleBytes + 256;
 }
 
 enum : uint32_t { kEpiBias = 1u, kEpiGeluTanh = 2u };
@@ -112,6 +119,7 @@ struct GemmParams {
   int32_t *acc_out;
   uint32_t M, N, K;
   uint32_t epilogue;
+  uint32_t split;   // CTAS = 1: CTAs of a cluster that share one tile's k-blocks (1 = no cluster)
   uint32_t tma_store; // 1: outputs leave through TMA stores (needs N % 8 == 0, aligned out)
   uint32_t withhold_kb; // test aid: the loads of this k-block are never issued (0xffffffff = none)
   unsigned long long wait_ns; // limit of every bounded wait
@@ -148,21 +156,22 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return packed;
 }
 
-template <int CTAS>
+template <int CTAS, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
-  constexpr int kStages = Cfg<CTAS>::kStages;
-  constexpr uint32_t kStageBytes = Cfg<CTAS>::kStageBytes;
-  constexpr uint32_t kTileM = Cfg<CTAS>::kTileM;
+  constexpr int kStages = Cfg<CTAS, BN>::kStages;
+  constexpr uint32_t kStageBytes = Cfg<CTAS, BN>::kStageBytes;
+  constexpr uint32_t kTileM = Cfg<CTAS, BN>::kTileM;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t cta_rank = CTAS == 2 ? ptx::cluster_ctarank() : 0u;  // 0 = leader of the pair
-  const uint32_t unit = CTAS == 2 ? blockIdx.x >> 1 : blockIdx.x;      // tile-scheduling unit
-  const uint32_t units = CTAS == 2 ? gridDim.x >> 1 : gridDim.x;
+  const uint32_t split = CTAS == 2 ? 1u : p.split, split_rank = split > 1 ? ptx::cluster_ctarank() : 0u;
+  const uint32_t unit = CTAS == 2 ? blockIdx.x >> 1 : blockIdx.x / split; // tile-scheduling unit
+  const uint32_t units = CTAS == 2 ? gridDim.x >> 1 : gridDim.x / split;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t staging_base = smem_base + kStages * kStageBytes;
-  const uint32_t scale_base = staging_base + Cfg<CTAS>::kStagingBytes;
-  const uint32_t bar_base = scale_base + kScaleBytes;
+  const uint32_t scale_base = staging_base + Cfg<CTAS, BN>::kStagingBytes;
+  const uint32_t bar_base = scale_base + Cfg<CTAS, BN>::kScaleBytes;
   // barrier layout (8 bytes each): full[kStages], empty[kStages], tmem_full[2], tmem_empty[2]; then a word
   // for the TMEM base address and a word for the abort flag.
   const uint32_t full_bar = bar_base, empty_bar = bar_base + 8 * kStages;
@@ -174,9 +183,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long wait_ns = p.wait_ns;
-  const uint32_t tiles_m = (p.M + kTileM - 1) / kTileM, tiles_n = (p.N + kBN - 1) / kBN;
+  const uint32_t tiles_m = (p.M + kTileM - 1) / kTileM, tiles_n = (p.N + BN - 1) / BN;
   const uint32_t num_tiles = tiles_m * tiles_n;
   const uint32_t k_blocks = (p.K + kBK - 1) / kBK;
+  // this CTA's k-blocks of every tile (all of them unless the tile is split; never empty: split <= k_blocks)
+  const uint32_t kb_first = k_blocks * split_rank / split, kb_end = k_blocks * (split_rank + 1u) / split;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -194,10 +205,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   if (warp == 1) {
     if (CTAS == 2) {
-      ptx::tmem_alloc_pair(tmem_slot, kTmemCols);
+      ptx::tmem_alloc_pair(tmem_slot, Cfg<CTAS, BN>::kTmemCols);
       ptx::tmem_relinquish_pair();
     } else {
-      ptx::tmem_alloc(tmem_slot, kTmemCols);
+      ptx::tmem_alloc(tmem_slot, Cfg<CTAS, BN>::kTmemCols);
       ptx::tmem_relinquish();
     }
   }
@@ -226,8 +237,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     for (uint32_t tile = unit; tile < num_tiles && ok; tile += units) {
       const int32_t m0 = (int32_t)((tile / tiles_n) * kTileM + cta_rank * kBM);
-      const int32_t n0 = (int32_t)((tile % tiles_n) * kBN + cta_rank * Cfg<CTAS>::kBRows);
-      for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+      const int32_t n0 = (int32_t)((tile % tiles_n) * BN + cta_rank * Cfg<CTAS, BN>::kBRows);
+      for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
         if (!ptx::mbar_wait_warp(empty_bar + 8 * stage, phase ^ 1u, abort_ptr, wait_ns)) {
           give_up(0, kb);
           ok = false;
@@ -269,7 +280,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 1) {
     if (cta_rank == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc(2 /*S32*/, 1 /*S8*/, 1 /*S8*/, 0, 0, kTileM, kBN);
+      constexpr uint32_t idesc = ptx::make_idesc(2 /*S32*/, 1 /*S8*/, 1 /*S8*/, 0, 0, kTileM, BN);
       const uint64_t desc0 = ptx::smem_desc_sw128(smem_base, 16, 1024);
       uint32_t stage = 0, phase = 0, local = 0;
       bool ok = true;
@@ -286,8 +297,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * kBN;
-        for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
           if (!ptx::mbar_wait_warp(full_bar + 8 * stage, phase, abort_ptr, wait_ns)) {
             give_up(1, kb);
             ok = false;
@@ -300,7 +311,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (ptx::elect_one()) {
 #pragma unroll
             for (int k = 0; k < kBK / kUmmaK; ++k) {
-              const uint32_t accumulate = k != 0 ? 1u : (kb != 0u ? 1u : 0u);
+              const uint32_t accumulate = k != 0 ? 1u : (kb != kb_first ? 1u : 0u);
               if (CTAS == 2)
                 ptx::mma_i8_ss_pair(d_tmem, a_desc + (uint64_t)(k * kUmmaK >> 4), b_desc + (uint64_t)(k * kUmmaK >> 4),
                                     idesc, accumulate);
@@ -326,38 +337,79 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t local = 0, store_buf = 0;
     uint8_t *generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
     float *scale_smem = reinterpret_cast<float *>(generic_base + (scale_base - smem_base));
-    const uint32_t my_staging = staging_base + ewarp * Cfg<CTAS>::kBoxes * kStoreBoxBytes;
+    const uint32_t my_staging = staging_base + ewarp * Cfg<CTAS, BN>::kBoxes * kStoreBoxBytes;
     uint8_t *my_staging_ptr = generic_base + (my_staging - smem_base);
     for (uint32_t tile = unit; tile < num_tiles; tile += units, ++local) {
       const uint32_t acc = local & 1u, acc_phase = (local >> 1) & 1u;
-      const uint32_t m0 = (tile / tiles_n) * kTileM + cta_rank * kBM, n0 = (tile % tiles_n) * kBN;
+      const uint32_t m0 = (tile / tiles_n) * kTileM + cta_rank * kBM, n0 = (tile % tiles_n) * BN;
       // column scales and biases of this tile -> this warp's private shared-memory copy
       // (warp-private so that no cross-warp barrier is needed)
-      float *cs = scale_smem + ewarp * kBN, *bs = cs + kBN / 2; // this warp's 128 columns
+      float *cs = scale_smem + ewarp * BN, *bs = cs + BN / 2; // this warp's 128 columns
       __syncwarp();
 #pragma unroll
-      for (int i = 0; i < kBN / 64; ++i) {
-        const uint32_t c = lane + 32u * i, n = n0 + col_half * (kBN / 2) + c;
+      for (int i = 0; i < BN / 64; ++i) {
+        const uint32_t c = lane + 32u * i, n = n0 + col_half * (BN / 2) + c;
         cs[c] = n < p.N ? __ldg(p.col_scales + n) : 0.0f;
         bs[c] = ((p.epilogue & kEpiBias) && n < p.N) ? bf16_bits_to_f32(__ldg(p.bias + n)) : 0.0f;
       }
       __syncwarp();
-      if (*abort_ptr || !ptx::mbar_wait(tfull_bar + 8 * acc, acc_phase, wait_ns)) {
+      const bool complete = ptx::mbar_wait_warp(tfull_bar + 8 * acc, acc_phase, abort_ptr, wait_ns);
+      if (!complete) {
         if (!*abort_ptr && lane == 0)
           report_timeout(p.status, 2, tile);
         *abort_ptr = 1;
-        break;
       }
+      if (split > 1) { // a split launch has one tile per cluster: every thread passes here once
+        __syncwarp();
+        ptx::cluster_sync(); // every CTA's MMAs are complete: the stage rings are free to receive partial sums
+        ptx::tc_fence_after();
+#pragma unroll 1
+        for (uint32_t sub = 0; sub < BN / 64; ++sub) {
+          const uint32_t chunk = col_half * (BN / 64) + sub, owner = chunk % split;
+          if (owner == split_rank)
+            continue;
+          uint32_t r[32];
+          ptx::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + acc * BN + chunk * 32u, r);
+          ptx::tmem_ld_wait();
+          const uint32_t slot = (chunk / split * split + split_rank) * 4u + quarter;
+          const uint32_t dst = ptx::mapa(smem_base + slot * kPartialBytes + lane * 16u, owner);
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            ptx::st_cluster_v4(dst + v * 512u, r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        }
+        __syncwarp();
+        ptx::cluster_sync(); // all partial sums have arrived
+      }
+      if (!complete)
+        break;
       ptx::tc_fence_after();
       const uint32_t row = m0 + quarter * 32u + lane;
       const bool row_ok = row < p.M;
       const float rs = row_ok ? __ldg(p.row_scales + row) : 0.0f;
 #pragma unroll 1
-      for (uint32_t sub = 0; sub < kBN / 64; ++sub) {
-        const uint32_t chunk = col_half * (kBN / 64) + sub; // 32-column chunk of the tile
+      for (uint32_t sub = 0; sub < BN / 64; ++sub) {
+        const uint32_t chunk = col_half * (BN / 64) + sub; // 32-column chunk of the tile
         uint32_t r[32];
-        ptx::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + acc * kBN + chunk * 32u, r);
+        ptx::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + acc * BN + chunk * 32u, r);
         ptx::tmem_ld_wait();
+        if (split > 1) {
+          if (chunk % split != split_rank)
+            continue; // finished by another CTA of the cluster
+          for (uint32_t from = 0; from < split; ++from) { // INT32 sums: exact in any order
+            if (from == split_rank)
+              continue;
+            const uint4 *part = reinterpret_cast<const uint4 *>(
+                generic_base + ((chunk / split * split + from) * 4u + quarter) * kPartialBytes) + lane;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+              const uint4 x = part[v * 32];
+              r[4 * v] += x.x;
+              r[4 * v + 1] += x.y;
+              r[4 * v + 2] += x.z;
+              r[4 * v + 3] += x.w;
+            }
+          }
+        }
         const uint32_t n_base = n0 + chunk * 32u;
         if (n_base >= p.N)
           continue; // (warp-uniform) whole chunk past the N edge
@@ -395,7 +447,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           // stage this warp's [32 x 32] box (64-byte rows, 16-byte chunk c of row r stored at
           // c ^ ((r >> 1) & 3): the 64B TMA swizzle, conflict-free), then one TMA store.
           if (lane == 0) { // the box about to be filled must have been read by its last store
-            if (Cfg<CTAS>::kBoxes == 2)
+            if (Cfg<CTAS, BN>::kBoxes == 2)
               asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
             else
               asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -416,7 +468,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
-          store_buf = Cfg<CTAS>::kBoxes == 2 ? store_buf ^ 1u : 0u;
+          store_buf = Cfg<CTAS, BN>::kBoxes == 2 ? store_buf ^ 1u : 0u;
         } else if (row_ok) {
           uint16_t *dst = p.out + (size_t)row * p.N + n_base;
           for (int i = 0; i < 32; ++i)
@@ -437,6 +489,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
+  if (split > 1 && warp < 2) { // the two barriers of the epilogue's exchange count every thread
+    __syncwarp();
+    ptx::cluster_sync();
+    ptx::cluster_sync();
+  }
   ptx::tc_fence_before();
   __syncthreads();
   if (CTAS == 2)
@@ -444,10 +501,117 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 1) {
     ptx::tc_fence_after();
     if (CTAS == 2)
-      ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+      ptx::tmem_dealloc_pair(tmem_base, Cfg<CTAS, BN>::kTmemCols);
     else
-      ptx::tmem_dealloc(tmem_base, kTmemCols);
+      ptx::tmem_dealloc(tmem_base, Cfg<CTAS, BN>::kTmemCols);
   }
+}
+
+// Tile form of a problem: CTAs per tile, tile columns, and the CTAs that share the k-blocks of a tile.
+struct Form {
+  int ctas, tile_n, split;
+};
+// The form with the least modelled time: waves of tiles x k-blocks per CTA x time of a k-block, plus what a
+// launch pays once (first loads, the last tile's epilogue, the exchange of a split). The figures, in ns, are
+// fitted to event times of every form at N 3072 / 9216 / 12288, K 3072 / 8192 / 12288 and 2 to 9216 rows with
+// cold caches. Large problems go to the 256 x 256 pair (fewest bytes per MAC). The narrower tiles and the
+// splits are for problems that leave SMs idle, where time is one CTA's serial chain of k-blocks: 2 rows,
+// K 12288, N 3072 45 -> 22.5 us (12 CTAs of 96 k-blocks -> 96 of 24), K 3072 20.5 -> 14.3 us; 512 rows, K 12288
+// 43 -> 31 us; 1600 rows, K 8192 53 -> 49 us; 1101 rows, N 12288 47 -> 43 us. A split costs more than it gives
+// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`.
+Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
+  struct Cost {
+    Form form;
+    uint64_t block_ns, launch_ns;
+  };
+  static const Cost costs[] = {{{2, 256, 1}, 320, 6000}, {{2, 128, 1}, 208, 4500}, {{1, 256, 1}, 363, 5100},
+                               {{1, 128, 1}, 245, 3200}, {{1, 128, 2}, 320, 3500}, {{1, 128, 4}, 450, 4600}};
+  const uint64_t sms = (uint64_t)sm_count(), k_blocks = (K + kBK - 1) / kBK;
+  // DIFB200_GEMM_FORM=ctas,columns,split forces one of the forms, DIFB200_GEMM_CTAS=1|2 a 256-column one
+  // (all give identical bits).
+  Form want{0, 0, 0}, best{1, 256, 1};
+  if (const char *force = std::getenv("DIFB200_GEMM_FORM"))
+    std::sscanf(force, "%d,%d,%d", &want.ctas, &want.tile_n, &want.split);
+  if (const char *force = std::getenv("DIFB200_GEMM_CTAS"))
+    if (force[0] == '1' || force[0] == '2')
+      want = Form{force[0] - '0', 256, 1};
+  uint64_t least = ~0ull;
+  for (const Cost &c : costs) {
+    const Form &f = c.form;
+    if ((uint64_t)f.split > k_blocks)
+      continue;
+    if (f.ctas == want.ctas && f.tile_n == want.tile_n && f.split == want.split)
+      return f;
+    const uint64_t tiles = ((M + kBM * f.ctas - 1) / (kBM * f.ctas)) * ((N + f.tile_n - 1) / f.tile_n);
+    const uint64_t resident = f.split > 2 ? sms * 7 / 8 / f.split : sms / (f.ctas * f.split); // wide clusters leave gaps
+    if ((f.ctas == 2 && M <= (uint64_t)kBM) || (f.split > 1 && tiles > resident))
+      continue;
+    const uint64_t waves = (tiles + resident - 1) / resident;
+    const uint64_t time = waves * ((k_blocks + f.split - 1) / f.split) * c.block_ns + c.launch_ns;
+    if (time < least) {
+      least = time;
+      best = f;
+    }
+  }
+  return best;
+}
+
+template <int CTAS, int BN>
+int launch_form(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorMap &map_c, const GemmParams &p,
+                cudaStream_t stream) {
+  // The dynamic shared-memory opt-in is an attribute of the function in one context, so it is
+  // made once per device (a process may hold plugin contexts on several GPUs).
+  static const char attr_key = 0;
+  if (int rc = current_device_once(&attr_key, [](void *, int *) -> int {
+        return check_cuda(cudaFuncSetAttribute(gemm_i8_kernel<CTAS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem_bytes<CTAS, BN>()),
+                          "cudaFuncSetAttribute(gemm_i8_kernel)");
+      }, nullptr, nullptr))
+    return rc;
+  const uint64_t tiles = (((uint64_t)p.M + Cfg<CTAS, BN>::kTileM - 1) / Cfg<CTAS, BN>::kTileM) *
+                         (((uint64_t)p.N + BN - 1) / BN);
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)sm_count());
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = smem_bytes<CTAS, BN>();
+  config.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CTAS == 2 ? 2u : p.split;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  uint64_t units = (uint64_t)sm_count();
+  if (CTAS == 2 || p.split > 1) {
+    config.attrs = &attr;
+    config.numAttrs = 1;
+  }
+  if (CTAS == 2) {
+    // The kernel is persistent: launch exactly as many CTA pairs as can be resident at once
+    // (SM pairs are formed inside a GPC, so this can be fewer than SMs / 2); a per-device figure.
+    static const char pairs_key = 0;
+    int resident_pairs = 0;
+    if (int rc = current_device_once(&pairs_key, [](void *arg, int *value) -> int {
+          int n = 0;
+          if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, gemm_i8_kernel<CTAS, BN>,
+                                                                 static_cast<cudaLaunchConfig_t *>(arg)),
+                                  "cudaOccupancyMaxActiveClusters"))
+            return rc;
+          *value = n > 0 ? n : 1;
+          return kOk;
+        }, &config, &resident_pairs))
+      return rc;
+    units = (uint64_t)resident_pairs;
+  }
+  if (CTAS == 1 && p.split > 1) {
+    // one cluster per tile: clusters do not wait for one another, so they need not all be resident
+    if (tiles * p.split > 0x7fffffffull)
+      return fail(kUnsupported, "LinearInt8Scaled: problem too large");
+    config.gridDim = dim3((unsigned)(tiles * p.split));
+  } else {
+    config.gridDim = dim3((unsigned)(CTAS * (units < tiles ? units : tiles)));
+  }
+  return launched(cudaLaunchKernelEx(&config, gemm_i8_kernel<CTAS, BN>, map_a, map_b, map_c, p),
+                  "gemm_i8_kernel launch");
 }
 
 } // namespace
@@ -474,21 +638,11 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   if (!status)
     return fail(kOutOfMemory, "LinearInt8Scaled: cannot allocate device status words");
 
-  // Form: the CTA-pair kernel moves a third less through shared memory per MAC and is the faster
-  // one whenever its 256x256 tiles fill the machine as well as 128x256 tiles do; the choice
-  // compares the number of tile waves (a pair wave costs about 0.94 of a single-CTA wave).
-  // DIFB200_GEMM_CTAS=1|2 forces a form (both give identical bits).
-  const uint64_t pair_tiles = ((M + 255) / 256) * ((N + kBN - 1) / kBN);
-  const uint64_t single_tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN);
-  const uint64_t sms = (uint64_t)sm_count();
-  const uint64_t single_waves = (single_tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
-  int ctas = (M > (uint64_t)kBM && 94 * pair_waves <= 100 * single_waves) ? 2 : 1;
-  if (const char *force = std::getenv("DIFB200_GEMM_CTAS"))
-    ctas = force[0] == '2' ? 2 : (force[0] == '1' ? 1 : ctas);
+  const Form form = choose_form(M, N, K);
   CUtensorMap map_a, map_b;
   const uint64_t dims_a[2] = {K, M}, dims_b[2] = {K, N};
   const uint64_t strides[1] = {K};
-  const uint32_t box_a[2] = {(uint32_t)kBK, (uint32_t)kBM}, box_b[2] = {(uint32_t)kBK, (uint32_t)(kBN / ctas)};
+  const uint32_t box_a[2] = {(uint32_t)kBK, (uint32_t)kBM}, box_b[2] = {(uint32_t)kBK, (uint32_t)(form.tile_n / form.ctas)};
   if (int rc = encode_tensor_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, x, dims_a, strides, box_a,
                                  CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
@@ -507,20 +661,6 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
       return rc;
   }
 
-  // The dynamic shared-memory opt-in is an attribute of the function in one context, so it is
-  // made once per device (a process may hold plugin contexts on several GPUs).
-  static const char attr_key = 0;
-  if (int rc = current_device_once(&attr_key, [](void *, int *) -> int {
-        if (int rc = check_cuda(cudaFuncSetAttribute(gemm_i8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)smem_bytes<1>()),
-                                "cudaFuncSetAttribute(gemm_i8_kernel<1>)"))
-          return rc;
-        return check_cuda(cudaFuncSetAttribute(gemm_i8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem_bytes<2>()),
-                          "cudaFuncSetAttribute(gemm_i8_kernel<2>)");
-      }, nullptr, nullptr))
-    return rc;
-
   GemmParams p{};
   p.row_scales = row_scales;
   p.col_scales = col_scales;
@@ -531,50 +671,16 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   p.N = (uint32_t)N;
   p.K = (uint32_t)K;
   p.epilogue = epilogue;
+  p.split = (uint32_t)form.split;
   p.tma_store = tma_store ? 1u : 0u;
   p.withhold_kb = take_withheld_gemm_load();
   p.wait_ns = wait_limit_ns();
   p.status = status;
-  if (ctas == 2) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3((unsigned)sm_count());
-    config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = smem_bytes<2>();
-    config.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    config.attrs = &attr;
-    config.numAttrs = 1;
-    // The kernel is persistent: launch exactly as many CTA pairs as can be resident at once
-    // (SM pairs are formed inside a GPC, so this can be fewer than SMs / 2); a per-device figure.
-    static const char pairs_key = 0;
-    int resident_pairs = 0;
-    if (int rc = current_device_once(&pairs_key, [](void *arg, int *value) -> int {
-          int n = 0;
-          if (int rc = check_cuda(cudaOccupancyMaxActiveClusters(&n, gemm_i8_kernel<2>,
-                                                                 static_cast<cudaLaunchConfig_t *>(arg)),
-                                  "cudaOccupancyMaxActiveClusters"))
-            return rc;
-          *value = n > 0 ? n : 1;
-          return kOk;
-        }, &config, &resident_pairs))
-      return rc;
-    uint64_t pairs = (uint64_t)resident_pairs;
-    if (pairs > pair_tiles)
-      pairs = pair_tiles;
-    config.gridDim = dim3((unsigned)(2 * pairs));
-    return launched(cudaLaunchKernelEx(&config, gemm_i8_kernel<2>, map_a, map_b, map_c, p),
-                      "gemm_i8_kernel<2> launch");
-  }
-  const uint64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN);
-  uint64_t grid = (uint64_t)sm_count();
-  if (grid > tiles)
-    grid = tiles;
-  gemm_i8_kernel<1><<<(unsigned)grid, kThreads, smem_bytes<1>(), stream>>>(map_a, map_b, map_c, p);
-  return launched(cudaGetLastError(), "gemm_i8_kernel launch");
+  if (form.ctas == 2)
+    return form.tile_n == 256 ? launch_form<2, 256>(map_a, map_b, map_c, p, stream)
+                              : launch_form<2, 128>(map_a, map_b, map_c, p, stream);
+  return form.tile_n == 256 ? launch_form<1, 256>(map_a, map_b, map_c, p, stream)
+                            : launch_form<1, 128>(map_a, map_b, map_c, p, stream);
 }
 
 } // namespace difb200

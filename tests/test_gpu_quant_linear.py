@@ -155,6 +155,31 @@ def test_linear_int8_scaled_bit_exact(ops, gemm_form, M, K, N):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("form", ["2,128,1", "1,128,1", "1,128,2", "1,128,4", None])
+@pytest.mark.parametrize("M,K,N", [(1, 3072, 3072), (2, 12288, 384), (127, 528, 128), (129, 656, 264), (257, 1168, 131),
+                                   (520, 512, 1032)])
+def test_linear_int8_scaled_narrow_and_split_tiles(ops, monkeypatch, form, M, K, N):
+    """The 128-column tiles and the splits over k-blocks (cluster exchange): tile edges in M and N, ragged k-blocks
+    (a split whose shares differ), odd N (no TMA stores); `None` is the form the dispatch picks."""
+    import torch
+    if form:
+        monkeypatch.setenv("DIFB200_GEMM_FORM", form)
+    g = torch.Generator().manual_seed(M + N + K)
+    x8, w8 = (torch.randint(-127, 128, s, dtype=torch.int8, generator=g) for s in ((M, K), (N, K)))
+    xs, ws = torch.rand(M, generator=g), torch.rand(N, generator=g)
+    bias = torch.randn(N, generator=g).to(torch.bfloat16)
+    want_acc = (x8.double() @ w8.double().T).to(torch.int32)  # exact: below 2^53
+    want = ((want_acc.float() * xs[:, None]) * ws[None]).to(torch.bfloat16)
+    dev = [t.cuda() for t in (x8, w8, xs, ws)]
+    for _ in range(2):
+        got, acc = ops.linear_int8_scaled(*dev, want_acc=True)
+        assert torch.equal(acc.cpu(), want_acc)
+        assert torch.equal(got.cpu(), want)
+        got = ops.linear_int8_scaled(*dev, bias=bias.cuda())
+        assert torch.equal(got.cpu(), (want.float() + bias.float()[None]).to(torch.bfloat16))
+    ops.poll_status()
+
+
 def test_w8a8_linear_end_to_end_single_layer(ops):
     """The single-layer benchmark case (M=1024, K=N=3072, H256ConvRot activations, bias): GPU quant + GEMM chained."""
     import torch
