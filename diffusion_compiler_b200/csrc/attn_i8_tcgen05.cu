@@ -34,7 +34,8 @@
 // so when a softmax warp finishes a step the scores of the next one are already there.
 // Tensor memory (512 columns): per query tile two score buffers of 64 columns (INT32; the bf16 P
 // of a step overwrites the first 32 columns of its buffer and is the TMEM A operand of P.V),
-// then O0 | O1 (fp32, 128 columns each).
+// then O0 | O1 (fp32, 128 columns each). Items that would not fill a last wave are shared by clusters of CTAs that
+// take a part of the keys each (plan_split).
 //
 // Chunked form (the token-sharded block, where keys arrive from other GPUs one slice at a time):
 // a launch covers up to two ranges of 128-key tiles and may carry the unnormalised state of every
@@ -60,6 +61,7 @@ constexpr uint32_t kVBytes = 128 * 128 * 2;    // bf16 [128 keys x 128] as two 6
 constexpr uint32_t kKsBytes = 128 * 8;         // (key scale, mask bias) per key, as float4 per key pair
 constexpr uint32_t kStageBytes = kKBytes + kVBytes + kKsBytes;
 constexpr int kThreads = 384;
+constexpr uint32_t kPartialBytes = 32 * 32 * 4; // split form: a [32 rows x 32 columns] fp32 partial output
 constexpr uint32_t kOutBoxBytes = 32 * 128;    // a warp's output staging: two [32 rows x 64 bf16] boxes
 constexpr size_t kSmemBytes = 1024 + 2 * kQBytes + kStages * kStageBytes + 256;
 
@@ -68,6 +70,7 @@ struct AttnParams {
   const float2 *ksmb;    // [B,KV,S_pad/2] x float4 (ks'_j, ks'_j+1, bias_j, bias_j+1)
   const float *tile_bound; // [B,KV,S_pad/128] max over the tile's valid keys of |k8_j| * ks'_j
   uint32_t B, Sq, Sk, H, KV, S_pad; // Sq query tokens, Sk key tokens (S_pad = Sk rounded up to 128)
+  uint16_t *out;         // [B,Sq,H,128] bf16
   float scale_log2e;     // scale * log2(e)
   unsigned long long wait_ns; // limit of every bounded wait
   DeviceStatus *status;
@@ -76,6 +79,7 @@ struct AttnParams {
   float *o_state;        // [B,Sq,H,128] fp32 unnormalised outputs carried between launches
   float2 *ml_state;      // [B,Sq,H] (m, l) carried between launches
   uint32_t carry_in, carry_out;
+  uint32_t item0, split; // first (batch, head, query block) of this launch; CTAs of a cluster that share its keys
 };
 
 __device__ __forceinline__ void report(DeviceStatus *status, uint32_t role, uint32_t detail) {
@@ -272,6 +276,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return packed;
 }
 
+// 32 outputs bf16(o / l) from RN(1 / l) and one correction by the residual (one rounding); where that has no
+// finite value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0.
+__device__ __forceinline__ void normalise(const uint32_t (&o)[32], float l, uint32_t (&w)[16]) {
+  const float y = __frcp_rn(l);
+  const uint64_t y2 = pack2(y, y), negl2 = pack2(-l, -l);
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    const uint64_t o2 = pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1]));
+    const uint64_t q2 = mul2(o2, y2);
+    float y0, y1, x0, x1;
+    unpack2(q2, y0, y1);
+    unpack2(fma2(fma2(q2, negl2, o2), y2, q2), x0, x1);
+    w[j >> 1] = l > 0.0f ? pack_bf16(x0 == x0 ? x0 : y0, x1 == x1 ? x1 : y1) : 0u;
+  }
+}
+
+// SPLIT: the launch whose items are shared by clusters (an instance of its own: run-time branches for it cost the
+// plain one 2 %).
+template <bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -298,14 +321,19 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long wait_ns = p.wait_ns;
   const uint32_t q_blocks = (p.Sq + 255u) / 256u;
-  const uint32_t qb = blockIdx.x % q_blocks;
-  const uint32_t head = (blockIdx.x / q_blocks) % p.H;
-  const uint32_t batch = blockIdx.x / (q_blocks * p.H);
+  const uint32_t split = SPLIT ? p.split : 1u, rank = SPLIT ? ptx::cluster_ctarank() : 0u;
+  const uint32_t item = SPLIT ? p.item0 + blockIdx.x / split : blockIdx.x;
+  const uint32_t qb = item % q_blocks;
+  const uint32_t head = (item / q_blocks) % p.H;
+  const uint32_t batch = item / (q_blocks * p.H);
   const uint32_t kvh = head / (p.H / p.KV);
   const uint32_t q0 = qb * 256u;
-  const uint32_t n_kv = p.tile_count[0] + p.tile_count[1];
+  const uint32_t tiles = p.tile_count[0] + p.tile_count[1], first = SPLIT ? tiles * rank / split : 0u;
+  const uint32_t n_kv = SPLIT ? tiles * (rank + 1u) / split - first : tiles; // of this CTA (at least one: split <= tiles)
   const uint32_t n_steps = 2u * n_kv;               // 64-key steps
-  auto key_tile = [&](uint32_t i) {                 // i-th key tile of this launch -> tile of the key axis
+  auto key_tile = [&](uint32_t i) {                 // i-th key tile of this CTA -> tile of the key axis
+    if (SPLIT)
+      i += first;
     return i < p.tile_count[0] ? p.tile_begin[0] + i : p.tile_begin[1] + (i - p.tile_count[0]);
   };
   auto score_col = [](uint32_t t, uint32_t b) { return t * 128u + b * 64u; }; // TMEM column of a score buffer
@@ -483,6 +511,12 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           }
         }
       }
+    }
+    if (SPLIT) { // the three barriers of the outputs' exchange count every thread of the cluster
+      __syncwarp();
+      ptx::cluster_sync();
+      ptx::cluster_sync();
+      ptx::cluster_sync();
     }
   } else {
     // ---------------- softmax + epilogue, one thread per query row ----------------
@@ -681,7 +715,88 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::tc_fence_before();
       ptx::mbar_arrive(p_full + 16 * t + 8 * h);
     }
-    if (alive && n_kv > 0) {
+    if (SPLIT) {
+      // The CTAs of the cluster hold the unnormalised outputs of the same queries over parts of the keys. Every m
+      // is an integer, so all move to the largest one by exact powers of two. Unit u = (query tile, 32 columns) is
+      // finished by CTA u % split: the others send it their scaled fp32 sums through distributed shared memory.
+      // Three cluster barriers, passed by every thread on every path.
+      alive = __all_sync(0xffffffffu, alive);
+      if (alive && !ptx::mbar_wait_warp(o_done + 8 * t, 0, abort_ptr, wait_ns)) {
+        if (!*abort_ptr && lane == 0)
+          report(p.status, 7 + t, 0);
+        *abort_ptr = 1;
+        alive = false;
+      }
+      __syncwarp();
+      ptx::cluster_sync(); // all MMAs of all CTAs are done: Q and the stage ring are free
+      ptx::tc_fence_after();
+      const uint32_t row = t * 128u + row_in_tile;
+      for (uint32_t r = 0; r < split; ++r) // (m, l) of every CTA and row, where Q was
+        ptx::st_cluster_v2(ptx::mapa(q_addr + (rank * 256u + row) * 8u, r), __float_as_uint(m_run), __float_as_uint(l));
+      __syncwarp();
+      ptx::cluster_sync();
+      const float2 *mls = reinterpret_cast<const float2 *>(base_ptr + (q_addr - base)) + row;
+      float m_all = -INFINITY, l_all = 0.0f;
+      for (uint32_t r = 0; r < split; ++r)
+        m_all = fmaxf(m_all, mls[r * 256u].x);
+      for (uint32_t r = 0; r < split; ++r)
+        l_all += mls[r * 256u].x == -INFINITY ? 0.0f : mls[r * 256u].y * ex2(mls[r * 256u].x - m_all);
+      const float factor = m_run == -INFINITY ? 0.0f : ex2(m_run - m_all);
+      auto scaled = [&](uint32_t c, uint32_t(&o)[32]) {
+        ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          o[j] = __float_as_uint(__uint_as_float(o[j]) * factor);
+      };
+      // slot of (unit, sending CTA, lane quarter) in the ring of the unit's owner: at most 9 x 4 of 4 KB
+      auto slot = [&](uint32_t u, uint32_t from) {
+        return stage_addr + ((u / split * split + from) * 4u + quarter) * kPartialBytes + lane * 16u;
+      };
+#pragma unroll 1
+      for (uint32_t c = 0; c < 4; ++c) {
+        const uint32_t u = t * 4u + c, owner = u % split;
+        if (owner == rank)
+          continue;
+        uint32_t o[32];
+        scaled(c, o);
+        const uint32_t dst = ptx::mapa(slot(u, rank), owner);
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          ptx::st_cluster_v4(dst + v * 512u, o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
+      }
+      __syncwarp();
+      ptx::cluster_sync();
+#pragma unroll 1
+      for (uint32_t c = 0; c < 4; ++c) {
+        const uint32_t u = t * 4u + c;
+        if (u % split != rank)
+          continue;
+        uint32_t o[32];
+        scaled(c, o);
+        for (uint32_t from = 0; from < split; ++from) {
+          if (from == rank)
+            continue;
+          const uint4 *part = reinterpret_cast<const uint4 *>(base_ptr + (slot(u, from) - base));
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            const uint4 x = part[v * 32];
+            o[4 * v] = __float_as_uint(__uint_as_float(o[4 * v]) + __uint_as_float(x.x));
+            o[4 * v + 1] = __float_as_uint(__uint_as_float(o[4 * v + 1]) + __uint_as_float(x.y));
+            o[4 * v + 2] = __float_as_uint(__uint_as_float(o[4 * v + 2]) + __uint_as_float(x.z));
+            o[4 * v + 3] = __float_as_uint(__uint_as_float(o[4 * v + 3]) + __uint_as_float(x.w));
+          }
+        }
+        uint32_t w[16];
+        normalise(o, l_all, w);
+        if (alive && row_ok) { // one launch's tail only: plain stores of 64 bytes per row
+          uint4 *dst = reinterpret_cast<uint4 *>(p.out + (((uint64_t)batch * p.Sq + qrow) * p.H + head) * kTile + 32u * c);
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            dst[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+        }
+      }
+    } else if (alive && n_kv > 0) {
       if (!ptx::mbar_wait(o_done + 8 * t, 0, wait_ns)) {
         if (lane == 0)
           report(p.status, 7 + t, 0);
@@ -714,25 +829,13 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const uint32_t stage = (n_kv + t) % kStages;
           const uint32_t staging = stage_addr + stage * kStageBytes + quarter * (2u * kOutBoxBytes);
           uint8_t *staging_ptr = base_ptr + (staging - base);
-          // o / l from RN(1 / l) and one correction by the residual (one rounding); where that has no finite
-          // value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0.
-          const float y = __frcp_rn(l);
-          const uint64_t y2 = pack2(y, y), negl2 = pack2(-l, -l);
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t o[32];
             ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
             ptx::tmem_ld_wait();
             uint32_t w[16];
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const uint64_t o2 = pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1]));
-              const uint64_t q2 = mul2(o2, y2);
-              float y0, y1, x0, x1;
-              unpack2(q2, y0, y1);
-              unpack2(fma2(fma2(q2, negl2, o2), y2, q2), x0, x1);
-              w[j >> 1] = l > 0.0f ? pack_bf16(x0 == x0 ? x0 : y0, x1 == x1 ? x1 : y1) : 0u;
-            }
+            normalise(o, l, w);
             uint8_t *box = staging_ptr + (c >> 1) * kOutBoxBytes + lane * 128;
 #pragma unroll
             for (int v = 0; v < 4; ++v)
@@ -759,6 +862,69 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
+}
+
+void split_config(cudaLaunchConfig_t &config, cudaLaunchAttribute &attr, uint32_t split) {
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmemBytes;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = split;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  config.attrs = &attr;
+  config.numAttrs = split > 1 ? 1 : 0;
+}
+
+// Clusters of `split` CTAs that fit on the device at once (one CTA per SM, clusters inside a GPC).
+int resident_clusters(uint32_t split, int &count) {
+  static const char keys[9] = {};
+  return current_device_once(&keys[split], [](void *arg, int *value) -> int {
+    cudaLaunchConfig_t config{};
+    cudaLaunchAttribute attr{};
+    const uint32_t ctas = *static_cast<uint32_t *>(arg);
+    split_config(config, attr, ctas);
+    config.gridDim = dim3((unsigned)sm_count() / ctas * ctas); // the grid has to be a multiple of the cluster
+    return check_cuda(cudaOccupancyMaxActiveClusters(value, attn_i8_kernel<true>, &config), "cudaOccupancyMaxActiveClusters");
+  }, &split, &count);
+}
+
+// Items (batch, head, 256 queries) that run as one CTA each, and the split over the keys of the others. A last wave
+// that is nearly empty costs as much as a full one: 3120 items of the 33272-token block are 21.08 waves of 148 SMs.
+// Its items (or those of the last two waves) are split 2, 3, 4 or 8 ways over the key tiles by clusters. Modelled
+// times in ns, measured on B200: 1660 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
+// and the exchange, at least four tiles per CTA; a split has to give 3 %. H24, without -> with: 1 x 1700 tokens
+// (1.14 waves) 75 -> 70 us, 2 x 2500 (3.24) 188 -> 178 us, 1 x 8000 (5.19) 707 -> 645 us.
+int plan_split(uint64_t items, uint64_t tiles, uint64_t &whole, uint32_t &split) {
+  constexpr uint64_t kTileNs = 1660, kItemNs = 6000, kExchangeNs = 8000;
+  const uint64_t sms = (uint64_t)sm_count(), item_ns = kItemNs + tiles * kTileNs;
+  whole = items;
+  split = 1;
+  uint64_t least = (items + sms - 1) / sms * item_ns * 97 / 100;
+  for (uint64_t back = 0; back < 2; ++back) {
+    if (items / sms < back)
+      break;
+    const uint64_t waves = items / sms - back, rest = items - waves * sms;
+    if (rest == 0)
+      continue;
+    for (uint32_t s : {2u, 3u, 4u, 8u}) {
+      if (tiles < 4ull * s)
+        break;
+      int resident = (int)(sms / s); // at most; asked for only where that would do
+      auto time = [&]() {
+        return waves * item_ns +
+               (rest + resident - 1) / resident * (kItemNs + kExchangeNs + (tiles + s - 1) / s * kTileNs);
+      };
+      if (time() >= least)
+        continue;
+      if (int rc = resident_clusters(s, resident))
+        return rc;
+      if (resident > 0 && time() < least) {
+        least = time();
+        whole = waves * sms;
+        split = s;
+      }
+    }
+  }
+  return kOk;
 }
 
 } // namespace
@@ -850,9 +1016,12 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
   }
   static const char attr_key = 0; // the opt-in belongs to the function in one context: once per device
   if (int rc = current_device_once(&attr_key, [](void *, int *) -> int {
-        return check_cuda(cudaFuncSetAttribute(attn_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)kSmemBytes),
-                          "cudaFuncSetAttribute(attn_i8_kernel)");
+        for (auto *kernel : {attn_i8_kernel<false>, attn_i8_kernel<true>})
+          if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)kSmemBytes),
+                                  "cudaFuncSetAttribute(attn_i8_kernel)"))
+            return rc;
+        return kOk;
       }, nullptr, nullptr))
     return rc;
 
@@ -898,6 +1067,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
   p.qs = qs;
   p.ksmb = table;
   p.tile_bound = tile_bound;
+  p.out = static_cast<uint16_t *>(out_bf16);
   p.B = (uint32_t)B;
   p.Sq = (uint32_t)Sq;
   p.Sk = (uint32_t)S;
@@ -918,9 +1088,28 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     p.carry_in = chunk->carry_in ? 1u : 0u;
     p.carry_out = chunk->carry_out ? 1u : 0u;
   }
-  const uint64_t grid = B * H * ((Sq + 255) / 256);
-  attn_i8_kernel<<<(unsigned)grid, kThreads, kSmemBytes, stream>>>(map_q, map_k, map_v, map_o, p);
-  return launched(cudaGetLastError(), "attn_i8_kernel launch");
+  const uint64_t items = B * H * ((Sq + 255) / 256);
+  uint64_t whole = items;
+  uint32_t split = 1;
+  if (!chunk)
+    if (int rc = plan_split(items, all_tiles, whole, split))
+      return rc;
+  auto launch = [&](uint64_t first, uint64_t count, uint32_t ctas) {
+    p.item0 = (uint32_t)first;
+    p.split = ctas;
+    cudaLaunchConfig_t config{};
+    cudaLaunchAttribute attr{};
+    split_config(config, attr, ctas);
+    config.gridDim = dim3((unsigned)(count * ctas));
+    config.stream = stream;
+    return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k,
+                                       map_v, map_o, p),
+                    "attn_i8_kernel launch");
+  };
+  if (whole)
+    if (int rc = launch(0, whole, 1))
+      return rc;
+  return whole < items ? launch(whole, items - whole, split) : kOk;
 }
 
 } // namespace difb200

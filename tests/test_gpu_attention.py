@@ -193,3 +193,46 @@ def test_attention_launch_plans_of_every_rank_match_the_single_launch(ops, size,
         assert np.all(np.abs(a - b) <= 2.0 ** -7 * np.abs(b) + 1e-3 * np.abs(b).max()), (size, rank)
         assert np.mean(a != b) <= 0.01, (size, rank, float(np.mean(a != b)))
     ops.poll_status()
+
+
+@pytest.mark.parametrize("B,Sq,Sk,H,KV,masked,q_gain", [
+    (1, 700, 1100 + 3 * 512, 24, 8, True, 1.0),    # 72 items, 21 ragged tiles: two CTAs per item
+    (2, 300, 1700, 12, 12, False, 1.0),            # 48 items of 14 tiles: three where their clusters fit
+    (1, 130, 4096 + 77, 6, 2, True, 6.0),          # 6 items of 33 tiles: eight, running maximum
+    (1, 1, 2048, 5, 5, True, 1.0),                 # one query row
+    (1, 1400, 2500, 25, 25, False, 1.0),           # 150 items: one whole wave, then the rest split
+])
+def test_attention_split_over_keys_matches_the_plain_launch(ops, B, Sq, Sk, H, KV, masked, q_gain):
+    """Items that would leave most SMs idle are split over the keys by clusters; the chunked form with one range is
+    the same launch without the split. Powers of two scale exactly, so only the order of the fp32 sums differs:
+    the bars of the launch plans above. The mask hides all keys of one CTA's share, and in the last entry of the
+    batch all but one key."""
+    import torch
+    rng = np.random.default_rng(700 + Sk)
+    q, _, _ = _qkv(rng, B, Sq, H, KV)
+    _, k, v = _qkv(rng, B, Sk, H, KV)
+    if q_gain != 1.0:
+        q = ob.f32_to_bf16(ob.bf16_to_f32(q) * np.float32(q_gain))
+    tv = None
+    if masked:
+        valid = np.ones((B, Sk), np.uint8)
+        valid[:, :Sk // 2 + 200] = 0
+        valid[:, Sk - 37:] = 0
+        tv = torch.from_numpy(valid).cuda()
+    q8, qs = ob.orc().quantize_int8_rows([q.reshape(-1, 128)], 1)
+    k8, ks = ob.orc().quantize_int8_rows([k.reshape(-1, 128)], 1)
+    t = lambda a: torch.from_numpy(a).cuda()
+    args = (t(q8.reshape(B, Sq, H, 128)), t(qs), t(k8.reshape(B, Sk, KV, 128)), t(ks), to_torch_bf16(v))
+    split = ops.attention_int8(*args, tv)
+    again = ops.attention_int8(*args, tv)
+    plain = ops.attention_int8_chunked(*args, [[(0, (Sk + 127) // 128)]], tv)
+    torch.cuda.synchronize()
+    ops.poll_status()
+    assert torch.equal(split.view(torch.int16), again.view(torch.int16))
+    a, b = (ob.bf16_to_f32(from_torch_bf16(x)) for x in (split, plain))
+    assert np.isfinite(a).all() and rel_l2(a, b) <= 3e-4, rel_l2(a, b)
+    assert np.all(np.abs(a - b) <= 2.0 ** -7 * np.abs(b) + 1e-3 * np.abs(b).max())
+    assert np.mean(a != b) <= 0.01, float(np.mean(a != b))
+    if masked:  # nothing valid anywhere: zeros
+        none = ops.attention_int8(*args, torch.zeros_like(tv))
+        assert torch.count_nonzero(none.float()) == 0
