@@ -541,8 +541,15 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
 // One block of 1024 columns per warp: the fp32 and residual forms, narrow rows, and calls of few rows.
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
 int launch_single(const QuantParams &p, cudaStream_t stream) {
-  if (((p.columns >> 8) + 3u) / 4u > 8u)
+  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+  // A row is a CTA of 9 to 16 warps: two of them per SM, or its barriers leave the SM idle (128 registers and one
+  // CTA: 3333 x 12288 fp32 60 us, two CTAs 47 us; 3333 x 15360 73 us and 58 us).
+  if (blocks > 8u) {
+    if constexpr (EXTRA == kPlain && !RESIDUAL)
+      return blocks <= 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 384, 2>(p, stream)
+                           : launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 512, 2>(p, stream);
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
+  }
   if constexpr (EXTRA == kNorm)
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream); // 24 warps, three tensors in flight
   else if constexpr (EXTRA != kPlain || (RESIDUAL && !F32))
@@ -569,17 +576,18 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     return launch_single<SIGNED, false, true, kPlain>(p, stream);
   if (norm)
     return launch_single<SIGNED, false, false, kNorm>(p, stream);
-  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, so calls
-  // whose rows fill the machine less than once with one block per warp keep that form, and so do
-  // rows of up to 8 blocks that three do not divide (8192 columns: 34.3 us against 41.5 us for 4159
-  // rows, the last warp would idle on a third of its slots). Wider rows take three in any case:
-  // one block per warp would make CTAs of up to 16 warps that meet at one barrier (4608 x 15360: 92 us
-  // against 73 us).
+  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, at half the
+  // occupancy: worth it from three rounds of the machine (9216 x 3072 30.2 -> 28.8 us; below, the last round is
+  // mostly empty: 3333 x 3072 signed 18.9 us with three, under 14.9 with one). Rows of up to 8 blocks that three
+  // do not divide keep one (8192 columns: 34.3 us against 41.5 us for 4159 rows, the last warp would idle on
+  // a third of its slots). Packing without the scale search follows the same line (3072 x 3072 27.4 -> 22.0 us);
+  // the search is arithmetic that the form for few rows need not hide.
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
   const bool few = p.rows * blocks <= (uint64_t)sm_count() * 24u;
-  const bool three = (blocks % 3u == 0 || blocks > 8u) && !few;
+  const uint64_t round = (uint64_t)sm_count() * 16u * 3u; // blocks that run at once with three per warp
+  const bool three = (blocks % 3u == 0 || blocks > 8u) && p.rows * blocks >= 3u * round;
   if (pack)
-    return few || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
+    return few || blocks == 1u || (!p.mse && p.rows * blocks < 3u * round) ? launch_single<SIGNED, false, false, kPack>(p, stream)
                                : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
   return three ? launch_form<SIGNED, false, false, kPlain, 3, true, 256, 2>(p, stream)
                : launch_single<SIGNED, false, false, kPlain>(p, stream);
