@@ -408,9 +408,6 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
     p.norm_bias = static_cast<const uint16_t *>(norm->bias);
     p.minus_zero2 = 0x8000000080000000ull;
     p.norm_rows_per_mod = norm->rows_per_modulation;
-    if (rows > 0) // the row statistic, by its own kernel in front
-      if (int rc = glue::row_stats(parts[0], rows, columns, norm->epsilon, norm->bias != nullptr, &p.norm_stats, stream))
-        return rc;
   }
   if (rows == 0)
     return kOk;
@@ -447,6 +444,9 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
     return fail(kUnsupported,
                 "QuantizeInt8Rows: ConvRot path needs 16-byte aligned pointers and part widths "
                 "that are multiples of 16");
+  if (norm) // the row statistic, by its own kernel in front: only now that nothing above refuses the call
+    if (int rc = glue::row_stats(parts[0], rows, columns, norm->epsilon, norm->bias != nullptr, &p.norm_stats, stream))
+      return rc;
   if (!h4096)
     return launch_convrot256(p, implementation, stream);
   return implementation == 4 ? launch_convrot4096<false>(p, stream) : launch_convrot4096<true>(p, stream);

@@ -54,8 +54,8 @@ int linear(const void *x, const void *w, const void *bias, void *o, uint32_t dt,
 // x is not 16-byte aligned or DIFB200_EXACT_NORM=0 asks for the parallel sums.
 bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats,
                           cudaStream_t s, int *rc);
-// The same statistics for a consumer that always reads them (16-byte aligned rows, cols a multiple of
-// 8): in the sequential order, or as parallel sums when DIFB200_EXACT_NORM=0 asks for them.
+// The same statistics for a consumer that always reads them: in the sequential order, or as parallel sums when
+// DIFB200_EXACT_NORM=0 asks for them. Refuses x that is not 16-byte aligned and cols that 8 does not divide.
 int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats, cudaStream_t s);
 
 // bf16 fast paths (glue_fast.cu). Each returns false when dtype, widths or alignment are not

@@ -583,6 +583,9 @@ bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps
 }
 
 int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats, cudaStream_t s) {
+  *stats = nullptr;
+  if (!aligned16(x) || cols == 0 || cols % 8 != 0 || cols > 0xffffff00ull) // both kernels read 16 bytes at a time
+    return fail(kUnsupported, "row statistics: rows must start on 16 bytes");
   int rc = 0;
   if (row_stats_sequential(x, rows, cols, eps, layer, stats, s, &rc))
     return rc;
