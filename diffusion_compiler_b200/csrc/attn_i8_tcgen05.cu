@@ -576,7 +576,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         l = ml.y;
       }
       const float m_both = fmaxf(m_prev, m_fixed);
-      fixed_max = __all_sync(0xffffffffu, m_both <= 60.0f);
+      // (a bound far above what the carried state holds would push that state towards underflow)
+      fixed_max = __all_sync(0xffffffffu, m_both <= 60.0f && (m_prev == -INFINITY || m_both - m_prev <= 60.0f));
       m_run = fixed_max ? m_both : m_prev;
       if (p.carry_in) {
         const float factor = (fixed_max && m_prev != -INFINITY) ? ex2(m_prev - m_run) : (fixed_max ? 0.0f : 1.0f);
@@ -715,6 +716,21 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::tc_fence_before();
       ptx::mbar_arrive(p_full + 16 * t + 8 * h);
     }
+    // A row that other keys still join, in this cluster or in a later launch, is handed on as what its own keys
+    // gave: no valid key counts as no maximum at all, and an m fixed at a bound far above the scores (l small)
+    // comes down by the power of two that brings l to [1/2, 1). So every joined l is at least 1/2, and what a factor
+    // flushes (2^-127 and less) is too small to reach the sum.
+    float m_out = m_run, up = 1.0f;
+    if (SPLIT || p.carry_out) {
+      if (l == 0.0f) {
+        m_out = -INFINITY;
+      } else if (l < 0.5f) {
+        const int e = (int)(__float_as_uint(l) >> 23) - 126;
+        m_out = m_run + (float)e;
+        up = __uint_as_float((uint32_t)(127 - e) << 23);
+        l *= up;
+      }
+    }
     if (SPLIT) {
       // The CTAs of the cluster hold the unnormalised outputs of the same queries over parts of the keys. Every m
       // is an integer, so all move to the largest one by exact powers of two. Unit u = (query tile, 32 columns) is
@@ -732,7 +748,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::tc_fence_after();
       const uint32_t row = t * 128u + row_in_tile;
       for (uint32_t r = 0; r < split; ++r) // (m, l) of every CTA and row, where Q was
-        ptx::st_cluster_v2(ptx::mapa(q_addr + (rank * 256u + row) * 8u, r), __float_as_uint(m_run), __float_as_uint(l));
+        ptx::st_cluster_v2(ptx::mapa(q_addr + (rank * 256u + row) * 8u, r), __float_as_uint(m_out), __float_as_uint(l));
       __syncwarp();
       ptx::cluster_sync();
       const float2 *mls = reinterpret_cast<const float2 *>(base_ptr + (q_addr - base)) + row;
@@ -741,7 +757,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         m_all = fmaxf(m_all, mls[r * 256u].x);
       for (uint32_t r = 0; r < split; ++r)
         l_all += mls[r * 256u].x == -INFINITY ? 0.0f : mls[r * 256u].y * ex2(mls[r * 256u].x - m_all);
-      const float factor = m_run == -INFINITY ? 0.0f : ex2(m_run - m_all);
+      const float factor = m_out == -INFINITY ? 0.0f : ex2(m_run - m_all);
       auto scaled = [&](uint32_t c, uint32_t(&o)[32]) {
         ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
         ptx::tmem_ld_wait();
@@ -805,7 +821,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         ptx::tc_fence_after();
         if (p.carry_out) {
           if (row_ok)
-            p.ml_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = make_float2(m_run, l);
+            p.ml_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = make_float2(m_out, l);
           float4 *carry = reinterpret_cast<float4 *>(p.o_state + (((uint64_t)batch * p.Sq + qrow) * p.H + head) * kTile);
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
@@ -815,8 +831,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (row_ok) {
 #pragma unroll
               for (int v = 0; v < 8; ++v)
-                carry[8 * c + v] = make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]),
-                                               __uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3]));
+                carry[8 * c + v] = make_float4(__uint_as_float(o[4 * v]) * up, __uint_as_float(o[4 * v + 1]) * up,
+                                               __uint_as_float(o[4 * v + 2]) * up, __uint_as_float(o[4 * v + 3]) * up);
             }
           }
         } else {

@@ -236,3 +236,48 @@ def test_attention_split_over_keys_matches_the_plain_launch(ops, B, Sq, Sk, H, K
     if masked:  # nothing valid anywhere: zeros
         none = ops.attention_int8(*args, torch.zeros_like(tv))
         assert torch.count_nonzero(none.float()) == 0
+
+
+@pytest.mark.parametrize("case", ["share_masked", "bounds_apart", "bounds_apart_reversed"])
+def test_attention_joins_key_ranges_whose_scores_are_far_below_their_maxima(ops, case):
+    """Keys against their queries: every score is -50 or less in units of log2. In `share_masked` the first half of
+    the keys is masked and the others score about -130, so a range without a valid key must not set a maximum.
+    In the other two one key of one half scores -59 (a bound that the fixed maximum takes as +60) and all keys of the
+    other half -69 (running maximum), which together outweigh it. The split, the plain and the chunked launches in
+    both orders against the oracle, at the bar of the path (rel-L2 2e-3)."""
+    import torch
+    B, Sq, Sk, H, KV = 1, 130, 4096, 6, 2  # 6 items of 32 tiles: eight CTAs each
+    rng = np.random.default_rng(11)
+    half = Sk // 2
+    q8 = np.full((B, Sq, H, 128), 100, np.int8) + rng.integers(-1, 2, (B, Sq, H, 128), dtype=np.int8)
+    k8 = np.full((B, Sk, KV, 128), -100, np.int8)
+    valid = np.ones((B, Sk), np.uint8)
+    score = np.full((B, Sk, KV), -69.0)
+    if case == "share_masked":
+        k8 += rng.integers(-3, 4, k8.shape, dtype=np.int8)
+        valid[:, :half] = 0
+        score[:] = -130.0
+    else:
+        near = slice(0, half) if case == "bounds_apart" else slice(half, Sk)
+        valid[:, near] = 0
+        valid[:, near.start + 300] = 1
+        score[:, near] = -59.0
+    qs = np.full((B, Sq, H), 0.03, np.float32)
+    unit = 128 * 100 * 100 * 0.03 / np.sqrt(128.0) * np.log2(np.e)  # what a key scale of 1 scores
+    ks = (-score / unit).astype(np.float32)
+    v = bf16_normal(rng, (B, Sk, KV, 128))
+    want = ob.bf16_to_f32(ob.orc().attention_int8_rows(q8, qs.reshape(-1), k8, ks.reshape(-1), v, valid))
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    args = (t(q8), t(qs.reshape(-1)), t(k8), t(ks.reshape(-1)), to_torch_bf16(v))
+    tiles = Sk // 128
+    low, high = (0, tiles // 2), (tiles // 2, tiles // 2)
+    got = {"split": ops.attention_int8(*args, t(valid)),
+           "plain": ops.attention_int8_chunked(*args, [[(0, tiles)]], t(valid)),
+           "low first": ops.attention_int8_chunked(*args, [[low], [high]], t(valid)),
+           "high first": ops.attention_int8_chunked(*args, [[high], [low]], t(valid)),
+           "single tiles": ops.attention_int8_chunked(*args, [[(i, 1)] for i in range(tiles)], t(valid))}
+    torch.cuda.synchronize()
+    ops.poll_status()
+    for name, out in got.items():
+        r = rel_l2(ob.bf16_to_f32(from_torch_bf16(out)), want)
+        assert r <= 2e-3, (name, r)
