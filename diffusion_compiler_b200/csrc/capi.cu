@@ -63,7 +63,20 @@ int attention_bf16_via_int8(const void *q, const void *k, const void *v, const u
   if (!scratch || scratch_bytes < attention_scratch_bytes(B, S, H, KV))
     return fail(kInvalidArgument, "Attention(INT8): scratch buffer too small");
   const AttentionScratch l = attention_scratch_layout(scratch, B, S, H, KV);
-  const AttentionSource source{q, k};
+  AttentionSource source{q, k};
+  // The attention's own launch reads its bf16 operands 16 bytes at a time; one that starts elsewhere goes through
+  // the general quantiser first (the same codes).
+  const uint64_t width[1] = {128};
+  if (q && (reinterpret_cast<uintptr_t>(q) & 15)) {
+    source.q = nullptr;
+    if (int rc = quantize_int8_rows(&q, width, 1, B * S * H, 1, 1.0f, nullptr, l.q8, l.qs, nullptr, nullptr, stream))
+      return rc;
+  }
+  if (k && (reinterpret_cast<uintptr_t>(k) & 15)) {
+    source.k = nullptr;
+    if (int rc = quantize_int8_rows(&k, width, 1, B * S * KV, 1, 1.0f, nullptr, l.k8, l.ks, nullptr, nullptr, stream))
+      return rc;
+  }
   return attention_int8(l.q8, l.qs, l.k8, l.ks, v, key_valid, B, S, S, H, KV, D, scale, l.rest,
                         attention_int8_scratch_bytes(B, S, KV), out_bf16, stream, nullptr, &source);
 }

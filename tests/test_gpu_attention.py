@@ -281,3 +281,20 @@ def test_attention_joins_key_ranges_whose_scores_are_far_below_their_maxima(ops,
     for name, out in got.items():
         r = rel_l2(ob.bf16_to_f32(from_torch_bf16(out)), want)
         assert r <= 2e-3, (name, r)
+
+
+@pytest.mark.parametrize("moved", ["q", "k", "both"])
+def test_attention_takes_operands_that_start_on_two_bytes(ops, moved):
+    """Contiguous bf16 q or k at an odd element offset goes through the general quantiser: the same bits."""
+    import torch
+    B, S, H, KV = 1, 300, 4, 2
+    q, k, v = (to_torch_bf16(a) for a in _qkv(np.random.default_rng(8), B, S, H, KV))
+    want = ops.attention(q, k, v)
+
+    def shifted(a):
+        return torch.empty(a.numel() + 1, dtype=a.dtype, device="cuda")[1:].view(a.shape).copy_(a)
+
+    got = ops.attention(shifted(q) if moved != "k" else q, shifted(k) if moved != "q" else k, v)
+    torch.cuda.synchronize()
+    ops.poll_status()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
