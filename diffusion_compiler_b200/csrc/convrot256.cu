@@ -258,7 +258,9 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             // tools/difflux2sample.cpp:3005-3014; the sign flip commutes with the division).
             // One Markstein step from the approximate reciprocal: the quotient of two 8-bit
             // significands is never within 2^-33 of a rounding boundary of fp32, far outside the
-            // 2^-44 error of fma(r, y, q).
+            // 2^-44 error of fma(r, y, q). Where w or the quotient is not finite the step gives NaN and the product,
+            // which then is the quotient, stands. Subnormal quotients may be off by 2^-149: the row scale
+            // is at least 1e-30.
             const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
             const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + c);
             const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z,
@@ -274,7 +276,10 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
                 asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(e0));
                 asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(e1));
                 const uint64_t y2 = pack2(y0, y1), q2 = mul2(P[i], y2);
-                P[i] = fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2);
+                float q0, q1, x0, x1;
+                unpack2(q2, q0, q1);
+                unpack2(fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2), x0, x1);
+                P[i] = pack2(x0 == x0 ? x0 : q0, x1 == x1 ? x1 : q1);
               } else {
                 float w0, w1;
                 unpack2(P[i], w0, w1);

@@ -86,3 +86,22 @@ def test_norm_prologue_equals_the_two_ops(rows, K, impl):
     want = ops.quantize_int8_rows([normed], impl)
     got = ops.layer_norm_modulate_quant(x, w, b, s, h, 1e-6, impl)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("impl,mse", [(2, True), (2, False), (3, True), (5, False), (6, True)])
+def test_equalised_packing_of_weights_that_are_not_finite(impl, mse):
+    """Division by an equalisation entry keeps infinities and NaNs: a vector of ones (or of twos with doubled weights)
+    gives the bits of packing without one, scale of the row included."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(impl)
+    w = to_torch_bf16(bf16_normal(rng, (8, 2816), 0.02))
+    w[1, 5], w[2, 300], w[2, 2700], w[3, 7], w[4] = float("inf"), float("-inf"), float("inf"), float("nan"), 0.0
+    w[5, 9] = 3.0e38 / 2  # finite, and its double too
+    want = ops.quantize_weight_rows(w, impl, mse_scale=mse)
+    assert not torch.isfinite(want[1][1]) and torch.isfinite(want[1][5])
+    for by in (1.0, 2.0):
+        vector = torch.full((2816,), by, dtype=torch.bfloat16, device="cuda")
+        got = ops.quantize_weight_rows(w * by, impl, mse_scale=mse, input_scale=vector)
+        assert torch.equal(got[0], want[0]), by
+        assert torch.equal(got[1].view(torch.int32), want[1].view(torch.int32)), by
