@@ -104,12 +104,18 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   // Weight packing: may the fast quotient be used for every entry of this thread's columns?
   bool equalise_fast = true;
   if (EXTRA == kPack && p.equalise) {
-#pragma unroll 1
-    for (int q = 0; q < 32 * NIT; ++q) {
-      const uint32_t c = col0 + (uint32_t)(q >> 5) * 1024u + (uint32_t)((q >> 4) & 1) * 256u + (q & 15);
+#pragma unroll
+    for (int q = 0; q < 2 * NIT; ++q) {
+      const uint32_t c = col0 + (uint32_t)(q >> 1) * 1024u + (uint32_t)(q & 1) * 256u;
       if (c < columns) {
-        const float e = fabsf(bf16_bits_to_f32(__ldg(p.equalise + c)));
-        equalise_fast = equalise_fast && e > 1.0e-9f && e < 1.0e9f;
+        const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + c);
+        const uint4 e0 = __ldg(ep), e1 = __ldg(ep + 1);
+        const uint32_t w[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float lo = fabsf(__uint_as_float(w[i] << 16)), hi = fabsf(__uint_as_float(w[i] & 0xffff0000u));
+          equalise_fast = equalise_fast && lo > 1.0e-9f && lo < 1.0e9f && hi > 1.0e-9f && hi < 1.0e9f;
+        }
       }
     }
   }
@@ -563,12 +569,26 @@ int launch_single(const QuantParams &p, cudaStream_t stream) {
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, RESIDUAL ? 3 : 4>(p, stream);
 }
 
+// Packing without the scale search: the division by the equalisation vector wants warps, not registers or blocks
+// per warp (three blocks with 168 registers -> this: 12288 x 3072 77 -> 57 us, 8192 x 8192 138 -> 95 us,
+// 3333 x 10240 86 -> 57 us; fp32 12288 x 3072 72 -> 59 us).
+template <bool SIGNED, bool F32>
+int launch_equalised(const QuantParams &p, cudaStream_t stream) {
+  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+  if (blocks > 12u)
+    return launch_single<SIGNED, F32, false, kPack>(p, stream);
+  return blocks <= 8u ? launch_form<SIGNED, F32, false, kPack, 1, false, 256, 3>(p, stream)
+                      : launch_form<SIGNED, F32, false, kPack, 1, false, 384, 2>(p, stream);
+}
+
 template <bool SIGNED>
 int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
   const bool pack = p.mse || p.equalise, norm = p.norm_scale != nullptr;
   if ((pack || norm) && p.rcodes)
     return fail(kUnsupported, "QuantizeInt8Rows: weight packing (MSE scale, input equalisation) exists for "
                               "the 256-wide variants without residual outputs");
+  if (pack && !p.mse)
+    return f32 ? launch_equalised<SIGNED, true>(p, stream) : launch_equalised<SIGNED, false>(p, stream);
   if (f32) {
     if (pack)
       return launch_single<SIGNED, true, false, kPack>(p, stream);
@@ -585,14 +605,13 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
   // occupancy: worth it from three rounds of the machine (9216 x 3072 30.2 -> 28.8 us; below, the last round is
   // mostly empty: 3333 x 3072 signed 18.9 us with three, under 14.9 with one). Rows of up to 8 blocks that three
   // do not divide keep one (8192 columns: 34.3 us against 41.5 us for 4159 rows, the last warp would idle on
-  // a third of its slots). Packing without the scale search follows the same line (3072 x 3072 27.4 -> 22.0 us);
-  // the search is arithmetic that the form for few rows need not hide.
+  // a third of its slots). The scale search of packing is arithmetic that the form for few rows need not hide.
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
   const bool few = p.rows * blocks <= (uint64_t)sm_count() * 24u;
   const uint64_t round = (uint64_t)sm_count() * 16u * 3u; // blocks that run at once with three per warp
   const bool three = (blocks % 3u == 0 || blocks > 8u) && p.rows * blocks >= 3u * round;
   if (pack)
-    return few || blocks == 1u || (!p.mse && p.rows * blocks < 3u * round) ? launch_single<SIGNED, false, false, kPack>(p, stream)
+    return few || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
                                : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
   return three ? launch_form<SIGNED, false, false, kPlain, 3, true, 256, 2>(p, stream)
                : launch_single<SIGNED, false, false, kPlain>(p, stream);
