@@ -130,14 +130,33 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       c -= p.width[i++];
     return reinterpret_cast<const uint4 *>(p.part[i] + row * p.width[i] + c);
   };
+  // With one block per warp the runs of a thread are in the same place of every row: looked up once. (Not where
+  // registers are short: the fp32 form with 64 of them spills, 9216 x 15360 147 -> 156 us.)
+  constexpr bool kPlaced = NIT == 1 && EXTRA == kPlain && !RESIDUAL && !(F32 && !SIGNED && MAXT * MINB > 768);
+  const uint16_t *src_a = p.part[0] + col0, *src_b = src_a + 256;
+  uint32_t pitch_a = columns, pitch_b = columns;
+  if (kPlaced && p.part_count > 1) {
+    auto place = [&](uint32_t c, const uint16_t *&src, uint32_t &pitch) {
+      uint32_t i = 0;
+      while (c >= p.width[i])
+        c -= p.width[i++];
+      src = p.part[i] + c;
+      pitch = p.width[i];
+    };
+    if (col0 < columns)
+      place(col0, src_a, pitch_a);
+    if (col0 + 256u < columns)
+      place(col0 + 256u, src_b, pitch_b);
+  }
   auto fetch = [&](uint64_t row, int it, uint4 (&v)[4]) {
     v[0] = v[1] = v[2] = v[3] = make_uint4(0, 0, 0, 0);
     const uint32_t c = col0 + 1024u * it;
     if (row < p.rows) {
       if (c < columns)
-        load_run(run_of(row, c), p.wide != 0, v[0], v[1]);
+        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_a + row * pitch_a) : run_of(row, c), p.wide != 0, v[0], v[1]);
       if (c + 256u < columns)
-        load_run(run_of(row, c + 256u), p.wide != 0, v[2], v[3]);
+        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_b + row * pitch_b) : run_of(row, c + 256u), p.wide != 0, v[2],
+                 v[3]);
     }
   };
   auto row_barrier = [&]() { // the warps of one row only; rows in flight do not wait for each other
@@ -549,29 +568,43 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   return launched(cudaGetLastError(), "convrot256_kernel launch");
 }
 
-// One block of 1024 columns per warp: the fp32 and residual forms, narrow rows, and calls of few rows.
+// One block of 1024 columns per warp: the fp32, residual and norm forms, packing, and calls of few rows.
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
 int launch_single(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
-  // A row is a CTA of 9 to 16 warps: two of them per SM, or its barriers leave the SM idle (128 registers and one
-  // CTA: 3333 x 12288 fp32 60 us, two CTAs 47 us; 3333 x 15360 73 us and 58 us).
+  // Plain rows of more than 8 blocks are a CTA each, and several CTAs per SM hide one another's barriers: three of 9 or
+  // 10 warps, two of 11 or more (64 registers; 11 and 12 warps leave 80). 3333 rows, two CTAs with a prefetch ->
+  // this: 10240 columns 39.2 -> 35.6 us, fp32 41.9 -> 39.2; 12288 columns 43.8 -> 42.4 us, fp32 47.4 -> 45.3.
   if (blocks > 8u) {
     if constexpr (EXTRA == kPlain && !RESIDUAL)
-      return blocks <= 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 384, 2>(p, stream)
-                           : launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 512, 2>(p, stream);
+      return blocks == 11u || blocks == 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 384, 2>(p, stream)
+                                            : launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 512, 2>(p, stream);
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
   }
-  if constexpr (EXTRA == kNorm)
+  if constexpr (EXTRA == kNorm) {
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream); // 24 warps, three tensors in flight
-  else if constexpr (EXTRA != kPlain || (RESIDUAL && !F32))
+  } else if constexpr (EXTRA != kPlain || (RESIDUAL && !F32)) {
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
-  else // 64 registers and 32 warps per SM hide the load latency without a prefetch
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, RESIDUAL ? 3 : 4>(p, stream);
+  } else if constexpr (RESIDUAL) {
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
+  } else {
+    // 64 registers and 32 warps per SM hide the load latency without a prefetch. Sign masks and the fp32 division on
+    // short rows want 80 registers and 24 warps (16384 x 3072: fp32 53.0 -> 51.6 us, both 55.6 -> 53.7 us; 4000 x 1024
+    // signed 9.8 -> 8.6 us; but 9216 x 8192 fp32 72.8 -> 77.2 us), and signed rows that are all resident at once the
+    // shortest path (700 x 3072 7.5 -> 6.4 us, 77 x 8192 fp32 6.4 -> 5.4 us).
+    if constexpr (SIGNED)
+      if (p.rows * blocks <= (uint64_t)sm_count() * 16u)
+        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
+    if constexpr (SIGNED || F32)
+      if (blocks <= 3u)
+        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 4>(p, stream);
+  }
 }
 
 // Packing without the scale search: the division by the equalisation vector wants warps, not registers or blocks
-// per warp (three blocks with 168 registers -> this: 12288 x 3072 77 -> 57 us, 8192 x 8192 138 -> 95 us,
-// 3333 x 10240 86 -> 57 us; fp32 12288 x 3072 72 -> 59 us).
+// per warp (three blocks with 168 registers -> this: 9216 x 3072 59.7 -> 41.2 us, 3072 x 8192 57.9 -> 37.1 us,
+// 3333 x 10240 83.8 -> 53.5 us).
 template <bool SIGNED, bool F32>
 int launch_equalised(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
@@ -601,18 +634,21 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     return launch_single<SIGNED, false, true, kPlain>(p, stream);
   if (norm)
     return launch_single<SIGNED, false, false, kNorm>(p, stream);
-  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, at half the
-  // occupancy: worth it from three rounds of the machine (9216 x 3072 30.2 -> 28.8 us; below, the last round is
-  // mostly empty: 3333 x 3072 signed 18.9 us with three, under 14.9 with one). Rows of up to 8 blocks that three
-  // do not divide keep one (8192 columns: 34.3 us against 41.5 us for 4159 rows, the last warp would idle on
-  // a third of its slots). The scale search of packing is arithmetic that the form for few rows need not hide.
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
-  const bool few = p.rows * blocks <= (uint64_t)sm_count() * 24u;
-  const uint64_t round = (uint64_t)sm_count() * 16u * 3u; // blocks that run at once with three per warp
-  const bool three = (blocks % 3u == 0 || blocks > 8u) && p.rows * blocks >= 3u * round;
-  if (pack)
-    return few || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
-                               : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
+  const uint64_t all = p.rows * blocks, sms = (uint64_t)sm_count();
+  if (pack) // the scale search is arithmetic that the form for few rows need not hide
+    return all <= sms * 24u || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
+                                            : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
+  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, at half the
+  // occupancy, and the last round of the machine is mostly empty. Rows of up to 8 blocks that three divide: from
+  // three rounds (9216 x 3072 30.2 -> 28.8 us; below, 3333 x 3072 signed takes 18.9 us with three, under 14.9 with
+  // one). Others of up to 8 keep one (4159 x 8192: 34.3 us against 41.5 us, the last warp would idle on a third of its
+  // slots). Wider rows have one CTA per row with one block, the better form for longer. One against three, 12288
+  // columns: 3333 rows 42.4 / 43.3 us, 4159 rows 52.8 / 50.6, 6000 rows 71.6 / 69.4; 15360 columns: 3333 rows
+  // 53.5 / 51.6. Signed: 12288 columns 3333 rows 45.3 / 47.5, 6000 rows 75.2 / 75.2, 16384 rows 191.8 / 188.0;
+  // 15360 columns 9216 rows 138.5 / 142.3.
+  const uint64_t rounds = all / (sms * 16u * 3u); // of the blocks that run at once with three per warp
+  const bool three = blocks <= 8u ? blocks % 3u == 0 && rounds >= 3u : SIGNED ? blocks <= 12u && rounds >= 10u : rounds >= 5u;
   return three ? launch_form<SIGNED, false, false, kPlain, 3, true, 256, 2>(p, stream)
                : launch_single<SIGNED, false, false, kPlain>(p, stream);
 }

@@ -105,3 +105,37 @@ def test_equalised_packing_of_weights_that_are_not_finite(impl, mse):
         got = ops.quantize_weight_rows(w * by, impl, mse_scale=mse, input_scale=vector)
         assert torch.equal(got[0], want[0]), by
         assert torch.equal(got[1].view(torch.int32), want[1].view(torch.int32)), by
+
+
+@pytest.mark.parametrize("impl,rows,widths", [
+    (3, 50, [1040, 2032]),    # inputs that meet between the two runs of a thread; all rows resident
+    (6, 900, [1040, 2032]),   # the same, more rows than are resident
+    (3, 2500, [1024]),        # one block per row, signed
+    (5, 60, [2048, 7168]),    # nine blocks, fp32: three CTAs per SM
+    (2, 70, [10240]),         # ten blocks
+    (5, 40, [16, 11248]),     # eleven blocks, a first input of one run
+    (6, 300, [5008, 10352]),  # fifteen blocks, signed fp32
+    (3, 480, [15360]),        # fifteen blocks, signed
+    (3, 40, [256, 528, 752]),  # three inputs
+])
+def test_one_block_forms_bit_exact(impl, rows, widths):
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(rows + sum(widths))
+    x = activations(rng, rows, sum(widths))
+    cuts = np.cumsum([0] + widths)
+    parts = [np.ascontiguousarray(x[:, cuts[i]:cuts[i + 1]]) for i in range(len(widths))]
+    tensors = [to_torch_bf16(p) for p in parts]
+    want = ob.orc().quantize_int8_rows(parts, impl, 1.0, False)
+    got = ops.quantize_int8_rows(tensors, impl)
+    assert _bits_equal(want[0], got[0]) and _bits_equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("N,K,impl", [(77, 3072, 3), (30, 8192, 5), (25, 9216, 2), (12, 11264, 6), (9, 15360, 3)])
+def test_equalised_packing_without_search_bit_exact(N, K, impl):
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(N + K)
+    w = bf16_normal(rng, (N, K), 0.02)
+    eq = ob.orc().weight_equalization(w)
+    want_codes, want_scales = ob.orc().quantize_weight_rows(w, impl, mse=False, equalise=eq)
+    codes, scales = ops.quantize_weight_rows(to_torch_bf16(w), impl, input_scale=to_torch_bf16(eq))
+    assert _bits_equal(want_scales, scales) and _bits_equal(want_codes, codes)
