@@ -547,7 +547,7 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   const uint32_t groups = p.columns >> 8;
   const int warps_per_row = (int)((groups + 4u * NIT - 1u) / (4u * NIT));
   if (warps_per_row > MAXT / 32)
-    return fail(kUnsupported, "QuantizeInt8Rows: ConvRot width above 16384 is not supported");
+    return fail(kInternalError, "QuantizeInt8Rows: row too wide for this form");
   constexpr int kWarps = MAXT / 32 < 8 ? MAXT / 32 : 8;
   int rows_per_cta = kWarps / warps_per_row;
   rows_per_cta = rows_per_cta < 1 ? 1 : rows_per_cta;
@@ -655,6 +655,7 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
 
 } // namespace
 
+// Rows of at most 16384 columns.
 int launch_convrot256(const QuantParams &p, int implementation, cudaStream_t stream) {
   const bool is_signed = implementation == 3 || implementation == 6, f32 = implementation >= 5;
   return is_signed ? launch_variant<true>(p, f32, stream) : launch_variant<false>(p, f32, stream);

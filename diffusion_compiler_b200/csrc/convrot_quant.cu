@@ -243,8 +243,6 @@ int launch_convrot4096(const QuantParams &p, cudaStream_t stream) {
     return fail(kUnsupported, "QuantizeInt8Rows: weight packing (MSE scale, input equalisation) exists for "
                               "the 256-wide variants without residual outputs");
   const int warps = (int)(p.columns >> 10), threads = 32 * warps;
-  if (warps > 16)
-    return fail(kUnsupported, "QuantizeInt8Rows: ConvRot width above 16384 is not supported");
   const size_t smem = (size_t)warps * (kWarpBytes + 16 + 32 * 64) + 64;
   auto kernel = threads <= 256   ? (p.rcodes ? convrot4096_kernel<F32, true, 256> : convrot4096_kernel<F32, false, 256>)
                 : threads <= 384 ? (p.rcodes ? convrot4096_kernel<F32, true, 384> : convrot4096_kernel<F32, false, 384>)
@@ -439,6 +437,8 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
   const bool h4096 = implementation == 4 || implementation == 7;
   if (columns % (h4096 ? 4096u : 256u) != 0)
     return fail(kInvalidArgument, "QuantizeInt8Rows: width is not a multiple of the rotation group");
+  if (columns > 16384) // 16 warps of 1024 columns: one limit for every form, whatever the number of rows
+    return fail(kUnsupported, "QuantizeInt8Rows: ConvRot width above 16384 is not supported");
   if (!aligned16 || (reinterpret_cast<uintptr_t>(codes) & 15) != 0 ||
       (rcodes && (reinterpret_cast<uintptr_t>(rcodes) & 15) != 0))
     return fail(kUnsupported,

@@ -34,3 +34,20 @@ def test_norm_prologue_refuses_an_unaligned_input(lib, layer, offset):
         call = lambda: lib.difb200_rms_norm_modulate_quant(x, w, s, h, 64, 3072, 1e-5, 2, 1.0, codes, scales,  # noqa: E731
                                                            None)
     _refused(lib, call, "16-byte aligned")
+
+
+@pytest.mark.parametrize("rows", [3, 1000000])
+@pytest.mark.parametrize("columns,impl", [(16640, 2), (24576, 3), (18432, 5), (20480, 4)])
+def test_convrot_width_limit_does_not_depend_on_the_rows(lib, rows, columns, impl):
+    """Rows of more than 16384 columns are refused whatever their number: plain, residual and packing forms."""
+    at = lambda k: C.c_void_p(0x700000000000 + 0x10000000000 * k)  # noqa: E731
+    parts, widths = (C.c_void_p * 1)(at(1).value), (C.c_uint64 * 1)(columns)
+    for residual in (False, True):
+        _refused(lib, lambda: lib.difb200_quantize_int8_rows(parts, widths, 1, rows, impl, 1.0, None, at(2), at(3),
+                                                             at(4) if residual else None, at(5) if residual else None,
+                                                             None), "16384")
+    if impl != 4:
+        _refused(lib, lambda: lib.difb200_quantize_weight_rows(at(1), None, rows, columns, impl, 1, at(2), at(3), None),
+                 "16384")
+        _refused(lib, lambda: lib.difb200_rms_norm_modulate_quant(at(1), at(2), at(3), at(4), rows, columns, 1e-5, impl,
+                                                                  1.0, at(5), at(6), None), "16384")
