@@ -248,6 +248,12 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
 #pragma unroll
           for (int e = 0; e < 16; ++e)
             P[e] = round_bf16_2(P[e]);
+          if ((columns & 1023u) != 0) { // groups that do not exist hold -mean / deviation: not for the row's maximum
+            const uint64_t keep = (act_a ? 0xffffffffull : 0ull) | (act_b ? 0xffffffff00000000ull : 0ull);
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              P[e] &= keep;
+          }
           if (SIGNED) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {

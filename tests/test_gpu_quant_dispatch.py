@@ -139,3 +139,26 @@ def test_equalised_packing_without_search_bit_exact(N, K, impl):
     want_codes, want_scales = ob.orc().quantize_weight_rows(w, impl, mse=False, equalise=eq)
     codes, scales = ops.quantize_weight_rows(to_torch_bf16(w), impl, input_scale=to_torch_bf16(eq))
     assert _bits_equal(want_scales, scales) and _bits_equal(want_codes, codes)
+
+
+@pytest.mark.parametrize("K", [256, 1280, 2816])
+@pytest.mark.parametrize("impl", [2, 3, 5])
+def test_layer_norm_prologue_of_rows_with_a_large_mean(K, impl):
+    """Widths that leave groups of a warp's 1024 columns without elements, and a mean far above the deviation: what
+    stands in those groups must not enter the row's maximum. Equal to the two separate ops, bit for bit."""
+    import ctypes as C
+
+    import torch
+    from diffusion_compiler_b200 import _lib, ops
+    rng = np.random.default_rng(K + impl)
+    t = lambda *shape, std=1.0: to_torch_bf16(bf16_normal(rng, shape, std))  # noqa: E731
+    rows = 40
+    x, w, b, s, h = t(rows, K) + 8.0, t(K, std=0.1), t(K, std=0.01), t(rows, K, std=0.1), t(rows, K, std=0.01)
+    p = lambda v: C.c_void_p(v.data_ptr())  # noqa: E731
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    normed = torch.empty_like(x)
+    _lib.check(_lib.lib().difb200_layer_norm_modulate(p(x), p(w), p(b), p(s), p(h), p(normed), 2, rows, K, rows, 1e-6,
+                                                      stream))
+    want = ops.quantize_int8_rows([normed], impl)
+    got = ops.layer_norm_modulate_quant(x, w, b, s, h, 1e-6, impl)
+    assert torch.equal(want[1], got[1]) and torch.equal(want[0], got[0])
