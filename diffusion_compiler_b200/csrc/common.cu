@@ -128,25 +128,38 @@ int sm_count() {
   return count;
 }
 
-void *device_scratch(size_t bytes) {
-  static std::unordered_map<int, std::pair<void *, size_t>> areas;
+int StreamScratch::allocate(size_t bytes, const char *what) {
+  static std::unordered_map<int, cudaMemPool_t> pools;
   int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess)
-    return nullptr;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  auto &area = areas[device];
-  if (area.second >= bytes && area.first)
-    return area.first;
-  if (area.first)
-    cudaFree(area.first); // waits for everything that may still read the old area
-  area = {nullptr, 0};
-  const size_t rounded = (bytes + (1u << 20) - 1) & ~(size_t)((1u << 20) - 1);
-  if (cudaMalloc(&area.first, rounded) != cudaSuccess) {
-    area.first = nullptr;
-    return nullptr;
+  if (int rc = check_cuda(cudaGetDevice(&device), what))
+    return rc;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    const auto it = pools.find(device);
+    if (it != pools.end()) {
+      pool = it->second;
+    } else {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      if (int rc = check_cuda(cudaMemPoolCreate(&pool, &props), what))
+        return rc;
+      unsigned long long kept = 4ull << 20; // the statistics of half a million rows
+      if (int rc = check_cuda(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept), what)) {
+        cudaMemPoolDestroy(pool);
+        return rc;
+      }
+      pools[device] = pool;
+    }
   }
-  area.second = rounded;
-  return area.first;
+  return check_cuda(cudaMallocFromPoolAsync(&data_, bytes, pool, stream_), what);
+}
+
+StreamScratch::~StreamScratch() {
+  if (data_)
+    cudaFreeAsync(data_, stream_);
 }
 
 DeviceStatus *device_status_words() {

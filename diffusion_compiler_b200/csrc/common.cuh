@@ -55,9 +55,23 @@ void set_wait_limit_ns(unsigned long long ns); // 0 restores the default
 // k-block. take_...() returns that k-block (0xffffffff = none) and disarms.
 void withhold_next_gemm_load(uint32_t k_block);
 uint32_t take_withheld_gemm_load();
-// Per-device scratch that only grows (reallocated, which synchronises the device, when a call
-// needs more than any call before it): small work areas whose size follows the row count.
-void *device_scratch(size_t bytes);
+// Device memory for one call: allocated and freed in the order of the call's stream, so that neither
+// another stream nor another thread can hold the same bytes meanwhile (also under stream capture, where the two become
+// nodes of the graph). It comes from a pool of this library that keeps at most 4 MB per device across
+// synchronisations. The consumer is launched on the same stream before the object goes.
+class StreamScratch {
+public:
+  explicit StreamScratch(cudaStream_t stream) : stream_(stream) {}
+  ~StreamScratch();
+  StreamScratch(const StreamScratch &) = delete;
+  StreamScratch &operator=(const StreamScratch &) = delete;
+  int allocate(size_t bytes, const char *what); // once per object
+  void *get() const { return data_; }
+
+private:
+  cudaStream_t stream_;
+  void *data_ = nullptr;
+};
 DeviceStatus *device_status_words();      // per-device, allocated once
 int poll_device_status(const char *what); // copies back, clears, maps to kExecutionError
 

@@ -55,6 +55,7 @@ __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, 
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
 convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_per_cta) {
+  static_assert(EXTRA != kNorm || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -176,7 +177,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     float m = 0.0f;
     float mean = 0.0f, inv = 0.0f;
     if (EXTRA == kNorm) {
-      const float2 st = __ldg(p.norm_stats + row);
+      // stands where this row's codes go: written behind the barrier of the row maximum, when all its warps have read it
+      const float2 st = glue::row_stat(p.norm_stats, row);
       mean = st.x;
       inv = st.y;
     }

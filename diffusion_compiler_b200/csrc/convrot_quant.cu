@@ -444,9 +444,14 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
     return fail(kUnsupported,
                 "QuantizeInt8Rows: ConvRot path needs 16-byte aligned pointers and part widths "
                 "that are multiples of 16");
-  if (norm) // the row statistic, by its own kernel in front: only now that nothing above refuses the call
-    if (int rc = glue::row_stats(parts[0], rows, columns, norm->epsilon, norm->bias != nullptr, &p.norm_stats, stream))
+  StreamScratch scratch(stream);
+  if (norm) { // the row statistic, by its own kernel in front: only now that nothing above refuses the call
+    const uint64_t vector = columns * 2, mods = (rows + norm->rows_per_modulation - 1) / norm->rows_per_modulation * vector;
+    if (int rc = glue::row_stats(parts[0], rows, columns, norm->epsilon, norm->bias != nullptr, true, codes, columns,
+                                 {{norm->weight, vector}, {norm->bias, vector}, {norm->scale, mods}, {norm->shift, mods}},
+                                 scratch, &p.norm_stats, stream))
       return rc;
+  }
   if (!h4096)
     return launch_convrot256(p, implementation, stream);
   return implementation == 4 ? launch_convrot4096<false>(p, stream) : launch_convrot4096<true>(p, stream);

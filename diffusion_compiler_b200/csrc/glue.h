@@ -5,7 +5,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 namespace difb200 {
+
+class StreamScratch; // common.cuh
 namespace glue {
 
 int binary(const void *a, const void *b, void *o, uint32_t dt, uint64_t n, bool multiply, cudaStream_t s);
@@ -48,15 +52,33 @@ int linear(const void *x, const void *w, const void *bias, void *o, uint32_t dt,
 
 // Row statistics of a bf16 [rows, cols] tensor in the reference's own order (one sequential fp32
 // chain per row, cpu_executor.cpp:1051-1062, 1119-1129, 1250-1256), so that a normalisation built on
-// them has the reference's bits: stats[r] = (0, 1 / sqrt(sum x^2 / cols + eps)) or, with `layer`,
-// (mean, 1 / sqrt(sum (x - mean)^2 / cols + eps)). *stats points into per-device scratch that the
-// next call of this function reuses. False (nothing launched) when cols is not a multiple of 64,
-// x is not 16-byte aligned or DIFB200_EXACT_NORM=0 asks for the parallel sums.
-bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats,
-                          cudaStream_t s, int *rc);
-// The same statistics for a consumer that always reads them: in the sequential order, or as parallel sums when
-// DIFB200_EXACT_NORM=0 asks for them. Refuses x that is not 16-byte aligned and cols that 8 does not divide.
-int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats, cudaStream_t s);
+// them has the reference's bits: per row (0, 1 / sqrt(sum x^2 / cols + eps)) or, with `layer`,
+// (mean, 1 / sqrt(sum (x - mean)^2 / cols + eps)).
+// The pair of row r stands at `at` + r * pitch: in the first bytes of row r of the consumer's output, which belongs
+// to this call alone (no area shared by streams or threads, nothing to allocate) and which the consumer overwrites
+// once every thread of the row has read the pair.
+struct RowStats {
+  unsigned char *at = nullptr; // nullptr: none, the consumer computes its own
+  uint64_t pitch = 0;
+};
+struct Span {
+  const void *start;
+  uint64_t bytes;
+};
+// out / out_pitch: the consumer's output rows; `reads`: what the consumer reads beside x. Where the output shares
+// bytes with one of them (an op in place) or is not 8-byte aligned, the pairs go to `scratch` instead.
+// Without `always`, nothing happens (stats->at stays null) when cols is not a multiple of 64, x is not 16-byte
+// aligned or DIFB200_EXACT_NORM=0 asks for the parallel sums; with it the parallel sums are computed here in
+// the last case, and x that is not 16-byte aligned or cols that 8 does not divide are refused.
+int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, bool always, void *out,
+              uint64_t out_pitch, std::initializer_list<Span> reads, StreamScratch &scratch, RowStats *stats,
+              cudaStream_t s);
+#ifdef __CUDACC__
+// Read by the warp (or the CTA, with its own barrier) that owns the row, before any of it writes the row.
+__device__ __forceinline__ float2 row_stat(const RowStats &stats, uint64_t row) {
+  return *reinterpret_cast<const float2 *>(stats.at + row * stats.pitch);
+}
+#endif
 
 // bf16 fast paths (glue_fast.cu). Each returns false when dtype, widths or alignment are not
 // covered (nothing launched; the caller runs the generic kernel), else true with the launch

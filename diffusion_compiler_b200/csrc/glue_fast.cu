@@ -124,7 +124,7 @@ __device__ __forceinline__ float accumulate_word(uint32_t word, float mean, floa
 
 template <bool LAYER, int STAGES>
 __global__ void __launch_bounds__(32 * kStatWarps)
-k_row_stats_sequential(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols, float eps) {
+k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps) {
   extern __shared__ uint4 stat_smem[];
   auto tile = reinterpret_cast<uint4 (*)[STAGES][32 * kStatPitch]>(stat_smem); // [kStatWarps]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -197,13 +197,14 @@ k_row_stats_sequential(const uint4 *x, float2 *stats, uint64_t rows, uint32_t co
       pass(std::integral_constant<int, 1>{});
     }
     if (row < rows)
-      stats[row] = make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(acc, (float)cols), eps))));
+      *reinterpret_cast<float2 *>(stats.at + row * stats.pitch) =
+          make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(acc, (float)cols), eps))));
   }
 }
 
 // The statistics as parallel sums, one warp per row.
 __global__ void __launch_bounds__(256)
-k_row_stats_parallel(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols, float eps, int layer) {
+k_row_stats_parallel(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps, int layer) {
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t cols8 = cols >> 3;
@@ -230,7 +231,8 @@ k_row_stats_parallel(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols
     }
     sum = warp_sum(sum);
     if (lane == 0)
-      stats[r] = make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps))));
+      *reinterpret_cast<float2 *>(stats.at + r * stats.pitch) =
+          make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps))));
   }
 }
 
@@ -240,7 +242,7 @@ k_row_stats_parallel(const uint4 *x, float2 *stats, uint64_t rows, uint32_t cols
 template <int CHUNKS>
 __global__ void __launch_bounds__(256)
 k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const uint4 *b, uint4 *o, uint64_t rows,
-                         uint32_t cols, float eps, const float2 *stats) {
+                         uint32_t cols, float eps, const RowStats stats) {
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -261,9 +263,11 @@ k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const u
         sum = __fmaf_rn(f[e], f[e], sum);
     }
     sum = warp_sum(sum);
-    // `stats`: the statistic in the reference's sequential order (row_stats_sequential), which
+    // `stats`: the statistic in the reference's sequential order (row_stats), which
     // makes every output bit the reference's; else the warp's parallel sum (last bit may differ)
-    const float inv = stats ? stats[r].y : __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps)));
+    const float inv = stats.at ? row_stat(stats, r).y
+                               : __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps)));
+    __syncwarp(); // every lane has its copy: the row may be written
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
       const uint32_t c = lane + 32u * k;
@@ -289,7 +293,7 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(256)
 k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const uint4 *scale, const uint4 *shift,
                            uint4 *o, uint64_t rows, uint32_t cols, uint64_t rows_per_mod, float eps,
-                           const float2 *stats) {
+                           const RowStats stats) {
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -309,7 +313,9 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
       for (int e = 0; e < 8; ++e)
         mean += f[e];
     }
-    mean = stats ? stats[r].x : __fdiv_rn(warp_sum(mean), (float)cols);
+    const float2 given = stats.at ? row_stat(stats, r) : make_float2(0.0f, 0.0f);
+    __syncwarp(); // every lane has its copy: the row may be written
+    mean = stats.at ? given.x : __fdiv_rn(warp_sum(mean), (float)cols);
     float var = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
@@ -322,7 +328,7 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
       }
     }
     var = warp_sum(var);
-    const float inv = stats ? stats[r].y : __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(var, (float)cols), eps)));
+    const float inv = stats.at ? given.y : __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(var, (float)cols), eps)));
     const uint64_t mrow = (r / rows_per_mod) * cols8;
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
@@ -549,19 +555,39 @@ bool swiglu_fast(const void *x, void *o, uint32_t dt, uint64_t rows, uint64_t wi
   return true;
 }
 
-bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats,
-                          cudaStream_t s, int *rc) {
-  *stats = nullptr;
-  *rc = 0;
-  if (const char *v = std::getenv("DIFB200_EXACT_NORM"))
-    if (v[0] == '0')
-      return false;
-  if (rows == 0 || cols == 0 || cols % kStatCols != 0 || cols > 0xffffff00ull || !aligned16(x))
-    return false;
-  float2 *area = static_cast<float2 *>(device_scratch(rows * sizeof(float2)));
-  if (!area) {
-    *rc = fail(kOutOfMemory, "cannot allocate the row statistics scratch");
-    return true;
+int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, bool always, void *out,
+              uint64_t out_pitch, std::initializer_list<Span> reads, StreamScratch &scratch, RowStats *stats,
+              cudaStream_t s) {
+  *stats = RowStats{};
+  if (always && (!aligned16(x) || cols == 0 || cols % 8 != 0 || cols > 0xffffff00ull)) // 16 bytes at a time
+    return fail(kUnsupported, "row statistics: rows must start on 16 bytes");
+  const char *exact = std::getenv("DIFB200_EXACT_NORM");
+  const bool sequential = !(exact && exact[0] == '0') && cols != 0 && cols % kStatCols == 0 && cols <= 0xffffff00ull &&
+                          aligned16(x);
+  if (rows == 0 || (!sequential && !always))
+    return kOk;
+  const uintptr_t begin = reinterpret_cast<uintptr_t>(out), end = begin + rows * out_pitch;
+  auto meets = [&](const Span &r) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(r.start);
+    return r.start && b < end && begin < b + r.bytes;
+  };
+  bool shared = begin % 8 != 0 || out_pitch % 8 != 0 || out_pitch < sizeof(float2) || meets({x, rows * cols * 2});
+  for (const Span &r : reads)
+    shared = shared || meets(r);
+  if (shared) {
+    if (int rc = scratch.allocate(rows * sizeof(float2), "row statistics scratch"))
+      return rc;
+    *stats = RowStats{static_cast<unsigned char *>(scratch.get()), sizeof(float2)};
+  } else {
+    *stats = RowStats{static_cast<unsigned char *>(out), out_pitch};
+  }
+  const auto *X = static_cast<const uint4 *>(x);
+  if (!sequential) {
+    uint64_t blocks = (rows + 7) / 8;
+    const uint64_t cap = (uint64_t)sm_count() * 8;
+    blocks = blocks > cap ? cap : blocks;
+    k_row_stats_parallel<<<(unsigned)blocks, 256, 0, s>>>(X, *stats, rows, (uint32_t)cols, eps, layer ? 1 : 0);
+    return done("k_row_stats_parallel");
   }
   // Eight chunks in flight where a few warps per SM have to cover the latency alone, four where the rows
   // give an SM more than six warps (33272 x 3072: one wave of resident CTAs instead of two).
@@ -571,34 +597,13 @@ bool row_stats_sequential(const void *x, uint64_t rows, uint64_t cols, float eps
                      : (layer ? k_row_stats_sequential<true, 4> : k_row_stats_sequential<false, 4>);
   const size_t smem = sizeof(uint4) * kStatWarps * (deep ? 8 : 4) * 32 * kStatPitch;
   int resident = 1;
-  if ((*rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * kStatWarps, smem, &resident)))
-    return true;
+  if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * kStatWarps, smem, &resident))
+    return rc;
   uint64_t blocks = (warps + kStatWarps - 1) / kStatWarps;
   const uint64_t cap = (uint64_t)sm_count() * resident;
   blocks = blocks > cap ? cap : blocks;
-  kernel<<<(unsigned)blocks, 32 * kStatWarps, smem, s>>>(static_cast<const uint4 *>(x), area, rows, (uint32_t)cols, eps);
-  *rc = done("k_row_stats_sequential");
-  *stats = area;
-  return true;
-}
-
-int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer, const float2 **stats, cudaStream_t s) {
-  *stats = nullptr;
-  if (!aligned16(x) || cols == 0 || cols % 8 != 0 || cols > 0xffffff00ull) // both kernels read 16 bytes at a time
-    return fail(kUnsupported, "row statistics: rows must start on 16 bytes");
-  int rc = 0;
-  if (row_stats_sequential(x, rows, cols, eps, layer, stats, s, &rc))
-    return rc;
-  float2 *area = static_cast<float2 *>(device_scratch(rows * sizeof(float2)));
-  if (!area)
-    return fail(kOutOfMemory, "cannot allocate the row statistics scratch");
-  uint64_t blocks = (rows + 7) / 8;
-  const uint64_t cap = (uint64_t)sm_count() * 8;
-  blocks = blocks > cap ? cap : blocks;
-  k_row_stats_parallel<<<(unsigned)blocks, 256, 0, s>>>(static_cast<const uint4 *>(x), area, rows, (uint32_t)cols, eps,
-                                                        layer ? 1 : 0);
-  *stats = area;
-  return done("k_row_stats_parallel");
+  kernel<<<(unsigned)blocks, 32 * kStatWarps, smem, s>>>(X, *stats, rows, (uint32_t)cols, eps);
+  return done("k_row_stats_sequential");
 }
 
 bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const void *b, void *o, uint32_t dt,
@@ -611,8 +616,11 @@ bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const v
   blocks = blocks < 1 ? 1 : (blocks > cap ? cap : blocks);
   const auto X = static_cast<const uint4 *>(x), W = static_cast<const uint4 *>(w), A = static_cast<const uint4 *>(a),
              B = static_cast<const uint4 *>(b);
-  const float2 *stats = nullptr;
-  if (row_stats_sequential(x, rows, cols, eps, false, &stats, s, rc) && *rc)
+  RowStats stats;
+  StreamScratch scratch(s);
+  const uint64_t row_bytes = cols * 2;
+  if ((*rc = row_stats(x, rows, cols, eps, false, false, o, row_bytes, {{w, row_bytes}, {a, rows * row_bytes}, {b, rows * row_bytes}},
+                       scratch, &stats, s)))
     return true;
   if (cols == 3072)
     k_rms_norm_modulate_bf16<12><<<(unsigned)blocks, 256, 0, s>>>(X, W, A, B, static_cast<uint4 *>(o), rows,
@@ -635,8 +643,11 @@ bool layer_norm_modulate_fast(const void *x, const void *w, const void *b, const
   blocks = blocks < 1 ? 1 : (blocks > cap ? cap : blocks);
   const auto X = static_cast<const uint4 *>(x), W = static_cast<const uint4 *>(w), B = static_cast<const uint4 *>(b),
              SC = static_cast<const uint4 *>(scale), SH = static_cast<const uint4 *>(shift);
-  const float2 *stats = nullptr;
-  if (row_stats_sequential(x, rows, cols, eps, true, &stats, s, rc) && *rc)
+  RowStats stats;
+  StreamScratch scratch(s);
+  const uint64_t row_bytes = cols * 2, mod_bytes = (rows + rows_per_mod - 1) / rows_per_mod * row_bytes;
+  if ((*rc = row_stats(x, rows, cols, eps, true, false, o, row_bytes,
+                       {{w, row_bytes}, {b, row_bytes}, {scale, mod_bytes}, {shift, mod_bytes}}, scratch, &stats, s)))
     return true;
   if (cols == 3072)
     k_layer_norm_modulate_bf16<12><<<(unsigned)blocks, 256, 0, s>>>(X, W, B, SC, SH, static_cast<uint4 *>(o), rows,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "glue.h"
 
 namespace difb200 {
 
@@ -28,7 +29,7 @@ struct QuantParams {
   const uint16_t *norm_shift;  // [rows, columns]
   const uint16_t *norm_bias;   // [columns]: LayerNormModulate (mean removed, weight and bias); nullptr = RMS
   uint64_t norm_rows_per_mod;  // rows that share one row of scale / shift
-  const float2 *norm_stats;    // per row (mean, inverse deviation)
+  glue::RowStats norm_stats;   // per row (mean, inverse deviation)
   // Two fp32 -0, added to products of the norm. The assembler contracts mul.rn.f32x2 followed by add.rn.f32x2
   // into one fused operation (seen as single codes off by one), and an fma with a constant -0 as well; with
   // a -0 it cannot see, the product keeps its own rounding (x + -0 = x for every x, signed zeros included).

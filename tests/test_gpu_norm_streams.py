@@ -1,0 +1,115 @@
+"""Norm ops whose row statistic passes through scratch memory, used from several streams and threads at once and
+under stream capture: the scratch belongs to one call, so every result equals the one of a call by itself."""
+import threading
+
+import numpy as np
+import pytest
+
+from helpers import bf16_normal, to_torch_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(seed, rows, K):
+    rng = np.random.default_rng(seed)
+    t = lambda *shape, std=1.0: to_torch_bf16(bf16_normal(rng, shape, std))  # noqa: E731
+    return t(rows, K, std=1.0 + seed), t(K), t(K, std=0.1), t(rows, K, std=0.1), t(rows, K, std=0.1)
+
+
+def _call(ops, layer, x, w, b, s, h):
+    return ops.layer_norm_modulate_quant(x, w, b, s, h, 1e-6) if layer else ops.rms_norm_modulate_quant(x, w, s, h, 1e-5)
+
+
+def _same(a, b):
+    import torch
+    return torch.equal(a[0], b[0]) and torch.equal(a[1].view(torch.int32), b[1].view(torch.int32))
+
+
+@pytest.mark.parametrize("layer", [False, True])
+def test_two_streams_do_not_share_the_statistics(layer):
+    import torch
+    from diffusion_compiler_b200 import ops
+    sides = [_operands(k, 700 + 900 * k, 3072) for k in range(2)]  # the second needs more scratch than the first
+    alone = [_call(ops, layer, *o) for o in sides]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in sides]
+    got = [[], []]
+    for _ in range(20):
+        for k, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[k].append(_call(ops, layer, *sides[k]))
+    torch.cuda.synchronize()
+    assert all(_same(alone[k], g) for k in range(2) for g in got[k])
+
+
+def test_threads_with_streams_of_their_own():
+    import torch
+    from diffusion_compiler_b200 import ops
+    sides = [_operands(k, 100 + 400 * k, 1024) for k in range(4)]
+    alone = [_call(ops, k % 2 == 1, *o) for k, o in enumerate(sides)]
+    torch.cuda.synchronize()
+    got, errors = [None] * 4, []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                got[k] = [_call(ops, k % 2 == 1, *sides[k]) for _ in range(30)]
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    assert all(_same(alone[k], g) for k in range(4) for g in got[k])
+
+
+def test_captured_call_keeps_its_statistics_apart_from_later_calls():
+    """A captured call replays on another stream while plain calls with more rows run beside it."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    small, large = _operands(1, 300, 1024), _operands(2, 5000, 1024)
+    want, beside = _call(ops, True, *small), _call(ops, True, *large)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _call(ops, True, *small)
+    side = torch.cuda.Stream()
+    others = []
+    for _ in range(10):
+        graph.replay()
+        with torch.cuda.stream(side):
+            others.append(_call(ops, True, *large))
+    torch.cuda.synchronize()
+    assert _same(want, got) and all(_same(beside, o) for o in others)
+
+
+@pytest.mark.parametrize("K", [3072, 1280])
+@pytest.mark.parametrize("over", ["x", "scale", "shift"])
+def test_norm_ops_in_place(K, over):
+    """The output in the place of an input: the statistic then cannot stand in the output's rows."""
+    import ctypes as C
+
+    import torch
+    from diffusion_compiler_b200 import _lib
+    lib = _lib.lib()
+    x, w, b, s, h = _operands(3, 200, K)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def run(layer, out, x, s, h):
+        if layer:
+            _lib.check(lib.difb200_layer_norm_modulate(p(x), p(w), p(b), p(s), p(h), p(out), 2, 200, K, 200, 1e-6, stream))
+        else:
+            _lib.check(lib.difb200_rms_norm_modulate(p(x), p(w), p(s), p(h), p(out), 2, 200, K, 1e-5, stream))
+        return out
+
+    for layer in (False, True):
+        want = run(layer, torch.empty_like(x), x, s, h)
+        own = {"x": x.clone(), "scale": s.clone(), "shift": h.clone()}
+        got = run(layer, own[over], own["x"], own["scale"], own["shift"])
+        torch.cuda.synchronize()
+        assert torch.equal(want.view(torch.int16), got.view(torch.int16)), layer
