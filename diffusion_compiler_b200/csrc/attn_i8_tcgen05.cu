@@ -276,8 +276,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return packed;
 }
 
-// 32 outputs bf16(o / l) from RN(1 / l) and one correction by the residual (one rounding); where that has no
-// finite value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0.
+// 32 outputs bf16(o / l) from RN(1 / l) and one Markstein step (the product corrected by its residual, one rounding);
+// where that has no finite value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0.
 __device__ __forceinline__ void normalise(const uint32_t (&o)[32], float l, uint32_t (&w)[16]) {
   const float y = __frcp_rn(l);
   const uint64_t y2 = pack2(y, y), negl2 = pack2(-l, -l);
@@ -531,6 +531,9 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const uint32_t lane_base = (quarter * 32u) << 16;
     const uint32_t s_tmem = tmem + lane_base + t * 128u, o_tmem = tmem + lane_base + 256u + t * 128u;
     float m_run = -INFINITY, l = 0.0f;
+    // Whether the warp goes on. Only waits that end in a vote decide it, so that the warp goes one way: lanes that gave
+    // up alone would leave the others in a warp-wide instruction. (A vote behind each of the other two waits
+    // costs 0.7 us a call and more.)
     bool alive = true;
     // A bound on every score of this row: |q8_i| * max_j(|k8_j| * ks'_j) * A. When it is small
     // for the whole warp, its ceiling is the fixed maximum m of the row and a key tile needs one
@@ -544,11 +547,10 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
         kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-      if (!ptx::mbar_wait(q_full, 0, wait_ns)) {
+      if (!ptx::mbar_wait(q_full, 0, wait_ns)) { // the first wait for scores then ends the loop, for the whole warp
         if (lane == 0)
           report(p.status, 9 + t, 0);
         *abort_ptr = 1;
-        alive = false;
       }
       // the row's 128 codes: eight 16-byte chunks of one 128-byte row (the swizzle permutes
       // chunks inside the row, and the sum does not care); lanes start at different chunks
@@ -607,7 +609,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // The scores of this step. The stage's key table needs no wait of its own: it arrives on
       // the barrier of the V tile, which the MMA warp has seen complete before it issued the
       // Q.K^T whose completion is awaited here.
-      if (!ptx::mbar_wait_abortable(s_full + 16 * t + 8 * h, use & 1u, abort_ptr, wait_ns)) {
+      if (!ptx::mbar_wait_warp(s_full + 16 * t + 8 * h, use & 1u, abort_ptr, wait_ns)) {
         if (!*abort_ptr && lane == 0)
           report(p.status, 3 + t, g);
         *abort_ptr = 1;
@@ -668,12 +670,10 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (__any_sync(0xffffffffu, grow)) {
           // rescale O (and l) by an exact power of two; needs P.V of the previous step finished
           // (grow implies an earlier step with a valid key, so g > 0)
-          if (!ptx::mbar_wait(pv_done + 8 * t, (g - 1u) & 1u, wait_ns)) {
+          if (!ptx::mbar_wait(pv_done + 8 * t, (g - 1u) & 1u, wait_ns)) { // a later wait of the warp ends the loop
             if (lane == 0)
               report(p.status, 5 + t, g);
             *abort_ptr = 1;
-            alive = false;
-            break;
           }
           ptx::tc_fence_after();
           const float factor = grow ? ex2(m_run - m_new) : 1.0f;
@@ -719,9 +719,10 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // A row that other keys still join, in this cluster or in a later launch, is handed on as what its own keys
     // gave: no valid key counts as no maximum at all, and an m fixed at a bound far above the scores (l small)
     // comes down by the power of two that brings l to [1/2, 1). So every joined l is at least 1/2, and what a factor
-    // flushes (2^-127 and less) is too small to reach the sum.
-    float m_out = m_run, up = 1.0f;
-    if (SPLIT || p.carry_out) {
+    // flushes (2^-127 and less) is too small to reach the sum. Gives the power of two.
+    auto hand_on = [&](float &m_out) {
+      float up = 1.0f;
+      m_out = m_run;
       if (l == 0.0f) {
         m_out = -INFINITY;
       } else if (l < 0.5f) {
@@ -730,13 +731,13 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         up = __uint_as_float((uint32_t)(127 - e) << 23);
         l *= up;
       }
-    }
+      return up;
+    };
     if (SPLIT) {
       // The CTAs of the cluster hold the unnormalised outputs of the same queries over parts of the keys. Every m
       // is an integer, so all move to the largest one by exact powers of two. Unit u = (query tile, 32 columns) is
       // finished by CTA u % split: the others send it their scaled fp32 sums through distributed shared memory.
       // Three cluster barriers, passed by every thread on every path.
-      alive = __all_sync(0xffffffffu, alive);
       if (alive && !ptx::mbar_wait_warp(o_done + 8 * t, 0, abort_ptr, wait_ns)) {
         if (!*abort_ptr && lane == 0)
           report(p.status, 7 + t, 0);
@@ -747,6 +748,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::cluster_sync(); // all MMAs of all CTAs are done: Q and the stage ring are free
       ptx::tc_fence_after();
       const uint32_t row = t * 128u + row_in_tile;
+      float m_out;
+      hand_on(m_out);
       for (uint32_t r = 0; r < split; ++r) // (m, l) of every CTA and row, where Q was
         ptx::st_cluster_v2(ptx::mapa(q_addr + (rank * 256u + row) * 8u, r), __float_as_uint(m_out), __float_as_uint(l));
       __syncwarp();
@@ -813,13 +816,15 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
       }
     } else if (alive && n_kv > 0) {
-      if (!ptx::mbar_wait(o_done + 8 * t, 0, wait_ns)) {
-        if (lane == 0)
+      if (!ptx::mbar_wait_warp(o_done + 8 * t, 0, abort_ptr, wait_ns)) {
+        if (!*abort_ptr && lane == 0)
           report(p.status, 7 + t, 0);
         *abort_ptr = 1;
       } else {
         ptx::tc_fence_after();
         if (p.carry_out) {
+          float m_out;
+          const float up = hand_on(m_out);
           if (row_ok)
             p.ml_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = make_float2(m_out, l);
           float4 *carry = reinterpret_cast<float4 *>(p.o_state + (((uint64_t)batch * p.Sq + qrow) * p.H + head) * kTile);
