@@ -333,7 +333,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else {
     const uint32_t quarter = (uint32_t)warp & 3u;        // TMEM lane quarter of this warp
     const uint32_t ewarp = (uint32_t)warp - 2u;          // 0..7
-    const uint32_t col_half = ewarp >> 2;                // columns [128 col_half, 128 col_half + 128)
+    const uint32_t col_half = ewarp >> 2;                // columns [BN/2 col_half, BN/2 col_half + BN/2)
     uint32_t local = 0, store_buf = 0;
     uint8_t *generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
     float *scale_smem = reinterpret_cast<float *>(generic_base + (scale_base - smem_base));
@@ -344,7 +344,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t m0 = (tile / tiles_n) * kTileM + cta_rank * kBM, n0 = (tile % tiles_n) * BN;
       // column scales and biases of this tile -> this warp's private shared-memory copy
       // (warp-private so that no cross-warp barrier is needed)
-      float *cs = scale_smem + ewarp * BN, *bs = cs + BN / 2; // this warp's 128 columns
+      float *cs = scale_smem + ewarp * BN, *bs = cs + BN / 2; // this warp's BN / 2 columns
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < BN / 64; ++i) {

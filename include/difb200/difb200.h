@@ -100,9 +100,9 @@ DIFB200_EXPORT int difb200_quantize_int8_rows(const void *const *parts, const ui
  * QuantizeInt8Rows (a 256-wide ConvRot variant, static clip) in one kernel: the bf16 tensor between
  * the two ops is never written. The reference runs them as two ops on its generic path and has a
  * fused producer of its own for one model (src/runtime/cuda_executor.cpp:5417-5466). x, scale,
- * shift: bf16 [rows, columns]; weight: bf16 [columns] or NULL. The row statistic is summed in
- * parallel, as in difb200_rms_norm_modulate (a different order than there, so the two forms agree
- * to the last bit of the statistic, not beyond).
+ * shift: bf16 [rows, columns]; weight: bf16 [columns] or NULL. The row statistic is summed in the
+ * reference's sequential order (DIFB200_EXACT_NORM=0: as parallel sums), so codes and scales have the bits of the
+ * two separate calls. x must start on 16 bytes. The statistic passes through the rows of `codes`.
  */
 DIFB200_EXPORT int difb200_rms_norm_modulate_quant(const void *x, const void *weight, const void *scale,
                                                    const void *shift, uint64_t rows, uint64_t columns,
@@ -114,8 +114,7 @@ DIFB200_EXPORT int difb200_rms_norm_modulate_quant(const void *x, const void *we
  * (1 + scale) * h + shift with the reference's intermediate bf16 roundings) and QuantizeInt8Rows
  * (a 256-wide ConvRot variant, static clip) in one kernel. x: bf16 [rows, columns]; weight, bias:
  * bf16 [columns]; scale, shift: bf16 [rows / rows_per_modulation, columns] (one modulation row per
- * batch item). Mean and centred second moment are parallel sums, as in
- * difb200_layer_norm_modulate.
+ * batch item). Mean and centred second moment as the statistic above.
  */
 DIFB200_EXPORT int difb200_layer_norm_modulate_quant(const void *x, const void *weight, const void *bias,
                                                      const void *scale, const void *shift, uint64_t rows,
