@@ -518,14 +518,16 @@ struct Form {
 // splits are for problems that leave SMs idle, where time is one CTA's serial chain of k-blocks: 2 rows,
 // K 12288, N 3072 45 -> 22.5 us (12 CTAs of 96 k-blocks -> 96 of 24), K 3072 20.5 -> 14.3 us; 512 rows, K 12288
 // 43 -> 31 us; 1600 rows, K 8192 53 -> 49 us; 1101 rows, N 12288 47 -> 43 us. A split costs more than it gives
-// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`.
+// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`. Up to 16 rows a
+// k-block of the 128-column tiles takes about 200 ns more, one of the 256-column tiles does not (2 rows, N 12288,
+// K 3072: 20.6 us a call with the former and 18.6 with the latter; 64 rows 16.5 and 18.6).
 Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
   struct Cost {
     Form form;
     uint64_t block_ns, launch_ns;
   };
   static const Cost costs[] = {{{2, 256, 1}, 320, 6000}, {{2, 128, 1}, 208, 4500}, {{1, 256, 1}, 363, 5100},
-                               {{1, 128, 1}, 245, 3200}, {{1, 128, 2}, 320, 3500}, {{1, 128, 4}, 450, 4600}};
+                               {{1, 128, 1}, 258, 3200}, {{1, 128, 2}, 320, 3500}, {{1, 128, 4}, 450, 4600}};
   const uint64_t sms = (uint64_t)sm_count(), k_blocks = (K + kBK - 1) / kBK;
   // DIFB200_GEMM_FORM=ctas,columns,split forces one of the forms, DIFB200_GEMM_CTAS=1|2 a 256-column one
   // (all give identical bits).
@@ -547,7 +549,8 @@ Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
     if ((f.ctas == 2 && M <= (uint64_t)kBM) || (f.split > 1 && tiles > resident))
       continue;
     const uint64_t waves = (tiles + resident - 1) / resident;
-    const uint64_t time = waves * ((k_blocks + f.split - 1) / f.split) * c.block_ns + c.launch_ns;
+    const uint64_t block_ns = c.block_ns + (M <= 16 && f.tile_n == 128 ? 200 : 0);
+    const uint64_t time = waves * ((k_blocks + f.split - 1) / f.split) * block_ns + c.launch_ns;
     if (time < least) {
       least = time;
       best = f;
