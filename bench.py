@@ -415,12 +415,12 @@ def projection_set_extra(torch, ops, device, local_rank, peaks, i8_peak, steps=2
                               "gemm_i8_kernel",
                               sum(M_TOKENS * K + N * K for _, K, N, _ in PROJECTIONS) / len(PROJECTIONS),
                               sum(2.0 * M_TOKENS * N for _, K, N, _ in PROJECTIONS) / len(PROJECTIONS))},
-        "roofline_quant": {"bound": "hbm", "kernel": "convrot_quant_kernel",
+        "roofline_quant": {"bound": "hbm", "kernel": "convrot256_kernel",
                            "achieved": quant_bytes / (quant_ms * 1e-3) / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                            "frac": quant_bytes / (quant_ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
                            "peak_source": "%s copy bandwidth" % peaks["source"],
                            "traffic": recorded_traffic(
-                               "convrot_quant_kernel",
+                               "convrot256_kernel",
                                sum(2.0 * M_TOKENS * K for _, K, _, _ in PROJECTIONS) / len(PROJECTIONS),
                                sum(M_TOKENS * K + 4.0 * M_TOKENS for _, K, _, _ in PROJECTIONS) / len(PROJECTIONS))},
         "sustained": {"steps": n, "ms_per_step": sus_ms, "int8_tops": total_ops / (sus_ms * 1e-3) / 1e12,

@@ -155,8 +155,8 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
 // quantiser and key_table_kernel would give one after the other, bit for bit. 8 lanes hold a row
 // (16 elements each), so every access is a full 32-byte sector; HBM-bound (3 bytes per element). The first
 // `key_blocks` CTAs each take the 128 keys of one (batch, kv head, tile), the others 128 query rows each.
-// Replaces two thread-per-row quantiser launches (uncoalesced: 2.4 TB/s) and the table's own pass over the
-// codes: B2 S4608 H24 72 + 9 us before.
+// (Two thread-per-row quantiser launches and the table's own pass over the codes: B2 S4608 H24 81 us.) Bound by the
+// latency of its loads with half of the warps resident: B1 S4608 H16 16.5 us.
 struct OperandParams {
   const uint4 *q, *k;
   int8_t *q8, *k8;

@@ -15,20 +15,18 @@
 // thread's own 16 elements; a 16x16 transpose through shared memory (XOR-swizzled, conflict-free)
 // gives the thread the 16 elements of stride 16, on which stages 2-3 run.
 //
-// What bounds it: the SM's arithmetic and its issue slots, not HBM (3 bytes per element against about 16
-// thread instructions, 5 of them packed additions that take two clocks each). A warp therefore takes
+// What bounds it: not HBM (3 bytes per element) and not the issue slots alone (about 16 thread instructions per
+// element, 5 of them packed additions that take two clocks each: half of the slots), but the chain of a row -- load,
+// rotation, maximum, division, codes -- with 14 to 32 warps per SM to cover for one another. A warp takes
 // up to three such blocks of its row (NIT) before it needs the row's scale: the scale arithmetic, the
 // reductions and the loop overhead are paid once per 96 elements of a thread instead of once per 32, and
 // a row of up to 3072 columns needs no barrier at all. Between rotation and quantisation the bf16
 // variants keep the values as packed bf16 (their result is defined on the rounded values), half the
 // registers of fp32. The one-block form instead fits 64 registers, so that 32 warps per SM hide the
-// load latency without a prefetch. Measured against the one-block form with 80 registers and fp32
-// values that came before: 33272 x 3072 93.4 -> 86.9 us, 33272 x 8192 249 -> 226 us, 9216 x 12288 (signed)
-// 124 -> 111 us, 9216 x 3072 30.2 -> 28.8 us; the scale search of the weight form 12288 x 3072 454 -> 78 us
-// (all lanes evaluate samples, doubles only where the square needs them), with input equalisation
-// 478 -> 118 us; with RmsNormModulate in front 33272 x 3072 262 -> 145 us (packed arithmetic, 24 warps
-// instead of 16). Staging the input with bulk copies through shared memory instead of registers gave
-// nothing (30.0 us and 93.7 us for the first and third shape): loads are not what it waits for.
+// load latency without a prefetch. 33272 x 3072 takes 87 us (3.5 TB/s), 33272 x 8192 226 us, 9216 x 3072 29 us, the
+// scale search of the weight form 12288 x 3072 78 us (all lanes evaluate samples, doubles only where the square needs
+// them), with input equalisation 109 us, RmsNormModulate in front of 33272 x 3072 145 us with its statistic. Staging
+// the input with bulk copies through shared memory instead of registers gave nothing (30.0 us for the third shape).
 #include "quant_common.cuh"
 
 namespace difb200 {
