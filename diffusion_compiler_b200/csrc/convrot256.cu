@@ -151,11 +151,15 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     v[0] = v[1] = v[2] = v[3] = make_uint4(0, 0, 0, 0);
     const uint32_t c = col0 + 1024u * it;
     if (row < p.rows) {
+      // A prefetch must not wait for what it requests: its loads are predicated, without a branch that they would have
+      // to return from (one width, places known).
+      constexpr bool kPredicated = PREFETCH && kPlaced;
       if (c < columns)
-        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_a + row * pitch_a) : run_of(row, c), p.wide != 0, v[0], v[1]);
+        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_a + row * pitch_a) : run_of(row, c),
+                 !kPredicated && p.wide != 0, v[0], v[1]);
       if (c + 256u < columns)
-        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_b + row * pitch_b) : run_of(row, c + 256u), p.wide != 0, v[2],
-                 v[3]);
+        load_run(kPlaced ? reinterpret_cast<const uint4 *>(src_b + row * pitch_b) : run_of(row, c + 256u),
+                 !kPredicated && p.wide != 0, v[2], v[3]);
     }
   };
   auto row_barrier = [&]() { // the warps of one row only; rows in flight do not wait for each other
@@ -580,10 +584,13 @@ int launch_single(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
   // Plain rows of more than 8 blocks are a CTA each, and several CTAs per SM hide one another's barriers: three of 9 or
   // 10 warps, two of 11 or more (64 registers; 11 and 12 warps leave 80). 3333 rows, two CTAs with a prefetch ->
-  // this: 10240 columns 39.2 -> 35.6 us, fp32 41.9 -> 39.2; 12288 columns 43.8 -> 42.4 us, fp32 47.4 -> 45.3.
+  // this: 10240 columns 39.2 -> 35.6 us, fp32 41.9 -> 39.2; 12288 columns 43.8 -> 42.4 us, fp32 47.4 -> 45.3. The
+  // fp32 values of 13 warps and more do not leave room for a second CTA: one with a prefetch (9216 x 15360, two
+  // CTAs -> this, 147 -> 142 us, in two inputs 152 -> 142).
   if (blocks > 8u) {
     if constexpr (EXTRA == kPlain && !RESIDUAL)
-      return blocks == 11u || blocks == 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 384, 2>(p, stream)
+      return F32 && blocks > 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream)
+             : blocks == 11u || blocks == 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 384, 2>(p, stream)
                                             : launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 512, 2>(p, stream);
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
   }
