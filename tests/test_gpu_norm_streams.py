@@ -1,5 +1,6 @@
-"""Norm ops whose row statistic passes through scratch memory, used from several streams and threads at once and
-under stream capture: the scratch belongs to one call, so every result equals the one of a call by itself."""
+"""Norm ops whose row statistic passes from one kernel to the next, used from several streams and threads at once, under
+stream capture and in place: the memory it passes through belongs to one call, so every result equals the one of a
+call by itself."""
 import threading
 
 import numpy as np
