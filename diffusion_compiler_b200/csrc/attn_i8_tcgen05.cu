@@ -26,16 +26,18 @@
 // q8/qs and k8/ks are QuantizeInt8Rows(Direct) of the [B,S,H,128] / [B,S,KV,128] tensors.
 //
 // Structure: one CTA per (batch, head, 256 queries) = two 128-query tiles that share every K/V
-// tile. Warpgroup 0: warp 0 = TMA producer, warp 1 = MMA issuer (warps 2-3 idle). Warpgroups 1
-// and 2: softmax + epilogue of query tile 0 / 1, one thread per query row (its scores live in
-// registers, so no shuffles). K/V arrive in 128-key stages; the score / softmax / P.V pipeline
-// works in 64-key steps with the scores of each query tile double-buffered in tensor memory:
-// Q.K^T of step g+2 is issued right after P.V of step g, into the buffer that step's P just left,
-// so when a softmax warp finishes a step the scores of the next one are already there.
-// Tensor memory (512 columns): per query tile two score buffers of 64 columns (INT32; the bf16 P
-// of a step overwrites the first 32 columns of its buffer and is the TMEM A operand of P.V),
-// then O0 | O1 (fp32, 128 columns each). Items that would not fill a last wave are shared by clusters of CTAs that
-// take a part of the keys each (plan_split).
+// tile. Warp 0 = TMA producer, warps 1 and 2 = MMA issuers of query tile 0 / 1 (warp 3 idle). Warps 4-11 and 12-19:
+// softmax + epilogue of query tile 0 / 1, two threads per query row that take 32 columns of a step each (a thread's
+// scores live in registers, so no shuffles). K/V arrive in 128-key stages; the score / softmax / P.V pipeline
+// works in 64-key steps. Scores and P have their own columns of tensor memory, so the scores of step g + 1 are
+// made while those of step g are worked on in registers: at the end of a step a warp takes the next scores,
+// leaves its P and arrives once; the MMA warp then issues P.V of the step and Q.K^T of the one after the next.
+// Tensor memory per query tile (256 columns): scores of one step (64), P (32 columns of bf16 pairs, the A operand
+// of P.V), Q codes (32 columns, the A operand of Q.K^T: read from shared memory for every 64 keys they alone took its
+// bandwidth for 128 clocks, 387 against 259 clocks for the Q.K^T of both tiles), output (fp32, 128). Items that would
+// not fill a last wave are shared by clusters of CTAs that take a part of the keys each (plan_split).
+// The scores start from the bits of the float 1.5 * 2^23 (a bf16 MMA of constants in front of the INT8 ones), so the
+// INT32 sums are already floats when they are read: no instruction converts them.
 //
 // Chunked form (the token-sharded block, where keys arrive from other GPUs one slice at a time):
 // a launch covers up to two ranges of 128-key tiles and may carry the unnormalised state of every
@@ -54,19 +56,21 @@ namespace difb200 {
 namespace {
 
 constexpr int kTile = 128;          // queries per tile, keys per tile, head dim
-constexpr int kStages = 3;          // K/V ring depth
-constexpr uint32_t kQBytes = 128 * 128;        // int8 [128 x 128]
+constexpr int kStages = 4;          // K/V ring depth (Q passes through stages 2 and 3 first)
 constexpr uint32_t kKBytes = 128 * 128;        // int8 [128 keys x 128]
 constexpr uint32_t kVBytes = 128 * 128 * 2;    // bf16 [128 keys x 128] as two 64-wide halves
 constexpr uint32_t kKsBytes = 128 * 8;         // (key scale, mask bias) per key, as float4 per key pair
 constexpr uint32_t kStageBytes = kKBytes + kVBytes + kKsBytes;
-constexpr int kThreads = 384;
+constexpr int kThreads = 640;      // 4 control warps, 2 x 8 softmax warps
 constexpr uint32_t kPartialBytes = 32 * 32 * 4; // split form: a [32 rows x 32 columns] fp32 partial output
 constexpr uint32_t kOutBoxBytes = 32 * 128;    // a warp's output staging: two [32 rows x 64 bf16] boxes
-constexpr size_t kSmemBytes = 1024 + 2 * kQBytes + kStages * kStageBytes + 256;
+constexpr uint32_t kConstBytes = 6144;         // bf16 [128 x 16] of 1024 and [64 x 16] of 768: 16 products = 1.5 * 2^23
+constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
+constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + kConstBytes + 256 + kPairBytes;
 
 struct AttnParams {
-  const float *qs;       // [B,S,H]
+  const int8_t *q8;      // [B,Sq,H,128]
+  const float *qs;       // [B,Sq,H]
   const float2 *ksmb;    // [B,KV,S_pad/2] x float4 (ks'_j, ks'_j+1, bias_j, bias_j+1)
   const float *tile_bound; // [B,KV,S_pad/128] max over the tile's valid keys of |k8_j| * ks'_j
   uint32_t B, Sq, Sk, H, KV, S_pad; // Sq query tokens, Sk key tokens (S_pad = Sk rounded up to 128)
@@ -77,7 +81,8 @@ struct AttnParams {
   // key tiles of this launch: [tile_begin[0], +tile_count[0]) then [tile_begin[1], +tile_count[1])
   uint32_t tile_begin[2], tile_count[2];
   float *o_state;        // [B,Sq,H,128] fp32 unnormalised outputs carried between launches
-  float2 *ml_state;      // [B,Sq,H] (m, l) carried between launches
+  float2 *ml_state;      // [B,Sq,H] (m, l of the even half of the columns) carried between launches
+  float *l2_state;       // [B,Sq,H] l of the other half: a sequence of launches continues the very same sums
   uint32_t carry_in, carry_out;
   uint32_t item0, split; // first (batch, head, query block) of this launch; CTAs of a cluster that share its keys
 };
@@ -303,18 +308,18 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t *base_ptr = smem_raw + (base - raw_addr);
-  const uint32_t q_addr = base;                       // 2 x 16 KB
-  const uint32_t stage_addr = base + 2 * kQBytes;     // kStages x (K | V | ksmb)
-  const uint32_t bar = stage_addr + kStages * kStageBytes;
+  const uint32_t stage_addr = base;                   // kStages x (K | V | ksmb)
+  const uint32_t const_addr = stage_addr + kStages * kStageBytes;
+  const uint32_t bar = const_addr + kConstBytes;
   // barriers (8 bytes each)
-  const uint32_t q_full = bar;
-  const uint32_t k_full = bar + 8, k_empty = k_full + 8 * kStages;
-  const uint32_t v_full = k_empty + 8 * kStages, v_empty = v_full + 8 * kStages;
-  const uint32_t s_full = v_empty + 8 * kStages;      // [2 tiles][2 buffers]
-  const uint32_t p_full = s_full + 32;                // [2][2]
-  const uint32_t pv_done = p_full + 32;               // [2] one phase per step (rescaling waits on it)
-  const uint32_t o_done = pv_done + 16;               // [2] completes once, after the last P.V
-  const uint32_t tmem_slot = o_done + 16;
+  const uint32_t q_tma = bar;                         // Q codes are in shared memory
+  const uint32_t q_full = bar + 8;                    // [2 tiles] they stand in tensor memory
+  const uint32_t kv_full = q_full + 16, kv_empty = kv_full + 8 * kStages;
+  const uint32_t s_full = kv_empty + 8 * kStages;     // [2] phase g: Q.K^T of step g is done, and P.V of step g - 2
+  const uint32_t p_full = s_full + 16;                // [2] phase 0: scores of step 0 read; phase g + 1: P of step g stored, scores of g + 1 read
+  const uint32_t pair_bar = p_full + 16;              // [2][4] the two warps of 32 rows have exchanged a word per row
+  const uint32_t tmem_slot = pair_bar + 64;
+  const uint32_t pair_mem = bar + 256;
   volatile uint32_t *slot_ptr = reinterpret_cast<volatile uint32_t *>(base_ptr + (tmem_slot - base));
   volatile uint32_t *abort_ptr = slot_ptr + 1;
 
@@ -336,31 +341,57 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       i += first;
     return i < p.tile_count[0] ? p.tile_begin[0] + i : p.tile_begin[1] + (i - p.tile_count[0]);
   };
-  auto score_col = [](uint32_t t, uint32_t b) { return t * 128u + b * 64u; }; // TMEM column of a score buffer
 
+  auto load_tile = [&](uint32_t i, uint32_t s) { // K, V and the key table of this CTA's i-th tile into stage s
+    const uint32_t k_dst = stage_addr + s * kStageBytes, v_dst = k_dst + kKBytes, t_dst = v_dst + kVBytes;
+    const uint32_t tile = key_tile(i);
+    const int32_t key0 = (int32_t)(tile * kTile);
+    const float2 *table = p.ksmb + ((uint64_t)batch * p.KV + kvh) * p.S_pad;
+    ptx::mbar_expect_tx(kv_full + 8 * s, kKBytes + kVBytes + kKsBytes);
+    ptx::tma_load_4d(k_dst, &map_k, kv_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
+    ptx::tma_load_4d(v_dst, &map_v, kv_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
+    ptx::tma_load_4d(v_dst + kVBytes / 2, &map_v, kv_full + 8 * s, 64, (int32_t)kvh, key0, (int32_t)batch);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+                     "r"(t_dst), "l"(reinterpret_cast<uint64_t>(table + (uint64_t)tile * kTile)),
+                 "r"(kKsBytes), "r"(kv_full + 8 * s)
+                 : "memory");
+  };
+  const uint32_t early = min(n_kv, 2u); // tiles whose loads thread 0 issues during the set-up (0.6 us of a CTA's 6 us around its steps)
+  // What the softmax warps need first is requested before the set-up: the row's scale, the bounds of the keys.
+  float A = 0.0f, kmax = 0.0f;
+  if (warp >= 4) {
+    const uint32_t qr = q0 + (uint32_t)((warp - 4) >> 3) * 128u + (warp & 3) * 32u + lane;
+    A = __ldg(p.qs + ((uint64_t)batch * p.Sq + (qr < p.Sq ? qr : 0u)) * p.H + head);
+    const float *bounds = p.tile_bound + ((uint64_t)batch * p.KV + kvh) * (p.S_pad / kTile);
+    for (uint32_t i = lane; i < n_kv; i += 32)
+      kmax = fmaxf(kmax, __ldg(bounds + key_tile(i)));
+  }
   if (threadIdx.x == 0) {
-    ptx::mbar_init(q_full, 1);
+    ptx::mbar_init(q_full, 8);
+    ptx::mbar_init(q_full + 8, 8);
+    ptx::mbar_init(q_tma, 1);
+    for (int i = 0; i < 8; ++i)
+      ptx::mbar_init(pair_bar + 8 * i, 2);
     for (int s = 0; s < kStages; ++s) {
-      ptx::mbar_init(k_full + 8 * s, 1);
-      ptx::mbar_init(k_empty + 8 * s, 1);
-      ptx::mbar_init(v_full + 8 * s, 1);
-      ptx::mbar_init(v_empty + 8 * s, 1);
+      ptx::mbar_init(kv_full + 8 * s, 1);
+      ptx::mbar_init(kv_empty + 8 * s, 2);
     }
     for (int t = 0; t < 2; ++t) {
-      for (int b = 0; b < 2; ++b) {
-        ptx::mbar_init(s_full + 16 * t + 8 * b, 1);
-        ptx::mbar_init(p_full + 16 * t + 8 * b, 128);
-      }
-      ptx::mbar_init(pv_done + 8 * t, 1);
-      ptx::mbar_init(o_done + 8 * t, 1);
+      ptx::mbar_init(s_full + 8 * t, 1);
+      ptx::mbar_init(p_full + 8 * t, 8);
     }
     *abort_ptr = 0;
     ptx::fence_barrier_init();
-    ptx::prefetch_tensormap(&map_q);
-    ptx::prefetch_tensormap(&map_k);
-    ptx::prefetch_tensormap(&map_v);
+    ptx::mbar_expect_tx(q_tma, 2 * kKBytes); // Q codes: staged where the ring is still free
+    for (uint32_t t = 0; t < 2; ++t)
+      ptx::tma_load_4d(stage_addr + (2u + t) * kStageBytes, &map_q, q_tma, 0, (int32_t)head, (int32_t)(q0 + t * 128u), (int32_t)batch);
+    for (uint32_t i = 0; i < early; ++i)
+      load_tile(i, i);
     ptx::prefetch_tensormap(&map_o);
   }
+  for (uint32_t i = threadIdx.x; i < kConstBytes / 4; i += kThreads)
+    *reinterpret_cast<uint32_t *>(base_ptr + (const_addr - base) + i * 4u) = i < 1024u ? 0x44804480u : 0x44404440u;
+  ptx::fence_proxy_async();
   if (warp == 1) {
     ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
@@ -371,12 +402,14 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const uint32_t tmem = *slot_ptr;
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-    // The producer and the MMA warp run their loops with all 32 lanes and warp-uniform control
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    // The producer and the MMA warps run their loops with all 32 lanes and warp-uniform control
     // flow (every wait ends in a vote); one elected lane issues the asynchronous instructions.
     // Addresses, descriptors and loop state are then warp-uniform values. As single-lane
-    // (divergent) loops every TMA / MMA operand was first moved between register files, and
-    // issuing the 12 MMAs of one tile step took about twice the 768 clocks they execute in.
+    // (divergent) loops every TMA / MMA operand was first moved between register files. One warp for both
+    // query tiles was the bound of the whole kernel: its control instructions are a serial chain of about 1500 clocks
+    // per 64-key step, in which the MMAs themselves execute for 770. Two warps with the shortest loop (one wait, one
+    // commit per step): B2 S4608 H24 443 -> 404 us.
     auto give_up = [&](uint32_t role, uint32_t detail) {
       if (lane == 0) {
         if (!*abort_ptr)
@@ -386,128 +419,91 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     };
     if (warp == 0) {
       // ---------------- TMA producer ----------------
-      if (ptx::elect_one()) {
-        ptx::mbar_expect_tx(q_full, 2 * kQBytes);
-        ptx::tma_load_4d(q_addr, &map_q, q_full, 0, (int32_t)head, (int32_t)q0, (int32_t)batch);
-        ptx::tma_load_4d(q_addr + kQBytes, &map_q, q_full, 0, (int32_t)head, (int32_t)(q0 + 128u),
-                         (int32_t)batch);
-      }
-      const float2 *table = p.ksmb + ((uint64_t)batch * p.KV + kvh) * p.S_pad;
-      uint32_t s = 0, phase = 0;
-      for (uint32_t i = 0; i < n_kv; ++i) {
-        const uint32_t k_dst = stage_addr + s * kStageBytes, v_dst = k_dst + kKBytes,
-                       t_dst = v_dst + kVBytes;
-        const uint32_t tile = key_tile(i);
-        const int32_t key0 = (int32_t)(tile * kTile);
-        if (!ptx::mbar_wait_warp(k_empty + 8 * s, phase ^ 1u, abort_ptr, wait_ns)) {
+      uint32_t s = early, phase = 0;
+      for (uint32_t i = early; i < n_kv; ++i) {
+        if (!ptx::mbar_wait_uniform(kv_empty + 8 * s, phase ^ 1u, abort_ptr, wait_ns) ||
+            ((i == 2u || i == 3u) && !ptx::mbar_wait_uniform(q_full + 8 * (i - 2u), 0, abort_ptr, wait_ns))) {
           give_up(0, i);
           break;
         }
-        if (ptx::elect_one()) {
-          ptx::mbar_expect_tx(k_full + 8 * s, kKBytes);
-          ptx::tma_load_4d(k_dst, &map_k, k_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
-        }
-        if (!ptx::mbar_wait_warp(v_empty + 8 * s, phase ^ 1u, abort_ptr, wait_ns)) {
-          give_up(1, i);
-          break;
-        }
-        if (ptx::elect_one()) {
-          ptx::mbar_expect_tx(v_full + 8 * s, kVBytes + kKsBytes);
-          ptx::tma_load_4d(v_dst, &map_v, v_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
-          ptx::tma_load_4d(v_dst + kVBytes / 2, &map_v, v_full + 8 * s, 64, (int32_t)kvh, key0,
-                           (int32_t)batch);
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-                           "r"(t_dst), "l"(reinterpret_cast<uint64_t>(table + (uint64_t)tile * kTile)),
-                       "r"(kKsBytes), "r"(v_full + 8 * s)
-                       : "memory");
-        }
+        if (ptx::elect_one())
+          load_tile(i, s);
         if (++s == kStages) {
           s = 0;
           phase ^= 1u;
         }
       }
-    } else if (warp == 1) {
-      // ---------------- MMA issuer ----------------
+    } else if (warp < 3) {
+      // ---------------- MMA issuers, one per query tile ----------------
+      const uint32_t t = __shfl_sync(0xffffffffu, (uint32_t)warp - 1u, 0);
       constexpr uint32_t idesc_qk = ptx::make_idesc(2 /*S32*/, 1 /*S8*/, 1 /*S8*/, 0, 0, 128, 64);
       constexpr uint32_t idesc_pv = ptx::make_idesc(1 /*F32*/, 1 /*BF16*/, 1 /*BF16*/, 0, 1 /*V is N-major*/, 128, 128);
-      const uint64_t q_desc = ptx::smem_desc_sw128(q_addr, 16, 1024);
       const uint64_t k_desc0 = ptx::smem_desc_sw128(stage_addr, 16, 1024);
       // V tile, N-major: 64-wide halves 16 KB apart (leading offset), 8-key groups 1 KB apart.
       const uint64_t v_desc0 = ptx::smem_desc_sw128(stage_addr + kKBytes, kVBytes / 2, 1024);
-      bool ok = true;
-      // (both are called inside the elected lane's branch) step g covers keys 64 g .. 64 g + 63,
-      // i.e. half g & 1 of the 128-key stage (g / 2) % kStages, and score buffer g & 1.
-      auto issue_qk = [&](uint32_t t, uint32_t g) {
-        const uint32_t h = g & 1u, st = (g >> 1) % kStages;
-        const uint64_t a = q_desc + (uint64_t)((t * kQBytes) >> 4);
-        const uint64_t b = k_desc0 + (uint64_t)((st * kStageBytes + h * 64u * 128u) >> 4);
+      // constants, no swizzle: [8 x 16 bytes] core matrices 128 bytes apart along K, 256 along the rows
+      constexpr uint32_t idesc_c = ptx::make_idesc(1 /*F32*/, 1 /*BF16*/, 1 /*BF16*/, 0, 0, 128, 64);
+      const uint64_t ca_desc = ptx::smem_desc_plain(const_addr, 128, 256), cb_desc = ptx::smem_desc_plain(const_addr + 4096u, 128, 256);
+      // Step g covers keys 64 g .. 64 g + 63, i.e. half g & 1 of the 128-key stage (g / 2) % kStages.
+      // (called inside the elected lane's branch) Q.K^T of a step, keys from descriptor address b
+      const uint32_t d_s = tmem + t * 256u, d_o = d_s + 128u, a_p = d_s + 64u, a_q = d_s + 96u;
+      const uint32_t s_bar = s_full + 8 * t, p_bar = p_full + 8 * t;
+      auto issue_qk = [&](uint32_t b) {
+        const uint64_t kd = k_desc0 + b;
+        ptx::mma_f16_ss(d_s, ca_desc, cb_desc, idesc_c, 0); // every score = the bits of 1.5 * 2^23
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          ptx::mma_i8_ss(tmem + score_col(t, h), a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc_qk, k != 0);
-        ptx::mma_commit(s_full + 16 * t + 8 * h);
+          ptx::mma_i8_ts(d_s, a_q + 8u * k, kd + (uint64_t)(2 * k), idesc_qk, 1);
+        ptx::mma_commit(s_bar);
       };
-      auto issue_pv = [&](uint32_t t, uint32_t g) {
-        // A = P in tensor memory (32 columns of bf16 pairs at the start of the score buffer);
-        // B = the 64 keys of the V stage: 16 keys per MMA = 8 TMEM columns, 2048 bytes of V
-        const uint32_t h = g & 1u, st = (g >> 1) % kStages;
-        const uint64_t b = v_desc0 + (uint64_t)((st * kStageBytes + h * 64u * 128u) >> 4);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          ptx::mma_f16_ts(tmem + 256u + t * 128u, tmem + score_col(t, h) + 8u * k, b + (uint64_t)(128 * k),
-                          idesc_pv, k != 0 ? 1u : ((g != 0u || p.carry_in) ? 1u : 0u));
-        ptx::mma_commit(pv_done + 8 * t);
-      };
-      if (!ptx::mbar_wait_warp(q_full, 0, abort_ptr, wait_ns)) {
+      bool ok = ptx::mbar_wait_uniform(kv_full, 0, abort_ptr, wait_ns) && ptx::mbar_wait_uniform(q_full + 8 * t, 0, abort_ptr, wait_ns);
+      if (!ok)
         give_up(2, 0);
-        ok = false;
-      }
-      if (ok && (!ptx::mbar_wait_warp(k_full, 0, abort_ptr, wait_ns) || !ptx::mbar_wait_warp(v_full, 0, abort_ptr, wait_ns))) {
-        give_up(2, 1);
-        ok = false;
-      }
       if (ok) {
         ptx::tc_fence_after();
-        if (ptx::elect_one()) {
-          issue_qk(0, 0);
-          issue_qk(1, 0);
-          issue_qk(0, 1);
-          issue_qk(1, 1);
-          ptx::mma_commit(k_empty);
-        }
+        if (ptx::elect_one())
+          issue_qk(0);
+        ok = ptx::mbar_wait_uniform(p_bar, 0, abort_ptr, wait_ns);
+        if (!ok)
+          give_up(2, 1);
+        ptx::tc_fence_after();
+        if (ok && ptx::elect_one())
+          issue_qk(512u);
       }
-      for (uint32_t g = 0; g < n_steps && ok; ++g) {
-        const uint32_t h = g & 1u, use = g >> 1;               // use-th time this score buffer is filled
-        const uint32_t st = use % kStages;
-        const uint32_t use_n = use + 1u, st_n = use_n % kStages, phase_n = (use_n / kStages) & 1u;
-        const bool more = g + 2u < n_steps;
-        // K, V and the key table of the next stage, before the first Q.K^T on it (the softmax
-        // warps take the completion of that Q.K^T as their signal for the table, and this
-        // stage's V was awaited the same way one stage earlier)
-        if (h == 0u && more &&
-            (!ptx::mbar_wait_warp(k_full + 8 * st_n, phase_n, abort_ptr, wait_ns) ||
-             !ptx::mbar_wait_warp(v_full + 8 * st_n, phase_n, abort_ptr, wait_ns))) {
+      uint32_t st = 0, st_n = 1, phase_n = 0, acc = p.carry_in; // stages of the P.V and Q.K^T that come next
+      for (uint32_t i = 0; i < n_steps && ok; ++i) {
+        const uint32_t h = i & 1u;
+        const bool more = i + 2u < n_steps;
+        if (h == 0u && more && !ptx::mbar_wait_uniform(kv_full + 8 * st_n, phase_n, abort_ptr, wait_ns)) {
           give_up(2, 5);
           break;
         }
+        if (!ptx::mbar_wait_uniform(p_bar, h ^ 1u, abort_ptr, wait_ns)) { // phase i + 1
+          give_up(2, 3 + t);
+          break;
+        }
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          const uint64_t b = v_desc0 + (uint64_t)(st * (kStageBytes >> 4) + h * 512u);
+          // A = P in tensor memory (32 columns of bf16 pairs);
+          // B = the 64 keys of the V stage: 16 keys per MMA = 8 TMEM columns, 2048 bytes of V
+          ptx::mma_f16_ts(d_o, a_p, b, idesc_pv, acc);
 #pragma unroll
-        for (uint32_t t = 0; t < 2; ++t) {
-          if (!ptx::mbar_wait_warp(p_full + 16 * t + 8 * h, use & 1u, abort_ptr, wait_ns)) {
-            give_up(2, 3 + t);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          if (ptx::elect_one()) {
-            issue_pv(t, g);
-            if (g + 1u == n_steps)
-              ptx::mma_commit(o_done + 8 * t);
-            if (t == 1 && h == 1u)
-              ptx::mma_commit(v_empty + 8 * st);
-            if (more) {
-              issue_qk(t, g + 2u); // into the buffer P of step g is being read from: same pipe, in order
-              if (t == 1 && h == 1u)
-                ptx::mma_commit(k_empty + 8 * st_n);
-            }
+          for (int k = 1; k < 4; ++k)
+            ptx::mma_f16_ts(d_o, a_p + 8u * k, b + (uint64_t)(128 * k), idesc_pv, 1);
+          if (more)
+            issue_qk(st_n * (kStageBytes >> 4) + h * 512u);
+          else
+            ptx::mma_commit(s_bar);
+          if (h != 0u)
+            ptx::mma_commit(kv_empty + 8 * st);
+        }
+        acc = 1u;
+        if (h != 0u) {
+          st = st_n;
+          if (++st_n == kStages) {
+            st_n = 0;
+            phase_n ^= 1u;
           }
         }
       }
@@ -519,52 +515,69 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::cluster_sync();
     }
   } else {
-    // ---------------- softmax + epilogue, one thread per query row ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-    const uint32_t t = (uint32_t)(warp - 4) >> 2;       // query tile 0 / 1
+    // ---------------- softmax + epilogue, two threads per query row ----------------
+    // Four warps per scheduler: the ld / st / barrier time of one is covered by the others. With one thread per row
+    // (two warps per scheduler, 64 columns each): B2 S4608 H24 398 us, with two 352. 32 x 128 + 112 x 512 registers are
+    // what the launch has (96 x 640).
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    const uint32_t t = (uint32_t)(warp - 4) >> 3, hf = ((uint32_t)(warp - 4) >> 2) & 1u; // query tile 0 / 1; half of the columns
     const uint32_t quarter = (uint32_t)warp & 3u;
     const uint32_t row_in_tile = quarter * 32u + lane;
     const uint32_t qrow = q0 + t * 128u + row_in_tile;
     const bool row_ok = qrow < p.Sq;
-    const float A = (row_ok ? __ldg(p.qs + ((uint64_t)batch * p.Sq + qrow) * p.H + head) : 1.0f) *
-                    p.scale_log2e;
+    A = (row_ok ? A : 1.0f) * p.scale_log2e;
     const uint32_t lane_base = (quarter * 32u) << 16;
-    const uint32_t s_tmem = tmem + lane_base + t * 128u, o_tmem = tmem + lane_base + 256u + t * 128u;
+    const uint32_t s_tmem = tmem + lane_base + t * 256u, p_tmem = s_tmem + 64u, o_tmem = s_tmem + 128u;
     float m_run = -INFINITY, l = 0.0f;
     // Whether the warp goes on. Only waits that end in a vote decide it, so that the warp goes one way: lanes that gave
-    // up alone would leave the others in a warp-wide instruction. (A vote behind each of the other two waits
-    // costs 0.7 us a call and more.)
+    // up alone would leave the others in a warp-wide instruction.
     bool alive = true;
     // A bound on every score of this row: |q8_i| * max_j(|k8_j| * ks'_j) * A. When it is small
     // for the whole warp, its ceiling is the fixed maximum m of the row and a key tile needs one
     // pass (no maximum, no rescaling); otherwise the warp keeps a running maximum.
     bool fixed_max = false;
     {
-      float kmax = 0.0f;
-      const float *bounds = p.tile_bound + ((uint64_t)batch * p.KV + kvh) * (p.S_pad / kTile);
-      for (uint32_t i = lane; i < n_kv; i += 32)
-        kmax = fmaxf(kmax, __ldg(bounds + key_tile(i)));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
         kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-      if (!ptx::mbar_wait(q_full, 0, wait_ns)) { // the first wait for scores then ends the loop, for the whole warp
+      // the row's 128 codes: A operand of Q.K^T, 32 columns of which each of the row's threads brings half
+      if (!ptx::mbar_wait_uniform(q_tma, 0, abort_ptr, wait_ns)) {
         if (lane == 0)
           report(p.status, 9 + t, 0);
         *abort_ptr = 1;
+        alive = false;
       }
-      // the row's 128 codes: eight 16-byte chunks of one 128-byte row (the swizzle permutes
-      // chunks inside the row, and the sum does not care); lanes start at different chunks
-      const uint4 *qrow = reinterpret_cast<const uint4 *>(base_ptr + (q_addr - base) + t * kQBytes +
-                                                          row_in_tile * 128u);
+      const uint8_t *codes = base_ptr + (stage_addr - base) + (2u + t) * kStageBytes + row_in_tile * 128u;
       int n2 = 0;
+      {
+        uint32_t mine[16];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint4 w = qrow[(c + lane) & 7];
-        n2 = __dp4a((int)w.x, (int)w.x, n2);
-        n2 = __dp4a((int)w.y, (int)w.y, n2);
-        n2 = __dp4a((int)w.z, (int)w.z, n2);
-        n2 = __dp4a((int)w.w, (int)w.w, n2);
+        for (int c = 0; c < 4; ++c) {
+          const uint4 w = *reinterpret_cast<const uint4 *>(codes + (((hf * 4u + c) ^ (lane & 7u)) << 4));
+          mine[4 * c] = w.x;
+          mine[4 * c + 1] = w.y;
+          mine[4 * c + 2] = w.z;
+          mine[4 * c + 3] = w.w;
+        }
+        ptx::tmem_st_32x16(s_tmem + 96u + 16u * hf, mine);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint4 w = *reinterpret_cast<const uint4 *>(codes + ((((hf ^ 1u) * 4u + c) ^ (lane & 7u)) << 4));
+          n2 = __dp4a((int)w.x, (int)w.x, n2);
+          n2 = __dp4a((int)w.y, (int)w.y, n2);
+          n2 = __dp4a((int)w.z, (int)w.z, n2);
+          n2 = __dp4a((int)w.w, (int)w.w, n2);
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          n2 = __dp4a((int)mine[c], (int)mine[c], n2);
       }
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before();
+      ptx::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0)
+        ptx::mbar_arrive(q_full + 8 * t);
       const float bound = __fmul_rn(__fmul_rn(A, __fsqrt_rn((float)n2)), kmax);
       const float m_fixed = ceilf(__fadd_rn(bound, 0.001f));
       // State carried in from the launch over the previous key ranges. m only ever grows, and
@@ -575,7 +588,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (p.carry_in && row_ok) {
         const float2 ml = __ldg(p.ml_state + ((uint64_t)batch * p.Sq + (q0 + t * 128u + row_in_tile)) * p.H + head);
         m_prev = ml.x;
-        l = ml.y;
+        l = hf == 0u ? ml.y : __ldg(p.l2_state + ((uint64_t)batch * p.Sq + qrow) * p.H + head);
       }
       const float m_both = fmaxf(m_prev, m_fixed);
       // (a bound far above what the carried state holds would push that state towards underflow)
@@ -587,7 +600,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const float4 *src = reinterpret_cast<const float4 *>(
             p.o_state + (((uint64_t)batch * p.Sq + (q0 + t * 128u + row_in_tile)) * p.H + head) * kTile);
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 2 * hf; c < 2 * hf + 2; ++c) {
           uint32_t o[32];
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
@@ -603,74 +616,98 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
     }
     const uint64_t A2 = pack2(A, A);
-    for (uint32_t g = 0; g < n_steps && alive; ++g) {
-      const uint32_t h = g & 1u, use = g >> 1;
-      const uint32_t s = use % kStages;
-      // The scores of this step. The stage's key table needs no wait of its own: it arrives on
-      // the barrier of the V tile, which the MMA warp has seen complete before it issued the
-      // Q.K^T whose completion is awaited here.
-      if (!ptx::mbar_wait_warp(s_full + 16 * t + 8 * h, use & 1u, abort_ptr, wait_ns)) {
+    uint32_t r[32];
+    uint32_t pair_phase = 0;
+    float *pair_slot = reinterpret_cast<float *>(base_ptr + (pair_mem - base)) + t * 256u + row_in_tile;
+    // A word of each of the row's two threads to the other (bounded like every wait).
+    auto exchange = [&](float x) {
+      float *slot = pair_slot + (pair_phase & 1u) * 512u;
+      slot[hf * 128u] = x;
+      __syncwarp();
+      if (lane == 0)
+        ptx::mbar_arrive(pair_bar + 8u * (t * 4u + quarter));
+      if (!ptx::mbar_wait_uniform(pair_bar + 8u * (t * 4u + quarter), pair_phase & 1u, abort_ptr, wait_ns)) {
+        if (!*abort_ptr && lane == 0)
+          report(p.status, 11 + t, 0);
+        *abort_ptr = 1;
+        alive = false;
+      }
+      ++pair_phase;
+      return slot[(hf ^ 1u) * 128u];
+    };
+    // The scores of step g, when its Q.K^T is done. The stage's key table needs no wait of its own: it arrives on
+    // the barrier of the V tile, which the MMA warp has seen complete before it issued the
+    // Q.K^T whose completion is awaited here.
+    auto await_scores = [&](uint32_t g) {
+      if (!ptx::mbar_wait_uniform(s_full + 8 * t, g & 1u, abort_ptr, wait_ns)) {
         if (!*abort_ptr && lane == 0)
           report(p.status, 3 + t, g);
         *abort_ptr = 1;
         alive = false;
-        break;
       }
+      return alive;
+    };
+    if (n_steps != 0u && alive && await_scores(0)) {
       ptx::tc_fence_after();
-      const uint32_t sc_tmem = s_tmem + h * 64u;
-      uint32_t r[2][32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-        ptx::tmem_ld_32x32(sc_tmem + 32u * c, r[c]);
+      ptx::tmem_ld_32x32(s_tmem + 32u * hf, r);
       ptx::tmem_ld_wait();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        ptx::mbar_arrive(p_full + 8 * t);
+    }
+    for (uint32_t g = 0; g < n_steps && alive; ++g) {
+      const uint32_t h = g & 1u;
+      const uint32_t s = (g >> 1) % kStages;
       const float4 *tab = reinterpret_cast<const float4 *>(base_ptr + (stage_addr - base) + s * kStageBytes +
-                                                           kKBytes + kVBytes) + h * 32u;
-      uint32_t pk[32];
+                                                           kKBytes + kVBytes) + h * 32u + hf * 16u;
+      uint32_t pk[16];
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull}; // 8 partial row sums as packed fp32 pairs
       if (fixed_max) {
         const uint64_t negm2 = pack2(-m_run, -m_run);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float4 kk = tab[(c * 32 + j) >> 1]; // (ks'_j, ks'_j+1, -C ks'_j, -C ks'_j+1)
-            const float f0 = __int_as_float((int32_t)r[c][j] + 0x4B400000);     // C + acc, exact
-            const float f1 = __int_as_float((int32_t)r[c][j + 1] + 0x4B400000);
-            const uint64_t u2 = fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w));
-            float e0, e1;
-            unpack2(fma2(u2, A2, negm2), e0, e1);
-            const float p0 = ex2(e0), p1 = ex2(e1);
-            sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
-            pk[(c * 32 + j) >> 1] = pack_bf16(p0, p1);
-          }
+        for (int j = 0; j < 32; j += 2) {
+          const float4 kk = tab[j >> 1]; // (ks'_j, ks'_j+1, -C ks'_j, -C ks'_j+1)
+          const float f0 = __uint_as_float(r[j]);     // C + acc, exact
+          const float f1 = __uint_as_float(r[j + 1]);
+          const uint64_t u2 = fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w));
+          float e0, e1;
+          unpack2(fma2(u2, A2, negm2), e0, e1);
+          const float p0 = ex2(e0), p1 = ex2(e1);
+          sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
+          pk[j >> 1] = pack_bf16(p0, p1);
         }
       } else {
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float4 kk = tab[(c * 32 + j) >> 1];
-            const float f0 = __int_as_float((int32_t)r[c][j] + 0x4B400000);
-            const float f1 = __int_as_float((int32_t)r[c][j + 1] + 0x4B400000);
-            float u0, u1;
-            unpack2(fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w)), u0, u1);
-            r[c][j] = __float_as_uint(u0);
-            r[c][j + 1] = __float_as_uint(u1);
-            float &acc_max = mx4[(j >> 1) & 3];
-            asm("max.f32 %0, %0, %1, %2;" : "+f"(acc_max) : "f"(u0), "f"(u1));
-          }
+        for (int j = 0; j < 32; j += 2) {
+          const float4 kk = tab[j >> 1];
+          const float f0 = __uint_as_float(r[j]);
+          const float f1 = __uint_as_float(r[j + 1]);
+          float u0, u1;
+          unpack2(fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w)), u0, u1);
+          r[j] = __float_as_uint(u0);
+          r[j + 1] = __float_as_uint(u1);
+          float &acc_max = mx4[(j >> 1) & 3];
+          asm("max.f32 %0, %0, %1, %2;" : "+f"(acc_max) : "f"(u0), "f"(u1));
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        // power-of-two running maximum
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        // power-of-two running maximum, of the whole row
+        mx = fmaxf(mx, exchange(mx));
+        if (!alive)
+          break;
         float m_new = m_run;
         if (mx != -INFINITY)
-          m_new = fmaxf(m_run, ceilf(mx * A));
+          m_new = ceilf(mx * A);
+        // It may lag behind the scores by 16, which makes a P at most 2^16: most warps had a row with a larger ceiling in
+        // most steps, and each moved 128 output columns (B2 S4608 H24 with 8 times larger scores: 674 us, with a lag of 8
+        // 600, 24 538). m_run = -inf: the first valid key sets it.
+        m_new = m_new > m_run + 16.0f ? m_new : m_run;
         const bool grow = m_new > m_run && m_run != -INFINITY;
         if (__any_sync(0xffffffffu, grow)) {
           // rescale O (and l) by an exact power of two; needs P.V of the previous step finished
           // (grow implies an earlier step with a valid key, so g > 0)
-          if (!ptx::mbar_wait(pv_done + 8 * t, (g - 1u) & 1u, wait_ns)) { // a later wait of the warp ends the loop
+          if (!ptx::mbar_wait(s_full + 8 * t, (g + 1u) & 1u, wait_ns)) { // a later wait of the warp ends the loop
             if (lane == 0)
               report(p.status, 5 + t, g);
             *abort_ptr = 1;
@@ -679,7 +716,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const float factor = grow ? ex2(m_run - m_new) : 1.0f;
           l *= factor;
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (uint32_t c = 2u * hf; c < 2u * hf + 2u; ++c) {
             uint32_t o[32];
             ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
             ptx::tmem_ld_wait();
@@ -694,15 +731,12 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const float neg_m = (m_run == -INFINITY) ? 0.0f : -m_run;
         const uint64_t negm2 = pack2(neg_m, neg_m);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float e0, e1;
-            unpack2(fma2(pack2(__uint_as_float(r[c][j]), __uint_as_float(r[c][j + 1])), A2, negm2), e0, e1);
-            const float p0 = ex2(e0), p1 = ex2(e1);
-            sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
-            pk[(c * 32 + j) >> 1] = pack_bf16(p0, p1);
-          }
+        for (int j = 0; j < 32; j += 2) {
+          float e0, e1;
+          unpack2(fma2(pack2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), A2, negm2), e0, e1);
+          const float p0 = ex2(e0), p1 = ex2(e1);
+          sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
+          pk[j >> 1] = pack_bf16(p0, p1);
         }
       }
       {
@@ -711,11 +745,26 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         unpack2(add2(sum2[2], sum2[3]), b0, b1);
         l += (a0 + a1) + (b0 + b1);
       }
-      ptx::tmem_st_32x32(sc_tmem, pk);
+      // P of this step takes the place of the last one's when that one's P.V is done: the Q.K^T of step g + 1 was issued
+      // behind it, so its completion says so.
+      if (!await_scores(g + 1u))
+        break;
+      if (g + 1u < n_steps) {
+        ptx::tc_fence_after();
+        ptx::tmem_ld_32x32(s_tmem + 32u * hf, r);
+      }
+      ptx::tmem_st_32x16(p_tmem + 16u * hf, pk);
+      ptx::tmem_ld_wait();
       ptx::tmem_st_wait();
       ptx::tc_fence_before();
-      ptx::mbar_arrive(p_full + 16 * t + 8 * h);
+      __syncwarp();
+      if (lane == 0)
+        ptx::mbar_arrive(p_full + 8 * t);
     }
+    const float l_own = l;
+    if (alive)
+      l += exchange(l);
+    const uint32_t done_bar = s_full + 8 * t, done_parity = (n_steps + 1u) & 1u;
     // A row that other keys still join, in this cluster or in a later launch, is handed on as what its own keys
     // gave: no valid key counts as no maximum at all, and an m fixed at a bound far above the scores (l small)
     // comes down by the power of two that brings l to [1/2, 1). So every joined l is at least 1/2, and what a factor
@@ -738,7 +787,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // is an integer, so all move to the largest one by exact powers of two. Unit u = (query tile, 32 columns) is
       // finished by CTA u % split: the others send it their scaled fp32 sums through distributed shared memory.
       // Three cluster barriers, passed by every thread on every path.
-      if (alive && !ptx::mbar_wait_warp(o_done + 8 * t, 0, abort_ptr, wait_ns)) {
+      if (alive && !ptx::mbar_wait_warp(done_bar, done_parity, abort_ptr, wait_ns)) {
         if (!*abort_ptr && lane == 0)
           report(p.status, 7 + t, 0);
         *abort_ptr = 1;
@@ -750,11 +799,11 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       const uint32_t row = t * 128u + row_in_tile;
       float m_out;
       hand_on(m_out);
-      for (uint32_t r = 0; r < split; ++r) // (m, l) of every CTA and row, where Q was
-        ptx::st_cluster_v2(ptx::mapa(q_addr + (rank * 256u + row) * 8u, r), __float_as_uint(m_out), __float_as_uint(l));
+      for (uint32_t r = hf; r < split; r += 2u) // (m, l) of every CTA and row, behind the slots
+        ptx::st_cluster_v2(ptx::mapa(stage_addr + 36u * kPartialBytes + (rank * 256u + row) * 8u, r), __float_as_uint(m_out), __float_as_uint(l));
       __syncwarp();
       ptx::cluster_sync();
-      const float2 *mls = reinterpret_cast<const float2 *>(base_ptr + (q_addr - base)) + row;
+      const float2 *mls = reinterpret_cast<const float2 *>(base_ptr + (stage_addr - base) + 36u * kPartialBytes) + row;
       float m_all = -INFINITY, l_all = 0.0f;
       for (uint32_t r = 0; r < split; ++r)
         m_all = fmaxf(m_all, mls[r * 256u].x);
@@ -773,7 +822,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         return stage_addr + ((u / split * split + from) * 4u + quarter) * kPartialBytes + lane * 16u;
       };
 #pragma unroll 1
-      for (uint32_t c = 0; c < 4; ++c) {
+      for (uint32_t c = 2u * hf; c < 2u * hf + 2u; ++c) {
         const uint32_t u = t * 4u + c, owner = u % split;
         if (owner == rank)
           continue;
@@ -787,7 +836,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       __syncwarp();
       ptx::cluster_sync();
 #pragma unroll 1
-      for (uint32_t c = 0; c < 4; ++c) {
+      for (uint32_t c = 2u * hf; c < 2u * hf + 2u; ++c) {
         const uint32_t u = t * 4u + c;
         if (u % split != rank)
           continue;
@@ -816,7 +865,14 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
       }
     } else if (alive && n_kv > 0) {
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(o_done + 8 * t, 0, wait_ns))) { // (0.5 us a call less than mbar_wait_warp)
+      // Outputs are staged in a ring stage: tile 0 in the one after the last one used, tile 1 in the one after that. The
+      // other query tile runs on its own and may still need what the stage held last (key tile n_kv - 4 + t, or Q codes).
+      const uint32_t stage = (n_kv + t) % kStages;
+      const bool free = n_kv + t >= (uint32_t)kStages
+                            ? ptx::mbar_wait_uniform(kv_empty + 8 * stage, ((n_kv + t - kStages) / kStages) & 1u, abort_ptr, wait_ns)
+                            : ptx::mbar_wait_uniform(q_full, 0, abort_ptr, wait_ns) &&
+                                  ptx::mbar_wait_uniform(q_full + 8, 0, abort_ptr, wait_ns);
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(done_bar, done_parity, wait_ns)) || !free) {
         if (!*abort_ptr && lane == 0)
           report(p.status, 7 + t, 0);
         *abort_ptr = 1;
@@ -825,11 +881,13 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (p.carry_out) {
           float m_out;
           const float up = hand_on(m_out);
-          if (row_ok)
-            p.ml_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = make_float2(m_out, l);
+          if (row_ok && hf == 0u)
+            p.ml_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = make_float2(m_out, l_own * up);
+          else if (row_ok)
+            p.l2_state[((uint64_t)batch * p.Sq + qrow) * p.H + head] = l_own * up;
           float4 *carry = reinterpret_cast<float4 *>(p.o_state + (((uint64_t)batch * p.Sq + qrow) * p.H + head) * kTile);
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 2 * (int)hf; c < 2 * (int)hf + 2; ++c) {
             uint32_t o[32];
             ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
             ptx::tmem_ld_wait();
@@ -842,16 +900,11 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           }
         } else {
           // Rows leave through shared memory and TMA stores of [32 rows x 64 columns] (rows past Sq are
-          // clipped); a thread's own stores touched 32 lines per instruction. Tile 0 stages in the ring stage
-          // after the last one used, tile 1 in the one after that: nothing is in flight there any more, while
-          // the last stage may still feed tile 1's final P.V.
-          // With the shorter division below: B2 S4608 H24 518 -> 488 us, 1101 tokens 35.9 -> 32.0 us a call
-          // (a CTA's fixed cost was about 13 us, 72 steps of the first shape take 60).
-          const uint32_t stage = (n_kv + t) % kStages;
+          // clipped); a thread's own stores touched 32 lines per instruction.
           const uint32_t staging = stage_addr + stage * kStageBytes + quarter * (2u * kOutBoxBytes);
           uint8_t *staging_ptr = base_ptr + (staging - base);
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 2 * (int)hf; c < 2 * (int)hf + 2; ++c) {
             uint32_t o[32];
             ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
             ptx::tmem_ld_wait();
@@ -871,7 +924,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
           }
           if (lane == 0)
-            ptx::tma_store_wait();
+            ptx::tma_store_read_wait();
         }
       }
     }
@@ -911,11 +964,12 @@ int resident_clusters(uint32_t split, int &count) {
 // Items (batch, head, 256 queries) that run as one CTA each, and the split over the keys of the others. A last wave
 // that is nearly empty costs as much as a full one: 3120 items of the 33272-token block are 21.08 waves of 148 SMs.
 // Its items (or those of the last two waves) are split 2, 3, 4 or 8 ways over the key tiles by clusters. Modelled
-// times in ns, measured on B200: 1660 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
+// times in ns, measured on B200: 1380 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
 // and the exchange, at least four tiles per CTA; a split has to give 3 %. H24, without -> with: 1 x 1700 tokens
-// (1.14 waves) 75 -> 70 us, 2 x 2500 (3.24) 188 -> 178 us, 1 x 8000 (5.19) 707 -> 645 us.
+// (1.14 waves) 60.2 -> 57.4 us, 2 x 2500 (3.24) 145 -> 141 us, 1 x 6400 (4.05) 381 -> 344 us, 1 x 8000 (5.19) 566 -> 529 us;
+// where the rule takes none, a split costs: 1 x 4608 (2.92) 178 -> 202 us.
 int plan_split(uint64_t items, uint64_t tiles, uint64_t &whole, uint32_t &split) {
-  constexpr uint64_t kTileNs = 1660, kItemNs = 6000, kExchangeNs = 8000;
+  constexpr uint64_t kTileNs = 1380, kItemNs = 6000, kExchangeNs = 8000;
   const uint64_t sms = (uint64_t)sm_count(), item_ns = kItemNs + tiles * kTileNs;
   whole = items;
   split = 1;
@@ -957,7 +1011,7 @@ size_t attention_int8_scratch_bytes(uint64_t B, uint64_t S, uint64_t KV) {
 }
 
 size_t attention_int8_state_bytes(uint64_t B, uint64_t Sq, uint64_t H) {
-  return (size_t)(B * Sq * H * (kTile * sizeof(float) + sizeof(float2)));
+  return (size_t)(B * Sq * H * (kTile * sizeof(float) + sizeof(float2) + sizeof(float)));
 }
 
 int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const float *ks, const void *v_bf16,
@@ -1085,6 +1139,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       return rc;
   }
   AttnParams p{};
+  p.q8 = q8;
   p.qs = qs;
   p.ksmb = table;
   p.tile_bound = tile_bound;
@@ -1103,9 +1158,10 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     p.tile_count[i] = count[i];
   }
   if (chunk && (chunk->carry_in || chunk->carry_out)) {
-    // state buffer: fp32 outputs [B,Sq,H,128], then (m, l) per row
+    // state buffer: fp32 outputs [B,Sq,H,128], then (m, l) and the other half's l per row
     p.o_state = static_cast<float *>(chunk->state);
     p.ml_state = reinterpret_cast<float2 *>(p.o_state + B * Sq * H * kTile);
+    p.l2_state = reinterpret_cast<float *>(p.ml_state + B * Sq * H);
     p.carry_in = chunk->carry_in ? 1u : 0u;
     p.carry_out = chunk->carry_out ? 1u : 0u;
   }
@@ -1123,8 +1179,8 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     split_config(config, attr, ctas);
     config.gridDim = dim3((unsigned)(count * ctas));
     config.stream = stream;
-    return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k,
-                                       map_v, map_o, p),
+    return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k, map_v,
+                                       map_o, p),
                     "attn_i8_kernel launch");
   };
   if (whole)

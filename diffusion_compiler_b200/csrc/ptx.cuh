@@ -94,6 +94,23 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   }
   return __all_sync(0xffffffffu, ok);
 }
+// The same with the least code (one loop that votes on every poll): for the serial loops of single warps, where
+// every instruction between two waits counts.
+__device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
+                                                  unsigned long long limit_ns) {
+  uint32_t polls = 0;
+  unsigned long long start = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++polls & 255u) == 0u) {
+      const unsigned long long now = global_timer();
+      if (polls == 256u)
+        start = now;
+      else if (__any_sync(0xffffffffu, *abort_flag != 0u || now - start > limit_ns))
+        return false;
+    }
+  }
+  return true;
+}
 
 // 2-D tiled TMA load, global -> this CTA's shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar,
@@ -117,7 +134,7 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
                "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
-// 4-D tiled TMA store, shared memory -> global, as its own bulk group; the wait is for all groups' completion.
+// 4-D tiled TMA store, shared memory -> global, as its own bulk group.
 __device__ __forceinline__ void tma_store_4d(uint32_t src, const CUtensorMap *map, int32_t c0, int32_t c1, int32_t c2,
                                              int32_t c3) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
@@ -126,8 +143,9 @@ __device__ __forceinline__ void tma_store_4d(uint32_t src, const CUtensorMap *ma
                : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void tma_store_wait() {
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+// Waits until the sources of all groups have been read (the CTA may go then; the writes end with the kernel).
+__device__ __forceinline__ void tma_store_read_wait() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
@@ -161,6 +179,17 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint
                "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n"
                "}" ::"r"(d_tmem),
                "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]; INT8 operands, INT32 accumulator.
+__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                          uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n"
+               ".reg .pred p;\n"
+               "setp.ne.b32 p, %4, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n"
+               "}" ::"r"(d_tmem),
+               "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem]; bf16/f16 operands, fp32 accumulator.
@@ -320,6 +349,12 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t
                                                     uint32_t sbo_bytes) {
   return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// The same without a swizzle (for operands whose layout does not matter).
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
+         ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
 // Instruction descriptor (32-bit) for kind::i8 / kind::f16:

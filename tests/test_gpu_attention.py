@@ -298,3 +298,32 @@ def test_attention_takes_operands_that_start_on_two_bytes(ops, moved):
     torch.cuda.synchronize()
     ops.poll_status()
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("q_gain", [1.0, 6.0])
+@pytest.mark.parametrize("Sq,tiles", [(130, 1), (130, 2), (256, 3), (130, 4), (257, 5), (130, 9)])
+def test_attention_ring_and_query_tiles(ops, Sq, tiles, q_gain):
+    """The two query tiles of a CTA run on their own and share the K/V ring, which also carries the query codes at the
+    start and the outputs at the end: key tiles around the depth of the ring (4), a second query tile of one or two
+    rows (it finishes first), keys whose first half is masked, with the fixed and the running maximum. Against the
+    oracle at the bar of the path (rel-L2 2e-3); the same bits again."""
+    import torch
+    Sk = 128 * tiles - 5
+    rng = np.random.default_rng(900 + tiles)
+    q, _, _ = _qkv(rng, 1, Sq, 4, 2)
+    _, k, v = _qkv(rng, 1, Sk, 4, 2)
+    if q_gain != 1.0:
+        q = ob.f32_to_bf16(ob.bf16_to_f32(q) * np.float32(q_gain))
+    valid = np.ones((1, Sk), np.uint8)
+    valid[:, :Sk // 2 + 11] = 0
+    q8, qs = ob.orc().quantize_int8_rows([q.reshape(-1, 128)], 1)
+    k8, ks = ob.orc().quantize_int8_rows([k.reshape(-1, 128)], 1)
+    q8, k8 = q8.reshape(1, Sq, 4, 128), k8.reshape(1, Sk, 2, 128)
+    want = ob.bf16_to_f32(ob.orc().attention_int8_rows(q8, qs, k8, ks, v, valid))
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    args = (t(q8), t(qs), t(k8), t(ks), to_torch_bf16(v), t(valid))
+    first, again = ops.attention_int8(*args), ops.attention_int8(*args)
+    torch.cuda.synchronize()
+    ops.poll_status()
+    assert torch.equal(first.view(torch.int16), again.view(torch.int16))
+    assert rel_l2(ob.bf16_to_f32(from_torch_bf16(first)), want) <= 2e-3
