@@ -160,8 +160,7 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
 // quantiser and key_table_kernel would give one after the other, bit for bit. 8 lanes hold a row
 // (16 elements each), so every access is a full 32-byte sector; HBM-bound (3 bytes per element). The first
 // `key_blocks` CTAs each take the 128 keys of one (batch, kv head, tile), the others 128 query rows each.
-// (Two thread-per-row quantiser launches and the table's own pass over the codes: B2 S4608 H24 81 us.) Bound by the
-// latency of its loads with half of the warps resident: B1 S4608 H16 16.5 us.
+// (Two thread-per-row quantiser launches and the table's own pass over the codes: B2 S4608 H24 81 us.)
 struct OperandParams {
   const uint4 *q, *k;
   int8_t *q8, *k8;
@@ -193,20 +192,8 @@ attention_operands_kernel(const OperandParams p) {
     for (int o = 4; o > 0; o >>= 1)
       m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     scale = row_scale(m, 1.0f);
-    const float recip = __frcp_rn(scale);
-    const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-scale, -scale);
     uint32_t out[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float f[4];
-      unpack2(div2_exact(v[2 * i], y2, nb2), f[0], f[1]);
-      unpack2(div2_exact(v[2 * i + 1], y2, nb2), f[2], f[3]);
-      uint32_t c[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        c[e] = (uint32_t)max(sat_s8(f[e]), -127);
-      out[i] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
-    }
+    direct_codes(v, scale, out);
     codes = make_uint4(out[0], out[1], out[2], out[3]);
   };
   if (blockIdx.x < p.key_blocks) {

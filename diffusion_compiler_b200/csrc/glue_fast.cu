@@ -7,6 +7,7 @@
 #include "glue.h"
 
 #include "common.cuh"
+#include "quant_common.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -353,9 +354,14 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
 
 // ---- QkNormPartialRope on 128-wide heads (cpu_executor.cpp:1741-1837), optionally followed by
 // QuantizeInt8Rows(Direct) of the result (cpu_executor.cpp:124-307, Direct branch) ----
-// One thread per (token, head) row: the sum of squares runs in the reference's sequential order
-// (multiply, then add), so the statistic has the reference's bits; rotation partners are in the
-// same thread. ROTARY and the layout are compile-time so that the row stays in registers.
+// A warp takes ROWS (token, head) rows of 256 bytes through shared memory. First a lane sums the squares of a row
+// in the reference's sequential order (squares of bf16 values are exact, so the fused operation is the reference's
+// multiply then add): the statistic has the reference's bits. Then 8 lanes share a row, two runs of 8 elements
+// each, chosen so that rotation partners are in the same lane: every access to HBM is a full 128-byte line, and
+// the codes come from direct_codes. HBM-bound by its bytes (3 per element), by its arithmetic in practice:
+// 33272 x 24 rows with rotary 96 and codes take 127 us (230 us as one thread per row with
+// IEEE divisions), 4096 x 24 with rotary 128 in pairs 21 us (37 us). Few rows take 8 per warp, for more warps in flight
+// (256 x 24: 12.6 -> 6.3 us a call).
 struct RowRopeParams {
   const uint4 *x;
   const uint4 *w;       // [128] bf16
@@ -379,112 +385,166 @@ __device__ __forceinline__ void load_table8(const void *table, uint32_t f32, uin
     unpack8(__ldg(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(table) + index)), v);
   }
 }
-__device__ __forceinline__ int sat_s8(float v) {
-  int r;
-  asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(r) : "f"(v));
-  return r;
-}
+constexpr int kRopePitch = 17;  // uint4 per row in shared memory (16 + 1 pad)
+constexpr int kRopeWarps = 4;
 
-template <int ROTARY, bool V2>
-__global__ void __launch_bounds__(128)
+template <int ROTARY, bool V2, int ROWS>
+__global__ void __launch_bounds__(32 * kRopeWarps)
 k_qk_norm_rope_row128(const RowRopeParams p) {
-  const uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= p.rows)
+  __shared__ uint4 tile[kRopeWarps][ROWS * kRopePitch];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t row0 = ((uint64_t)blockIdx.x * kRopeWarps + warp) * ROWS;
+  if (row0 >= p.rows)
     return;
-  const uint64_t token = row / p.heads, head = row - token * p.heads;
-  const uint4 *src = p.x + token * p.in_token_stride16 + p.in_offset16 + head * 16;
-  const uint64_t out_row = ((token / p.input_seq) * p.out_seq + p.out_start + token % p.input_seq) * p.heads + head;
-  float n[128];
+  // this lane's row of the first pass
+  const uint64_t mine = row0 + (lane % ROWS) < p.rows ? row0 + (lane % ROWS) : p.rows - 1;
+  const uint64_t token = mine / p.heads, head = mine - token * p.heads, sequence = token / p.input_seq;
+  const uint64_t in_sequence = token - sequence * p.input_seq;
+  const uint64_t src = token * p.in_token_stride16 + p.in_offset16 + head * 16;
+  const uint64_t out_row = (sequence * p.out_seq + p.out_start + in_sequence) * p.heads + head;
+  const uint64_t trow = (sequence * p.table_seq + p.table_start + in_sequence) * p.table_width;
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    float f[8];
-    unpack8(__ldg(src + c), f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      n[8 * c + e] = f[e];
+  for (int i = 0; i < ROWS; i += 2) { // half a warp copies a row
+    const int r = i + (lane >> 4);
+    const uint64_t from = __shfl_sync(0xffffffffu, src, r) + (lane & 15);
+    cp_async16(smem_u32(&tile[warp][r * kRopePitch + (lane & 15)]), p.x + from, true);
   }
+  // runs of 8 elements of this lane in the second pass: partners of a half-split rotation are ROTARY / 2 apart
+  constexpr int kRun = ROTARY / 8; // runs that rotate
+  const int j = lane & 7;
+  const bool rotates = V2 ? 2 * j < kRun : j < kRun / 2;
+  const int c0 = V2 ? 2 * j : j < kRun / 2 ? j : kRun + 2 * (j - kRun / 2);
+  const int c1 = V2 || !rotates ? c0 + 1 : j + kRun / 2;
+  uint64_t w[8];
+  {
+    const uint4 a = __ldg(p.w + c0), b = __ldg(p.w + c1);
+    const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      w[i] = unpack_bf16_pair(u[i]);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
   float sum = 0.0f;
-#pragma unroll
-  for (int d = 0; d < 128; ++d)
-    sum = __fadd_rn(sum, __fmul_rn(n[d], n[d]));
-  const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, 128.0f), p.eps)));
-#pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    float wv[8];
-    unpack8(__ldg(p.w + c), wv);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float scaled = __fmul_rn(n[8 * c + e], inv);
-      n[8 * c + e] = V2 ? round_bf16(__fmul_rn(round_bf16(scaled), wv[e])) : __fmul_rn(scaled, wv[e]);
-    }
-  }
-  const uint64_t trow = ((token / p.input_seq) * p.table_seq + p.table_start + token % p.input_seq) * p.table_width;
-  if (V2) { // interleaved pairs (2 i, 2 i + 1), one table entry per pair
-#pragma unroll
-    for (int pc = 0; pc < ROTARY / 16; ++pc) {
-      float c[8], s[8];
-      load_table8(p.cosv, p.table_f32, trow + 8 * pc, c);
-      load_table8(p.sinv, p.table_f32, trow + 8 * pc, s);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float even = n[16 * pc + 2 * e], odd = n[16 * pc + 2 * e + 1];
-        n[16 * pc + 2 * e] = __fsub_rn(__fmul_rn(even, c[e]), __fmul_rn(odd, s[e]));
-        n[16 * pc + 2 * e + 1] = __fadd_rn(__fmul_rn(even, s[e]), __fmul_rn(odd, c[e]));
-      }
-    }
-  } else { // half-split pairs (d, d + ROTARY / 2)
-    constexpr int kHalf = ROTARY / 2;
-    const bool wide = p.table_width == (uint32_t)ROTARY; // second half of the pair has its own entries
-#pragma unroll
-    for (int dc = 0; dc < kHalf / 8; ++dc) {
-      float c1[8], s1[8], c2[8], s2[8];
-      load_table8(p.cosv, p.table_f32, trow + 8 * dc, c1);
-      load_table8(p.sinv, p.table_f32, trow + 8 * dc, s1);
-      load_table8(p.cosv, p.table_f32, trow + 8 * dc + (wide ? kHalf : 0), c2);
-      load_table8(p.sinv, p.table_f32, trow + 8 * dc + (wide ? kHalf : 0), s2);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float a = n[8 * dc + e], b = n[8 * dc + e + kHalf];
-        n[8 * dc + e] = __fsub_rn(__fmul_rn(a, c1[e]), __fmul_rn(b, s1[e]));
-        n[8 * dc + e + kHalf] = __fadd_rn(__fmul_rn(b, c2[e]), __fmul_rn(a, s2[e]));
-      }
-    }
-  }
-  // the stored bf16 values (what a consumer of the unfused op would read back)
-  float m = 0.0f;
-#pragma unroll
-  for (int d = 0; d < 128; ++d) {
-    n[d] = round_bf16(n[d]);
-    m = fmaxf(m, fabsf(n[d]));
-  }
-  if (p.o) {
+  {
+    const uint4 *row = tile[warp] + (lane % ROWS) * kRopePitch;
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      float f[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        f[e] = n[8 * c + e];
-      p.o[out_row * 16 + c] = pack8(f);
+      const uint4 v = row[c];
+      sum = accumulate_word<1>(v.x, 0.0f, sum);
+      sum = accumulate_word<1>(v.y, 0.0f, sum);
+      sum = accumulate_word<1>(v.z, 0.0f, sum);
+      sum = accumulate_word<1>(v.w, 0.0f, sum);
     }
   }
-  if (p.codes) {
-    const float scale = fmaxf(__fdiv_rn(m, 127.0f), 1.0e-30f); // clip 1: max * 1 / 127
-    p.scales[out_row] = scale;
-    uint4 *dst = reinterpret_cast<uint4 *>(p.codes + out_row * 128);
+  const float inv_mine = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, 128.0f), p.eps)));
+  // Rows it .. it + 3. The bf16 conversions keep NaN, where the reference's rounding of the bits makes zeros of the
+  // NaN that arithmetic gives: RAW rounds as the reference does. Returns whether a NaN was met (NaN spreads to the end).
+  auto process = [&](int it, auto raw) {
+    constexpr bool RAW = decltype(raw)::value;
+    auto bf16_bits = [](uint64_t v) -> uint32_t {
+      float lo, hi;
+      unpack2(v, lo, hi);
+      return RAW ? f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16) : pack_bf16_pair(lo, hi);
+    };
+    const int r = it + (lane >> 3);
+    const float inv = __shfl_sync(0xffffffffu, inv_mine, r);
+    const uint64_t out = __shfl_sync(0xffffffffu, out_row, r), at = __shfl_sync(0xffffffffu, trow, r);
+    const bool exists = row0 + r < p.rows;
+    uint64_t n[8]; // run c0, then run c1
+    {
+      const uint4 a = tile[warp][r * kRopePitch + c0], b = tile[warp][r * kRopePitch + c1];
+      const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const uint64_t inv2 = pack2(inv, inv);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint32_t word[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t packed = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          packed |= (uint32_t)(max(sat_s8(__fdiv_rn(n[16 * c + 4 * q + e], scale)), -127) & 0xff) << (8 * e);
-        word[q] = packed;
+      for (int i = 0; i < 8; ++i) {
+        const uint64_t scaled = mul2(unpack_bf16_pair(u[i]), inv2);
+        n[i] = V2 ? unpack_bf16_pair(bf16_bits(mul2(unpack_bf16_pair(bf16_bits(scaled)), w[i]))) : mul2(scaled, w[i]);
       }
-      dst[c] = make_uint4(word[0], word[1], word[2], word[3]);
     }
-  }
+    if (rotates) {
+      float a[8], b[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        unpack2(n[i], a[2 * i], a[2 * i + 1]);
+        unpack2(n[4 + i], b[2 * i], b[2 * i + 1]);
+      }
+      if (V2) { // interleaved pairs (2 i, 2 i + 1), one table entry per pair: 8 entries for the two runs
+        float c[8], s[8];
+        load_table8(p.cosv, p.table_f32, at + 4 * c0, c);
+        load_table8(p.sinv, p.table_f32, at + 4 * c0, s);
+        auto rotate = [&](float (&x)[8], int first) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float even = x[2 * e], odd = x[2 * e + 1];
+            x[2 * e] = __fsub_rn(__fmul_rn(even, c[first + e]), __fmul_rn(odd, s[first + e]));
+            x[2 * e + 1] = __fadd_rn(__fmul_rn(even, s[first + e]), __fmul_rn(odd, c[first + e]));
+          }
+        };
+        rotate(a, 0);
+        rotate(b, 4);
+      } else { // half-split pairs (d, d + ROTARY / 2)
+        const uint64_t second = at + 8 * c0 + (p.table_width == (uint32_t)ROTARY ? ROTARY / 2 : 0); // its own entries, or the same
+        float c[8], s[8], first[8];
+        load_table8(p.cosv, p.table_f32, at + 8 * c0, c);
+        load_table8(p.sinv, p.table_f32, at + 8 * c0, s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          first[e] = __fsub_rn(__fmul_rn(a[e], c[e]), __fmul_rn(b[e], s[e]));
+        load_table8(p.cosv, p.table_f32, second, c);
+        load_table8(p.sinv, p.table_f32, second, s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          b[e] = __fadd_rn(__fmul_rn(b[e], c[e]), __fmul_rn(a[e], s[e]));
+          a[e] = first[e];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        n[i] = pack2(a[2 * i], a[2 * i + 1]);
+        n[4 + i] = pack2(b[2 * i], b[2 * i + 1]);
+      }
+    }
+    // the stored bf16 values (what a consumer of the unfused op would read back)
+    uint32_t bits[8], most = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      bits[i] = bf16_bits(n[i]);
+      if (RAW)
+        asm("max.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(bits[i] & 0x7fff7fffu));
+      else
+        asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(bits[i] & 0x7fff7fffu));
+    }
+    float m = fmaxf(__uint_as_float(most << 16), __uint_as_float(most & 0xffff0000u));
+    if (!RAW && __any_sync(0xffffffffu, ((most & 0x7fffu) > 0x7f80u) | ((most >> 16) > 0x7f80u)))
+      return true;
+    if (p.o && exists) {
+      p.o[out * 16 + c0] = make_uint4(bits[0], bits[1], bits[2], bits[3]);
+      p.o[out * 16 + c1] = make_uint4(bits[4], bits[5], bits[6], bits[7]);
+    }
+    if (p.codes) {
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const float scale = row_scale(m, 1.0f); // clip 1: max * 1 / 127
+      uint32_t words[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        n[i] = unpack_bf16_pair(bits[i]);
+      direct_codes(n, scale, words);
+      if (exists) {
+        *reinterpret_cast<uint2 *>(p.codes + out * 128 + 8 * c0) = make_uint2(words[0], words[1]);
+        *reinterpret_cast<uint2 *>(p.codes + out * 128 + 8 * c1) = make_uint2(words[2], words[3]);
+        if (j == 0)
+          p.scales[out] = scale;
+      }
+    }
+    return false;
+  };
+#pragma unroll 1
+  for (int it = 0; it < ROWS; it += 4)
+    if (process(it, std::false_type{}))
+      process(it, std::true_type{});
 }
 
 // ---- QuantizeInt8Rows(Direct) of 128-wide rows, one thread per row (same arithmetic as the
@@ -684,12 +744,20 @@ bool qk_norm_rope_fast(const void *x, const void *w, const void *cosv, const voi
   RowRopeParams p{static_cast<const uint4 *>(x), static_cast<const uint4 *>(w), cosv, sinv, static_cast<uint4 *>(o),
                   codes, scales, tokens * heads, heads, input_seq, table_seq, table_start, l.in_token_stride / 8,
                   l.in_offset / 8, l.out_seq, l.out_start, (uint32_t)table_width, dt_table == 1 ? 1u : 0u, eps};
-  const unsigned blocks = (unsigned)((p.rows + 127) / 128);
-  if (p.rows + 127 > 0x7fffffffull * 128ull)
+  if (p.rows == 0) { // nothing to launch
+    *rc = kOk;
+    return true;
+  }
+  const bool few = p.rows <= (uint64_t)sm_count() * 12 * 32; // less than three warps of 32 rows per scheduler
+  const uint64_t blocks = (p.rows + (few ? 8 : 32) * kRopeWarps - 1) / ((few ? 8 : 32) * kRopeWarps);
+  if (blocks > 0x7fffffffull)
     return false;
 #define DIFB200_ROPE_CASE(R, V)                                                                   \
   if (rotary == R && interleaved_v2 == V) {                                                       \
-    k_qk_norm_rope_row128<R, V><<<blocks, 128, 0, s>>>(p);                                        \
+    if (few)                                                                                      \
+      k_qk_norm_rope_row128<R, V, 8><<<(unsigned)blocks, 32 * kRopeWarps, 0, s>>>(p);             \
+    else                                                                                          \
+      k_qk_norm_rope_row128<R, V, 32><<<(unsigned)blocks, 32 * kRopeWarps, 0, s>>>(p);            \
     *rc = done("k_qk_norm_rope_row128");                                                          \
     return true;                                                                                  \
   }

@@ -72,6 +72,14 @@ __device__ __forceinline__ float absmax2(float m, uint64_t v) {
   return m;
 }
 
+// The same with NaN as the result once one is NaN.
+__device__ __forceinline__ float absmax2_nan(float m, uint64_t v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(lo)), "f"(fabsf(hi)));
+  return m;
+}
+
 // Correctly rounded fp32 quotient a/b from y = RN(1/b): two Markstein refinements.
 __device__ __forceinline__ uint64_t div2_exact(uint64_t a, uint64_t y, uint64_t negb) {
   uint64_t q = mul2(a, y);
@@ -126,6 +134,42 @@ __device__ __forceinline__ float row_scale(float maximum, float clip) {
   if (!(a < 3.0e38f)) // inf and NaN as the plain division treats them
     q = a / 127.0f;
   return fmaxf(q, 1.0e-30f);
+}
+
+// QuantizeInt8Rows(Direct) codes of 2 N neighbouring values |v| <= 127 scale (or not finite), N even: the nearest even
+// integer to the IEEE quotient RN(v / scale), four codes per word. v times RN(1 / scale) is within 8e-6 of the quotient's
+// exact value and RN within 4e-6, so where it lies no nearer than 2e-5 to the middle between two integers, all three
+// round to the same one: three packed operations and a maximum per pair, against a division (ten and more) and two
+// float to integer conversions, which run at a quarter of the rate. Else, or with NaN, the codes are made from the
+// quotient itself (about one warp in fifty).
+template <int N>
+__device__ __forceinline__ void direct_codes(const uint64_t (&v)[N], float scale, uint32_t (&words)[N / 2]) {
+  constexpr float kBias = 12582912.0f; // 1.5 * 2^23: adding it rounds to integers
+  const float recip = __frcp_rn(scale);
+  const uint64_t y2 = pack2(recip, recip), bias2 = pack2(kBias, kBias);
+  float worst = 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const uint64_t a = fma2(v[i], y2, bias2), b = fma2(v[i + 1], y2, bias2);
+    worst = absmax2_nan(worst, fma2(v[i], y2, sub2(bias2, a))); // v y - n
+    worst = absmax2_nan(worst, fma2(v[i + 1], y2, sub2(bias2, b)));
+    words[i >> 1] = __byte_perm(__byte_perm((uint32_t)a, (uint32_t)(a >> 32), 0x0040),
+                                __byte_perm((uint32_t)b, (uint32_t)(b >> 32), 0x0040), 0x5410);
+  }
+  if (!(worst < 0.49998f)) {
+    const uint64_t nb2 = pack2(-scale, -scale);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      float f[4];
+      unpack2(div2_exact(v[i], y2, nb2), f[0], f[1]);
+      unpack2(div2_exact(v[i + 1], y2, nb2), f[2], f[3]);
+      uint32_t c[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        c[e] = (uint32_t)max(sat_s8(f[e]), -127);
+      words[i >> 1] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
+    }
+  }
 }
 
 // ---- shared-memory access through 32-bit shared addresses (cheap address arithmetic) ----
