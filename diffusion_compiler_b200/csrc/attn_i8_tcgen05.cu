@@ -84,6 +84,7 @@ struct AttnParams {
   float2 *ml_state;      // [B,Sq,H] (m, l of the even half of the columns) carried between launches
   float *l2_state;       // [B,Sq,H] l of the other half: a sequence of launches continues the very same sums
   uint32_t carry_in, carry_out;
+  uint32_t behind_whole; // 1: launched behind the items that are not split, whose operands this launch shares
   uint32_t item0, split; // first (batch, head, query block) of this launch; CTAs of a cluster that share its keys
 };
 
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(128)
 key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, float *table,
                  float *tile_bound, uint32_t S, uint32_t KV, uint32_t S_pad, uint32_t begin0, uint32_t count0,
                  uint32_t begin1, uint32_t count1) {
+  grid_dependents_launch(); // (launched plainly)
   const uint32_t tiles = S_pad / kTile;     // tiles of the whole key axis (table layout)
   const uint32_t mine = count0 + count1;    // tiles this launch covers
   const uint32_t local = blockIdx.x % mine;
@@ -172,6 +174,7 @@ struct OperandParams {
 };
 __global__ void __launch_bounds__(256)
 attention_operands_kernel(const OperandParams p) {
+  grid_dependents_launch(); // (launched plainly)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
   // codes of this lane's 16 elements of a row, the row's scale and sum of squared codes (in every lane)
   auto quantise = [&](const uint4 *row, bool valid, uint4 &codes, float &scale) {
@@ -344,15 +347,6 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                  : "memory");
   };
   const uint32_t early = min(n_kv, 2u); // tiles whose loads thread 0 issues during the set-up (0.6 us of a CTA's 6 us around its steps)
-  // What the softmax warps need first is requested before the set-up: the row's scale, the bounds of the keys.
-  float A = 0.0f, kmax = 0.0f;
-  if (warp >= 4) {
-    const uint32_t qr = q0 + (uint32_t)((warp - 4) >> 3) * 128u + (warp & 3) * 32u + lane;
-    A = __ldg(p.qs + ((uint64_t)batch * p.Sq + (qr < p.Sq ? qr : 0u)) * p.H + head);
-    const float *bounds = p.tile_bound + ((uint64_t)batch * p.KV + kvh) * (p.S_pad / kTile);
-    for (uint32_t i = lane; i < n_kv; i += 32)
-      kmax = fmaxf(kmax, __ldg(bounds + key_tile(i)));
-  }
   if (threadIdx.x == 0) {
     ptx::mbar_init(q_full, 8);
     ptx::mbar_init(q_full + 8, 8);
@@ -369,6 +363,19 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
     *abort_ptr = 0;
     ptx::fence_barrier_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_slot, 512);
+    ptx::tmem_relinquish();
+  }
+  // The kernel in front makes the codes and the key table and may run up to here. A split launch behind the unsplit
+  // items is independent of them (they let it start when the operands were complete): it fills the SMs as they become
+  // free, and only its end waits for them.
+  if (!SPLIT || !p.behind_whole)
+    grid_dependency_wait();
+  if (!SPLIT)
+    grid_dependents_launch();
+  if (threadIdx.x == 0) {
     ptx::mbar_expect_tx(q_tma, 2 * kKBytes); // Q codes: staged where the ring is still free
     for (uint32_t t = 0; t < 2; ++t)
       ptx::tma_load_4d(stage_addr + (2u + t) * kStageBytes, &map_q, q_tma, 0, (int32_t)head, (int32_t)(q0 + t * 128u), (int32_t)batch);
@@ -376,13 +383,21 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       load_tile(i, i);
     ptx::prefetch_tensormap(&map_o);
   }
+  // What the softmax warps need first, requested here and used behind the barrier: the row's scale, the bounds of the
+  // first 128 key tiles.
+  const float *bounds = p.tile_bound + ((uint64_t)batch * p.KV + kvh) * (p.S_pad / kTile);
+  float A = 0.0f, near[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (warp >= 4) {
+    const uint32_t qr = q0 + (uint32_t)((warp - 4) >> 3) * 128u + (warp & 3) * 32u + lane;
+    A = load_produced(p.qs + ((uint64_t)batch * p.Sq + (qr < p.Sq ? qr : 0u)) * p.H + head);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (lane + 32u * u < n_kv)
+        near[u] = load_produced(bounds + key_tile(lane + 32u * u));
+  }
   for (uint32_t i = threadIdx.x; i < kConstBytes / 4; i += kThreads)
     *reinterpret_cast<uint32_t *>(base_ptr + (const_addr - base) + i * 4u) = i < 1024u ? 0x44804480u : 0x44404440u;
   ptx::fence_proxy_async();
-  if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, 512);
-    ptx::tmem_relinquish();
-  }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -524,6 +539,9 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // pass (no maximum, no rescaling); otherwise the warp keeps a running maximum.
     bool fixed_max = false;
     {
+      float kmax = fmaxf(fmaxf(near[0], near[1]), fmaxf(near[2], near[3]));
+      for (uint32_t i = lane + 128u; i < n_kv; i += 32u)
+        kmax = fmaxf(kmax, load_produced(bounds + key_tile(i)));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
         kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
@@ -923,16 +941,19 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
+  if (SPLIT && p.behind_whole)
+    grid_dependency_wait();
 }
 
-void split_config(cudaLaunchConfig_t &config, cudaLaunchAttribute &attr, uint32_t split) {
+void split_config(cudaLaunchConfig_t &config, cudaLaunchAttribute (&attrs)[2], uint32_t split) {
   config.blockDim = dim3(kThreads);
   config.dynamicSmemBytes = kSmemBytes;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = split;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  config.attrs = &attr;
-  config.numAttrs = split > 1 ? 1 : 0;
+  attrs[0] = dependent_launch();
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = split;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  config.attrs = attrs;
+  config.numAttrs = split > 1 ? 2 : 1;
 }
 
 // Clusters of `split` CTAs that fit on the device at once (one CTA per SM, clusters inside a GPC).
@@ -940,9 +961,9 @@ int resident_clusters(uint32_t split, int &count) {
   static const char keys[9] = {};
   return current_device_once(&keys[split], [](void *arg, int *value) -> int {
     cudaLaunchConfig_t config{};
-    cudaLaunchAttribute attr{};
+    cudaLaunchAttribute attrs[2]{};
     const uint32_t ctas = *static_cast<uint32_t *>(arg);
-    split_config(config, attr, ctas);
+    split_config(config, attrs, ctas);
     config.gridDim = dim3((unsigned)sm_count() / ctas * ctas); // the grid has to be a multiple of the cluster
     return check_cuda(cudaOccupancyMaxActiveClusters(value, attn_i8_kernel<true>, &config), "cudaOccupancyMaxActiveClusters");
   }, &split, &count);
@@ -952,9 +973,10 @@ int resident_clusters(uint32_t split, int &count) {
 // that is nearly empty costs as much as a full one: 3120 items of the 33272-token block are 21.08 waves of 148 SMs.
 // Its items (or those of the last two waves) are split 2, 3, 4 or 8 ways over the key tiles by clusters. Modelled
 // times in ns, measured on B200: 1380 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
-// and the exchange, at least four tiles per CTA; a split has to give 3 %. H24, without -> with: 1 x 1700 tokens
-// (1.14 waves) 60.2 -> 57.4 us, 2 x 2500 (3.24) 145 -> 141 us, 1 x 6400 (4.05) 381 -> 344 us, 1 x 8000 (5.19) 566 -> 529 us;
-// where the rule takes none, a split costs: 1 x 4608 (2.92) 178 -> 202 us.
+// and the exchange (an upper figure: the second launch fills the SMs as they become free), at least four tiles per CTA; a
+// split has to give 3 %. H24, without -> with: 1 x 1700 tokens (1.14 waves) 60 -> 52 us, 1 x 2304 (1.46) 72 -> 65 us,
+// 2 x 2500 (3.24) 145 -> 135 us, 1 x 3300 (2.11) 133 -> 114 us; where the rule takes none, a split costs: 1 x 2816 (1.78)
+// 83 -> 99 us, 1 x 4608 (2.92) 179 -> 196 us.
 int plan_split(uint64_t items, uint64_t tiles, uint64_t &whole, uint32_t &split) {
   constexpr uint64_t kTileNs = 1380, kItemNs = 6000, kExchangeNs = 8000;
   const uint64_t sms = (uint64_t)sm_count(), item_ns = kItemNs + tiles * kTileNs;
@@ -1160,12 +1182,21 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       return rc;
   auto launch = [&](uint64_t first, uint64_t count, uint32_t ctas) {
     p.item0 = (uint32_t)first;
+    // Clusters of three that start one by one, as SMs become free behind the unsplit items, leave gaps in the GPCs. Where
+    // nearly all SMs are needed the last ones then wait for a second round: 44 clusters (1 x 2048 tokens) take 70 us, and
+    // 64 when all start together; 20 (1 x 1700) 52 and 57, 36 (2 x 2500) 135 and 142.
+    const bool scattered = first != 0 && ctas == 3 && count * ctas > (uint64_t)sm_count() * 3 / 4;
+    p.behind_whole = first != 0 && !scattered ? 1u : 0u;
     p.split = ctas;
     cudaLaunchConfig_t config{};
-    cudaLaunchAttribute attr{};
-    split_config(config, attr, ctas);
+    cudaLaunchAttribute attrs[2]{};
+    split_config(config, attrs, ctas);
     config.gridDim = dim3((unsigned)(count * ctas));
     config.stream = stream;
+    if (scattered) {
+      config.attrs = attrs + 1;
+      config.numAttrs = 1;
+    }
     return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k, map_v,
                                        map_o, p),
                     "attn_i8_kernel launch");

@@ -27,7 +27,7 @@ int w8a8_linear(const void *x_bf16, const int8_t *w, const float *col_scales, co
                                   scales_scratch, nullptr, nullptr, stream))
     return rc;
   return linear_int8_scaled(codes_scratch, w, scales_scratch, col_scales, bias_bf16, epilogue, M, N, K,
-                            out_bf16, nullptr, stream, status_words);
+                            out_bf16, nullptr, stream, status_words, /*weights_ready=*/true);
 }
 
 namespace {

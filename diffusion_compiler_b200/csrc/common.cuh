@@ -77,6 +77,31 @@ int poll_device_status(const char *what); // copies back, clears, maps to kExecu
 
 #ifdef __CUDACC__
 
+// ---- programmatic dependent launch ----
+// A kernel launched with dependent_launch() may start while the one in front of it on the stream still runs: as soon as
+// all CTAs of that one have called grid_dependents_launch() (or ended) and there is room. Its set-up runs then; what
+// the kernel in front wrote is read behind grid_dependency_wait(), which every thread passes that touches global
+// memory, and through loads that the compiler cannot move up (load_produced or TMA). A kernel that lets dependents
+// start and is itself launched so waits first: when a kernel starts, the one two in front is complete.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ float load_produced(const float *p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_produced(const uint16_t *p) {
+  uint16_t v;
+  asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+inline cudaLaunchAttribute dependent_launch() {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  return attr;
+}
+
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t bits16) {
   return __uint_as_float(bits16 << 16);
 }

@@ -56,6 +56,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   static_assert(EXTRA != kNorm || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
+  grid_dependents_launch(); // (launched plainly)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = warp / warps_per_row;         // which row of this CTA's batch
   const int wrow = warp - slot * warps_per_row;  // warp index inside the row

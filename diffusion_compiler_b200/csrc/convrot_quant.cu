@@ -23,6 +23,7 @@ template <bool F32, bool RESIDUAL, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : (MAXT == 384 ? 2 : 1))
 convrot4096_kernel(const QuantParams p) {
   extern __shared__ __align__(128) uint32_t smem[];
+  grid_dependents_launch(); // (launched plainly)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = lane >> 4, a = lane & 15;
   const int warps = blockDim.x >> 5;
@@ -274,6 +275,7 @@ __device__ __forceinline__ float load_logical(const QuantParams &p, uint64_t row
 template <bool VEC8>
 __global__ void __launch_bounds__(256)
 direct_quant_kernel(const QuantParams p) {
+  grid_dependents_launch(); // (launched plainly)
   const int lane = threadIdx.x & 31;
   const uint64_t warp_global = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t warp_count = (uint64_t)gridDim.x * (blockDim.x >> 5);

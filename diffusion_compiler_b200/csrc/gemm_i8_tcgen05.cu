@@ -121,6 +121,7 @@ struct GemmParams {
   uint32_t epilogue;
   uint32_t split;   // CTAS = 1: CTAs of a cluster that share one tile's k-blocks (1 = no cluster)
   uint32_t tma_store; // 1: outputs leave through TMA stores (needs N % 8 == 0, aligned out)
+  uint32_t weights_first; // 1: w is not written by the kernel in front, its first blocks are requested before that one is done
   uint32_t withhold_kb; // test aid: the loads of this k-block are never issued (0xffffffff = none)
   unsigned long long wait_ns; // limit of every bounded wait
   DeviceStatus *status;
@@ -232,12 +233,40 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       *abort_ptr = 1;
     }
   };
+  // The kernel in front (the quantiser, as a rule) may still run up to here.
+  if (warp != 0)
+    grid_dependency_wait();
   if (warp == 0) {
+    // A pair counts the bytes of both CTAs on the leader's barrier: the leader expects
+    // them all, the peer's loads complete their bytes there (cta_group::2 form of the
+    // load) and the peer itself never arrives.
+    auto expect = [&](uint32_t bar) {
+      if (cta_rank == 0)
+        ptx::mbar_expect_tx(bar, CTAS * kStageBytes);
+    };
+    auto load = [&](const CUtensorMap *map, uint32_t dst, uint32_t bar, uint32_t kb, int32_t first) {
+      const int32_t k0 = (int32_t)(kb * kBK);
+      if (CTAS == 2 && cta_rank != 0)
+        ptx::tma_load_2d_pair(dst, map, ptx::mapa(bar, 0), k0, first);
+      else
+        ptx::tma_load_2d(dst, map, bar, k0, first);
+    };
+    auto rows_of = [&](uint32_t tile) { return (int32_t)((tile / tiles_n) * kTileM + cta_rank * kBM); };
+    auto columns_of = [&](uint32_t tile) { return (int32_t)((tile % tiles_n) * BN + cta_rank * Cfg<CTAS, BN>::kBRows); };
+    // k-blocks of the first tile whose weights are requested at once
+    const uint32_t early = p.weights_first && unit < num_tiles ? min(kb_end - kb_first, (uint32_t)kStages) : 0u;
+    if (early != 0u && ptx::elect_one())
+      for (uint32_t i = 0; i < early; ++i) {
+        expect(full_bar + 8 * i);
+        load(&map_b, smem_base + i * kStageBytes + kABytes, full_bar + 8 * i, kb_first + i, columns_of(unit));
+      }
+    grid_dependency_wait();
+    grid_dependents_launch();
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (uint32_t tile = unit; tile < num_tiles && ok; tile += units) {
-      const int32_t m0 = (int32_t)((tile / tiles_n) * kTileM + cta_rank * kBM);
-      const int32_t n0 = (int32_t)((tile % tiles_n) * BN + cta_rank * Cfg<CTAS, BN>::kBRows);
+      const int32_t m0 = rows_of(tile), n0 = columns_of(tile);
+      const uint32_t ahead = tile == unit ? kb_first + early : kb_first;
       for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
         if (!ptx::mbar_wait_warp(empty_bar + 8 * stage, phase ^ 1u, abort_ptr, wait_ns)) {
           give_up(0, kb);
@@ -246,31 +275,17 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         const uint32_t a_dst = smem_base + stage * kStageBytes, b_dst = a_dst + kABytes;
         const uint32_t bar = full_bar + 8 * stage;
-        const int32_t k0 = (int32_t)(kb * kBK);
         if (kb == p.withhold_kb) {
           // test aid: the bytes are announced but never loaded, so the consumer's wait on this
           // stage runs out and the kernel leaves through its give-up path
           if (cta_rank == 0 && ptx::elect_one())
             ptx::mbar_expect_tx(bar, CTAS * kStageBytes);
         } else if (ptx::elect_one()) {
-          if (CTAS == 2) {
-            // A pair counts the bytes of both CTAs on the leader's barrier: the leader expects
-            // them all, the peer's loads complete their bytes there (cta_group::2 form of the
-            // load) and the peer itself never arrives.
-            if (cta_rank == 0) {
-              ptx::mbar_expect_tx(bar, 2 * kStageBytes);
-              ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
-              ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
-            } else {
-              const uint32_t leader_bar = ptx::mapa(bar, 0);
-              ptx::tma_load_2d_pair(a_dst, &map_a, leader_bar, k0, m0);
-              ptx::tma_load_2d_pair(b_dst, &map_b, leader_bar, k0, n0);
-            }
-          } else {
-            ptx::mbar_expect_tx(bar, kStageBytes);
-            ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
-            ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
-          }
+          if (kb >= ahead)
+            expect(bar);
+          load(&map_a, a_dst, bar, kb, m0);
+          if (kb >= ahead)
+            load(&map_b, b_dst, bar, kb, n0);
         }
         if (++stage == kStages) {
           stage = 0;
@@ -349,8 +364,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
       for (int i = 0; i < BN / 64; ++i) {
         const uint32_t c = lane + 32u * i, n = n0 + col_half * (BN / 2) + c;
-        cs[c] = n < p.N ? __ldg(p.col_scales + n) : 0.0f;
-        bs[c] = ((p.epilogue & kEpiBias) && n < p.N) ? bf16_bits_to_f32(__ldg(p.bias + n)) : 0.0f;
+        cs[c] = n < p.N ? load_produced(p.col_scales + n) : 0.0f;
+        bs[c] = ((p.epilogue & kEpiBias) && n < p.N) ? bf16_bits_to_f32(load_produced(p.bias + n)) : 0.0f;
       }
       __syncwarp();
       const bool complete = ptx::mbar_wait_warp(tfull_bar + 8 * acc, acc_phase, abort_ptr, wait_ns);
@@ -385,7 +400,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       ptx::tc_fence_after();
       const uint32_t row = m0 + quarter * 32u + lane;
       const bool row_ok = row < p.M;
-      const float rs = row_ok ? __ldg(p.row_scales + row) : 0.0f;
+      const float rs = row_ok ? load_produced(p.row_scales + row) : 0.0f;
 #pragma unroll 1
       for (uint32_t sub = 0; sub < BN / 64; ++sub) {
         const uint32_t chunk = col_half * (BN / 64) + sub; // 32-column chunk of the tile
@@ -578,16 +593,14 @@ int launch_form(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtens
   config.blockDim = dim3(kThreads);
   config.dynamicSmemBytes = smem_bytes<CTAS, BN>();
   config.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = CTAS == 2 ? 2u : p.split;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
+  cudaLaunchAttribute attrs[2]{dependent_launch(), {}};
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = CTAS == 2 ? 2u : p.split;
+  attrs[1].val.clusterDim.y = 1;
+  attrs[1].val.clusterDim.z = 1;
   uint64_t units = (uint64_t)sm_count();
-  if (CTAS == 2 || p.split > 1) {
-    config.attrs = &attr;
-    config.numAttrs = 1;
-  }
+  config.attrs = attrs;
+  config.numAttrs = CTAS == 2 || p.split > 1 ? 2 : 1;
   if (CTAS == 2) {
     // The kernel is persistent: launch exactly as many CTA pairs as can be resident at once
     // (SM pairs are formed inside a GPC, so this can be fewer than SMs / 2); a per-device figure.
@@ -622,7 +635,7 @@ int launch_form(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtens
 int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales,
                        const float *col_scales, const void *bias_bf16, uint32_t epilogue, uint64_t M,
                        uint64_t N, uint64_t K, void *out_bf16, int32_t *acc_out, cudaStream_t stream,
-                       DeviceStatus *status_words) {
+                       DeviceStatus *status_words, bool weights_ready) {
   if (!x || !w || !row_scales || !col_scales || !out_bf16)
     return fail(kInvalidArgument, "LinearInt8Scaled: null pointer");
   if ((epilogue & kEpiBias) && !bias_bf16)
@@ -677,6 +690,7 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   p.split = (uint32_t)form.split;
   p.tma_store = tma_store ? 1u : 0u;
   p.withhold_kb = take_withheld_gemm_load();
+  p.weights_first = weights_ready && p.withhold_kb == 0xffffffffu ? 1u : 0u;
   p.wait_ns = wait_limit_ns();
   p.status = status;
   if (form.ctas == 2)

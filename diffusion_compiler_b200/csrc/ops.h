@@ -31,7 +31,9 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
 int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales,
                        const float *col_scales, const void *bias_bf16, uint32_t epilogue, uint64_t M,
                        uint64_t N, uint64_t K, void *out_bf16, int32_t *acc_out, cudaStream_t stream,
-                       DeviceStatus *status_words = nullptr);
+                       DeviceStatus *status_words = nullptr, bool weights_ready = false);
+// weights_ready: the kernel launched last on the stream does not write w, and was launched plainly or waits for the
+// one before it: the first blocks of w are requested while that kernel still runs.
 
 // QuantizeInt8Rows -> LinearInt8Scaled [-> BiasAdd -> Gelu] on a bf16 [M,K] input; codes [M,K]
 // and row scales [M] are scratch supplied by the caller.
