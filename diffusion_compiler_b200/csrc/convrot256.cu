@@ -24,8 +24,8 @@
 // variants keep the values as packed bf16 (their result is defined on the rounded values), half the
 // registers of fp32. The one-block form instead fits 64 registers, so that 32 warps per SM hide the
 // load latency without a prefetch. 33272 x 3072 takes 87 us (3.5 TB/s), 33272 x 8192 226 us, 9216 x 3072 29 us, the
-// scale search of the weight form 12288 x 3072 78 us (all lanes evaluate samples, doubles only where the square needs
-// them), with input equalisation 109 us, RmsNormModulate in front of 33272 x 3072 145 us with its statistic. Staging
+// scale search of the weight form 12288 x 3072 69 us (all lanes evaluate samples, in doubles only where candidates
+// are close), with input equalisation 99 us, RmsNormModulate in front of 33272 x 3072 145 us with its statistic. Staging
 // the input with bulk copies through shared memory instead of registers gave nothing (30.0 us for the third shape).
 #include "quant_common.cuh"
 
@@ -36,7 +36,8 @@ namespace {
 // code bytes and the sampled elements of the scale search.
 constexpr int kWarpBytes = 4096;
 
-enum Extra { kPlain = 0, kPack = 1, kNorm = 2 };
+// kPack: weight rows with the scale search (and input equalisation where given), kEqualise: without the search.
+enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3 };
 
 // 32 bytes of one thread: one 256-bit load where every run starts on 32 bytes, else two of 128 bits.
 __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, uint4 &b) {
@@ -57,6 +58,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
   grid_dependents_launch(); // (launched plainly)
+  constexpr bool kWeights = EXTRA == kPack || EXTRA == kEqualise;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = warp / warps_per_row;         // which row of this CTA's batch
   const int wrow = warp - slot * warps_per_row;  // warp index inside the row
@@ -103,7 +105,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   }
   // Weight packing: may the fast quotient be used for every entry of this thread's columns?
   bool equalise_fast = true;
-  if (EXTRA == kPack && p.equalise) {
+  if (kWeights && p.equalise) {
 #pragma unroll
     for (int q = 0; q < 2 * NIT; ++q) {
       const uint32_t c = col0 + (uint32_t)(q >> 1) * 1024u + (uint32_t)(q & 1) * 256u;
@@ -289,7 +291,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             P[2 * i] = pack2(__uint_as_float(wa[i] << 16), __uint_as_float(wb[i] << 16));
             P[2 * i + 1] = pack2(__uint_as_float(wa[i] & 0xffff0000u), __uint_as_float(wb[i] & 0xffff0000u));
           }
-          if (EXTRA == kPack && p.equalise) {
+          if (kWeights && p.equalise) {
             // weight rows with input equalisation: w / e in fp32 before anything else (reference
             // tools/difflux2sample.cpp:3005-3014; the sign flip commutes with the division).
             // One Markstein step from the approximate reciprocal: the quotient of two 8-bit
@@ -399,59 +401,123 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       }
       __syncwarp();
       float candidate[7], reciprocal[7];
-      double e[7];
 #pragma unroll
       for (int f = 0; f < 7; ++f) {
         candidate[f] = round_bf16(row_scale(maximum, factors[f])) * kCarry;
         reciprocal[f] = __frcp_rn(candidate[f]);
-        e[f] = 0.0;
       }
-#pragma unroll 1
-      for (int i = lane; i < 8 * samples; i += 32) {
-        uint32_t pair;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(pair) : "r"(warp_addr + 4u * i) : "memory");
-        const float v0 = __uint_as_float(pair << 16), v1 = __uint_as_float(pair & 0xffff0000u);
-#pragma unroll
-        for (int f = 0; f < 7; ++f) {
-          const uint32_t q = pack_bf16_pair(__fmul_rn(v0, reciprocal[f]), __fmul_rn(v1, reciprocal[f]));
-          // nearest-even integer by the magic constant 1.5 * 2^23 (|q| < 2^9)
-          const float n0 = __fadd_rn(fminf(fmaxf(__uint_as_float(q << 16), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
-          const float n1 =
-              __fadd_rn(fminf(fmaxf(__uint_as_float(q & 0xffff0000u), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
-          const double d0 = (double)__fmaf_rn(-n0, candidate[f], v0), d1 = (double)__fmaf_rn(-n1, candidate[f], v1);
-          e[f] = fma(d0, d0, e[f]); // the square is exact in double: one rounding, as multiply then add
-          e[f] = fma(d1, d1, e[f]);
-        }
-      }
+      // sums of the row's warps: doubles, then floats in an area of their own (rows of a CTA are not in step)
       double *errors = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(smem) +
                                                   (size_t)total_warps * (kWarpBytes + 16) + 64 +
                                                   (SIGNED ? (size_t)total_warps * 32 * 64 * NIT : 0));
+      float *sums = reinterpret_cast<float *>(errors + 7 * total_warps);
+      auto sample = [&](int i) {
+        uint32_t pair;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(pair) : "r"(warp_addr + 4u * i) : "memory");
+        return pair;
+      };
+      // First in fp32: the value minus code times candidate is exact, and the at most 48 additions of squares leave a
+      // sum within 3e-6 of the exact one. Where one candidate is better than the others by 1e-4 it is the answer;
+      // else, and where the sums left the range of fp32, the doubles decide. (Doubles for every row -> this:
+      // 12288 x 3072 78 -> 69 us, with input equalisation 110 -> 99 us.) Both barriers are passed on either way.
+      float chosen = candidate[0];
+      bool decided;
+      {
+        float e[7] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+        for (int i = lane; i < 8 * samples; i += 32) {
+          const uint64_t v2 = unpack_bf16_pair(sample(i));
+          float v0, v1;
+          unpack2(v2, v0, v1);
 #pragma unroll
-      for (int f = 0; f < 7; ++f) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-          e[f] = __dadd_rn(e[f], __shfl_xor_sync(0xffffffffu, e[f], o));
-        if (warps_per_row > 1 && lane == 0)
-          errors[f * total_warps + warp] = e[f];
-      }
-      if (warps_per_row > 1) {
-        row_barrier();
+          for (int f = 0; f < 7; ++f) {
+            uint32_t t0, t1;
+            code_words(pack_bf16_pair(mul2(v2, pack2(reciprocal[f], reciprocal[f]))), t0, t1);
+            const float d0 = __fmaf_rn(kCodeBias - __uint_as_float(t0), candidate[f], v0);
+            const float d1 = __fmaf_rn(kCodeBias - __uint_as_float(t1), candidate[f], v1);
+            e[f] = __fmaf_rn(d0, d0, e[f]);
+            e[f] = __fmaf_rn(d1, d1, e[f]);
+          }
+        }
 #pragma unroll
         for (int f = 0; f < 7; ++f) {
-          e[f] = 0.0;
-          for (int w = 0; w < warps_per_row; ++w)
-            e[f] = __dadd_rn(e[f], errors[f * total_warps + slot * warps_per_row + w]);
-        }
-        row_barrier(); // the error slots are reused by the next row
-      }
-      double best = e[0];
-      float chosen = candidate[0];
 #pragma unroll
-      for (int f = 1; f < 7; ++f)
-        if (e[f] < best) {
-          best = e[f];
-          chosen = candidate[f];
+          for (int o = 16; o > 0; o >>= 1)
+            e[f] += __shfl_xor_sync(0xffffffffu, e[f], o);
+          if (warps_per_row > 1 && lane == 0)
+            sums[f * total_warps + warp] = e[f];
         }
+        if (warps_per_row > 1) {
+          row_barrier();
+#pragma unroll
+          for (int f = 0; f < 7; ++f) {
+            e[f] = 0.0f;
+            for (int w = 0; w < warps_per_row; ++w)
+              e[f] += sums[f * total_warps + slot * warps_per_row + w];
+          }
+        }
+        float best = e[0], worst = e[0];
+#pragma unroll
+        for (int f = 1; f < 7; ++f) {
+          best = fminf(best, e[f]);
+          asm("max.NaN.f32 %0, %0, %1;" : "+f"(worst) : "f"(e[f]));
+        }
+        int close = 0;
+#pragma unroll
+        for (int f = 6; f >= 0; --f)
+          if (e[f] <= best * 1.0001f) {
+            ++close;
+            chosen = candidate[f];
+          }
+        decided = close == 1 && best > 1.0e-30f && worst < INFINITY; // the same for every thread of the row
+      }
+      double e[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      if (!decided) {
+#pragma unroll 1
+        for (int i = lane; i < 8 * samples; i += 32) {
+          const uint32_t pair = sample(i);
+          const float v0 = __uint_as_float(pair << 16), v1 = __uint_as_float(pair & 0xffff0000u);
+#pragma unroll
+          for (int f = 0; f < 7; ++f) {
+            const uint32_t q = pack_bf16_pair(__fmul_rn(v0, reciprocal[f]), __fmul_rn(v1, reciprocal[f]));
+            // nearest-even integer by the magic constant 1.5 * 2^23 (|q| < 2^9)
+            const float n0 = __fadd_rn(fminf(fmaxf(__uint_as_float(q << 16), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
+            const float n1 =
+                __fadd_rn(fminf(fmaxf(__uint_as_float(q & 0xffff0000u), -128.0f), 127.0f), 12582912.0f) - 12582912.0f;
+            const double d0 = (double)__fmaf_rn(-n0, candidate[f], v0), d1 = (double)__fmaf_rn(-n1, candidate[f], v1);
+            e[f] = fma(d0, d0, e[f]); // the square is exact in double: one rounding, as multiply then add
+            e[f] = fma(d1, d1, e[f]);
+          }
+        }
+#pragma unroll
+        for (int f = 0; f < 7; ++f) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+            e[f] = __dadd_rn(e[f], __shfl_xor_sync(0xffffffffu, e[f], o));
+          if (warps_per_row > 1 && lane == 0)
+            errors[f * total_warps + warp] = e[f];
+        }
+      }
+      if (warps_per_row > 1)
+        row_barrier(); // (also: every warp has read the sums; the barriers of the next row keep the errors until they are read)
+      if (!decided) {
+        if (warps_per_row > 1) {
+#pragma unroll
+          for (int f = 0; f < 7; ++f) {
+            e[f] = 0.0;
+            for (int w = 0; w < warps_per_row; ++w)
+              e[f] = __dadd_rn(e[f], errors[f * total_warps + slot * warps_per_row + w]);
+          }
+        }
+        double best = e[0];
+        chosen = candidate[0];
+#pragma unroll
+        for (int f = 1; f < 7; ++f)
+          if (e[f] < best) {
+            best = e[f];
+            chosen = candidate[f];
+          }
+      }
       scale = maximum == 0.0f ? 1.0e-30f : chosen * (1.0f / kCarry);
       __syncwarp(); // the samples are read before the codes overwrite them
     }
@@ -567,7 +633,7 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   const int warps = warps_per_row * rows_per_cta, threads = warps * 32;
   // per warp: transpose / staging area; row maxima; for the signed variants 16 XOR masks per thread and block
   const size_t smem = (size_t)warps * kWarpBytes + (size_t)warps * 4 * sizeof(float) + 64 +
-                      (SIGNED ? (size_t)warps * 32 * 64 * NIT : 0) + (EXTRA == kPack ? (size_t)warps * 7 * sizeof(double) : 0);
+                      (SIGNED ? (size_t)warps * 32 * 64 * NIT : 0) + (EXTRA == kPack ? (size_t)warps * 7 * (sizeof(double) + sizeof(float)) : 0);
   auto kernel = convrot256_kernel<SIGNED, F32, RESIDUAL, EXTRA, NIT, PREFETCH, MAXT, MINB>;
   int resident = 1;
   if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), threads, smem, &resident))
@@ -623,9 +689,9 @@ template <bool SIGNED, bool F32>
 int launch_equalised(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
   if (blocks > 12u)
-    return launch_single<SIGNED, F32, false, kPack>(p, stream);
-  return blocks <= 8u ? launch_form<SIGNED, F32, false, kPack, 1, false, 256, 3>(p, stream)
-                      : launch_form<SIGNED, F32, false, kPack, 1, false, 384, 2>(p, stream);
+    return launch_single<SIGNED, F32, false, kEqualise>(p, stream);
+  return blocks <= 8u ? launch_form<SIGNED, F32, false, kEqualise, 1, false, 256, 3>(p, stream)
+                      : launch_form<SIGNED, F32, false, kEqualise, 1, false, 384, 2>(p, stream);
 }
 
 template <bool SIGNED>

@@ -123,6 +123,20 @@ __device__ __forceinline__ void codes_of(uint32_t q, int &c0, int &c1) {
   c1 = sat_s8(__uint_as_float(q & 0xffff0000u));
 }
 
+// INT8 codes of a pair of bf16 quotients that are not NaN as (the bits of) two floats kCodeBias + code: clamped to
+// [-128, 127], then rounded to the nearest even integer by the addition of 1.5 * 2^23.
+constexpr float kCodeBias = 12582912.0f;
+__device__ __forceinline__ void code_words(uint32_t q, uint32_t &c0, uint32_t &c1) {
+  float f0, f1;
+  asm("max.bf16x2 %0, %0, %1;" : "+r"(q) : "r"(0xc300c300u));
+  asm("min.bf16x2 %0, %0, %1;" : "+r"(q) : "r"(0x42fe42feu));
+  asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\nadd.rn.f32.bf16 %0, lo, %3;\nadd.rn.f32.bf16 %1, hi, %3;\n}"
+      : "=f"(f0), "=f"(f1)
+      : "r"(q), "f"(kCodeBias));
+  c0 = __float_as_uint(f0);
+  c1 = __float_as_uint(f1);
+}
+
 // max * clip / 127 as the reference rounds it (IEEE product, IEEE quotient, then the guard): one
 // Markstein step from RN(1/127) gives the correctly rounded quotient for every fp32 mantissa
 // (checked exhaustively), and below 2^-90, where the residual could underflow, the guard decides.
@@ -144,9 +158,8 @@ __device__ __forceinline__ float row_scale(float maximum, float clip) {
 // quotient itself (about one warp in fifty).
 template <int N>
 __device__ __forceinline__ void direct_codes(const uint64_t (&v)[N], float scale, uint32_t (&words)[N / 2]) {
-  constexpr float kBias = 12582912.0f; // 1.5 * 2^23: adding it rounds to integers
   const float recip = __frcp_rn(scale);
-  const uint64_t y2 = pack2(recip, recip), bias2 = pack2(kBias, kBias);
+  const uint64_t y2 = pack2(recip, recip), bias2 = pack2(kCodeBias, kCodeBias);
   float worst = 0.0f;
 #pragma unroll
   for (int i = 0; i < N; i += 2) {

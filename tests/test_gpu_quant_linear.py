@@ -217,6 +217,33 @@ def test_w8a8_linear_single_call_matches_two_calls(ops):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("impl", [2, 3, 5, 6])
+@pytest.mark.parametrize("K", [256, 1024, 3072, 12288])  # rows of one warp and of several, one and three blocks per warp
+def test_weight_scale_search_where_its_fp32_sums_do_not_decide(ops, impl, K):
+    """The search compares fp32 sums first; rows in which candidates tie (constant magnitudes, one non-zero weight, zeros)
+    or whose squares leave the range of fp32 (1e-18, 1e18) are decided in doubles. Such rows between ordinary ones,
+    twice (rows of a CTA are not in step), bit for bit against the CPU restatement."""
+    import torch
+    rng = np.random.default_rng(impl + K)
+    N = 1400
+    w = (rng.standard_normal((N, K)) * 0.02).astype(np.float32)
+    w[0::7] = np.where(rng.random((len(w[0::7]), K)) < 0.5, -0.5, 0.5)
+    w[1::7] = 0
+    w[1::14, 3] = 1
+    w[2::7] *= 1e-18
+    w[3::7] *= 1e18
+    w[4::14] = 0.25
+    w = ob.f32_to_bf16(w)
+    want_codes, want_scales = ob.orc().quantize_weight_rows(w, impl, mse=True)
+    dw = torch.from_numpy(w.view(np.int16)).cuda().view(torch.bfloat16)
+    for _ in range(2):
+        codes, scales = ops.quantize_weight_rows(dw, impl, mse_scale=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(scales.cpu().numpy().view(np.uint32), want_scales.view(np.uint32))
+        assert np.array_equal(codes.cpu().numpy(), want_codes)
+    ops.poll_status()
+
+
 def test_weight_rows_equal_the_reference_packers_own_files(ops):
     """The GPU weight quantiser against whole runs of the reference's own offline packer
     (rewrite_named_linear_w8a8 of reference tools/difflux2sample.cpp; its cache tensors are the
