@@ -20,8 +20,9 @@
 //                                                    ceil(A * |q8_i| * max_j(|k8_j| * ks'_j)) when
 //                                                    that is at most 60 (one pass, no running
 //                                                    maximum, no rescaling of the output), else a
-//                                                    running maximum
-//   p_j   = exp2(fma(u_j, A, -m)),  P_j = bf16(p_j)
+//                                                    running maximum, which moves to 24 above the
+//                                                    scores where they exceed it
+//   p_j   = exp2(fma(u_j, A, -m)),  P_j = bf16(p_j)   (never above 1)
 //   out   = bf16((sum_j P_j * v_j) / (sum_j p_j))   fp32 accumulation; all keys masked -> 0
 // q8/qs and k8/ks are QuantizeInt8Rows(Direct) of the [B,S,H,128] / [B,S,KV,128] tensors.
 //
@@ -65,6 +66,8 @@ constexpr int kThreads = 640;      // 4 control warps, 2 x 8 softmax warps
 constexpr uint32_t kPartialBytes = 32 * 32 * 4; // split form: a [32 rows x 32 columns] fp32 partial output
 constexpr uint32_t kOutBoxBytes = 32 * 128;    // a warp's output staging: two [32 rows x 64 bf16] boxes
 constexpr uint32_t kConstBytes = 6144;         // bf16 [128 x 16] of 1024 and [64 x 16] of 768: 16 products = 1.5 * 2^23
+constexpr float kHeadroom = 24.0f;  // powers of two that the running maximum goes beyond a row's scores when it moves
+constexpr float kLeastSum = 1.0f / (1u << 25); // of a running maximum: its largest p is above 2^-(kHeadroom + 1)
 constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
 constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + kConstBytes + 256 + kPairBytes;
 
@@ -704,10 +707,13 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         float m_new = m_run;
         if (mx != -INFINITY)
           m_new = ceilf(mx * A);
-        // It may lag behind the scores by 16, which makes a P at most 2^16: most warps had a row with a larger ceiling in
-        // most steps, and each moved 128 output columns (B2 S4608 H24 with 8 times larger scores: 674 us, with a lag of 8
-        // 600, 24 538). m_run = -inf: the first valid key sets it.
-        m_new = m_new > m_run + 16.0f ? m_new : m_run;
+        // Where it moves it goes kHeadroom beyond the ceiling, so that most steps move nothing (a move scales 128 output
+        // columns, and without a headroom most warps had a row that moved in most steps) and no P exceeds 1: an output sum
+        // stays within l max |V|. B2 S4608 H24 with q 4, 8 and 30 times larger: 704, 716 and 725 us without one, 586, 630 and 682
+        // with 8, 566, 588 and 656 with 16, 566, 565 and 639 with 24, 566, 565 and 628 with 32. The rounding of the exponent's
+        // fma (2^-20) does not show in the error against 64 bits; products below 2^-149 are lost, which for |V| above
+        // 2^-115 is less than the rounding of the output (a maximum fixed at its bound may lie 60 above the scores).
+        m_new = m_new > m_run ? m_new + kHeadroom : m_run;
         const bool grow = m_new > m_run && m_run != -INFINITY;
         if (__any_sync(0xffffffffu, grow)) {
           // rescale O (and l) by an exact power of two; needs P.V of the previous step finished
@@ -771,15 +777,16 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       l += exchange(l);
     const uint32_t done_bar = s_full + 8 * t, done_parity = (n_steps + 1u) & 1u;
     // A row that other keys still join, in this cluster or in a later launch, is handed on as what its own keys
-    // gave: no valid key counts as no maximum at all, and an m fixed at a bound far above the scores (l small)
-    // comes down by the power of two that brings l to [1/2, 1). So every joined l is at least 1/2, and what a factor
-    // flushes (2^-127 and less) is too small to reach the sum. Gives the power of two.
+    // gave: no valid key counts as no maximum at all, and an m fixed at a bound so far above the scores that l is
+    // smaller than a running maximum leaves it (2^-25 at least, which stays as it is: the next launch continues the
+    // very same sums) comes down by the power of two that brings l to [1/2, 1). So every joined l is at least 2^-25, and
+    // what a factor flushes (2^-127 and less) is too small to reach the sum. Gives the power of two.
     auto hand_on = [&](float &m_out) {
       float up = 1.0f;
       m_out = m_run;
       if (l == 0.0f) {
         m_out = -INFINITY;
-      } else if (l < 0.5f) {
+      } else if (l < kLeastSum) {
         const int e = (int)(__float_as_uint(l) >> 23) - 126;
         m_out = m_run + (float)e;
         up = __uint_as_float((uint32_t)(127 - e) << 23);

@@ -327,3 +327,31 @@ def test_attention_ring_and_query_tiles(ops, Sq, tiles, q_gain):
     ops.poll_status()
     assert torch.equal(first.view(torch.int16), again.view(torch.int16))
     assert rel_l2(ob.bf16_to_f32(from_torch_bf16(first)), want) <= 2e-3
+
+
+@pytest.mark.parametrize("exponent", [122, 100, -100])
+@pytest.mark.parametrize("form", ["plain", "split", "chunked"])
+def test_attention_running_maximum_with_large_and_small_values(ops, exponent, form):
+    """No softmax weight is above 1, so values near the end of bf16's range stay finite where the maximum runs: V in
+    [2^e, 2^(e+1)) under scores that rise by hundreds of powers of two along the keys, against the oracle on the same
+    values without the power of two (rel-L2 2e-3, the bar of the path; the outputs themselves scale exactly)."""
+    import torch
+    rng = np.random.default_rng(31)
+    Sq, Sk, H, KV = (130, 2048, 6, 2) if form == "split" else (130, 700, 4, 2)
+    q = ob.f32_to_bf16(rng.standard_normal((1, Sq, H, 128)).astype(np.float32) * 8)
+    k = rng.standard_normal((1, Sk, KV, 128)).astype(np.float32) * np.linspace(0.2, 3.0, Sk, dtype=np.float32)[:, None, None]
+    v = ob.f32_to_bf16((1 + rng.random((1, Sk, KV, 128))).astype(np.float32))
+    q8, qs = ob.orc().quantize_int8_rows([q.reshape(-1, 128)], 1)
+    k8, ks = ob.orc().quantize_int8_rows([ob.f32_to_bf16(k).reshape(-1, 128)], 1)
+    q8, k8 = q8.reshape(1, Sq, H, 128), k8.reshape(1, Sk, KV, 128)
+    want = ob.bf16_to_f32(ob.orc().attention_int8_rows(q8, qs, k8, ks, v, np.ones((1, Sk), np.uint8)))
+    scaled = ob.f32_to_bf16(ob.bf16_to_f32(v) * np.float32(2.0 ** exponent))
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    args = (t(q8), t(qs), t(k8), t(ks), to_torch_bf16(scaled))
+    tiles = (Sk + 127) // 128
+    got = ops.attention_int8_chunked(*args, [[(0, 2)], [(2, tiles - 2)]]) if form == "chunked" else ops.attention_int8(*args)
+    torch.cuda.synchronize()
+    ops.poll_status()
+    got = ob.bf16_to_f32(from_torch_bf16(got)).astype(np.float64)
+    assert np.isfinite(got).all()
+    assert rel_l2(got * 2.0 ** -exponent, want) <= 2e-3
