@@ -237,37 +237,38 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp != 0)
     grid_dependency_wait();
   if (warp == 0) {
-    // A pair counts the bytes of both CTAs on the leader's barrier: the leader expects
-    // them all, the peer's loads complete their bytes there (cta_group::2 form of the
-    // load) and the peer itself never arrives.
-    auto expect = [&](uint32_t bar) {
-      if (cta_rank == 0)
-        ptx::mbar_expect_tx(bar, CTAS * kStageBytes);
-    };
-    auto load = [&](const CUtensorMap *map, uint32_t dst, uint32_t bar, uint32_t kb, int32_t first) {
-      const int32_t k0 = (int32_t)(kb * kBK);
-      if (CTAS == 2 && cta_rank != 0)
-        ptx::tma_load_2d_pair(dst, map, ptx::mapa(bar, 0), k0, first);
-      else
-        ptx::tma_load_2d(dst, map, bar, k0, first);
-    };
     auto rows_of = [&](uint32_t tile) { return (int32_t)((tile / tiles_n) * kTileM + cta_rank * kBM); };
     auto columns_of = [&](uint32_t tile) { return (int32_t)((tile % tiles_n) * BN + cta_rank * Cfg<CTAS, BN>::kBRows); };
-    // k-blocks of the first tile whose weights are requested at once
+    // One operand's part of k-block kb. A pair counts the bytes of both CTAs on the leader's barrier: the leader
+    // expects them all, the peer's loads complete their bytes there (cta_group::2 form of the load) and the peer
+    // itself never arrives.
+    auto load = [&](const CUtensorMap *map, uint32_t dst, uint32_t bar, uint32_t kb, int32_t first) {
+      if (CTAS == 2 && cta_rank != 0)
+        ptx::tma_load_2d_pair(dst, map, ptx::mapa(bar, 0), (int32_t)(kb * kBK), first);
+      else
+        ptx::tma_load_2d(dst, map, bar, (int32_t)(kb * kBK), first);
+    };
+    // The first k-blocks of the first tile, as many as the ring holds, whose weights are requested before the wait and
+    // whose rows behind it: a loop of its own, since a test for them in every k-block of the loop below cost the
+    // 256 x 128 pairs 18 % (2048 x 12288 x 3072: 61 -> 72 us; a k-block of theirs takes 210 ns).
     const uint32_t early = p.weights_first && unit < num_tiles ? min(kb_end - kb_first, (uint32_t)kStages) : 0u;
     if (early != 0u && ptx::elect_one())
       for (uint32_t i = 0; i < early; ++i) {
-        expect(full_bar + 8 * i);
+        if (cta_rank == 0)
+          ptx::mbar_expect_tx(full_bar + 8 * i, CTAS * kStageBytes);
         load(&map_b, smem_base + i * kStageBytes + kABytes, full_bar + 8 * i, kb_first + i, columns_of(unit));
       }
     grid_dependency_wait();
     grid_dependents_launch();
-    uint32_t stage = 0, phase = 0;
+    if (early != 0u && ptx::elect_one())
+      for (uint32_t i = 0; i < early; ++i)
+        load(&map_a, smem_base + i * kStageBytes, full_bar + 8 * i, kb_first + i, rows_of(unit));
+    uint32_t stage = early == (uint32_t)kStages ? 0u : early, phase = early == (uint32_t)kStages ? 1u : 0u;
+    uint32_t kb = kb_first + early;
     bool ok = true;
     for (uint32_t tile = unit; tile < num_tiles && ok; tile += units) {
       const int32_t m0 = rows_of(tile), n0 = columns_of(tile);
-      const uint32_t ahead = tile == unit ? kb_first + early : kb_first;
-      for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
+      for (; kb < kb_end; ++kb) {
         if (!ptx::mbar_wait_warp(empty_bar + 8 * stage, phase ^ 1u, abort_ptr, wait_ns)) {
           give_up(0, kb);
           ok = false;
@@ -275,23 +276,35 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         const uint32_t a_dst = smem_base + stage * kStageBytes, b_dst = a_dst + kABytes;
         const uint32_t bar = full_bar + 8 * stage;
+        const int32_t k0 = (int32_t)(kb * kBK);
         if (kb == p.withhold_kb) {
           // test aid: the bytes are announced but never loaded, so the consumer's wait on this
           // stage runs out and the kernel leaves through its give-up path
           if (cta_rank == 0 && ptx::elect_one())
             ptx::mbar_expect_tx(bar, CTAS * kStageBytes);
         } else if (ptx::elect_one()) {
-          if (kb >= ahead)
-            expect(bar);
-          load(&map_a, a_dst, bar, kb, m0);
-          if (kb >= ahead)
-            load(&map_b, b_dst, bar, kb, n0);
+          if (CTAS == 2) {
+            if (cta_rank == 0) {
+              ptx::mbar_expect_tx(bar, 2 * kStageBytes);
+              ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
+              ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
+            } else {
+              const uint32_t leader_bar = ptx::mapa(bar, 0);
+              ptx::tma_load_2d_pair(a_dst, &map_a, leader_bar, k0, m0);
+              ptx::tma_load_2d_pair(b_dst, &map_b, leader_bar, k0, n0);
+            }
+          } else {
+            ptx::mbar_expect_tx(bar, kStageBytes);
+            ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
+            ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
+          }
         }
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
         }
       }
+      kb = kb_first;
     }
   } else if (warp == 1) {
     if (cta_rank == 0) {

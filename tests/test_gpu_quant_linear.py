@@ -217,6 +217,33 @@ def test_w8a8_linear_single_call_matches_two_calls(ops):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("form", ["2,256,1", "2,128,1", "1,256,1", "1,128,1", "1,128,2", "1,128,4"])
+@pytest.mark.parametrize("blocks", [1, 3, 4, 5, 6, 7, 8, 9, 15])
+def test_w8a8_linear_with_k_blocks_around_the_ring_depth(ops, monkeypatch, form, blocks):
+    """The single call requests the weights of the first k-blocks of a CTA's first tile ahead of everything else: fewer
+    k-blocks than the ring has stages (4 to 7), as many, more, a last one that is not full, and several tiles per CTA. The
+    same bits as the two calls, whose GEMM requests nothing ahead."""
+    import torch
+    split = int(form[-1])
+    if split > blocks:
+        pytest.skip("a split form needs a k-block per CTA")
+    monkeypatch.setenv("DIFB200_GEMM_FORM", form)
+    g = torch.Generator(device="cuda").manual_seed(blocks)
+    M, N, K = (300, 640, 128 * blocks - 16) if split > 1 else (2700, 2600, 128 * blocks - 16)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    w8 = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(N, generator=g, device="cuda") * 0.01
+    codes, scales = ops.quantize_int8_rows([x], 1)
+    want = ops.linear_int8_scaled(codes, w8, scales, ws)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = ops.w8a8_linear(x, w8, ws, implementation=1)
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    acc = (codes.double() @ w8.double().T).float()  # exact: |sum| < 2^24
+    assert torch.equal(((acc * scales[:, None]) * ws[None]).to(torch.bfloat16).view(torch.int16), want.view(torch.int16))
+    ops.poll_status()
+
+
 @pytest.mark.parametrize("impl", [2, 3, 5, 6])
 @pytest.mark.parametrize("K", [256, 1024, 3072, 12288])  # rows of one warp and of several, one and three blocks per warp
 def test_weight_scale_search_where_its_fp32_sums_do_not_decide(ops, impl, K):
