@@ -37,8 +37,6 @@
 // of P.V), Q codes (32 columns, the A operand of Q.K^T: read from shared memory for every 64 keys they alone took its
 // bandwidth for 128 clocks, 387 against 259 clocks for the Q.K^T of both tiles), output (fp32, 128). Items that would
 // not fill a last wave are shared by clusters of CTAs that take a part of the keys each (plan_split).
-// The scores start from the bits of the float 1.5 * 2^23 (a bf16 MMA of constants in front of the INT8 ones), so the
-// INT32 sums are already floats when they are read: no instruction converts them.
 //
 // Chunked form (the token-sharded block, where keys arrive from other GPUs one slice at a time):
 // a launch covers up to two ranges of 128-key tiles and may carry the unnormalised state of every
@@ -65,11 +63,15 @@ constexpr uint32_t kStageBytes = kKBytes + kVBytes + kKsBytes;
 constexpr int kThreads = 640;      // 4 control warps, 2 x 8 softmax warps
 constexpr uint32_t kPartialBytes = 32 * 32 * 4; // split form: a [32 rows x 32 columns] fp32 partial output
 constexpr uint32_t kOutBoxBytes = 32 * 128;    // a warp's output staging: two [32 rows x 64 bf16] boxes
-constexpr uint32_t kConstBytes = 6144;         // bf16 [128 x 16] of 1024 and [64 x 16] of 768: 16 products = 1.5 * 2^23
 constexpr float kHeadroom = 24.0f;  // powers of two that the running maximum goes beyond a row's scores when it moves
 constexpr float kLeastSum = 1.0f / (1u << 25); // of a running maximum: its largest p is above 2^-(kHeadroom + 1)
+// The bits of the float C = 1.5 * 2^23: added to an INT32 score they make the float C + score. One integer addition per
+// score (B2 S4608 H24 374 -> 387 us, 1101 tokens 27.2 -> 27.0); a bf16 MMA that puts them under the scores takes it out,
+// but the INT8 MMAs that add to its result are of another kind and K, between which no order is promised, and with a wait
+// for its completion in between the same calls took 439 and 27.7 us.
+constexpr uint32_t kScoreBias = 0x4B400000u;
 constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
-constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + kConstBytes + 256 + kPairBytes;
+constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + 256 + kPairBytes;
 
 struct AttnParams {
   const int8_t *q8;      // [B,Sq,H,128]
@@ -302,8 +304,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t *base_ptr = smem_raw + (base - raw_addr);
   const uint32_t stage_addr = base;                   // kStages x (K | V | ksmb)
-  const uint32_t const_addr = stage_addr + kStages * kStageBytes;
-  const uint32_t bar = const_addr + kConstBytes;
+  const uint32_t bar = stage_addr + kStages * kStageBytes;
   // barriers (8 bytes each)
   const uint32_t q_tma = bar;                         // Q codes are in shared memory
   const uint32_t q_full = bar + 8;                    // [2 tiles] they stand in tensor memory
@@ -398,9 +399,6 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (lane + 32u * u < n_kv)
         near[u] = load_produced(bounds + key_tile(lane + 32u * u));
   }
-  for (uint32_t i = threadIdx.x; i < kConstBytes / 4; i += kThreads)
-    *reinterpret_cast<uint32_t *>(base_ptr + (const_addr - base) + i * 4u) = i < 1024u ? 0x44804480u : 0x44404440u;
-  ptx::fence_proxy_async();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -446,19 +444,15 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       const uint64_t k_desc0 = ptx::smem_desc_sw128(stage_addr, 16, 1024);
       // V tile, N-major: 64-wide halves 16 KB apart (leading offset), 8-key groups 1 KB apart.
       const uint64_t v_desc0 = ptx::smem_desc_sw128(stage_addr + kKBytes, kVBytes / 2, 1024);
-      // constants, no swizzle: [8 x 16 bytes] core matrices 128 bytes apart along K, 256 along the rows
-      constexpr uint32_t idesc_c = ptx::make_idesc(1 /*F32*/, 1 /*BF16*/, 1 /*BF16*/, 0, 0, 128, 64);
-      const uint64_t ca_desc = ptx::smem_desc_plain(const_addr, 128, 256), cb_desc = ptx::smem_desc_plain(const_addr + 4096u, 128, 256);
       // Step g covers keys 64 g .. 64 g + 63, i.e. half g & 1 of the 128-key stage (g / 2) % kStages.
       // (called inside the elected lane's branch) Q.K^T of a step, keys from descriptor address b
       const uint32_t d_s = tmem + t * 256u, d_o = d_s + 128u, a_p = d_s + 64u, a_q = d_s + 96u;
       const uint32_t s_bar = s_full + 8 * t, p_bar = p_full + 8 * t;
       auto issue_qk = [&](uint32_t b) {
         const uint64_t kd = k_desc0 + b;
-        ptx::mma_f16_ss(d_s, ca_desc, cb_desc, idesc_c, 0); // every score = the bits of 1.5 * 2^23
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          ptx::mma_i8_ts(d_s, a_q + 8u * k, kd + (uint64_t)(2 * k), idesc_qk, 1);
+          ptx::mma_i8_ts(d_s, a_q + 8u * k, kd + (uint64_t)(2 * k), idesc_qk, k != 0);
         ptx::mma_commit(s_bar);
       };
       bool ok = ptx::mbar_wait_uniform(kv_full, 0, abort_ptr, wait_ns) && ptx::mbar_wait_uniform(q_full + 8 * t, 0, abort_ptr, wait_ns);
@@ -676,8 +670,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float4 kk = tab[j >> 1]; // (ks'_j, ks'_j+1, -C ks'_j, -C ks'_j+1)
-          const float f0 = __uint_as_float(r[j]);     // C + acc, exact
-          const float f1 = __uint_as_float(r[j + 1]);
+          const float f0 = __uint_as_float(r[j] + kScoreBias); // C + acc, exact
+          const float f1 = __uint_as_float(r[j + 1] + kScoreBias);
           const uint64_t u2 = fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w));
           float e0, e1;
           unpack2(fma2(u2, A2, negm2), e0, e1);
@@ -690,8 +684,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float4 kk = tab[j >> 1];
-          const float f0 = __uint_as_float(r[j]);
-          const float f1 = __uint_as_float(r[j + 1]);
+          const float f0 = __uint_as_float(r[j] + kScoreBias);
+          const float f1 = __uint_as_float(r[j + 1] + kScoreBias);
           float u0, u1;
           unpack2(fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w)), u0, u1);
           r[j] = __float_as_uint(u0);

@@ -192,17 +192,6 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint
                "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem]; bf16/f16 operands, fp32 accumulator.
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                           uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n"
-               ".reg .pred p;\n"
-               "setp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-               "}" ::"r"(d_tmem),
-               "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
 // D[tmem] (+)= A[tmem] * B[smem]; bf16/f16 operands, fp32 accumulator.
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                            uint32_t idesc, uint32_t accumulate) {
@@ -349,12 +338,6 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t
                                                     uint32_t sbo_bytes) {
   return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// The same without a swizzle (for operands whose layout does not matter).
-__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
-         ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
 // Instruction descriptor (32-bit) for kind::i8 / kind::f16:

@@ -355,3 +355,35 @@ def test_attention_running_maximum_with_large_and_small_values(ops, exponent, fo
     got = ob.bf16_to_f32(from_torch_bf16(got)).astype(np.float64)
     assert np.isfinite(got).all()
     assert rel_l2(got * 2.0 ** -exponent, want) <= 2e-3
+
+
+@pytest.mark.parametrize("q_gain", [1.0, 6.0])
+@pytest.mark.parametrize("masked", [False, True])
+def test_attention_shows_every_score(ops, q_gain, masked):
+    """Values that are one unit vector per key of one 128-key tile and zero elsewhere: output d of a query is the softmax
+    weight of key d of that tile alone, so a score that was not made whole (or stood where another belongs) shows. Tile by
+    tile, 72 CTAs, both query tiles, against the softmax in 64 bits: bf16 rounds a weight and the output once each (2^-8
+    each), and the exponent's product and sum, at most 2^7 in fp32, move it by less than 2^-15."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(3)
+    B, Sq, Sk, H, KV = 3, 257, 600, 12, 4
+    q = torch.randn((B, Sq, H, 128), generator=g, device="cuda") * q_gain
+    k = torch.randn((B, Sk, KV, 128), generator=g, device="cuda")
+    q8, qs = ops.quantize_int8_rows([q.to(torch.bfloat16).view(-1, 128)], 1)
+    k8, ks = ops.quantize_int8_rows([k.to(torch.bfloat16).view(-1, 128)], 1)
+    q8, k8 = q8.view(B, Sq, H, 128), k8.view(B, Sk, KV, 128)
+    valid = (torch.rand((B, Sk), generator=g, device="cuda") < 0.7).to(torch.uint8) if masked else None
+    rep = lambda a: a.double().repeat_interleave(H // KV, 2)  # noqa: E731
+    scores = torch.einsum("bqhd,bkhd->bhqk", q8.double() * qs.view(B, Sq, H, 1).double(),
+                          rep(k8 * ks.view(B, Sk, KV, 1).double())) / 128 ** 0.5
+    if masked:
+        scores = scores.masked_fill(valid[:, None, None, :] == 0, -float("inf"))
+    want = torch.softmax(scores, -1)
+    for tile in range(0, Sk, 128):
+        n = min(128, Sk - tile)
+        v = torch.zeros((B, Sk, KV, 128), dtype=torch.bfloat16, device="cuda")
+        v[:, tile:tile + n, :, :n] = torch.eye(n, dtype=torch.bfloat16, device="cuda")[None, :, None, :]
+        out = ops.attention_int8(q8, qs, k8, ks, v, valid).double().permute(0, 2, 1, 3)[..., :n]
+        w = want[..., tile:tile + n]
+        assert bool(((out - w).abs() <= w * (2.0 ** -7 + 2.0 ** -10) + 1e-30).all()), tile
+    ops.poll_status()
