@@ -90,6 +90,7 @@ struct AttnParams {
   float *l2_state;       // [B,Sq,H] l of the other half: a sequence of launches continues the very same sums
   uint32_t carry_in, carry_out;
   uint32_t behind_whole; // 1: launched behind the items that are not split, whose operands this launch shares
+  uint32_t split_follows; // 1: such a launch comes next
   uint32_t item0, split; // first (batch, head, query block) of this launch; CTAs of a cluster that share its keys
 };
 
@@ -372,13 +373,19 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
   }
-  // The kernel in front makes the codes and the key table and may run up to here. A split launch behind the unsplit
-  // items is independent of them (they let it start when the operands were complete): it fills the SMs as they become
-  // free, and only its end waits for them.
+  // The kernel in front makes the codes and the key table and may run up to here. A split launch behind the unsplit items
+  // is independent of them: it fills the SMs as they become free, and only its end waits for them. It reads the operands
+  // without a wait of its own. Every CTA of the unsplit launch lets it start only behind its own wait, when the operands'
+  // kernel is complete and its writes are performed, and hands them on with a fence; the reader has the other half.
   if (!SPLIT || !p.behind_whole)
     grid_dependency_wait();
-  if (!SPLIT)
+  else
+    ptx::fence_device_and_tma();
+  if (!SPLIT && warp == 3) { // (the idle one)
+    if (p.split_follows)
+      ptx::fence_device_and_tma();
     grid_dependents_launch();
+  }
   if (threadIdx.x == 0) {
     ptx::mbar_expect_tx(q_tma, 2 * kKBytes); // Q codes: staged where the ring is still free
     for (uint32_t t = 0; t < 2; ++t)
@@ -1188,6 +1195,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     // 64 when all start together; 20 (1 x 1700) 52 and 57, 36 (2 x 2500) 135 and 142.
     const bool scattered = first != 0 && ctas == 3 && count * ctas > (uint64_t)sm_count() * 3 / 4;
     p.behind_whole = first != 0 && !scattered ? 1u : 0u;
+    p.split_follows = first == 0 && count < items ? 1u : 0u;
     p.split = ctas;
     cudaLaunchConfig_t config{};
     cudaLaunchAttribute attrs[2]{};

@@ -83,6 +83,11 @@ int poll_device_status(const char *what); // copies back, clears, maps to kExecu
 // the kernel in front wrote is read behind grid_dependency_wait(), which every thread passes that touches global
 // memory, and through loads that the compiler cannot move up (load_produced or TMA). A kernel that lets dependents
 // start and is itself launched so waits first: when a kernel starts, the one two in front is complete.
+// Two reads are not behind such a wait. Both are of what a kernel further in front wrote, and both hold only because
+// the kernel in between was launched plainly or waited before it let anything start (then that kernel is complete):
+// * the first weights of a GEMM, requested ahead in w8a8_linear, whose quantiser, the kernel in between, is launched plainly;
+// * the operands of the attention's split launch: the unsplit one waits for their kernel, then fences, then lets it start.
+// Every kernel that calls grid_dependents_launch() in its first lines is launched plainly, and has to stay so.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ float load_produced(const float *p) {

@@ -19,6 +19,11 @@ __device__ __forceinline__ void fence_barrier_init() {
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// Between writes of others that this thread knows to be performed and what is read, by TMA too, by a kernel that it lets
+// start (or between that and the reads of the kernel started so).
+__device__ __forceinline__ void fence_device_and_tma() {
+  asm volatile("fence.acq_rel.gpu;\nfence.proxy.async.global;" ::: "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
