@@ -87,7 +87,7 @@ extern "C" {
 
 const char *difb200_last_error(void) { return last_error().c_str(); }
 
-int difb200_version(void) { return 3; }
+int difb200_version(void) { return 4; }
 
 uint64_t difb200_launch_count(void) { return launch_count(); }
 

@@ -31,6 +31,8 @@ extern "C" {
 #define DIFB200_EPILOGUE_GELU_TANH 2u /* Gelu, tanh form: y = bf16(gelu(y)) */
 
 DIFB200_EXPORT const char *difb200_last_error(void);
+/* Raised whenever a buffer that a caller sizes changes its size or layout. 4: the state of difb200_attention_int8_chunk has
+ * 524 bytes per query row and head (520 before). */
 DIFB200_EXPORT int difb200_version(void);
 /* Kernels of this library launched by this process so far (every entry point and the plugin count). */
 DIFB200_EXPORT uint64_t difb200_launch_count(void);
@@ -189,7 +191,9 @@ DIFB200_EXPORT int difb200_attention_int8(const int8_t *q8, const float *qs, con
  *   [begin0, begin0 + count0) and [begin1, begin1 + count1) of the key axis (Sk rounded up to 128).
  *   carry_in != 0: start from the state an earlier launch left in `state`; carry_out != 0: leave
  *   the state there instead of writing `out`. state: difb200_attention_int8_state_bytes(B,Sq,H)
- *   bytes, 16-byte aligned (per query row: m, l and 128 unnormalised fp32 outputs).
+ *   bytes, 16-byte aligned: 524 per query row and head (m, two partial sums l and 128 unnormalised fp32 outputs). The
+ *   call has no size to check, and size and layout belong to the library's version: ask for the size, and hand a state
+ *   only from one launch of this library to another.
  * A sequence of launches over disjoint tile ranges -- the first without carry_in, the last
  * without carry_out, all on one stream or ordered by events -- gives the result of the single
  * launch over all tiles up to the order of the fp32 sums (every m is an integer, so moving a row

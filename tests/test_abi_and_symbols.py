@@ -59,6 +59,19 @@ def test_api_tables(lib):
             assert C.cast(getattr(api, field), C.c_void_p).value
 
 
+def test_sizes_that_callers_allocate_belong_to_the_version(lib):
+    """Buffers whose size a caller asks for: the sizes that this version of the library stands for, and what the header
+    says of them. A size that changes raises difb200_version()."""
+    assert lib.difb200_version() == 4
+    for B, Sq, H in ((1, 1, 1), (2, 257, 24), (1, 33272, 24)):
+        assert lib.difb200_attention_int8_state_bytes(B, Sq, H) == 524 * B * Sq * H
+    for B, S, KV in ((1, 1, 1), (2, 4608, 24), (1, 1101, 8)):
+        tiles = (S + 127) // 128
+        assert lib.difb200_attention_int8_scratch_bytes(B, S, KV) == B * KV * tiles * 1024 + (4 * B * KV * tiles + 15) // 16 * 16
+    header = open(os.path.join(INCLUDE, "difb200", "difb200.h")).read()
+    assert "524 per query row and head" in header
+
+
 def test_per_device_bookkeeping_selftest(lib):
     """One-time kernel set-up (shared-memory opt-in, resident CTA pairs) is keyed by device
     ordinal, a failed set-up is retried, and the wait-limit state round-trips: the library's
