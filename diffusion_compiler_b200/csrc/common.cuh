@@ -111,13 +111,20 @@ __device__ __forceinline__ float bf16_bits_to_f32(uint32_t bits16) {
   return __uint_as_float(bits16 << 16);
 }
 // Round-to-nearest-even on the raw fp32 bits, the reference's bf16 store
-// (reference src/runtime/scalar.cpp:18-22).
-__device__ __forceinline__ uint32_t f32_to_bf16_bits(float v) {
-  const uint32_t b = __float_as_uint(v);
+// (reference src/runtime/scalar.cpp:18-22). The NaN of this GPU's arithmetic, 0x7fffffff, would overflow to -0 there, where
+// that of a CPU (0x7fc00000, 0xffc00000) stays a NaN: the minimum keeps it one (0x7fff) and changes nothing else.
+__device__ __forceinline__ uint32_t number_to_bf16_bits(uint32_t b) {
   return ((b + 0x7fffu + ((b >> 16) & 1u)) >> 16) & 0xffffu;
+}
+__device__ __forceinline__ uint32_t f32_to_bf16_bits(float v) {
+  return number_to_bf16_bits((uint32_t)min(__float_as_int(v), 0x7fff7fff));
 }
 __device__ __forceinline__ float round_bf16(float v) {
   return __uint_as_float(f32_to_bf16_bits(v) << 16);
+}
+// The same of what is never NaN (a row scale).
+__device__ __forceinline__ float round_bf16_number(float v) {
+  return __uint_as_float(number_to_bf16_bits(__float_as_uint(v)) << 16);
 }
 
 // ---- packed fp32x2 arithmetic (two independent fp32 lanes per 64-bit register) ----

@@ -403,7 +403,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       float candidate[7], reciprocal[7];
 #pragma unroll
       for (int f = 0; f < 7; ++f) {
-        candidate[f] = round_bf16(row_scale(maximum, factors[f])) * kCarry;
+        candidate[f] = round_bf16_number(row_scale(maximum, factors[f])) * kCarry;
         reciprocal[f] = __frcp_rn(candidate[f]);
       }
       // sums of the row's warps: doubles, then floats in an area of their own (rows of a CTA are not in step)
@@ -521,7 +521,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       scale = maximum == 0.0f ? 1.0e-30f : chosen * (1.0f / kCarry);
       __syncwarp(); // the samples are read before the codes overwrite them
     }
-    const float scale_bf16 = round_bf16(scale);
+    const float scale_bf16 = round_bf16_number(scale);
     const float stored = ((SIGNED || (EXTRA == kPack && p.mse)) && !F32) ? scale_bf16 : scale;
     const float divisor = (F32 ? scale : scale_bf16) * kCarry;
     const float recip = __frcp_rn(divisor);
@@ -592,7 +592,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       for (int w = 0; w < warps_per_row; ++w)
         rm = fmaxf(rm, redp[total_warps + slot * warps_per_row + w]);
       const float rscale = row_scale(rm, 1.0f);
-      const float rscale_bf16 = round_bf16(rscale);
+      const float rscale_bf16 = round_bf16_number(rscale);
       if (wrow == 0 && lane == 0)
         p.rscales[row] = (SIGNED && !F32) ? rscale_bf16 : rscale;
       const float rdivisor = F32 ? rscale : rscale_bf16, rrecip = __frcp_rn(rdivisor);

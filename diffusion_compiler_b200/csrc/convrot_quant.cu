@@ -149,7 +149,7 @@ convrot4096_kernel(const QuantParams p) {
     m = 0.0f;
     for (int w = 0; w < warps; ++w)
       m = fmaxf(m, redp[w]);
-    const float scale = row_scale(m * (1.0f / kCarry), clip), scale_bf16 = round_bf16(scale);
+    const float scale = row_scale(m * (1.0f / kCarry), clip), scale_bf16 = round_bf16_number(scale);
     const float stored = F32 ? scale : scale_bf16, divisor = stored * kCarry, recip = __frcp_rn(divisor);
     const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
     if (threadIdx.x == 0)
@@ -211,7 +211,7 @@ convrot4096_kernel(const QuantParams p) {
       rm = 0.0f;
       for (int w = 0; w < warps; ++w)
         rm = fmaxf(rm, redp[warps + w]);
-      const float rscale = row_scale(rm, 1.0f), rstored = F32 ? rscale : round_bf16(rscale);
+      const float rscale = row_scale(rm, 1.0f), rstored = F32 ? rscale : round_bf16_number(rscale);
       if (threadIdx.x == 0)
         p.rscales[row] = rstored;
       const float rrecip = __frcp_rn(rstored);

@@ -438,15 +438,8 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
     }
   }
   const float inv_mine = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, 128.0f), p.eps)));
-  // Rows it .. it + 3. The bf16 conversions keep NaN, where the reference's rounding of the bits makes zeros of the
-  // NaN that arithmetic gives: RAW rounds as the reference does. Returns whether a NaN was met (NaN spreads to the end).
-  auto process = [&](int it, auto raw) {
-    constexpr bool RAW = decltype(raw)::value;
-    auto bf16_bits = [](uint64_t v) -> uint32_t {
-      float lo, hi;
-      unpack2(v, lo, hi);
-      return RAW ? f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16) : pack_bf16_pair(lo, hi);
-    };
+#pragma unroll 1
+  for (int it = 0; it < ROWS; it += 4) { // rows it .. it + 3
     const int r = it + (lane >> 3);
     const float inv = __shfl_sync(0xffffffffu, inv_mine, r);
     const uint64_t out = __shfl_sync(0xffffffffu, out_row, r), at = __shfl_sync(0xffffffffu, trow, r);
@@ -459,7 +452,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const uint64_t scaled = mul2(unpack_bf16_pair(u[i]), inv2);
-        n[i] = V2 ? unpack_bf16_pair(bf16_bits(mul2(unpack_bf16_pair(bf16_bits(scaled)), w[i]))) : mul2(scaled, w[i]);
+        n[i] = V2 ? round_bf16_2(mul2(round_bf16_2(scaled), w[i])) : mul2(scaled, w[i]);
       }
     }
     if (rotates) {
@@ -509,15 +502,10 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
     uint32_t bits[8], most = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      bits[i] = bf16_bits(n[i]);
-      if (RAW)
-        asm("max.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(bits[i] & 0x7fff7fffu));
-      else
-        asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(bits[i] & 0x7fff7fffu));
+      bits[i] = pack_bf16_pair(n[i]);
+      asm("max.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(bits[i] & 0x7fff7fffu)); // NaN does not count
     }
     float m = fmaxf(__uint_as_float(most << 16), __uint_as_float(most & 0xffff0000u));
-    if (!RAW && __any_sync(0xffffffffu, ((most & 0x7fffu) > 0x7f80u) | ((most >> 16) > 0x7f80u)))
-      return true;
     if (p.o && exists) {
       p.o[out * 16 + c0] = make_uint4(bits[0], bits[1], bits[2], bits[3]);
       p.o[out * 16 + c1] = make_uint4(bits[4], bits[5], bits[6], bits[7]);
@@ -539,12 +527,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
           p.scales[out] = scale;
       }
     }
-    return false;
-  };
-#pragma unroll 1
-  for (int it = 0; it < ROWS; it += 4)
-    if (process(it, std::false_type{}))
-      process(it, std::true_type{});
+  }
 }
 
 // ---- QuantizeInt8Rows(Direct) of 128-wide rows, one thread per row (same arithmetic as the

@@ -1,6 +1,6 @@
 """The Direct codes (QuantizeInt8Rows variant 1) that QkNormPartialRope and the attention's operand kernel make without a
 division, against the oracle's quotients: rows whose quotients lie exactly in the middle between two integers, rows
-with infinity, and the rotation kernel at the edges of its rows per warp."""
+with infinity and NaN, and the rotation kernel at the edges of its rows per warp, with every part of its addressing."""
 import ctypes as C
 
 import numpy as np
@@ -61,6 +61,112 @@ def test_rope_codes_and_output(tokens, heads, interleaved, rotary, wide):
     assert np.array_equal(from_torch_bf16(out), want)
     assert np.array_equal(codes.cpu().numpy().reshape(-1, 128), want_codes)
     assert np.array_equal(scales.cpu().numpy().view(np.uint32), want_scales.view(np.uint32))
+
+
+def _rope_quant(x, w, cos, sin, rotary, interleaved, sequence, table_sequence, start):
+    """difb200_qk_norm_rope_quant on device tensors: (output bits, codes, scales) as host arrays."""
+    import torch
+    from diffusion_compiler_b200 import _lib
+    tokens, heads = x.shape[0], x.shape[1]
+    out = torch.zeros((tokens, heads, 128), dtype=torch.bfloat16, device="cuda")
+    codes = torch.full((tokens, heads, 128), 99, dtype=torch.int8, device="cuda")
+    scales = torch.zeros(tokens * heads, dtype=torch.float32, device="cuda")
+    p = lambda a: C.c_void_p(a.data_ptr())  # noqa: E731
+    _lib.check(_lib.lib().difb200_qk_norm_rope_quant(
+        p(x), p(w), p(cos), p(sin), p(out), p(codes), p(scales), 1 if cos.dtype == torch.float32 else 2, tokens, heads, rotary,
+        cos.shape[-1], sequence, table_sequence, start, 1e-5, int(interleaved), None))
+    torch.cuda.synchronize()
+    return from_torch_bf16(out), codes.cpu().numpy().reshape(-1, 128), scales.cpu().numpy()
+
+
+@pytest.mark.parametrize("sequence,heads", [(37, 5), (1201, 24)])  # 370 rows: 8 per warp; 57648: 32; neither fills the last
+@pytest.mark.parametrize("interleaved,rotary", [(False, 96), (True, 128)])
+@pytest.mark.parametrize("bf16_table", [False, True])
+def test_rope_of_two_sequences_with_longer_tables(sequence, heads, interleaved, rotary, bf16_table):
+    """Two sequences whose tables are longer than they are and start at a later row, with fp32 and bf16 tables."""
+    import torch
+    rng = np.random.default_rng(sequence + rotary)
+    table, start = sequence + 13, 9
+    x = bf16_normal(rng, (2 * sequence, heads, 128))
+    w = ob.f32_to_bf16((1 + 0.1 * rng.standard_normal(128)).astype(np.float32))
+    angle = rng.uniform(0, 6.28, (2, table, rotary // 2 if interleaved else rotary)).astype(np.float32)
+    cos, sin = np.cos(angle), np.sin(angle)
+    if bf16_table:
+        dc, ds = to_torch_bf16(ob.f32_to_bf16(cos)), to_torch_bf16(ob.f32_to_bf16(sin))
+        cos, sin = ob.bf16_to_f32(ob.f32_to_bf16(cos)), ob.bf16_to_f32(ob.f32_to_bf16(sin))
+    else:
+        dc, ds = torch.from_numpy(cos).cuda(), torch.from_numpy(sin).cuda()
+    rows = lambda a: np.ascontiguousarray(a[:, start:start + sequence]).reshape(2 * sequence, -1)  # noqa: E731
+    want = _rope(ob.bf16_to_f32(x), ob.bf16_to_f32(w), rows(cos), rows(sin), rotary, interleaved, 1e-5)
+    want_codes, want_scales = ob.orc().quantize_int8_rows([want.reshape(-1, 128)], 1)
+    out, codes, scales = _rope_quant(to_torch_bf16(x), to_torch_bf16(w), dc, ds, rotary, interleaved, sequence, table, start)
+    assert np.array_equal(out, want)
+    assert np.array_equal(codes, want_codes)
+    assert np.array_equal(scales.view(np.uint32), want_scales.view(np.uint32))
+
+
+@pytest.mark.parametrize("fusion", ["1", "0"])
+def test_rope_reads_a_slice_of_a_wider_tensor(monkeypatch, fusion):
+    """QkNormPartialRope on the middle third of a packed tensor [2, 37, 3 * 5 * 128], read in place and through a copy."""
+    from diffusion_compiler_b200 import diffir, plugin
+    from diffusion_compiler_b200.diffir import AttrKey, Attribute, DType, Opcode, Role
+    monkeypatch.setenv("DIFB200_ROPE_FUSION", fusion)
+    rng = np.random.default_rng(8)
+    T, H, table, start = 37, 5, 50, 9
+    x, w = bf16_normal(rng, (2, T, 3 * H * 128)), ob.f32_to_bf16((1 + 0.1 * rng.standard_normal(128)).astype(np.float32))
+    angle = rng.uniform(0, 6.28, (2, table, 64)).astype(np.float32)
+    cos, sin = np.cos(angle), np.sin(angle)
+    p = diffir.Program()
+    tx = p.add_tensor(DType.BF16, [2, T, 3 * H * 128], Role.Input)
+    tw = p.add_tensor(DType.BF16, [128], Role.Constant)
+    tc, ts = (p.add_tensor(DType.F32, [2, table, 64], Role.Input) for _ in range(2))
+    flat, shaped = p.add_tensor(DType.BF16, [2, T, H * 128]), p.add_tensor(DType.BF16, [2, T, H, 128])
+    to = p.add_tensor(DType.BF16, [2, T, H, 128], Role.Output)
+    p.add_op(Opcode.Slice, [tx], [flat], [Attribute.u64(AttrKey.Axis, 2), Attribute.u64(AttrKey.Start, H * 128)])
+    p.add_op(Opcode.Reshape, [flat], [shaped])
+    p.add_op(Opcode.QkNormPartialRope, [shaped, tw, tc, ts], [to],
+             [Attribute.f64(AttrKey.Epsilon, 1e-5), Attribute.u64(AttrKey.Implementation, 2),
+              Attribute.u64(AttrKey.BlockSize, 128), Attribute.u64(AttrKey.RotaryDim, 128),
+              Attribute.u64(AttrKey.Start, start), Attribute.u64(AttrKey.RotaryLayout, 1)])
+    ex = plugin.PluginExecutor(0)
+    got, _ = ex.prepare(p, {tw: w}).run({tx: x, tc: cos, ts: sin})
+    ex.close()
+    part = ob.bf16_to_f32(np.ascontiguousarray(x[:, :, H * 128:2 * H * 128])).reshape(2 * T, H, 128)
+    rows = lambda a: np.ascontiguousarray(a[:, start:start + T]).reshape(2 * T, -1)  # noqa: E731
+    want = _rope(part, ob.bf16_to_f32(w), rows(cos), rows(sin), 128, True, 1e-5)
+    assert np.array_equal(got[to].reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("tokens", [11, 2401])  # 8 and 32 rows per warp
+@pytest.mark.parametrize("interleaved,rotary", [(False, 96), (True, 128)])
+def test_rope_keeps_nan_and_infinity(tokens, interleaved, rotary):
+    """A NaN makes its row NaN, an infinity makes NaN of itself and of its partner in the rotation and zeros of the rest (its
+    norm is infinite), a NaN in a table those two elements: as on a CPU, so that a broken activation shows. Codes are zero
+    where the value is NaN, and the scale is that of the other elements."""
+    import torch
+    rng = np.random.default_rng(tokens)
+    heads = 24
+    x = bf16_normal(rng, (tokens, heads, 128))
+    for row, (at, bits) in {1: (5, 0x7fc0), 3: (100, 0xffc0), 4: (2, 0x7f80), 6: (97, 0xff80), 8: (0, 0x7f81)}.items():
+        x[row, 2, at] = bits
+        x[tokens - 1 - row, heads - 1, at] = bits
+    w = ob.f32_to_bf16((1 + 0.1 * rng.standard_normal(128)).astype(np.float32))
+    angle = rng.uniform(0, 6.28, (tokens, rotary // 2 if interleaved else rotary)).astype(np.float32)
+    cos, sin = np.cos(angle), np.sin(angle)
+    cos[7, 3] = np.nan
+    with np.errstate(invalid="ignore"):
+        want = _rope(ob.bf16_to_f32(x), ob.bf16_to_f32(w), cos, sin, rotary, interleaved, 1e-5)
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    out, codes, scales = _rope_quant(to_torch_bf16(x), to_torch_bf16(w), t(cos), t(sin), rotary, interleaved, tokens, tokens, 0)
+    nan = np.isnan(ob.bf16_to_f32(want))
+    assert 6 * 128 <= nan.sum() < want.size // 2
+    assert np.array_equal(np.isnan(ob.bf16_to_f32(out)), nan)
+    assert np.array_equal(out[~nan], want[~nan])
+    others = want.copy()
+    others[nan] = 0
+    want_codes, want_scales = ob.orc().quantize_int8_rows([others.reshape(-1, 128)], 1)
+    assert np.array_equal(codes, want_codes)
+    assert np.array_equal(scales.view(np.uint32), want_scales.view(np.uint32))
 
 
 def test_operand_codes_of_ties():
