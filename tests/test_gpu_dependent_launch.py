@@ -1,6 +1,6 @@
-"""Kernels that start while the one in front of them on the stream still runs (the GEMM behind a quantiser, the attention
-behind its operands, its split items behind the whole ones): results where the kernel in front has just written the
-operands, weights included, back to back without a synchronisation and replayed from a graph."""
+"""Kernels that start while the one in front of them on the stream still runs (the GEMM behind a quantiser or an attention,
+the attention behind its operands, its split items behind the whole ones): results where the kernel in front has just
+written the operands, weights included, back to back without a synchronisation and replayed from a graph."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -73,3 +73,98 @@ def test_attention_back_to_back_and_from_a_graph(tokens, heads):
     ops.poll_status()
     for i, o in enumerate(got):
         assert torch.equal(_bits(o), _bits(want[i % 3])), i
+
+
+@pytest.mark.parametrize("rows", [2, 130, 4159])
+def test_linear_from_a_graph_behind_new_weights(rows):
+    """The captured single call, which requests its first weights before its quantiser is done: between two replays the
+    inputs and the weights are overwritten on the stream, by copies and by a packing kernel that is captured in front."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    K, N = 1024, 1536
+    sets = [(normal(rows, K), normal(N, K)) for _ in range(4)]
+    want = []
+    for x, w in sets:
+        codes, scales = ops.quantize_weight_rows(w, 2)
+        torch.cuda.synchronize()
+        want.append(ops.w8a8_linear(x, codes, scales))
+        torch.cuda.synchronize()
+    x, w = (t.clone() for t in sets[0])
+    w8, ws = ops.quantize_weight_rows(w, 2)
+    graphs = []
+    for packed in (False, True):  # the weights as they stand; packed inside the graph
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            ops.w8a8_linear(x, w8, ws)
+        torch.cuda.current_stream().wait_stream(stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = ops.w8a8_linear(x, *(ops.quantize_weight_rows(w, 2) if packed else (w8, ws)))
+        graphs.append((graph, out))
+    got = []
+    for i, (nx, nw) in enumerate(sets + sets):
+        x.copy_(nx)
+        w.copy_(nw)
+        codes, scales = ops.quantize_weight_rows(w, 2)
+        w8.copy_(codes)
+        ws.copy_(scales)
+        graph, out = graphs[i // len(sets)]
+        graph.replay()
+        got.append(out.clone())
+    torch.cuda.synchronize()
+    ops.poll_status()
+    for i, o in enumerate(got):
+        assert torch.equal(_bits(o), _bits(want[i % len(sets)])), i
+
+
+@pytest.mark.parametrize("tokens", [130, 1700, 2048])  # no split; a split behind the whole items; one that starts together
+def test_gemm_directly_behind_an_attention(tokens):
+    """LinearInt8Scaled as the next launch after the attention's, with nothing in between: its scales are the attention's
+    output (reinterpreted), so that a GEMM that read before the attention was done would show; also from a graph."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    H, N, K = 24, 256, 1024
+    q, k, v = (torch.randn((1, tokens, H, 128), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3))
+    x8 = torch.randint(-127, 128, (tokens, K), generator=g, device="cuda", dtype=torch.int8)
+    w8 = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(N, generator=g, device="cuda")
+    out = torch.empty_like(q)
+    scales = out.view(torch.float32).view(-1)  # pairs of bf16 outputs as fp32 row scales, from the last rows of the output
+    scales = scales[scales.numel() - tokens:]
+    y = torch.empty((tokens, N), dtype=torch.bfloat16, device="cuda")
+
+    def both():
+        ops.attention(q, k, v, out=out)
+        ops.linear_int8_scaled(x8, w8, scales, ws, out=y)
+
+    ops.attention(q, k, v, out=out)
+    torch.cuda.synchronize()
+    want = ops.linear_int8_scaled(x8, w8, scales, ws).clone()
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(4):
+        out.zero_()
+        both()
+        got.append(y.clone())
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        both()
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        both()
+    for _ in range(4):
+        out.zero_()
+        y.zero_()
+        graph.replay()
+        got.append(y.clone())
+    torch.cuda.synchronize()
+    ops.poll_status()
+    assert bool(torch.isfinite(want.float()).all()) and bool(want.float().any())
+    for i, o in enumerate(got):
+        assert torch.equal(_bits(o), _bits(want)), i
