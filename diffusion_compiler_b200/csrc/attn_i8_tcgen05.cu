@@ -988,13 +988,13 @@ int resident_clusters(uint32_t split, int &count) {
 // Items (batch, head, 256 queries) that run as one CTA each, and the split over the keys of the others. A last wave
 // that is nearly empty costs as much as a full one: 3120 items of the 33272-token block are 21.08 waves of 148 SMs.
 // Its items (or those of the last two waves) are split 2, 3, 4 or 8 ways over the key tiles by clusters. Modelled
-// times in ns, measured on B200: 1380 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
+// times in ns, measured on B200: 1480 per 128-key tile of a CTA, 6000 around them, 8000 more for a second launch
 // and the exchange (an upper figure: the second launch fills the SMs as they become free), at least four tiles per CTA; a
-// split has to give 3 %. H24, without -> with: 1 x 1700 tokens (1.14 waves) 60 -> 52 us, 1 x 2304 (1.46) 72 -> 65 us,
-// 2 x 2500 (3.24) 145 -> 135 us, 1 x 3300 (2.11) 133 -> 114 us; where the rule takes none, a split costs: 1 x 2816 (1.78)
-// 83 -> 99 us, 1 x 4608 (2.92) 179 -> 196 us.
+// split has to give 3 %. H24, without -> with: 1 x 1700 tokens (1.14 waves) 56.0 -> 48.8 us, 1 x 2048 (1.30) 62.2 -> 56.8,
+// 1 x 2304 (1.46) 68.0 -> 61.9, 2 x 2500 (3.24) 144.6 -> 134.4, 1 x 3300 (2.11) 131.6 -> 113.5; where the rule takes none,
+// a split costs: 1 x 2560 (1.62) 74.6 -> 90.3, 1 x 2816 (1.78) 80.2 -> 96.9, 1 x 4608 (2.92) 182 -> 198.
 int plan_split(uint64_t items, uint64_t tiles, uint64_t &whole, uint32_t &split) {
-  constexpr uint64_t kTileNs = 1380, kItemNs = 6000, kExchangeNs = 8000;
+  constexpr uint64_t kTileNs = 1480, kItemNs = 6000, kExchangeNs = 8000;
   const uint64_t sms = (uint64_t)sm_count(), item_ns = kItemNs + tiles * kTileNs;
   whole = items;
   split = 1;
@@ -1198,11 +1198,20 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       return rc;
   auto launch = [&](uint64_t first, uint64_t count, uint32_t ctas) {
     p.item0 = (uint32_t)first;
-    // Clusters of three that start one by one, as SMs become free behind the unsplit items, leave gaps in the GPCs. Where
-    // nearly all SMs are needed the last ones then wait for a second round: 44 clusters (1 x 2048 tokens) take 70 us, and
-    // 64 when all start together; 20 (1 x 1700) 52 and 57, 36 (2 x 2500) 135 and 142.
-    const bool scattered = first != 0 && ctas == 3 && count * ctas > (uint64_t)sm_count() * 3 / 4;
-    p.behind_whole = first != 0 && !scattered ? 1u : 0u;
+    // Items that start one by one, as SMs become free behind the unsplit ones, are 3 to 5 % of a call faster than all
+    // together behind them, except where nearly all clusters of three that fit (45) are needed: started one by one they
+    // leave gaps in the GPCs, and the last ones wait for a second round. 148 + n items of 16 tiles, one by one / together:
+    // n = 40 69.5 / 72.3 us, 42 70.7 / 73.1, 43 74.7 / 73.5, 44 79.7 / 73.6, 45 81.7 / 73.6; of 32 tiles n = 42 116 / 118,
+    // 43 120 / 117. Clusters of two, four and eight leave none: 74 of two 76.5 / 78.1, 33 of four 69.5 / 72.3, 15 of eight
+    // (32 tiles) 104 / 107.
+    bool together = false;
+    if (first != 0 && ctas == 3) {
+      int resident = 0;
+      if (int rc = resident_clusters(ctas, resident))
+        return rc;
+      together = count + 2 >= (uint64_t)resident;
+    }
+    p.behind_whole = first != 0 && !together ? 1u : 0u;
     p.split_follows = first == 0 && count < items ? 1u : 0u;
     p.split = ctas;
     cudaLaunchConfig_t config{};
@@ -1210,7 +1219,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     split_config(config, attrs, ctas);
     config.gridDim = dim3((unsigned)(count * ctas));
     config.stream = stream;
-    if (scattered) {
+    if (together) {
       config.attrs = attrs + 1;
       config.numAttrs = 1;
     }

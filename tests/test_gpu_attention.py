@@ -387,3 +387,26 @@ def test_attention_shows_every_score(ops, q_gain, masked):
         w = want[..., tile:tile + n]
         assert bool(((out - w).abs() <= w * (2.0 ** -7 + 2.0 ** -10) + 1e-30).all()), tile
     ops.poll_status()
+
+
+@pytest.mark.parametrize("rest", [40, 42, 43, 45])  # clusters of three behind a whole wave: one by one, all together from 43
+def test_attention_split_where_its_clusters_fill_the_device(ops, rest):
+    """The clusters behind a whole wave, started as SMs become free or together, against the same launch without a split
+    (the bars of the split's test), back to back with new operands and the same bits again."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rest)
+    H, Sq, Sk = torch.cuda.get_device_properties(0).multi_processor_count + rest, 130, 2048
+    v = torch.randn((1, Sk, 1, 128), generator=g, device="cuda").to(torch.bfloat16)
+    runs = []
+    for _ in range(2):
+        q8, qs = ops.quantize_int8_rows([torch.randn((Sq * H, 128), generator=g, device="cuda").to(torch.bfloat16)], 1)
+        k8, ks = ops.quantize_int8_rows([torch.randn((Sk, 128), generator=g, device="cuda").to(torch.bfloat16)], 1)
+        args = (q8.view(1, Sq, H, 128), qs, k8.view(1, Sk, 1, 128), ks, v)
+        runs.append((args, ops.attention_int8(*args), ops.attention_int8(*args)))
+    for args, split, again in runs:
+        plain = ops.attention_int8_chunked(*args, [[(0, Sk // 128)]])
+        assert torch.equal(split.view(torch.int16), again.view(torch.int16))
+        a, b = split.double(), plain.double()
+        assert float((a - b).norm() / b.norm()) <= 3e-4
+        assert float((a != b).double().mean()) <= 0.01
+    ops.poll_status()
