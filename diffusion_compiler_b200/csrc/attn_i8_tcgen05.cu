@@ -421,8 +421,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // Addresses, descriptors and loop state are then warp-uniform values. As single-lane
     // (divergent) loops every TMA / MMA operand was first moved between register files. One warp for both
     // query tiles was the bound of the whole kernel: its control instructions are a serial chain of about 1500 clocks
-    // per 64-key step, in which the MMAs themselves execute for 770. Two warps with the shortest loop (one wait, one
-    // commit per step): B2 S4608 H24 443 -> 404 us.
+    // per 64-key step, in which the MMAs themselves execute for 770. With one thread per query row, B2 S4608 H24 took
+    // 443 us with one warp in the shortest loop (one wait, one commit per step) and 404 with two.
     auto give_up = [&](uint32_t role, uint32_t detail) {
       if (lane == 0) {
         if (!*abort_ptr)
@@ -525,9 +525,9 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
   } else {
     // ---------------- softmax + epilogue, two threads per query row ----------------
-    // Four warps per scheduler: the ld / st / barrier time of one is covered by the others. With one thread per row
-    // (two warps per scheduler, 64 columns each): B2 S4608 H24 398 us, with two 352. 32 x 128 + 112 x 512 registers are
-    // what the launch has (96 x 640).
+    // Four warps per scheduler: the ld / st / barrier time of one is covered by the others. B2 S4608 H24 398 us with one
+    // thread per row (two warps per scheduler, 64 columns each) and 367 with two. 32 x 128 + 112 x 512 registers are what
+    // the launch has (96 x 640); without spills, which the smaller share had, it went from 363 to 352.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const uint32_t t = (uint32_t)(warp - 4) >> 3, hf = ((uint32_t)(warp - 4) >> 2) & 1u; // query tile 0 / 1; half of the columns
     const uint32_t quarter = (uint32_t)warp & 3u;
