@@ -333,7 +333,7 @@ def test_attention_ring_and_query_tiles(ops, Sq, tiles, q_gain):
 @pytest.mark.parametrize("form", ["plain", "split", "chunked"])
 def test_attention_running_maximum_with_large_and_small_values(ops, exponent, form):
     """No softmax weight is above 1, so values near the end of bf16's range stay finite where the maximum runs: V in
-    [2^e, 2^(e+1)) under scores that rise by hundreds of powers of two along the keys, against the oracle on the same
+    [2^e, 2^(e+1)) under scores that rise by about a hundred powers of two along the keys, against the oracle on the same
     values without the power of two (rel-L2 2e-3, the bar of the path; the outputs themselves scale exactly)."""
     import torch
     rng = np.random.default_rng(31)
