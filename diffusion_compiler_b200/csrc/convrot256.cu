@@ -15,26 +15,28 @@
 // thread's own 16 elements; a 16x16 transpose through shared memory (XOR-swizzled, conflict-free)
 // gives the thread the 16 elements of stride 16, on which stages 2-3 run.
 //
-// What bounds it: not HBM (3 bytes per element) and not the issue slots alone (about 16 thread instructions per
-// element, 5 of them packed additions that take two clocks each: half of the slots), but the chain of a row -- load,
-// rotation, maximum, division, codes -- with 14 to 32 warps per SM to cover for one another. A warp takes
-// up to three such blocks of its row (NIT) before it needs the row's scale: the scale arithmetic, the
-// reductions and the loop overhead are paid once per 96 elements of a thread instead of once per 32, and
-// a row of up to 3072 columns needs no barrier at all. Between rotation and quantisation the bf16
-// variants keep the values as packed bf16 (their result is defined on the rounded values), half the
-// registers of fp32. The one-block form instead fits 64 registers, so that 32 warps per SM hide the
-// load latency without a prefetch. 33272 x 3072 takes 87 us (3.5 TB/s), 33272 x 8192 226 us, 9216 x 3072 29 us, the
-// scale search of the weight form 12288 x 3072 69 us (all lanes evaluate samples, in doubles only where candidates
-// are close), with input equalisation 99 us, RmsNormModulate in front of 33272 x 3072 145 us with its statistic. Staging
-// the input with bulk copies through shared memory instead of registers gave nothing (30.0 us for the third shape).
+// What bounds it: nothing alone. A warp's 1024 elements are about 430 instructions (13.5 per element and lane, 5 of them packed
+// additions of two clocks), and with 24 warps per SM the FMA pipe is 57 % busy, the issue slots 63 % and the L1 and shared-memory
+// pipe 69 % (9216 x 8192): 64 of its 112 accesses per block are the transpose, which fp32 sums between the stages need whole. Between
+// rotation and quantisation the bf16 variants keep the values as packed bf16 (their result is defined on the rounded
+// values), half the registers of fp32. The codes of a pair are made by one conversion and leave as 16 bits; as a
+// conversion and a byte store per element they kept the quarter-rate unit busy for 256 clocks of a block, and a warp took three
+// blocks at a time to save per-row work. Before -> now, us: 33272 x 3072 83.9 -> 71.8 (4.3 TB/s), 33272 x 8192 220.6 -> 181.7,
+// 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 55.4, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
+// 12288 x 3072 64.7 -> 61.6 (all lanes evaluate samples, in doubles only where candidates are close), with input
+// equalisation 94.5 -> 90.8, RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
+// copies through shared memory instead of registers gave nothing.
 #include "quant_common.cuh"
 
 namespace difb200 {
 namespace {
 
-// Shared memory per warp: 4 groups x 256 fp32 (two swizzled 16x32-word transposes), reused for the
-// code bytes and the sampled elements of the scale search.
-constexpr int kWarpBytes = 4096;
+// Shared memory per warp: 4 groups x 256 fp32 (two 16x32-word transposes whose rows are padded, so that every access is
+// free of conflicts at a constant offset), reused for the code pairs and the sampled elements of the scale search.
+constexpr int kWarpBytes = 4608;
+constexpr uint32_t kRowPitch = 144;                  // bytes of a row of 16 pairs in the transpose
+constexpr uint32_t kHalfBytes = 16 * kRowPitch;      // a half-warp's area
+constexpr uint32_t kCodeHalfBytes = 544, kCodeBytes = 2 * kCodeHalfBytes; // code pairs of a half-warp's two groups, of a block
 
 // kPack: weight rows with the scale search (and input equalisation where given), kEqualise: without the search.
 enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3 };
@@ -73,17 +75,13 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   const uint32_t col_warp = (uint32_t)wrow * (NIT * 1024u);
   const uint32_t col0 = col_warp + 512u * h + 16u * a; // this thread's run in the first group of block 0
 
-  // Transpose addressing (per half-warp area of 2048 bytes; rows of 128 bytes = 16 pairs):
-  // thread a writes its 8 chunks of 2 pairs at chunk position c ^ (a & 7), and reads pair a of
-  // every row j from chunk position (a >> 1) ^ (j & 7).
-  const uint32_t half_addr = warp_addr + h * 2048u;
-  const uint32_t wr_addr = half_addr + 128u * a + ((a & 7u) << 4);                // ^ (c << 4)
-  const uint32_t rd_addr = half_addr + ((uint32_t)(a >> 1) << 4) + 8u * (a & 1u); // ^ ((j&7)<<4), + 128 j
-  // Code bytes of one block are staged at index(col) = col + 64 * (col >> 9): a 64-byte skew per 512
-  // columns, so that the two half-warps hit different banks; blocks are 1152 bytes apart.
-  const uint32_t code_a = warp_addr + 512u * h + a + 64u * h, code_b = code_a + 256u;
-  const uint32_t copy_addr = warp_addr + 16u * lane;
-  const uint32_t copy_col = col_warp + 16u * lane;
+  // Transpose: thread a writes its 16 pairs as row a and reads pair a of every row j.
+  const uint32_t wr_addr = warp_addr + h * kHalfBytes + kRowPitch * a; // + 16 c
+  const uint32_t rd_addr = warp_addr + h * kHalfBytes + 8u * a;        // + kRowPitch j
+  // The two codes that belong together, of the same element of both groups, are staged as 16 bits: element 16 j + a in
+  // row j of 32 bytes, whose two 16-byte chunks change places in rows 4-7 and 12-15 (a thread reads whole rows).
+  const uint32_t code_wr = warp_addr + h * kCodeHalfBytes + ((uint32_t)(a >> 3) << 4) + 2u * (a & 7u); // ^ 16, + 32 j
+  const uint32_t code_rd = warp_addr + h * kCodeHalfBytes + 32u * a + (((uint32_t)a >> 2 & 1u) << 4);  // ^ 16 c
 
   // Sign flips of this thread's columns as XOR masks on the packed bf16 pairs (bits 15 and 31 of
   // word i: elements 2i and 2i+1), kept in shared memory: per block four 16-byte vectors per thread
@@ -341,10 +339,10 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
           float x0, x1, x2, x3;
           unpack2(P[2 * c], x0, x1);
           unpack2(P[2 * c + 1], x2, x3);
-          sts128(wr_addr ^ (uint32_t)(c << 4), x0, x1, x2, x3);
+          sts128(wr_addr + 16u * c, x0, x1, x2, x3);
         }
         __syncwarp();
-#define DIFB200_READ_PAIR(J) P[J] = lds64<(J) * 128>(rd_addr ^ (uint32_t)(((J) & 7) << 4));
+#define DIFB200_READ_PAIR(J) P[J] = lds64<(J) * kRowPitch>(rd_addr);
         DIFB200_READ_PAIR(0) DIFB200_READ_PAIR(1) DIFB200_READ_PAIR(2) DIFB200_READ_PAIR(3)
         DIFB200_READ_PAIR(4) DIFB200_READ_PAIR(5) DIFB200_READ_PAIR(6) DIFB200_READ_PAIR(7)
         DIFB200_READ_PAIR(8) DIFB200_READ_PAIR(9) DIFB200_READ_PAIR(10) DIFB200_READ_PAIR(11)
@@ -376,9 +374,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       if (lane == 0)
         redp[warp] = m;
       row_barrier();
-      m = 0.0f;
-      for (int w = 0; w < warps_per_row; ++w)
-        m = fmaxf(m, redp[slot * warps_per_row + w]);
+      m = lane < warps_per_row ? redp[slot * warps_per_row + lane] : 0.0f;
+      m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     }
     const float maximum = m * (1.0f / kCarry);
     float scale = row_scale(maximum, clip);
@@ -524,60 +521,88 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     const float scale_bf16 = round_bf16_number(scale);
     const float stored = ((SIGNED || (EXTRA == kPack && p.mse)) && !F32) ? scale_bf16 : scale;
     const float divisor = (F32 ? scale : scale_bf16) * kCarry;
-    const float recip = __frcp_rn(divisor);
-    const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
     if (wrow == 0 && lane == 0)
       p.scales[row] = stored;
+    // The bf16 variants' quotients as bf16: V r1 + V r2 with the two bf16 parts of r = (1 + 6 / 2^23) / divisor, a product
+    // and a fused sum that rounds once. For every pair of 8-bit significands that is the rounded quotient, with the
+    // reciprocal anywhere between 1 + 2^-25 and 1 + 43 / 2^25 times the exact one, and the approximate one is within 2^-23.
+    // Beside the fp32 product and its rounding it saves the conversions on either side. Rows whose divisor leaves no
+    // room for the low part, or whose quotients could overflow, get their quotients first, bounded, and the factors 1 and 0.
+    constexpr bool kSplitQuotient = !F32 && !RESIDUAL;
+    float recip;
+    uint32_t r1 = 0x3f803f80u, r2 = 0u;
+    if (kSplitQuotient && divisor < 0x1p110f && maximum < divisor * 0x1p40f) {
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(recip) : "f"(divisor));
+      recip *= 0x1.00000cp+0f;
+      r1 = pack_bf16_pair(recip, recip);
+      const float low = recip - __uint_as_float(r1 << 16);
+      r2 = pack_bf16_pair(low, low);
+    } else {
+      recip = __frcp_rn(divisor);
+      if (kSplitQuotient)
+#pragma unroll
+        for (int i = 0; i < (F32 ? 1 : 16 * NIT); ++i) {
+          V[i] = pack_bf16_pair(mul2(unpack_bf16_pair(V[i]), pack2(recip, recip)));
+          asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(V[i]) : "r"(0x44804480u)); // 1024
+          asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(V[i]) : "r"(0xc480c480u));
+        }
+    }
+    const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
 
-    auto code_pair = [&](int i, int &c0, int &c1) { // codes of pair i (block i / 16, element 16 (i % 16) + a)
+    // codes of pair i (block i / 16, element 16 (i % 16) + a), the first group's in the low byte
+    auto code_pair = [&](int i) {
       if (F32) {
         float q0, q1;
         unpack2(div2_exact(PF[F32 ? i : 0], y2, nb2), q0, q1);
-        c0 = max(sat_s8(q0), -127);
-        c1 = max(sat_s8(q1), -127);
-      } else {
-        codes_of(pack_bf16_pair(div2_bf16(unpack_bf16_pair(V[F32 ? 0 : i]), y2)), c0, c1);
+        return code_bytes_127(q0, q1);
       }
+      uint32_t q;
+      if (kSplitQuotient)
+        asm("{\n.reg .b32 t;\nmul.rn.bf16x2 t, %1, %3;\nfma.rn.bf16x2 %0, %1, %2, t;\n}" : "=r"(q) : "r"(V[F32 ? 0 : i]), "r"(r1), "r"(r2));
+      else
+        q = pack_bf16_pair(div2_bf16(unpack_bf16_pair(V[F32 ? 0 : i]), y2));
+      return code_bytes(q);
     };
-    auto flush_codes = [&](int8_t *dst) { // every lane copies 2 x 16 bytes of each block's 1024 columns
+    auto flush_codes = [&](int8_t *dst) { // every thread copies row a of both its groups
       __syncwarp();
+      int8_t *to = dst + row * columns + col0;
 #pragma unroll
-      for (int part = 0; part < 2 * NIT; ++part) {
-        const uint32_t col = copy_col + part * 512u;
-        if (col < columns)
-          *reinterpret_cast<uint4 *>(dst + row * columns + col) = lds128(copy_addr + part * 576u);
+      for (int it = 0; it < NIT; ++it) {
+        const uint4 x = lds128(code_rd + kCodeBytes * it), y = lds128((code_rd ^ 16u) + kCodeBytes * it);
+        if (col0 + 1024u * it < columns)
+          *reinterpret_cast<uint4 *>(to + 1024u * it) = make_uint4(__byte_perm(x.x, x.y, 0x6420), __byte_perm(x.z, x.w, 0x6420),
+                                                                   __byte_perm(y.x, y.y, 0x6420), __byte_perm(y.z, y.w, 0x6420));
+        if (col0 + 1024u * it + 256u < columns)
+          *reinterpret_cast<uint4 *>(to + 1024u * it + 256u) = make_uint4(__byte_perm(x.x, x.y, 0x7531), __byte_perm(x.z, x.w, 0x7531),
+                                                                          __byte_perm(y.x, y.y, 0x7531), __byte_perm(y.z, y.w, 0x7531));
       }
       __syncwarp();
     };
-#define DIFB200_STAGE(J)                     \
-  {                                          \
-    int ca, cb;                              \
-    emit(16 * it + (J), ca, cb);             \
-    sts8<16 * (J)>(code_a + 1152u * it, ca); \
-    sts8<16 * (J)>(code_b + 1152u * it, cb); \
-  }
+#define DIFB200_STAGE(J) sts16<32 * (J)>(((J) & 4) ? code_wr_odd : code_wr_even, emit(16 * it + (J)));
 #define DIFB200_STAGE_ALL                                                                                     \
   _Pragma("unroll") for (int it = 0; it < NIT; ++it) {                                                        \
+    const uint32_t code_wr_even = code_wr + kCodeBytes * it, code_wr_odd = (code_wr ^ 16u) + kCodeBytes * it; \
     DIFB200_STAGE(0) DIFB200_STAGE(1) DIFB200_STAGE(2) DIFB200_STAGE(3) DIFB200_STAGE(4) DIFB200_STAGE(5)     \
     DIFB200_STAGE(6) DIFB200_STAGE(7) DIFB200_STAGE(8) DIFB200_STAGE(9) DIFB200_STAGE(10) DIFB200_STAGE(11)   \
     DIFB200_STAGE(12) DIFB200_STAGE(13) DIFB200_STAGE(14) DIFB200_STAGE(15)                                   \
   }
     float rm = 0.0f;
-    // Residual of an element (reference cpu_executor.cpp:262-305): r = fma(-code, stored, value).
-    auto residual_pair = [&](int i, int c0, int c1, float &r0, float &r1) {
+    // Residuals of a pair (reference cpu_executor.cpp:262-305): r = fma(-code, stored, value).
+    auto residual_pair = [&](int i, uint32_t codes, float &r0, float &r1) {
       float x0, x1;
       unpack2(F32 ? PF[F32 ? i : 0] : unpack_bf16_pair(V[F32 ? 0 : i]), x0, x1);
-      r0 = __fmaf_rn(-(float)c0, stored, x0 * (1.0f / kCarry));
-      r1 = __fmaf_rn(-(float)c1, stored, x1 * (1.0f / kCarry));
+      r0 = __fmaf_rn(-(float)(int8_t)codes, stored, x0 * (1.0f / kCarry));
+      r1 = __fmaf_rn(-(float)(int8_t)(codes >> 8), stored, x1 * (1.0f / kCarry));
     };
     {
-      auto emit = [&](int i, int &c0, int &c1) {
-        code_pair(i, c0, c1);
+      auto emit = [&](int i) {
+        const uint32_t codes = code_pair(i);
         if (RESIDUAL) {
           float r0, r1;
-          residual_pair(i, c0, c1, r0, r1);
+          residual_pair(i, codes, r0, r1);
           asm("max.f32 %0, %0, %1, %2;" : "+f"(rm) : "f"(fabsf(r0)), "f"(fabsf(r1)));
         }
+        return codes;
       };
       DIFB200_STAGE_ALL
     }
@@ -588,28 +613,23 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       if (lane == 0)
         redp[total_warps + warp] = rm;
       row_barrier();
-      rm = 0.0f;
-      for (int w = 0; w < warps_per_row; ++w)
-        rm = fmaxf(rm, redp[total_warps + slot * warps_per_row + w]);
+      rm = lane < warps_per_row ? redp[total_warps + slot * warps_per_row + lane] : 0.0f;
+      rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
       const float rscale = row_scale(rm, 1.0f);
       const float rscale_bf16 = round_bf16_number(rscale);
       if (wrow == 0 && lane == 0)
         p.rscales[row] = (SIGNED && !F32) ? rscale_bf16 : rscale;
       const float rdivisor = F32 ? rscale : rscale_bf16, rrecip = __frcp_rn(rdivisor);
       const uint64_t ry2 = pack2(rrecip, rrecip), rnb2 = pack2(-rdivisor, -rdivisor);
-      auto emit = [&](int i, int &c0, int &c1) {
-        int f0, f1;
+      auto emit = [&](int i) {
         float r0, r1;
-        code_pair(i, f0, f1);
-        residual_pair(i, f0, f1, r0, r1);
+        residual_pair(i, code_pair(i), r0, r1);
         if (F32) {
           float q0, q1;
           unpack2(div2_exact(pack2(r0, r1), ry2, rnb2), q0, q1);
-          c0 = max(sat_s8(q0), -127);
-          c1 = max(sat_s8(q1), -127);
-        } else {
-          codes_of(pack_bf16_pair(div2_bf16(round_bf16_2(pack2(r0, r1)), ry2)), c0, c1);
+          return code_bytes_127(q0, q1);
         }
+        return code_bytes(pack_bf16_pair(div2_bf16(round_bf16_2(pack2(r0, r1)), ry2)));
       };
       DIFB200_STAGE_ALL
       flush_codes(p.rcodes);
@@ -645,53 +665,32 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   return launched(cudaGetLastError(), "convrot256_kernel launch");
 }
 
-// One block of 1024 columns per warp: the fp32, residual and norm forms, packing, and calls of few rows.
+// The form of a row of `blocks` blocks of 1024 columns, one per warp: threads and CTAs per SM, and whether a warp requests
+// its next row before it works on this one. Up to 8 blocks several rows share a CTA; wider rows are a CTA each, and two or
+// three CTAs per SM hide one another's barriers. us per call, one block per warp with 80 registers, 24 warps per SM and a
+// prefetch / 64 registers, 32 warps and none / 80 registers and none:
+//   33272 x 3072 72.8 / 78.5 / 76.6, 16384 x 8192 91.9 / 99.0 / 102.4, 4608 x 12288 42.1 / 49.2 / 48.2,
+//   9216 x 15360 (one CTA of 128 registers with a prefetch) 105.8 / 117.4 / -; signed 98.3 / 107.3 / 108.1 (8192),
+//   fp32 106.5 / 112.1 / 111.5 (8192), but 13.0 / 13.1 / 12.3 (4159 x 3072). Three blocks per warp, which save per-row work, were
+//   the best form before the codes were converted in pairs, and are no longer (9216 x 3072 23.2, now 21.5).
+// Signed rows that are all resident at once want the shortest path (333 x 3072 4.1 / 4.4 / 4.4).
+// A norm in front needs its registers for three tensors in flight (33272 x 3072 198 / 186 / 174), residual outputs
+// are arithmetic (4000 x 8192 46.8 / 43.0 / 41.6).
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
 int launch_single(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
-  // Plain rows of more than 8 blocks are a CTA each, and several CTAs per SM hide one another's barriers: three of 9 or
-  // 10 warps, two of 11 or more (64 registers; 11 and 12 warps leave 80). 3333 rows, two CTAs with a prefetch ->
-  // this: 10240 columns 39.2 -> 35.6 us, fp32 41.9 -> 39.2; 12288 columns 43.8 -> 42.4 us, fp32 47.4 -> 45.3. The
-  // fp32 values of 13 warps and more do not leave room for a second CTA: one with a prefetch (9216 x 15360, two
-  // CTAs -> this, 147 -> 142 us, in two inputs 152 -> 142).
-  if (blocks > 8u) {
-    if constexpr (EXTRA == kPlain && !RESIDUAL)
-      return F32 && blocks > 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream)
-             : blocks == 11u || blocks == 12u ? launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 384, 2>(p, stream)
-                                            : launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 512, 2>(p, stream);
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
-  }
-  if constexpr (EXTRA == kNorm) {
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream); // 24 warps, three tensors in flight
-  } else if constexpr (EXTRA != kPlain || (RESIDUAL && !F32)) {
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
-  } else if constexpr (RESIDUAL) {
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
-  } else {
-    // 64 registers and 32 warps per SM hide the load latency without a prefetch. Sign masks and the fp32 division on
-    // short rows want 80 registers and 24 warps (16384 x 3072: fp32 53.0 -> 51.6 us, both 55.6 -> 53.7 us; 4000 x 1024
-    // signed 9.8 -> 8.6 us; but 9216 x 8192 fp32 72.8 -> 77.2 us), and signed rows that are all resident at once the
-    // shortest path (700 x 3072 7.5 -> 6.4 us, 77 x 8192 fp32 6.4 -> 5.4 us).
-    if constexpr (SIGNED)
-      if (p.rows * blocks <= (uint64_t)sm_count() * 16u)
-        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
-    if constexpr (SIGNED || F32)
-      if (blocks <= 3u)
-        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
-    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 4>(p, stream);
-  }
-}
-
-// Packing without the scale search: the division by the equalisation vector wants warps, not registers or blocks
-// per warp (three blocks with 168 registers -> this: 9216 x 3072 59.7 -> 41.2 us, 3072 x 8192 57.9 -> 37.1 us,
-// 3333 x 10240 83.8 -> 53.5 us).
-template <bool SIGNED, bool F32>
-int launch_equalised(const QuantParams &p, cudaStream_t stream) {
-  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
   if (blocks > 12u)
-    return launch_single<SIGNED, F32, false, kEqualise>(p, stream);
-  return blocks <= 8u ? launch_form<SIGNED, F32, false, kEqualise, 1, false, 256, 3>(p, stream)
-                      : launch_form<SIGNED, F32, false, kEqualise, 1, false, 384, 2>(p, stream);
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
+  constexpr bool kArithmetic = EXTRA != kPlain || RESIDUAL;
+  if (blocks > 8u)
+    return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, !kArithmetic, 384, 2>(p, stream);
+  if constexpr (!kArithmetic && SIGNED)
+    if (p.rows * blocks <= (uint64_t)sm_count() * 16u)
+      return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
+  if constexpr (!kArithmetic && F32 && !SIGNED)
+    if (blocks <= 3u)
+      return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
+  return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, !kArithmetic, 256, 3>(p, stream);
 }
 
 template <bool SIGNED>
@@ -701,7 +700,7 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     return fail(kUnsupported, "QuantizeInt8Rows: weight packing (MSE scale, input equalisation) exists for "
                               "the 256-wide variants without residual outputs");
   if (pack && !p.mse)
-    return f32 ? launch_equalised<SIGNED, true>(p, stream) : launch_equalised<SIGNED, false>(p, stream);
+    return f32 ? launch_single<SIGNED, true, false, kEqualise>(p, stream) : launch_single<SIGNED, false, false, kEqualise>(p, stream);
   if (f32) {
     if (pack)
       return launch_single<SIGNED, true, false, kPack>(p, stream);
@@ -714,23 +713,16 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     return launch_single<SIGNED, false, true, kPlain>(p, stream);
   if (norm)
     return launch_single<SIGNED, false, false, kNorm>(p, stream);
-  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
-  const uint64_t all = p.rows * blocks, sms = (uint64_t)sm_count();
-  if (pack) // the scale search is arithmetic that the form for few rows need not hide
-    return all <= sms * 24u || blocks == 1u ? launch_single<SIGNED, false, false, kPack>(p, stream)
-                                            : launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream);
-  // Blocks per warp. Three save the per-row work of two warps but leave a third of the warps, at half the
-  // occupancy, and the last round of the machine is mostly empty. Rows of up to 8 blocks that three divide: from
-  // three rounds (9216 x 3072 30.2 -> 28.8 us; below, 3333 x 3072 signed takes 18.9 us with three, under 14.9 with
-  // one). Others of up to 8 keep one (4159 x 8192: 34.3 us against 41.5 us, the last warp would idle on a third of its
-  // slots). Wider rows have one CTA per row with one block, the better form for longer. One against three, 12288
-  // columns: 3333 rows 42.4 / 43.3 us, 4159 rows 52.8 / 50.6, 6000 rows 71.6 / 69.4; 15360 columns: 3333 rows
-  // 53.5 / 51.6. Signed: 12288 columns 3333 rows 45.3 / 47.5, 6000 rows 75.2 / 75.2, 16384 rows 191.8 / 188.0;
-  // 15360 columns 9216 rows 138.5 / 142.3.
-  const uint64_t rounds = all / (sms * 16u * 3u); // of the blocks that run at once with three per warp
-  const bool three = blocks <= 8u ? blocks % 3u == 0 && rounds >= 3u : SIGNED ? blocks <= 12u && rounds >= 10u : rounds >= 5u;
-  return three ? launch_form<SIGNED, false, false, kPlain, 3, true, 256, 2>(p, stream)
-               : launch_single<SIGNED, false, false, kPlain>(p, stream);
+  if (pack) {
+    // The scale search is arithmetic per row as well as per element: three blocks per warp where they divide the row
+    // (12288 x 3072 77.5 -> 62.1 us, 3072 x 12288 with equalisation 101.7 -> 94.9; 3072 x 8192 signed, whose last warp
+    // would be a third empty, 69.3 -> 75.2) and the rows are more than the machine holds at once.
+    const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+    return blocks % 3u == 0u && p.rows * blocks > (uint64_t)sm_count() * 24u
+               ? launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream)
+               : launch_single<SIGNED, false, false, kPack>(p, stream);
+  }
+  return launch_single<SIGNED, false, false, kPlain>(p, stream);
 }
 
 } // namespace

@@ -162,3 +162,25 @@ def test_layer_norm_prologue_of_rows_with_a_large_mean(K, impl):
     want = ops.quantize_int8_rows([normed], impl)
     got = ops.layer_norm_modulate_quant(x, w, b, s, h, 1e-6, impl)
     assert torch.equal(want[1], got[1]) and torch.equal(want[0], got[0])
+
+
+@pytest.mark.parametrize("impl", [2, 3])
+@pytest.mark.parametrize("K", [256, 3072, 9216])
+def test_quotients_out_of_the_two_part_products_range(impl, K):
+    """Rows whose scale is so large that the reciprocal's low part would be subnormal, and clips so small that quotients
+    overflow: such rows take the fp32 quotient. The rows beside them do not."""
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(K + impl)
+    x = ob.bf16_to_f32(activations(rng, 24, K))
+    x[3] *= np.float32(2.0 ** 113)
+    x[4] *= np.float32(2.0 ** 106)
+    x[5] *= np.float32(2.0 ** -120)
+    x[6] = 0
+    x = ob.f32_to_bf16(x)
+    for clip in (1.0, 1.0e-3, 1.0e-6):
+        want = ob.orc().quantize_int8_rows([x], impl, clip, False)
+        got = ops.quantize_int8_rows([to_torch_bf16(x)], impl, clip)
+        assert _bits_equal(want[1], got[1]) and _bits_equal(want[0], got[0]), clip
+    for clip in (1.0e-12, 1.0e-30):  # beyond the integers the reference converts to: saturated by sign
+        codes = ops.quantize_int8_rows([to_torch_bf16(x)], impl, clip)[0].cpu().numpy()
+        assert np.all(codes[want[0] > 0] == 127) and np.all(codes[want[0] < 0] == -128), clip

@@ -35,3 +35,22 @@ def test_bf16_quotient_for_every_pair_of_significands():
 
     product = v * (np.float32(1.0) / s)
     assert np.array_equal(bf16(product), bf16((v.astype(np.float64) / s.astype(np.float64)).astype(np.float32)))
+
+
+def test_bf16_quotient_in_two_bf16_parts_for_every_pair_of_significands():
+    """bf16(v / s) as fma(v, r1, bf16(v r2)) rounded once to bf16, with r1 = bf16(r), r2 = bf16(r - r1), as the 256-wide
+    quantiser forms it, for all 128 x 128 pairs. r is 1 + 6 / 2^23 times an approximate reciprocal that is within 2^-23
+    of the exact one: every r between 1 + 18 / 2^25 and 1 + 30 / 2^25 times the exact reciprocal has to do (steps of 2^-25)."""
+    def bf16(x):  # nearest even, 8 significant bits; x exact in float64
+        m, e = np.frexp(x)
+        return np.ldexp(np.rint(m * 256.0), e - 8)
+
+    v = np.arange(128, 256, dtype=np.float64)[:, None]
+    s = np.arange(128, 256, dtype=np.float64)[None, :]
+    want = bf16(v / s)  # no quotient is within 2^-17 of a rounding boundary
+    for step in range(16, 33):
+        r = (1.0 / s) * (1.0 + step * 2.0 ** -25)
+        r1 = bf16(r)
+        r2 = bf16(r - r1)
+        got = bf16(v * r1 + bf16(v * r2))  # 8 + 8 bits and a term at most 2^9 times smaller: exact in float64
+        assert np.array_equal(got, want), step
