@@ -58,25 +58,20 @@ constexpr int kTile = 128;          // queries per tile, keys per tile, head dim
 constexpr int kStages = 4;          // K/V ring depth (Q passes through stages 2 and 3 first)
 constexpr uint32_t kKBytes = 128 * 128;        // int8 [128 keys x 128]
 constexpr uint32_t kVBytes = 128 * 128 * 2;    // bf16 [128 keys x 128] as two 64-wide halves
-constexpr uint32_t kKsBytes = 128 * 8;         // (key scale, mask bias) per key, as float4 per key pair
+constexpr uint32_t kKsBytes = 128 * 8;         // the tile's 128 key scales, then its 128 mask entries
 constexpr uint32_t kStageBytes = kKBytes + kVBytes + kKsBytes;
 constexpr int kThreads = 640;      // 4 control warps, 2 x 8 softmax warps
 constexpr uint32_t kPartialBytes = 32 * 32 * 4; // split form: a [32 rows x 32 columns] fp32 partial output
 constexpr uint32_t kOutBoxBytes = 32 * 128;    // a warp's output staging: two [32 rows x 64 bf16] boxes
 constexpr float kHeadroom = 24.0f;  // powers of two that the running maximum goes beyond a row's scores when it moves
 constexpr float kLeastSum = 1.0f / (1u << 25); // of a running maximum: its largest p is above 2^-(kHeadroom + 1)
-// The bits of the float C = 1.5 * 2^23: added to an INT32 score they make the float C + score. One integer addition per
-// score (B2 S4608 H24 374 -> 387 us, 1101 tokens 27.2 -> 27.0); a bf16 MMA that puts them under the scores takes it out,
-// but the INT8 MMAs that add to its result are of another kind and K, between which no order is promised, and with a wait
-// for its completion in between the same calls took 439 and 27.7 us.
-constexpr uint32_t kScoreBias = 0x4B400000u;
 constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
 constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + 256 + kPairBytes;
 
 struct AttnParams {
   const int8_t *q8;      // [B,Sq,H,128]
   const float *qs;       // [B,Sq,H]
-  const float2 *ksmb;    // [B,KV,S_pad/2] x float4 (ks'_j, ks'_j+1, bias_j, bias_j+1)
+  const float *table;    // [B,KV,S_pad/128] x (128 key scales ks'_j, 128 mask entries)
   const float *tile_bound; // [B,KV,S_pad/128] max over the tile's valid keys of |k8_j| * ks'_j
   uint32_t B, Sq, Sk, H, KV, S_pad; // Sq query tokens, Sk key tokens (S_pad = Sk rounded up to 128)
   uint16_t *out;         // [B,Sq,H,128] bf16
@@ -105,23 +100,24 @@ __device__ __forceinline__ void report(DeviceStatus *status, uint32_t role, uint
   }
 }
 
-// The entry of one key: (ks', -C ks') and the key's contribution to its tile's bound, from the key scale
-// and the sum of squares of its codes.
-__device__ __forceinline__ void key_entry(float ks, int n2, float &k22, float &bias, float &bound) {
+// The scale of one key, rounded to the 22 significant bits of the contract, and the key's contribution to its tile's
+// bound, from the key scale and the sum of squares of its codes.
+__device__ __forceinline__ void key_entry(float ks, int n2, float &k22, float &bound) {
   uint32_t bits = __float_as_uint(ks);
   bits = (bits + 1u + ((bits >> 2) & 1u)) & ~3u; // nearest-even to 22 significant bits
   k22 = __uint_as_float(bits);
-  bias = -12582912.0f * k22;
   bound = __fmul_rn(__fsqrt_rn((float)n2), k22);
+  if (!(fabsf(k22) < INFINITY))
+    k22 = __int_as_float(0x7fc00000); // whatever the score, such a key makes its rows NaN
 }
 
-// Builds the per-key table [B,KV,S_pad] of (ks', -C * ks') with C = 1.5 * 2^23: the key scales of
-// the [B,S,KV] row order re-laid contiguous along keys, stored per key pair as
-// (ks'_j, ks'_j+1, bias_j, bias_j+1) so that one 16-byte load feeds one packed fma. The softmax
-// threads turn an INT32 score into fp32 with one integer add, f' = as_float(acc + bits(C)) =
-// C + acc exactly, and then u = fma(f', ks', -C * ks') = RN(acc * ks'): rounding ks to 22
-// significant bits makes C * ks' exact, so the fused form has the single rounding of a plain
-// multiply. Masked and padding keys carry (0, -inf), which yields u = -inf.
+// Builds the key table [B,KV,S_pad/128]: per 128-key tile its key scales, re-laid from the [B,S,KV] row order to be
+// contiguous along keys, then its mask entries. u = RN(float(acc) * ks') is the conversion and one multiplication; a
+// 16-byte load brings the scales of four keys. (An integer addition of the bits of 1.5 * 2^23 in the place of the
+// conversion, with -1.5 * 2^23 ks' beside every scale, takes twice the loads: B2 S4608 H24 390 us, now 382.) Masked and padding keys carry the scale 0 and the mask entry -inf, which
+// is added: u = -inf. The others' entry is 0, and a segment of 32 keys (what a softmax thread takes of a step) says in
+// its first entry whether it has such keys at all: +0 there means none, and the softmax leaves the entries unread. In
+// a segment that has some, the first key's entry is -inf or -0.
 // Also writes, per 128-key tile, the largest |k8_j|_2 * ks'_j of its valid keys: with |q8_i|_2 it
 // bounds every score of the tile (Cauchy-Schwarz on the integer codes).
 // One block of 128 threads per (batch, kv head, key tile), one thread per key.
@@ -137,7 +133,7 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
   const uint32_t kvh = (blockIdx.x / mine) % KV;
   const uint32_t b = blockIdx.x / (mine * KV);
   const uint32_t j = tile * kTile + threadIdx.x;
-  float k22 = 0.0f, bias = -INFINITY, bound = 0.0f;
+  float k22 = 0.0f, mask = -INFINITY, bound = 0.0f;
   if (j < S && (key_valid == nullptr || key_valid[(uint64_t)b * S + j] != 0)) {
     const uint4 *row = reinterpret_cast<const uint4 *>(k8 + (((uint64_t)b * S + j) * KV + kvh) * kTile);
     int n2 = 0;
@@ -149,11 +145,14 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
       n2 = __dp4a((int)w.z, (int)w.z, n2);
       n2 = __dp4a((int)w.w, (int)w.w, n2);
     }
-    key_entry(ks[((uint64_t)b * S + j) * KV + kvh], n2, k22, bias, bound);
+    key_entry(ks[((uint64_t)b * S + j) * KV + kvh], n2, k22, bound);
+    mask = 0.0f;
   }
-  float *t = table + (((uint64_t)b * KV + kvh) * S_pad + (j & ~1u)) * 2u + (j & 1u);
+  if (__any_sync(0xffffffffu, mask != 0.0f) && (threadIdx.x & 31) == 0 && mask == 0.0f)
+    mask = -0.0f;
+  float *t = table + (((uint64_t)b * KV + kvh) * tiles + tile) * (2u * kTile) + threadIdx.x;
   t[0] = k22;
-  t[2] = bias;
+  t[kTile] = mask;
   __shared__ float warp_max[4];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
@@ -211,7 +210,13 @@ attention_operands_kernel(const OperandParams p) {
   if (blockIdx.x < p.key_blocks) {
     const uint32_t tiles = p.S_pad / kTile, tile = blockIdx.x % tiles, kvh = (blockIdx.x / tiles) % p.KV,
                    b = blockIdx.x / (tiles * p.KV);
+    __shared__ uint32_t masked[4]; // whether a segment of 32 keys has masked ones
+    if (threadIdx.x < 4)
+      masked[threadIdx.x] = 0u;
+    __syncthreads();
+    float *t = p.table + (((uint64_t)b * p.KV + kvh) * tiles + tile) * (2u * kTile);
     float most = 0.0f;
+    uint32_t first_valid = 0; // (thread 0) of the four segments' first keys
 #pragma unroll
     for (int step = 0; step < 4; ++step) {
       const uint32_t j = tile * kTile + step * 32u + warp * 4u + (lane >> 3);
@@ -227,19 +232,24 @@ attention_operands_kernel(const OperandParams p) {
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1)
         n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-      float k22 = 0.0f, bias = -INFINITY, bound = 0.0f;
+      float k22 = 0.0f, mask = -INFINITY, bound = 0.0f;
       if (exists) {
         reinterpret_cast<uint4 *>(p.k8 + row * kTile)[part] = codes;
         if (part == 0)
           p.ks[row] = scale;
-        if (p.key_valid == nullptr || p.key_valid[(uint64_t)b * p.S + j] != 0)
-          key_entry(scale, n2, k22, bias, bound);
+        if (p.key_valid == nullptr || p.key_valid[(uint64_t)b * p.S + j] != 0) {
+          key_entry(scale, n2, k22, bound);
+          mask = 0.0f;
+        }
       }
       most = fmaxf(most, bound);
       if (part == 0) {
-        float *t = p.table + (((uint64_t)b * p.KV + kvh) * p.S_pad + (j & ~1u)) * 2u + (j & 1u);
-        t[0] = k22;
-        t[2] = bias;
+        t[j % kTile] = k22;
+        t[kTile + j % kTile] = mask;
+        if (mask != 0.0f)
+          masked[step] = 1u;
+        else
+          first_valid |= 1u << step;
       }
     }
     __shared__ float warp_max[8];
@@ -251,6 +261,9 @@ attention_operands_kernel(const OperandParams p) {
       for (int w = 1; w < 8; ++w)
         most = fmaxf(most, warp_max[w]);
       p.tile_bound[((uint64_t)b * p.KV + kvh) * tiles + tile] = most;
+      for (int step = 0; step < 4; ++step)
+        if (masked[step] != 0u && (first_valid >> step & 1u))
+          t[kTile + 32 * step] = -0.0f;
     }
   } else {
 #pragma unroll
@@ -344,13 +357,13 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const uint32_t k_dst = stage_addr + s * kStageBytes, v_dst = k_dst + kKBytes, t_dst = v_dst + kVBytes;
     const uint32_t tile = key_tile(i);
     const int32_t key0 = (int32_t)(tile * kTile);
-    const float2 *table = p.ksmb + ((uint64_t)batch * p.KV + kvh) * p.S_pad;
+    const float *table = p.table + ((uint64_t)batch * p.KV + kvh) * p.S_pad * 2u;
     ptx::mbar_expect_tx(kv_full + 8 * s, kKBytes + kVBytes + kKsBytes);
     ptx::tma_load_4d(k_dst, &map_k, kv_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
     ptx::tma_load_4d(v_dst, &map_v, kv_full + 8 * s, 0, (int32_t)kvh, key0, (int32_t)batch);
     ptx::tma_load_4d(v_dst + kVBytes / 2, &map_v, kv_full + 8 * s, 64, (int32_t)kvh, key0, (int32_t)batch);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-                     "r"(t_dst), "l"(reinterpret_cast<uint64_t>(table + (uint64_t)tile * kTile)),
+                     "r"(t_dst), "l"(reinterpret_cast<uint64_t>(table + (uint64_t)tile * (2u * kTile))),
                  "r"(kKsBytes), "r"(kv_full + 8 * s)
                  : "memory");
   };
@@ -633,6 +646,12 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
     const uint64_t A2 = pack2(A, A);
     uint32_t r[32];
+    uint32_t masked = 0; // the first mask entry of this thread's segment of the step whose scores are in r
+    // the key scales of this thread's 32 columns of a step; the mask entries stand kTile floats behind
+    auto segment = [&](uint32_t g) {
+      return reinterpret_cast<const float *>(base_ptr + (stage_addr - base) + ((g >> 1) % kStages) * kStageBytes + kKBytes +
+                                             kVBytes) + (g & 1u) * 64u + hf * 32u;
+    };
     uint32_t pair_phase = 0;
     float *pair_slot = reinterpret_cast<float *>(base_ptr + (pair_mem - base)) + t * 256u + row_in_tile;
     // A word of each of the row's two threads to the other (bounded like every wait).
@@ -671,42 +690,109 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       __syncwarp();
       if (lane == 0)
         ptx::mbar_arrive(p_full + 8 * t);
+      masked = __float_as_uint(segment(0)[kTile]);
     }
-    for (uint32_t g = 0; g < n_steps && alive; ++g) {
-      const uint32_t h = g & 1u;
-      const uint32_t s = (g >> 1) % kStages;
-      const float4 *tab = reinterpret_cast<const float4 *>(base_ptr + (stage_addr - base) + s * kStageBytes +
-                                                           kKBytes + kVBytes) + h * 32u + hf * 16u;
-      uint32_t pk[16];
-      uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull}; // 8 partial row sums as packed fp32 pairs
-      if (fixed_max) {
+    // A loop for each way to the maximum: with both in one the registers are shared out worse (B2 S4608 H24 with q 4 times
+    // larger, whose maximum runs, 588 us; 535 with a loop of its own).
+    if (fixed_max) {
+      for (uint32_t g = 0; g < n_steps && alive; ++g) {
+        const float4 *tab = reinterpret_cast<const float4 *>(segment(g));
+        // u of four neighbouring keys: float(acc) * ks', plus the mask entries where the segment has masked keys
+        auto scores4 = [&](int j, bool with_mask, uint64_t &u01, uint64_t &u23) {
+          const float4 ks = tab[j >> 2];
+          u01 = pack2((float)(int32_t)r[j], (float)(int32_t)r[j + 1]);
+          u23 = pack2((float)(int32_t)r[j + 2], (float)(int32_t)r[j + 3]);
+          if (with_mask) { // (a product of 0 and the entry -0 is the sum +0, as without an entry)
+            const float4 mask = tab[(kTile + j) >> 2];
+            u01 = fma2(u01, pack2(ks.x, ks.y), pack2(mask.x, mask.y));
+            u23 = fma2(u23, pack2(ks.z, ks.w), pack2(mask.z, mask.w));
+          } else {
+            u01 = mul2(u01, pack2(ks.x, ks.y));
+            u23 = mul2(u23, pack2(ks.z, ks.w));
+          }
+        };
+        uint32_t pk[16];
+        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull}; // 8 partial row sums as packed fp32 pairs
+        auto weights = [&](int j, uint64_t e2) {
+          float p0, p1;
+          unpack2(e2, p0, p1);
+          p0 = ex2(p0);
+          p1 = ex2(p1);
+          pk[j >> 1] = pack_bf16(p0, p1);
+          sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
+        };
         const uint64_t negm2 = pack2(-m_run, -m_run);
+        if (masked == 0u) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float4 kk = tab[j >> 1]; // (ks'_j, ks'_j+1, -C ks'_j, -C ks'_j+1)
-          const float f0 = __uint_as_float(r[j] + kScoreBias); // C + acc, exact
-          const float f1 = __uint_as_float(r[j + 1] + kScoreBias);
-          const uint64_t u2 = fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w));
-          float e0, e1;
-          unpack2(fma2(u2, A2, negm2), e0, e1);
-          const float p0 = ex2(e0), p1 = ex2(e1);
+          for (int j = 0; j < 32; j += 4) {
+            uint64_t u01, u23;
+            scores4(j, false, u01, u23);
+            weights(j, fma2(u01, A2, negm2));
+            weights(j + 2, fma2(u23, A2, negm2));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            uint64_t u01, u23;
+            scores4(j, true, u01, u23);
+            weights(j, fma2(u01, A2, negm2));
+            weights(j + 2, fma2(u23, A2, negm2));
+          }
+        }
+        {
+          float a0, a1, b0, b1;
+          unpack2(add2(sum2[0], sum2[1]), a0, a1);
+          unpack2(add2(sum2[2], sum2[3]), b0, b1);
+          l += (a0 + a1) + (b0 + b1);
+        }
+        // P of this step takes the place of the last one's when that one's P.V is done: the Q.K^T of step g + 1 was issued
+        // behind it, so its completion says so.
+        if (!await_scores(g + 1u))
+          break;
+        if (g + 1u < n_steps) {
+          ptx::tc_fence_after();
+          ptx::tmem_ld_32x32(s_tmem + 32u * hf, r);
+          masked = __float_as_uint(segment(g + 1u)[kTile]);
+        }
+        ptx::tmem_st_32x16(p_tmem + 16u * hf, pk);
+        ptx::tmem_ld_wait();
+        ptx::tmem_st_wait();
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          ptx::mbar_arrive(p_full + 8 * t);
+      }
+    } else {
+      for (uint32_t g = 0; g < n_steps && alive; ++g) {
+        const float4 *tab = reinterpret_cast<const float4 *>(segment(g));
+        uint32_t pk[16];
+        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull}; // 8 partial row sums as packed fp32 pairs
+        auto weights = [&](int j, uint64_t e2) {
+          float p0, p1;
+          unpack2(e2, p0, p1);
+          p0 = ex2(p0);
+          p1 = ex2(p1);
           sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
           pk[j >> 1] = pack_bf16(p0, p1);
-        }
-      } else {
+        };
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float4 kk = tab[j >> 1];
-          const float f0 = __uint_as_float(r[j] + kScoreBias);
-          const float f1 = __uint_as_float(r[j + 1] + kScoreBias);
-          float u0, u1;
-          unpack2(fma2(pack2(f0, f1), pack2(kk.x, kk.y), pack2(kk.z, kk.w)), u0, u1);
-          r[j] = __float_as_uint(u0);
-          r[j + 1] = __float_as_uint(u1);
-          float &acc_max = mx4[(j >> 1) & 3];
-          asm("max.f32 %0, %0, %1, %2;" : "+f"(acc_max) : "f"(u0), "f"(u1));
+        for (int j = 0; j < 32; j += 4) {
+          const float4 ks = tab[j >> 2];
+          float u[4];
+          unpack2(mul2(pack2((float)(int32_t)r[j], (float)(int32_t)r[j + 1]), pack2(ks.x, ks.y)), u[0], u[1]);
+          unpack2(mul2(pack2((float)(int32_t)r[j + 2], (float)(int32_t)r[j + 3]), pack2(ks.z, ks.w)), u[2], u[3]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            r[j + i] = __float_as_uint(u[i]);
         }
+        if (masked != 0u)
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            r[j] = __float_as_uint(__uint_as_float(r[j]) + reinterpret_cast<const float *>(tab)[kTile + j]);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2)
+          asm("max.f32 %0, %0, %1, %2;" : "+f"(mx4[(j >> 1) & 3]) : "f"(__uint_as_float(r[j])), "f"(__uint_as_float(r[j + 1])));
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         // power-of-two running maximum, of the whole row
         mx = fmaxf(mx, exchange(mx));
@@ -750,35 +836,31 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const float neg_m = (m_run == -INFINITY) ? 0.0f : -m_run;
         const uint64_t negm2 = pack2(neg_m, neg_m);
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          float e0, e1;
-          unpack2(fma2(pack2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), A2, negm2), e0, e1);
-          const float p0 = ex2(e0), p1 = ex2(e1);
-          sum2[(j >> 1) & 3] = add2(sum2[(j >> 1) & 3], pack2(p0, p1));
-          pk[j >> 1] = pack_bf16(p0, p1);
+        for (int j = 0; j < 32; j += 2)
+          weights(j, fma2(pack2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), A2, negm2));
+        {
+          float a0, a1, b0, b1;
+          unpack2(add2(sum2[0], sum2[1]), a0, a1);
+          unpack2(add2(sum2[2], sum2[3]), b0, b1);
+          l += (a0 + a1) + (b0 + b1);
         }
+        // P of this step takes the place of the last one's when that one's P.V is done: the Q.K^T of step g + 1 was issued
+        // behind it, so its completion says so.
+        if (!await_scores(g + 1u))
+          break;
+        if (g + 1u < n_steps) {
+          ptx::tc_fence_after();
+          ptx::tmem_ld_32x32(s_tmem + 32u * hf, r);
+          masked = __float_as_uint(segment(g + 1u)[kTile]);
+        }
+        ptx::tmem_st_32x16(p_tmem + 16u * hf, pk);
+        ptx::tmem_ld_wait();
+        ptx::tmem_st_wait();
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          ptx::mbar_arrive(p_full + 8 * t);
       }
-      {
-        float a0, a1, b0, b1;
-        unpack2(add2(sum2[0], sum2[1]), a0, a1);
-        unpack2(add2(sum2[2], sum2[3]), b0, b1);
-        l += (a0 + a1) + (b0 + b1);
-      }
-      // P of this step takes the place of the last one's when that one's P.V is done: the Q.K^T of step g + 1 was issued
-      // behind it, so its completion says so.
-      if (!await_scores(g + 1u))
-        break;
-      if (g + 1u < n_steps) {
-        ptx::tc_fence_after();
-        ptx::tmem_ld_32x32(s_tmem + 32u * hf, r);
-      }
-      ptx::tmem_st_32x16(p_tmem + 16u * hf, pk);
-      ptx::tmem_ld_wait();
-      ptx::tmem_st_wait();
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0)
-        ptx::mbar_arrive(p_full + 8 * t);
     }
     const float l_own = l;
     if (alive)
@@ -1125,8 +1207,8 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       }, nullptr, nullptr))
     return rc;
 
-  float2 *table = static_cast<float2 *>(scratch);
-  float *tile_bound = reinterpret_cast<float *>(table + B * KV * s_pad);
+  float *table = static_cast<float *>(scratch);
+  float *tile_bound = table + B * KV * s_pad * 2;
   // q / k still in bf16: one launch quantises them and, with k, also builds the key table
   if (source && (source->q || source->k)) {
     if (chunk || (reinterpret_cast<uintptr_t>(source->q) | reinterpret_cast<uintptr_t>(source->k)) & 15)
@@ -1139,7 +1221,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     o.qs = const_cast<float *>(qs);
     o.ks = const_cast<float *>(ks);
     o.key_valid = key_valid;
-    o.table = reinterpret_cast<float *>(table);
+    o.table = table;
     o.tile_bound = tile_bound;
     o.q_rows = source->q ? B * Sq * H : 0;
     o.S = (uint32_t)S;
@@ -1157,8 +1239,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     const uint64_t blocks = B * KV * (count[0] + count[1]);
     if (blocks > 0x7fffffffull)
       return fail(kUnsupported, "Attention(INT8): problem too large");
-    key_table_kernel<<<(unsigned)blocks, 128, 0, stream>>>(k8, ks, key_valid, reinterpret_cast<float *>(table),
-                                                           tile_bound, (uint32_t)S, (uint32_t)KV, s_pad, begin[0],
+    key_table_kernel<<<(unsigned)blocks, 128, 0, stream>>>(k8, ks, key_valid, table, tile_bound, (uint32_t)S, (uint32_t)KV, s_pad, begin[0],
                                                            count[0], begin[1], count[1]);
     if (int rc = launched(cudaGetLastError(), "key_table_kernel launch"))
       return rc;
@@ -1166,7 +1247,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
   AttnParams p{};
   p.q8 = q8;
   p.qs = qs;
-  p.ksmb = table;
+  p.table = table;
   p.tile_bound = tile_bound;
   p.out = static_cast<uint16_t *>(out_bf16);
   p.B = (uint32_t)B;

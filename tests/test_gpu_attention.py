@@ -410,3 +410,42 @@ def test_attention_split_where_its_clusters_fill_the_device(ops, rest):
         assert float((a - b).norm() / b.norm()) <= 3e-4
         assert float((a != b).double().mean()) <= 0.01
     ops.poll_status()
+
+
+@pytest.mark.parametrize("q_gain", [1.0, 6.0])
+@pytest.mark.parametrize("from_bf16", [False, True])
+def test_attention_masks_at_the_edges_of_the_tables_segments(ops, q_gain, from_bf16):
+    """Key masks against segments of 32 keys, whose first entry says whether any of them is masked: none, the first key
+    alone, the last alone, all but the first, all; both builders of the key table. Against the contract, and the same
+    bits as a call in which the masked keys' codes and values are others."""
+    import torch
+    rng = np.random.default_rng(17)
+    B, S, H, KV = 2, 300, 2, 1
+    q, k, v = _qkv(rng, B, S, H, KV)
+    q = ob.f32_to_bf16(ob.bf16_to_f32(q) * np.float32(q_gain))
+    valid = np.ones((B, S), np.uint8)
+    valid[0, 32] = 0           # first of a segment
+    valid[0, 95] = 0           # last of one
+    valid[0, 129:160] = 0      # all but the first
+    valid[0, 192:224] = 0      # a whole segment
+    valid[1, 0] = 0
+    valid[1, 255:] = 0
+    q8, qs = ob.orc().quantize_int8_rows([q.reshape(-1, 128)], 1)
+    k8, ks = ob.orc().quantize_int8_rows([k.reshape(-1, 128)], 1)
+    q8, k8 = q8.reshape(B, S, H, 128), k8.reshape(B, S, KV, 128)
+    want = ob.bf16_to_f32(ob.orc().attention_int8(q8, qs, k8, ks, v, valid))
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+
+    def run(k, v, k8, ks):
+        if from_bf16:
+            return ops.attention(to_torch_bf16(q), to_torch_bf16(k), to_torch_bf16(v), t(valid))
+        return ops.attention_int8(t(q8), t(qs), t(k8), t(ks), to_torch_bf16(v), t(valid))
+
+    got = run(k, v, k8, ks)
+    assert rel_l2(ob.bf16_to_f32(from_torch_bf16(got)), want) <= 2e-3
+    gone = valid == 0
+    k2, v2 = k.copy(), v.copy()
+    k2[gone], v2[gone] = ob.f32_to_bf16(np.float32([9.0]))[0], ob.f32_to_bf16(np.float32([-7.0]))[0]
+    k82, ks2 = ob.orc().quantize_int8_rows([k2.reshape(-1, 128)], 1)
+    assert torch.equal(run(k2, v2, k82.reshape(k8.shape), ks2).view(torch.int16), got.view(torch.int16))
+    ops.poll_status()
