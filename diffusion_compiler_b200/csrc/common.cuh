@@ -100,6 +100,17 @@ __device__ __forceinline__ uint32_t load_produced(const uint16_t *p) {
   asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ uint4 load_produced(const uint4 *p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// 16 bytes that are read once and were not written by a kernel that may still run.
+__device__ __forceinline__ uint4 load_streamed(const void *p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 inline cudaLaunchAttribute dependent_launch() {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -180,6 +180,50 @@ def test_linear_int8_scaled_narrow_and_split_tiles(ops, monkeypatch, form, M, K,
     ops.poll_status()
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32, 33])  # 8, 16 and 32 rows per form; 33 is the tile kernel's
+@pytest.mark.parametrize("K,N", [(16, 16), (48, 1), (80, 131), (3072, 40), (3136, 24), (12288, 17), (16, 3000)])
+def test_linear_of_few_rows_bit_exact(ops, M, K, N):
+    """The kernel of few rows: chunks of 64 k that end early, fewer chunks than warps, warps whose last batch is short,
+    columns that do not fill 16, and each number of 8-row groups; with codes of -128, bias, GELU and the accumulators."""
+    import torch
+    g = torch.Generator().manual_seed(M + N + K)
+    x8, w8 = (torch.randint(-128, 128, s, dtype=torch.int8, generator=g) for s in ((M, K), (N, K)))
+    xs, ws = torch.rand(M, generator=g) * 0.01, torch.rand(N, generator=g) * 0.01
+    bias = torch.randn(N, generator=g).to(torch.bfloat16)
+    want_acc = (x8.double() @ w8.double().T).to(torch.int32)  # exact: below 2^53
+    want = ((want_acc.float() * xs[:, None]) * ws[None]).to(torch.bfloat16)
+    want_b = (want.float() + bias.float()[None]).to(torch.bfloat16)
+    dev = [t.cuda() for t in (x8, w8, xs, ws)]
+    got, acc = ops.linear_int8_scaled(*dev, want_acc=True)
+    assert torch.equal(acc.cpu(), want_acc)
+    assert torch.equal(got.cpu(), want)
+    assert torch.equal(ops.linear_int8_scaled(*dev, bias=bias.cuda()).cpu(), want_b)
+    gelu = ops.linear_int8_scaled(*dev, bias=bias.cuda(), gelu=True).cpu()
+    want_g = ob.orc().gelu_tanh(want_b.view(torch.int16).numpy().view(np.uint16))
+    assert rel_l2(gelu.float().numpy(), ob.bf16_to_f32(want_g)) <= 2e-3
+    ops.poll_status()
+
+
+@pytest.mark.parametrize("rows", [1, 16, 30])
+def test_w8a8_linear_of_few_rows_matches_two_calls(ops, rows):
+    """The single call, whose weights are requested before the quantiser in front is complete, back to back."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = [torch.randn((rows, 3072), generator=g, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    w8 = torch.randint(-127, 128, (520, 3072), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(520, generator=g, device="cuda") * 0.01
+    want = []
+    for a in x:
+        codes, scales = ops.quantize_int8_rows([a], 2)
+        torch.cuda.synchronize()
+        want.append(ops.linear_int8_scaled(codes, w8, scales, ws))
+        torch.cuda.synchronize()
+    got = [ops.w8a8_linear(a, w8, ws) for a in x + x]
+    for i, out in enumerate(got):
+        assert torch.equal(out.view(torch.int16), want[i % 4].view(torch.int16)), i
+    ops.poll_status()
+
+
 def test_w8a8_linear_end_to_end_single_layer(ops):
     """The single-layer benchmark case (M=1024, K=N=3072, H256ConvRot activations, bias): GPU quant + GEMM chained."""
     import torch
