@@ -523,29 +523,15 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     const float divisor = (F32 ? scale : scale_bf16) * kCarry;
     if (wrow == 0 && lane == 0)
       p.scales[row] = stored;
-    // The bf16 variants' quotients as bf16: V r1 + V r2 with the two bf16 parts of r = (1 + 6 / 2^23) / divisor, a product
-    // and a fused sum that rounds once. For every pair of 8-bit significands that is the rounded quotient, with the
-    // reciprocal anywhere between 1 + 2^-25 and 1 + 43 / 2^25 times the exact one, and the approximate one is within 2^-23.
-    // Beside the fp32 product and its rounding it saves the conversions on either side. Rows whose divisor leaves no
-    // room for the low part, or whose quotients could overflow, get their quotients first, bounded, and the factors 1 and 0.
     constexpr bool kSplitQuotient = !F32 && !RESIDUAL;
-    float recip;
-    uint32_t r1 = 0x3f803f80u, r2 = 0u;
-    if (kSplitQuotient && divisor < 0x1p110f && maximum < divisor * 0x1p40f) {
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(recip) : "f"(divisor));
-      recip *= 0x1.00000cp+0f;
-      r1 = pack_bf16_pair(recip, recip);
-      const float low = recip - __uint_as_float(r1 << 16);
-      r2 = pack_bf16_pair(low, low);
-    } else {
+    float recip = 0.0f;
+    SplitReciprocal split;
+    if (!kSplitQuotient || !split.of(divisor, maximum)) {
       recip = __frcp_rn(divisor);
       if (kSplitQuotient)
 #pragma unroll
-        for (int i = 0; i < (F32 ? 1 : 16 * NIT); ++i) {
-          V[i] = pack_bf16_pair(mul2(unpack_bf16_pair(V[i]), pack2(recip, recip)));
-          asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(V[i]) : "r"(0x44804480u)); // 1024
-          asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(V[i]) : "r"(0xc480c480u));
-        }
+        for (int i = 0; i < (F32 ? 1 : 16 * NIT); ++i)
+          V[i] = bounded_quotients(V[i], recip);
     }
     const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
 
@@ -556,11 +542,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
         unpack2(div2_exact(PF[F32 ? i : 0], y2, nb2), q0, q1);
         return code_bytes_127(q0, q1);
       }
-      uint32_t q;
-      if (kSplitQuotient)
-        asm("{\n.reg .b32 t;\nmul.rn.bf16x2 t, %1, %3;\nfma.rn.bf16x2 %0, %1, %2, t;\n}" : "=r"(q) : "r"(V[F32 ? 0 : i]), "r"(r1), "r"(r2));
-      else
-        q = pack_bf16_pair(div2_bf16(unpack_bf16_pair(V[F32 ? 0 : i]), y2));
+      const uint32_t v = V[F32 ? 0 : i];
+      const uint32_t q = kSplitQuotient ? split.quotients(v) : pack_bf16_pair(div2_bf16(unpack_bf16_pair(v), y2));
       return code_bytes(q);
     };
     auto flush_codes = [&](int8_t *dst) { // every thread copies row a of both its groups

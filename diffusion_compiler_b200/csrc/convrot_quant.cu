@@ -146,24 +146,36 @@ convrot4096_kernel(const QuantParams p) {
     if (lane == 0)
       redp[warp] = m;
     __syncthreads(); // also: every read of the natural-order row is done before codes overwrite it
-    m = 0.0f;
-    for (int w = 0; w < warps; ++w)
-      m = fmaxf(m, redp[w]);
+    m = lane < warps ? redp[lane] : 0.0f;
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     const float scale = row_scale(m * (1.0f / kCarry), clip), scale_bf16 = round_bf16_number(scale);
-    const float stored = F32 ? scale : scale_bf16, divisor = stored * kCarry, recip = __frcp_rn(divisor);
+    const float stored = F32 ? scale : scale_bf16, divisor = stored * kCarry;
+    constexpr bool kSplitQuotient = !F32 && !RESIDUAL; // the rotated values are packed as bf16 pairs for it
+    uint32_t V[kSplitQuotient ? 16 : 1];
+    if (kSplitQuotient)
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        V[kSplitQuotient ? j : 0] = pack_bf16_pair(P[j]);
+    float recip = 0.0f;
+    SplitReciprocal split;
+    if (!kSplitQuotient || !split.of(divisor, m)) {
+      recip = __frcp_rn(divisor);
+      if (kSplitQuotient)
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          V[kSplitQuotient ? j : 0] = bounded_quotients(V[kSplitQuotient ? j : 0], recip);
+    }
     const uint64_t y2 = pack2(recip, recip), nb2 = pack2(-divisor, -divisor);
     if (threadIdx.x == 0)
       p.scales[row] = stored;
 
-    auto code_pair = [&](int i, int &ca, int &cb) {
+    auto code_pair = [&](int i) { // the codes of both positions, the first's in the low byte
       if (F32) {
         float q0, q1;
         unpack2(div2_exact(P[i], y2, nb2), q0, q1);
-        ca = max(sat_s8(q0), -127);
-        cb = max(sat_s8(q1), -127);
-      } else {
-        codes_of(pack_bf16_pair(div2_bf16(round_bf16_2(P[i]), y2)), ca, cb);
+        return code_bytes_127(q0, q1);
       }
+      return code_bytes(kSplitQuotient ? split.quotients(V[kSplitQuotient ? i : 0]) : pack_bf16_pair(div2_bf16(round_bf16_2(P[i]), y2)));
     };
     auto flush_codes = [&](int8_t *dst) { // every lane copies 2 x 16 bytes of its warp's 1024 columns
       __syncthreads();
@@ -175,30 +187,30 @@ convrot4096_kernel(const QuantParams p) {
     // group J of a block sits 256 J columns on; one byte per column with a 64-byte skew per 512 columns
 #define DIFB200_STAGE(J)                          \
   {                                               \
-    int ca, cb;                                   \
-    emit(J, ca, cb);                              \
-    sts8<256 * (J) + 64 * ((J) >> 1)>(code_a, ca); \
-    sts8<256 * (J) + 64 * ((J) >> 1)>(code_b, cb); \
+    const uint32_t codes = emit(J);               \
+    sts8<256 * (J) + 64 * ((J) >> 1)>(code_a, (int)codes); \
+    sts8<256 * (J) + 64 * ((J) >> 1)>(code_b, (int)(codes >> 8)); \
   }
 #define DIFB200_STAGE_ALL                                                                                   \
   DIFB200_STAGE(0) DIFB200_STAGE(1) DIFB200_STAGE(2) DIFB200_STAGE(3) DIFB200_STAGE(4) DIFB200_STAGE(5)     \
   DIFB200_STAGE(6) DIFB200_STAGE(7) DIFB200_STAGE(8) DIFB200_STAGE(9) DIFB200_STAGE(10) DIFB200_STAGE(11)   \
   DIFB200_STAGE(12) DIFB200_STAGE(13) DIFB200_STAGE(14) DIFB200_STAGE(15)
     float rm = 0.0f;
-    auto residual_pair = [&](int i, int ca, int cb, float &r0, float &r1) { // cpu_executor.cpp:262-305
+    auto residual_pair = [&](int i, uint32_t codes, float &r0, float &r1) { // cpu_executor.cpp:262-305
       float x0, x1;
       unpack2(F32 ? P[i] : round_bf16_2(P[i]), x0, x1);
-      r0 = __fmaf_rn(-(float)ca, stored, x0 * (1.0f / kCarry));
-      r1 = __fmaf_rn(-(float)cb, stored, x1 * (1.0f / kCarry));
+      r0 = __fmaf_rn(-(float)(int8_t)codes, stored, x0 * (1.0f / kCarry));
+      r1 = __fmaf_rn(-(float)(int8_t)(codes >> 8), stored, x1 * (1.0f / kCarry));
     };
     {
-      auto emit = [&](int i, int &ca, int &cb) {
-        code_pair(i, ca, cb);
+      auto emit = [&](int i) {
+        const uint32_t codes = code_pair(i);
         if (RESIDUAL) {
           float r0, r1;
-          residual_pair(i, ca, cb, r0, r1);
+          residual_pair(i, codes, r0, r1);
           asm("max.f32 %0, %0, %1, %2;" : "+f"(rm) : "f"(fabsf(r0)), "f"(fabsf(r1)));
         }
+        return codes;
       };
       DIFB200_STAGE_ALL
     }
@@ -208,27 +220,22 @@ convrot4096_kernel(const QuantParams p) {
       if (lane == 0)
         redp[warps + warp] = rm;
       __syncthreads();
-      rm = 0.0f;
-      for (int w = 0; w < warps; ++w)
-        rm = fmaxf(rm, redp[warps + w]);
+      rm = lane < warps ? redp[warps + lane] : 0.0f;
+      rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
       const float rscale = row_scale(rm, 1.0f), rstored = F32 ? rscale : round_bf16_number(rscale);
       if (threadIdx.x == 0)
         p.rscales[row] = rstored;
       const float rrecip = __frcp_rn(rstored);
       const uint64_t ry2 = pack2(rrecip, rrecip), rnb2 = pack2(-rstored, -rstored);
-      auto emit = [&](int i, int &ca, int &cb) {
-        int f0, f1;
+      auto emit = [&](int i) {
         float r0, r1;
-        code_pair(i, f0, f1);
-        residual_pair(i, f0, f1, r0, r1);
+        residual_pair(i, code_pair(i), r0, r1);
         if (F32) {
           float q0, q1;
           unpack2(div2_exact(pack2(r0, r1), ry2, rnb2), q0, q1);
-          ca = max(sat_s8(q0), -127);
-          cb = max(sat_s8(q1), -127);
-        } else {
-          codes_of(pack_bf16_pair(div2_bf16(round_bf16_2(pack2(r0, r1)), ry2)), ca, cb);
+          return code_bytes_127(q0, q1);
         }
+        return code_bytes(pack_bf16_pair(div2_bf16(round_bf16_2(pack2(r0, r1)), ry2)));
       };
       DIFB200_STAGE_ALL
       flush_codes(p.rcodes);

@@ -111,16 +111,42 @@ __device__ __forceinline__ uint64_t unpack_bf16_pair(uint32_t packed) {
 }
 __device__ __forceinline__ uint64_t round_bf16_2(uint64_t v) { return unpack_bf16_pair(pack_bf16_pair(v)); }
 
+// Quotients of packed bf16 pairs by one bf16 divisor, as bf16: v r1 + v r2 with the two bf16 parts of r = (1 + 6 / 2^23) / divisor,
+// a product and a fused sum that rounds once. For every pair of 8-bit significands that is the rounded quotient, with the
+// reciprocal anywhere between 1 + 2^-25 and 1 + 43 / 2^25 times the exact one, and the approximate one is within 2^-23.
+// Beside the fp32 product and its rounding it saves the conversions on either side.
+struct SplitReciprocal {
+  uint32_t r1 = 0x3f803f80u, r2 = 0u; // 1 and 0: quotients made before
+  // False where the divisor leaves no room for the low part, or quotients (of values up to `maximum`) could overflow.
+  __device__ __forceinline__ bool of(float divisor, float maximum) {
+    if (!(divisor < 0x1p110f && maximum < divisor * 0x1p40f))
+      return false;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(divisor));
+    r *= 0x1.00000cp+0f;
+    r1 = pack_bf16_pair(r, r);
+    const float low = r - __uint_as_float(r1 << 16);
+    r2 = pack_bf16_pair(low, low);
+    return true;
+  }
+  __device__ __forceinline__ uint32_t quotients(uint32_t v) const {
+    uint32_t q;
+    asm("{\n.reg .b32 t;\nmul.rn.bf16x2 t, %1, %3;\nfma.rn.bf16x2 %0, %1, %2, t;\n}" : "=r"(q) : "r"(v), "r"(r1), "r"(r2));
+    return q;
+  }
+};
+// The fp32 product's quotients, within +-1024 (NaN stays NaN): what codes are made of saturates long before.
+__device__ __forceinline__ uint32_t bounded_quotients(uint32_t v, float recip) {
+  uint32_t q = pack_bf16_pair(mul2(unpack_bf16_pair(v), pack2(recip, recip)));
+  asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(q) : "r"(0x44804480u));
+  asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(q) : "r"(0xc480c480u));
+  return q;
+}
+
 __device__ __forceinline__ int sat_s8(float v) {
   int r;
   asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(r) : "f"(v));
   return r;
-}
-
-// INT8 codes of a packed pair of bf16 quotients: round to nearest even, saturate.
-__device__ __forceinline__ void codes_of(uint32_t q, int &c0, int &c1) {
-  c0 = sat_s8(__uint_as_float(q << 16));
-  c1 = sat_s8(__uint_as_float(q & 0xffff0000u));
 }
 
 // INT8 codes of two quotients in the low 16 bits: round to nearest even, saturate, NaN gives 0. Two conversions to 32-bit integers
