@@ -4,11 +4,13 @@
 
 The shared library carries every CUDA kernel, the device-resident C entry points
 (include/difb200/difb200.h) and the reference-compatible backend plugin entry points
-(include/difb200/abi.h). nvcc cross-compiles without a GPU.
+(include/difb200/abi.h). nvcc cross-compiles without a GPU. Beside it stands _torch_calls.so, the binding
+that ops.py calls it through on torch tensors.
 """
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -18,6 +20,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "_obj")
 LIB_PATH = os.path.join(HERE, "libdifb200.so")
+CALLS_SOURCE = os.path.join(HERE, "binding", "torch_calls.cpp")
+CALLS_PATH = os.path.join(HERE, "_torch_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -56,7 +60,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def run(cmd):
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
-            raise RuntimeError("nvcc failed: %s\n%s\n%s" % (" ".join(cmd), res.stdout, res.stderr))
+            raise RuntimeError("%s failed: %s\n%s\n%s" % (cmd[0], " ".join(cmd), res.stdout, res.stderr))
         if verbose:
             sys.stderr.write(res.stderr)
 
@@ -64,7 +68,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
         list(pool.map(run, jobs))
     if jobs or force or _stale(LIB_PATH, objs):
         run([nvcc, "-shared", "-o", LIB_PATH] + objs + ["-Xlinker", "--no-undefined", "-ldl", "-lpthread"])
+    if force or _stale(CALLS_PATH, [CALLS_SOURCE] + headers):
+        run(_calls_command())
     return LIB_PATH
+
+
+def _calls_command():
+    """The binding for torch tensors: an extension module beside the library, which it finds there ($ORIGIN)."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"))
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"], os.path.join(ROOT, "include")]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+             "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
+            + ["-I" + d for d in includes] + [CALLS_SOURCE, "-o", CALLS_PATH, "-L" + os.path.join(root, "lib"), "-L" + HERE,
+                                              "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-l:libdifb200.so",
+                                              "-Wl,-rpath,$ORIGIN"])
 
 
 if __name__ == "__main__":

@@ -12,6 +12,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib
+from ._calls import calls as _calls
 
 EPILOGUE_BIAS = 1
 EPILOGUE_GELU_TANH = 2
@@ -19,6 +20,13 @@ EPILOGUE_GELU_TANH = 2
 
 _PTR_ARRAYS = [C.c_void_p * n for n in range(9)]
 _WIDTH_ARRAYS = [C.c_uint64 * n for n in range(9)]
+
+
+def _done(result):
+    """What the native binding made of a call: its outputs, or the status of one that failed."""
+    if type(result) is int:
+        _lib.check(result)
+    return result
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -54,6 +62,10 @@ def quantize_int8_rows(parts: Sequence[torch.Tensor], implementation: int = 2, c
     [, residual codes, residual scales]). ``implementation`` is the Int8RowQuantization value.
     ``out`` = (codes, scales) writes into existing contiguous buffers (e.g. a slice of an
     all-gather buffer)."""
+    if out is None and clip_tensor is None and not residual:
+        result = _calls().quantize_int8_rows(parts, implementation, clip)
+        if result is not None:
+            return _done(result)
     if isinstance(parts, torch.Tensor):
         parts = [parts]
     parts = [_require(p, torch.bfloat16, "input") for p in parts]
@@ -91,6 +103,9 @@ def rms_norm_modulate_quant(x: torch.Tensor, weight: Optional[torch.Tensor], sca
                             shift: torch.Tensor, epsilon: float = 1e-5, implementation: int = 2, clip: float = 1.0):
     """RmsNormModulate (explicit scale / shift) + QuantizeInt8Rows in one kernel: bf16 [M, K] inputs
     -> (codes i8 [M, K], row scales f32 [M]); the normalised tensor is never written."""
+    result = _calls().norm_modulate_quant(x, weight, None, scale, shift, epsilon, implementation, clip)
+    if result is not None:
+        return _done(result)
     x = _require(x, torch.bfloat16, "x")
     scale, shift = _require(scale, torch.bfloat16, "scale"), _require(shift, torch.bfloat16, "shift")
     if weight is not None:
@@ -111,6 +126,9 @@ def layer_norm_modulate_quant(x: torch.Tensor, weight: torch.Tensor, bias: torch
     """LayerNormModulate + QuantizeInt8Rows in one kernel: x bf16 [M, K], weight / bias bf16 [K],
     scale / shift bf16 [M / r, K] (r rows of x share one modulation row) -> (codes i8 [M, K], row
     scales f32 [M])."""
+    result = None if bias is None else _calls().norm_modulate_quant(x, weight, bias, scale, shift, epsilon, implementation, clip)
+    if result is not None:
+        return _done(result)
     x = _require(x, torch.bfloat16, "x")
     weight, bias = _require(weight, torch.bfloat16, "weight"), _require(bias, torch.bfloat16, "bias")
     scale, shift = _require(scale, torch.bfloat16, "scale"), _require(shift, torch.bfloat16, "shift")
@@ -192,6 +210,10 @@ def w8a8_linear(x: torch.Tensor, w8: torch.Tensor, col_scales: torch.Tensor,
                 scratch: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> torch.Tensor:
     """The W8A8 int8-convrot linear in one call: quantize x [..,K] bf16, multiply with w8 [N,K].
     ``scratch`` = (codes int8 [M,K], row scales f32 [M]) may be passed to reuse buffers."""
+    if out is None and scratch is None:
+        result = _calls().w8a8_linear(x, w8, col_scales, bias, gelu, implementation, clip)
+        if result is not None:
+            return _done(result)
     x = _require(x, torch.bfloat16, "x")
     w8 = _require(w8, torch.int8, "w8")
     col_scales = _require(col_scales, torch.float32, "col_scales")
@@ -294,6 +316,10 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key_valid: Opti
               scale: Optional[float] = None, out: Optional[torch.Tensor] = None,
               scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
     """DiffIR Attention on bf16 q [B,S,H,128], k/v [B,S,KV,128] through the INT8 lowering."""
+    if out is None and scratch is None:
+        result = _calls().attention(q, k, v, key_valid, scale)
+        if result is not None:
+            return _done(result)
     q = _require(q, torch.bfloat16, "q")
     k = _require(k, torch.bfloat16, "k")
     v = _require(v, torch.bfloat16, "v")
