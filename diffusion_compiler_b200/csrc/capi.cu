@@ -21,6 +21,10 @@ int w8a8_linear(const void *x_bf16, const int8_t *w, const float *col_scales, co
                 DeviceStatus *status_words) {
   if (!x_bf16 || !codes_scratch || !scales_scratch)
     return fail(kInvalidArgument, "w8a8_linear: null input or scratch pointer");
+  int rc = kOk;
+  if (w8a8_few_rows(x_bf16, w, col_scales, bias_bf16, epilogue, implementation, clip, M, N, K, codes_scratch, scales_scratch,
+                    out_bf16, stream, &rc))
+    return rc;
   const void *parts[1] = {x_bf16};
   const uint64_t widths[1] = {K};
   if (int rc = quantize_int8_rows(parts, widths, 1, M, implementation, clip, nullptr, codes_scratch,

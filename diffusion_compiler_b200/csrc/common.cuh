@@ -55,6 +55,7 @@ void set_wait_limit_ns(unsigned long long ns); // 0 restores the default
 // k-block. take_...() returns that k-block (0xffffffff = none) and disarms.
 void withhold_next_gemm_load(uint32_t k_block);
 uint32_t take_withheld_gemm_load();
+bool gemm_load_is_withheld();
 // Device memory for one call: allocated and freed in the order of the call's stream, so that neither
 // another stream nor another thread can hold the same bytes meanwhile (also under stream capture, where the two become
 // nodes of the graph). It comes from a pool of this library that keeps at most 4 MB per device across

@@ -31,11 +31,8 @@
 namespace difb200 {
 namespace {
 
-// Shared memory per warp: 4 groups x 256 fp32 (two 16x32-word transposes whose rows are padded, so that every access is
-// free of conflicts at a constant offset), reused for the code pairs and the sampled elements of the scale search.
-constexpr int kWarpBytes = 4608;
-constexpr uint32_t kRowPitch = 144;                  // bytes of a row of 16 pairs in the transpose
-constexpr uint32_t kHalfBytes = 16 * kRowPitch;      // a half-warp's area
+// Shared memory per warp: the rotation's transpose, reused for the code pairs and the sampled elements of the scale search.
+constexpr int kWarpBytes = kWarpBytes256;
 constexpr uint32_t kCodeHalfBytes = 544, kCodeBytes = 2 * kCodeHalfBytes; // code pairs of a half-warp's two groups, of a block
 
 // kPack: weight rows with the scale search (and input equalisation where given), kEqualise: without the search.
@@ -325,38 +322,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
           }
         }
       }
-      // stage 0 (stride 1) and stage 1 (stride 4)
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        bfly(P[4 * q], P[4 * q + 1], P[4 * q + 2], P[4 * q + 3]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        bfly(P[q], P[q + 4], P[q + 8], P[q + 12]);
-      // 16x16 transpose of pairs through shared memory.
-      {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float x0, x1, x2, x3;
-          unpack2(P[2 * c], x0, x1);
-          unpack2(P[2 * c + 1], x2, x3);
-          sts128(wr_addr + 16u * c, x0, x1, x2, x3);
-        }
-        __syncwarp();
-#define DIFB200_READ_PAIR(J) P[J] = lds64<(J) * kRowPitch>(rd_addr);
-        DIFB200_READ_PAIR(0) DIFB200_READ_PAIR(1) DIFB200_READ_PAIR(2) DIFB200_READ_PAIR(3)
-        DIFB200_READ_PAIR(4) DIFB200_READ_PAIR(5) DIFB200_READ_PAIR(6) DIFB200_READ_PAIR(7)
-        DIFB200_READ_PAIR(8) DIFB200_READ_PAIR(9) DIFB200_READ_PAIR(10) DIFB200_READ_PAIR(11)
-        DIFB200_READ_PAIR(12) DIFB200_READ_PAIR(13) DIFB200_READ_PAIR(14) DIFB200_READ_PAIR(15)
-#undef DIFB200_READ_PAIR
-        __syncwarp();
-      }
-      // Now P[j] = element 16*j + a of both groups. stage 2 (stride 16), stage 3 (stride 64).
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        bfly(P[4 * q], P[4 * q + 1], P[4 * q + 2], P[4 * q + 3]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        bfly(P[q], P[q + 4], P[q + 8], P[q + 12]);
+      rotate_pairs(P, wr_addr, rd_addr);
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         m = absmax2(m, P[j]);

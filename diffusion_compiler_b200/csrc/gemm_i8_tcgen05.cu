@@ -32,7 +32,8 @@
 //             CTAs. The only remaining software signal across the pair is the epilogue's arrive
 //             on the leader's accumulator-empty barrier, with CTA-scope release: a cluster-scope
 //             release arrive per k-block costs microseconds while TMA traffic is in flight.
-#include "common.cuh"
+// Problems of few rows have kernels of their own (linear_few_rows.cu).
+#include "gemm_common.cuh"
 #include "ptx.cuh"
 
 #include <cstdio>
@@ -109,52 +110,12 @@ constexpr size_t smem_bytes() {
          Cfg<CTAS, BN>::kStagingBytes + Cfg<CTAS, BN>::kScaleBytes + 256;
 }
 
-enum : uint32_t { kEpiBias = 1u, kEpiGeluTanh = 2u };
-
-struct GemmParams {
-  const float *row_scales;
-  const float *col_scales;
-  const uint16_t *bias;
-  uint16_t *out;
-  int32_t *acc_out;
-  uint32_t M, N, K;
-  uint32_t epilogue;
-  uint32_t split;   // CTAS = 1: CTAs of a cluster that share one tile's k-blocks (1 = no cluster)
-  uint32_t tma_store; // 1: outputs leave through TMA stores (needs N % 8 == 0, aligned out)
-  uint32_t weights_first; // 1: w is not written by the kernel in front, its first blocks are requested before that one is done
-  uint32_t withhold_kb; // test aid: the loads of this k-block are never issued (0xffffffff = none)
-  unsigned long long wait_ns; // limit of every bounded wait
-  DeviceStatus *status;
-};
-
 __device__ __forceinline__ void report_timeout(DeviceStatus *status, uint32_t role, uint32_t detail) {
   if (atomicExch(&status->flag, 1u) == 0u) {
     status->kernel = 2u;
     status->role = role;
     status->detail = detail;
   }
-}
-
-__device__ __forceinline__ float gelu_tanh(float v) {
-  // Reference form (cpu_executor.cpp:93-113): 0.5 * v * (1 + tanh(u)), u = 0.79788456 * (v +
-  // 0.044715 * v^3). The reference's fp32 sum 1 + tanh(u) cancels for negative v, and that
-  // rounding is part of its result, so the same three roundings are kept here and only tanh
-  // itself is computed differently: tanh|u| = 1 - 2 / (e^(2|u|) + 1) with two MUFU ops
-  // (ex2, rcp), absolute error below one ulp of 1.
-  constexpr float kA = 0.7978845608028654f * 2.0f * 1.4426950408889634f;
-  constexpr float kB = kA * 0.044715f;
-  const float t = fmaf(kB, v * v, kA) * v; // 2u * log2(e), same sign as v
-  float e, r;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(fabsf(t)));
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
-  const float th = copysignf(fmaf(-2.0f, r, 1.0f), v);
-  return __fmul_rn(__fmul_rn(0.5f, v), __fadd_rn(1.0f, th));
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  uint32_t packed;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
-  return packed;
 }
 
 template <int CTAS, int BN>
@@ -535,119 +496,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// ---- few rows ----
-// A problem of at most 32 rows reads every weight for next to no arithmetic, and what the tile kernel spends around its
-// main loop (tensor memory, barriers, the first loads' latency, a chain of k-blocks, a cluster's exchange) is most of its
-// time. Here a CTA takes 16 columns, whose weights go from global memory straight into the registers of warp-wide integer MMAs
-// (16 columns x 32 k x 8 rows; which k stands in which slot is the same for both operands and otherwise free, so every lane
-// loads 16 contiguous bytes), all of a warp's first loads before it waits for the quantiser. Eight warps share the k
-// range in turns of 64 bytes and add their INT32 sums through shared memory.
-constexpr int kFewWarps = 8, kFewBatch = 6; // chunks of 64 bytes of k that a warp requests at once
-struct FewParams {
-  const int8_t *x, *w;
-  GemmParams g;
-};
-
-__device__ __forceinline__ void mma_s8_16x8x32(int32_t (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-template <int GROUPS> // of 8 rows
-__global__ void __launch_bounds__(32 * kFewWarps, 2)
-gemm_i8_few_rows_kernel(const FewParams f) {
-  const GemmParams &p = f.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint32_t n0 = blockIdx.x * 16u;
-  const bool low_ok = n0 + g < p.N, high_ok = n0 + 8u + g < p.N;
-  const int8_t *low = f.w + (size_t)(low_ok ? n0 + g : 0) * p.K, *high = f.w + (size_t)(high_ok ? n0 + 8u + g : 0) * p.K;
-  const uint32_t chunks = (p.K + 63u) / 64u;
-  uint4 wl[kFewBatch], wh[kFewBatch];
-  auto at = [&](uint32_t first, int u) { return (first + warp + kFewWarps * u) * 64u + 16u * t; }; // this lane's k of a chunk
-  auto load_weights = [&](uint32_t first) {
-#pragma unroll
-    for (int u = 0; u < kFewBatch; ++u) {
-      const uint32_t k = at(first, u);
-      wl[u] = wh[u] = make_uint4(0, 0, 0, 0);
-      if (k < p.K) {
-        if (low_ok)
-          wl[u] = load_streamed(low + k);
-        if (high_ok)
-          wh[u] = load_streamed(high + k);
-      }
-    }
-  };
-  if (p.weights_first)
-    load_weights(0);
-  grid_dependency_wait();
-  grid_dependents_launch();
-  if (!p.weights_first)
-    load_weights(0);
-  int32_t c[GROUPS][4] = {};
-  for (uint32_t first = 0; first < chunks; first += kFewWarps * kFewBatch) {
-    if (first != 0u)
-      load_weights(first);
-#pragma unroll
-    for (int q = 0; q < GROUPS; ++q) {
-      const uint32_t row = 8u * q + g;
-      uint4 x[kFewBatch];
-#pragma unroll
-      for (int u = 0; u < kFewBatch; ++u) {
-        const uint32_t k = at(first, u);
-        x[u] = make_uint4(0, 0, 0, 0);
-        if (k < p.K && row < p.M)
-          x[u] = load_produced(reinterpret_cast<const uint4 *>(f.x + (size_t)row * p.K + k));
-      }
-#pragma unroll
-      for (int u = 0; u < kFewBatch; ++u) {
-        mma_s8_16x8x32(c[q], wl[u].x, wh[u].x, wl[u].y, wh[u].y, x[u].x, x[u].y);
-        mma_s8_16x8x32(c[q], wl[u].z, wh[u].z, wl[u].w, wh[u].w, x[u].z, x[u].w);
-      }
-    }
-  }
-  __shared__ int32_t sums[kFewWarps][GROUPS * 8][16]; // [warp][row][column]
-#pragma unroll
-  for (int q = 0; q < GROUPS; ++q) {
-    sums[warp][8 * q + 2 * t][g] = c[q][0];
-    sums[warp][8 * q + 2 * t + 1][g] = c[q][1];
-    sums[warp][8 * q + 2 * t][g + 8] = c[q][2];
-    sums[warp][8 * q + 2 * t + 1][g + 8] = c[q][3];
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < 16u * p.M; i += 32 * kFewWarps) {
-    const uint32_t row = i >> 4, n = n0 + (i & 15u);
-    if (n >= p.N)
-      continue;
-    int32_t acc = 0;
-#pragma unroll
-    for (int w = 0; w < kFewWarps; ++w)
-      acc += sums[w][row][i & 15u];
-    if (p.acc_out)
-      p.acc_out[(size_t)row * p.N + n] = acc;
-    float y = __fmul_rn(__fmul_rn((float)acc, load_produced(p.row_scales + row)), load_produced(p.col_scales + n));
-    uint32_t bits = pack_bf16x2(y, 0.0f);
-    if (p.epilogue & kEpiBias)
-      bits = pack_bf16x2(__fadd_rn(__uint_as_float(bits << 16), bf16_bits_to_f32(load_produced(p.bias + n))), 0.0f);
-    if (p.epilogue & kEpiGeluTanh)
-      bits = pack_bf16x2(gelu_tanh(__uint_as_float(bits << 16)), 0.0f);
-    p.out[(size_t)row * p.N + n] = (uint16_t)bits;
-  }
-}
-
-template <int GROUPS>
-int launch_few_rows(const FewParams &f, cudaStream_t stream) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3((f.g.N + 15u) / 16u);
-  config.blockDim = dim3(32 * kFewWarps);
-  config.stream = stream;
-  cudaLaunchAttribute attr = dependent_launch();
-  config.attrs = &attr;
-  config.numAttrs = 1;
-  return launched(cudaLaunchKernelEx(&config, gemm_i8_few_rows_kernel<GROUPS>, f), "gemm_i8_few_rows_kernel launch");
-}
-
 // Tile form of a problem: CTAs per tile, tile columns, and the CTAs that share the k-blocks of a tile.
 struct Form {
   int ctas, tile_n, split;
@@ -698,16 +546,6 @@ Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
     }
   }
   return best;
-}
-
-// Whether the few-rows kernel takes a problem. Every CTA reads all rows' codes, which come from the same few lines of L2, so
-// its time grows with the rows and, beyond 16, with the weights. us of a linear, tile kernel -> this (K x N): 2 rows
-// 3072 x 3072 10.8 -> 5.3, 3072 x 9216 12.5 -> 7.8, 3072 x 16384 17.2 -> 11.5, 12288 x 3072 15.9 -> 10.6; 16 rows 11.2 -> 6.4,
-// 13.9 -> 10.8, 16.4 -> 14.9, 14.7 -> 13.3; 32 rows 11.0 -> 8.3, 14.0 -> 14.5, 17.2 -> 21.0, 15.1 -> 17.5.
-bool few_rows(uint64_t M, uint64_t N, uint64_t K) {
-  if (std::getenv("DIFB200_GEMM_FORM") || std::getenv("DIFB200_GEMM_CTAS"))
-    return false; // a tile form is forced
-  return M <= 16 || (M <= 32 && N * K <= (1ull << 24));
 }
 
 template <int CTAS, int BN>
@@ -804,10 +642,8 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   p.weights_first = weights_ready && p.withhold_kb == 0xffffffffu ? 1u : 0u;
   p.wait_ns = wait_limit_ns();
   p.status = status;
-  if (p.withhold_kb == 0xffffffffu && few_rows(M, N, K)) {
-    const FewParams f{x, w, p};
-    return M <= 8 ? launch_few_rows<1>(f, stream) : M <= 16 ? launch_few_rows<2>(f, stream) : launch_few_rows<4>(f, stream);
-  }
+  if (p.withhold_kb == 0xffffffffu && few_rows(M, N, K))
+    return launch_few_rows(x, w, p, stream);
 
   const Form form = choose_form(M, N, K);
   CUtensorMap map_a, map_b;

@@ -35,6 +35,11 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
 // weights_ready: the kernel launched last on the stream does not write w, and was launched plainly or waits for the
 // one before it: the first blocks of w are requested while that kernel still runs.
 
+// The same pair for the fewest rows in one launch; false: not a problem for it (or a call that the general way refuses).
+bool w8a8_few_rows(const void *x_bf16, const int8_t *w, const float *col_scales, const void *bias_bf16, uint32_t epilogue,
+                   int implementation, float clip, uint64_t M, uint64_t N, uint64_t K, int8_t *codes, float *scales,
+                   void *out_bf16, cudaStream_t stream, int *rc);
+
 // QuantizeInt8Rows -> LinearInt8Scaled [-> BiasAdd -> Gelu] on a bf16 [M,K] input; codes [M,K]
 // and row scales [M] are scratch supplied by the caller.
 int w8a8_linear(const void *x_bf16, const int8_t *w, const float *col_scales, const void *bias_bf16,

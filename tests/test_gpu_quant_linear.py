@@ -224,6 +224,37 @@ def test_w8a8_linear_of_few_rows_matches_two_calls(ops, rows):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("M,K", [(1, 256), (8, 768), (8, 1024), (4, 2048), (2, 3072), (3, 3072), (2, 2816), (1, 8192), (1, 9216),
+                                 (2, 4096), (9, 1024)])
+@pytest.mark.parametrize("N", [1, 17, 520, 9000])  # fewer tiles than the machine holds CTAs, and more
+def test_w8a8_linear_in_one_launch_bit_exact(ops, M, K, N):
+    """The one launch for the fewest rows (up to a block of 1024 columns for every warp, partial blocks, just too many
+    of them) against quantise + linear: outputs, the codes and scales left in the caller's scratch, a clip, an input whose
+    quotients leave the split product's range, and a call in place."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M * K + N)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    x[0, :7] = 2.0 ** 113 if M > 2 else 40.0
+    w8 = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(N, generator=g, device="cuda") * 0.01
+    bias = torch.randn(N, generator=g, device="cuda").to(torch.bfloat16)
+    for clip in (1.0, 0.9):
+        codes, scales = ops.quantize_int8_rows([x], 2, clip)
+        want = ops.linear_int8_scaled(codes, w8, scales, ws, bias=bias, gelu=True)
+        scratch = (torch.zeros_like(codes), torch.zeros_like(scales))
+        got = ops.w8a8_linear(x, w8, ws, bias=bias, gelu=True, clip=clip, scratch=scratch)
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+        assert torch.equal(scratch[0], codes) and torch.equal(scratch[1], scales)
+        assert torch.equal(ops.w8a8_linear(x, w8, ws, clip=clip).view(torch.int16),
+                           ops.linear_int8_scaled(codes, w8, scales, ws).view(torch.int16))
+    if N <= K:
+        room = x.clone()
+        want = ops.w8a8_linear(x, w8, ws)
+        got = ops.w8a8_linear(room, w8, ws, out=room.view(-1)[:M * N].view(M, N))
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    ops.poll_status()
+
+
 def test_w8a8_linear_end_to_end_single_layer(ops):
     """The single-layer benchmark case (M=1024, K=N=3072, H256ConvRot activations, bias): GPU quant + GEMM chained."""
     import torch
