@@ -15,6 +15,7 @@ struct GemmParams {
   int32_t *acc_out;
   uint32_t M, N, K;
   uint32_t epilogue;
+  uint32_t a_rows;  // rows of a load of x
   uint32_t split;   // CTAS = 1: CTAs of a cluster that share one tile's k-blocks (1 = no cluster)
   uint32_t tma_store; // 1: outputs leave through TMA stores (needs N % 8 == 0, aligned out)
   uint32_t weights_first; // 1: w is not written by the kernel in front, its first blocks are requested before that one is done

@@ -20,7 +20,7 @@
 //             sums are exact, so the bits do not depend on the split.
 //   CTAS = 2: a CTA pair (cluster of 2) computes a 256 x BN tile with cta_group::2 MMAs: each CTA
 //             stages its 128 rows of A and only its BN / 2 rows (half) of the B tile, 5 stages of
-//             32 KB (BN 256) or 7 of 24 KB (BN 128). This halves the B bytes every SM moves through
+//             32 KB (BN 256), 6 of 28 KB (BN 192) or 7 of 24 KB (BN 128). This halves the B bytes every SM moves through
 //             shared memory per MAC -- at 8192 INT8 MACs/clk/SM the 128x256 single-CTA tile needs
 //             48 KB written plus 48 KB read per 512 clocks, which is what bounds the CTAS = 1 form.
 //             The leader CTA (cluster rank 0) issues the MMAs; both CTAs load, and both run the
@@ -91,14 +91,14 @@ struct Cfg {
   static constexpr uint32_t kBRows = BN / CTAS;                  // rows of the B tile this CTA stages
   static constexpr uint32_t kBBytes = kBRows * kBK;
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = kStageBytes <= 24 * 1024 ? 7 : kStageBytes <= 32 * 1024 ? 5 : 4; // 160-192 KB
+  static constexpr int kStages = kStageBytes <= 24 * 1024 ? 7 : kStageBytes <= 28 * 1024 ? 6 : kStageBytes <= 32 * 1024 ? 5 : 4; // 160-192 KB
   // staging boxes per epilogue warp (two let a TMA store drain while the next box is filled;
   // the 128x256 form has room for one)
   static constexpr uint32_t kBoxes = kStageBytes <= 32 * 1024 ? 2 : 1;
   static constexpr uint32_t kStagingBytes = kEpilogueWarps * kBoxes * 32 * 64;
   static constexpr uint32_t kScaleBytes = kEpilogueWarps * BN * 4; // per warp: scales and biases of its BN / 2 columns
   static constexpr uint32_t kTileM = kBM * CTAS;                 // rows of the (pair's) output tile
-  static constexpr uint32_t kTmemCols = 2 * BN;                  // two accumulators
+  static constexpr uint32_t kTmemCols = BN == 192 ? 512 : 2 * BN; // two accumulators; a power of two
 };
 // Epilogue staging: per epilogue warp one or two [32 rows x 32 bf16] boxes (64-byte rows, 64B TMA swizzle).
 constexpr uint32_t kStoreBoxBytes = 32 * 64;
@@ -198,6 +198,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp != 0)
     grid_dependency_wait();
   if (warp == 0) {
+    const uint32_t stage_tx = CTAS == 2 ? 2 * kStageBytes : Cfg<CTAS, BN>::kBBytes + p.a_rows * kBK; // bytes of a stage's loads
     auto rows_of = [&](uint32_t tile) { return (int32_t)((tile / tiles_n) * kTileM + cta_rank * kBM); };
     auto columns_of = [&](uint32_t tile) { return (int32_t)((tile % tiles_n) * BN + cta_rank * Cfg<CTAS, BN>::kBRows); };
     // One operand's part of k-block kb. A pair counts the bytes of both CTAs on the leader's barrier: the leader
@@ -216,7 +217,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (early != 0u && ptx::elect_one())
       for (uint32_t i = 0; i < early; ++i) {
         if (cta_rank == 0)
-          ptx::mbar_expect_tx(full_bar + 8 * i, CTAS * kStageBytes);
+          ptx::mbar_expect_tx(full_bar + 8 * i, stage_tx);
         load(&map_b, smem_base + i * kStageBytes + kABytes, full_bar + 8 * i, kb_first + i, columns_of(unit));
       }
     grid_dependency_wait();
@@ -242,11 +243,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           // test aid: the bytes are announced but never loaded, so the consumer's wait on this
           // stage runs out and the kernel leaves through its give-up path
           if (cta_rank == 0 && ptx::elect_one())
-            ptx::mbar_expect_tx(bar, CTAS * kStageBytes);
+            ptx::mbar_expect_tx(bar, stage_tx);
         } else if (ptx::elect_one()) {
           if (CTAS == 2) {
             if (cta_rank == 0) {
-              ptx::mbar_expect_tx(bar, 2 * kStageBytes);
+              ptx::mbar_expect_tx(bar, stage_tx);
               ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
               ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
             } else {
@@ -255,7 +256,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               ptx::tma_load_2d_pair(b_dst, &map_b, leader_bar, k0, n0);
             }
           } else {
-            ptx::mbar_expect_tx(bar, kStageBytes);
+            ptx::mbar_expect_tx(bar, stage_tx);
             ptx::tma_load_2d(a_dst, &map_a, bar, k0, m0);
             ptx::tma_load_2d(b_dst, &map_b, bar, k0, n0);
           }
@@ -449,7 +450,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
           ptx::fence_proxy_async();
           __syncwarp();
-          if (lane == 0) {
+          if (lane == 0 && m0 + quarter * 32u < p.M) {
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                              reinterpret_cast<uint64_t>(&map_c)),
                          "r"(my_staging + store_buf * kStoreBoxBytes), "r"((int32_t)n_base),
@@ -502,20 +503,20 @@ struct Form {
 };
 // The form with the least modelled time: waves of tiles x k-blocks per CTA x time of a k-block, plus what a
 // launch pays once (first loads, the last tile's epilogue, the exchange of a split). The figures, in ns, are
-// fitted to event times of every form at N 3072 / 9216 / 12288, K 3072 / 8192 / 12288 and 2 to 9216 rows with
-// cold caches. Large problems go to the 256 x 256 pair (fewest bytes per MAC). The narrower tiles and the
+// fitted to event times of every form at N 3072 / 9216 / 12288 / 16384, K 3072 / 8192 / 12288 and 17 to 12000 rows; over 160
+// such problems the form chosen is within 5 % of the best one, and within 2 % of it for all but 20. Large problems go to the 256 x 256 pair (fewest bytes per MAC). The narrower tiles and the
 // splits are for problems that leave SMs idle, where time is one CTA's serial chain of k-blocks: 2 rows,
 // K 12288, N 3072 45 -> 22.5 us (12 CTAs of 96 k-blocks -> 96 of 24), K 3072 20.5 -> 14.3 us; 512 rows, K 12288
 // 43 -> 31 us; 1600 rows, K 8192 53 -> 49 us; 1101 rows, N 12288 47 -> 43 us. A split costs more than it gives
-// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`. Up to 16 rows a
-// k-block of the 128-column tiles takes about 200 ns more, one of the 256-column tiles does not (2 rows, N 12288,
-// K 3072: 20.6 us a call with the former and 18.6 with the latter; 64 rows 16.5 and 18.6).
+// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`. Pairs of 192 columns
+// fill waves that the others leave half empty (the GEMM alone, best of the others -> 192: 512 rows, N 12288, K 3072
+// 21.9 -> 19.8 us; 900 rows, K 8192 26 -> 21; 1024 rows, K 12288 36 -> 29; 2048 rows, K 8192 41 -> 35).
 Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
   struct Cost {
     Form form;
     uint64_t block_ns, launch_ns;
   };
-  static const Cost costs[] = {{{2, 256, 1}, 320, 6000}, {{2, 128, 1}, 208, 4500}, {{1, 256, 1}, 363, 5100},
+  static const Cost costs[] = {{{2, 256, 1}, 320, 6000}, {{2, 192, 1}, 265, 5200}, {{2, 128, 1}, 208, 4500}, {{1, 256, 1}, 363, 5100},
                                {{1, 128, 1}, 258, 3200}, {{1, 128, 2}, 320, 3500}, {{1, 128, 4}, 450, 4600}};
   const uint64_t sms = (uint64_t)sm_count(), k_blocks = (K + kBK - 1) / kBK;
   // DIFB200_GEMM_FORM=ctas,columns,split forces one of the forms, DIFB200_GEMM_CTAS=1|2 a 256-column one
@@ -538,8 +539,7 @@ Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
     if ((f.ctas == 2 && M <= (uint64_t)kBM) || (f.split > 1 && tiles > resident))
       continue;
     const uint64_t waves = (tiles + resident - 1) / resident;
-    const uint64_t block_ns = c.block_ns + (M <= 16 && f.tile_n == 128 ? 200 : 0);
-    const uint64_t time = waves * ((k_blocks + f.split - 1) / f.split) * block_ns + c.launch_ns;
+    const uint64_t time = waves * ((k_blocks + f.split - 1) / f.split) * c.block_ns + c.launch_ns;
     if (time < least) {
       least = time;
       best = f;
@@ -649,7 +649,11 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   CUtensorMap map_a, map_b;
   const uint64_t dims_a[2] = {K, M}, dims_b[2] = {K, N};
   const uint64_t strides[1] = {K};
-  const uint32_t box_a[2] = {(uint32_t)kBK, (uint32_t)kBM}, box_b[2] = {(uint32_t)kBK, (uint32_t)(form.tile_n / form.ctas)};
+  // Where all rows are one tile of a CTA, loads end with them (a multiple of 8 rows, the swizzle's period): rows beyond
+  // the tensor are not free, 17 x 3072 x 16384 took 16.6 us with boxes of 128 rows and 9.9 with boxes of 32. What stands in the
+  // others' place meets only rows of the accumulator that are never read.
+  p.a_rows = form.ctas == 1 && M < (uint64_t)kBM ? (uint32_t)(M + 7) / 8 * 8 : (uint32_t)kBM;
+  const uint32_t box_a[2] = {(uint32_t)kBK, p.a_rows}, box_b[2] = {(uint32_t)kBK, (uint32_t)(form.tile_n / form.ctas)};
   if (int rc = encode_tensor_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, x, dims_a, strides, box_a,
                                  CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
@@ -671,8 +675,9 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   p.split = (uint32_t)form.split;
   p.tma_store = tma_store ? 1u : 0u;
   if (form.ctas == 2)
-    return form.tile_n == 256 ? launch_form<2, 256>(map_a, map_b, map_c, p, stream)
-                              : launch_form<2, 128>(map_a, map_b, map_c, p, stream);
+    return form.tile_n == 256   ? launch_form<2, 256>(map_a, map_b, map_c, p, stream)
+           : form.tile_n == 192 ? launch_form<2, 192>(map_a, map_b, map_c, p, stream)
+                                : launch_form<2, 128>(map_a, map_b, map_c, p, stream);
   return form.tile_n == 256 ? launch_form<1, 256>(map_a, map_b, map_c, p, stream)
                             : launch_form<1, 128>(map_a, map_b, map_c, p, stream);
 }

@@ -305,14 +305,14 @@ int launch_groups(const FewParams &f, cudaStream_t stream) {
 
 } // namespace
 
-// Whether the few-rows kernel takes a problem. Every CTA reads all rows' codes, which come from the same few lines of L2, so
-// its time grows with the rows and, beyond 16, with the weights. us of a linear, tile kernel -> this (K x N): 2 rows
-// 3072 x 3072 10.8 -> 5.3, 3072 x 9216 12.5 -> 7.8, 3072 x 16384 17.2 -> 11.5, 12288 x 3072 15.9 -> 10.6; 16 rows 11.2 -> 6.4,
-// 13.9 -> 10.8, 16.4 -> 14.9, 14.7 -> 13.3; 32 rows 11.0 -> 8.3, 14.0 -> 14.5, 17.2 -> 21.0, 15.1 -> 17.5.
+// Whether the few-rows kernels take a problem. Every CTA reads all rows' codes, which come from the same few lines of L2, so
+// the time grows with the rows and, the more of them, with the weights. us of a linear, tile kernel / this (K x N): 8 rows
+// 3072 x 3072 10.4 / 5.3, 3072 x 9216 10.2 / 7.9, 3072 x 16384 11.5 / 11.9, 12288 x 3072 14.4 / 11.4; 16 rows 10.4 / 6.3, 10.2 / 10.5,
+// 11.5 / 15.2, 14.4 / 13.2, 3072 x 12288 12.9 / 12.8; 32 rows 10.4 / 8.3, 10.4 / 14.5.
 bool few_rows(uint64_t M, uint64_t N, uint64_t K) {
   if (std::getenv("DIFB200_GEMM_FORM") || std::getenv("DIFB200_GEMM_CTAS"))
     return false; // a tile form is forced
-  return M <= 16 || (M <= 32 && N * K <= (1ull << 24));
+  return M <= 8 || (M <= 16 && N * K <= (5ull << 23)) || (M <= 32 && N * K <= (1ull << 24));
 }
 
 int launch_few_rows(const int8_t *x, const int8_t *w, const GemmParams &p, cudaStream_t stream) {

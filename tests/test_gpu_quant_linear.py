@@ -155,11 +155,12 @@ def test_linear_int8_scaled_bit_exact(ops, gemm_form, M, K, N):
     ops.poll_status()
 
 
-@pytest.mark.parametrize("form", ["2,128,1", "1,128,1", "1,128,2", "1,128,4", None])
-@pytest.mark.parametrize("M,K,N", [(1, 3072, 3072), (2, 12288, 384), (127, 528, 128), (129, 656, 264), (257, 1168, 131),
-                                   (520, 512, 1032)])
+@pytest.mark.parametrize("form", ["2,192,1", "2,128,1", "1,256,1", "1,128,1", "1,128,2", "1,128,4", None])
+@pytest.mark.parametrize("M,K,N", [(1, 3072, 3072), (2, 12288, 384), (33, 640, 256), (40, 656, 200), (127, 528, 128), (129, 656, 264),
+                                   (257, 1168, 131), (520, 512, 1032), (300, 768, 577)])
 def test_linear_int8_scaled_narrow_and_split_tiles(ops, monkeypatch, form, M, K, N):
-    """The 128-column tiles and the splits over k-blocks (cluster exchange): tile edges in M and N, ragged k-blocks
+    """The 128- and 192-column tiles and the splits over k-blocks (cluster exchange): tile edges in M and N, loads that end
+    with the rows, ragged k-blocks
     (a split whose shares differ), odd N (no TMA stores); `None` is the form the dispatch picks."""
     import torch
     if form:
@@ -292,7 +293,7 @@ def test_w8a8_linear_single_call_matches_two_calls(ops):
     ops.poll_status()
 
 
-@pytest.mark.parametrize("form", ["2,256,1", "2,128,1", "1,256,1", "1,128,1", "1,128,2", "1,128,4"])
+@pytest.mark.parametrize("form", ["2,256,1", "2,192,1", "2,128,1", "1,256,1", "1,128,1", "1,128,2", "1,128,4"])
 @pytest.mark.parametrize("blocks", [1, 3, 4, 5, 6, 7, 8, 9, 15])
 def test_w8a8_linear_with_k_blocks_around_the_ring_depth(ops, monkeypatch, form, blocks):
     """The single call requests the weights of the first k-blocks of a CTA's first tile ahead of everything else: fewer
