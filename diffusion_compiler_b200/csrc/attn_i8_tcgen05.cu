@@ -184,13 +184,19 @@ __global__ void __launch_bounds__(256)
 attention_operands_kernel(const OperandParams p) {
   grid_dependents_launch(); // (launched plainly)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
-  // codes of this lane's 16 elements of a row, the row's scale and sum of squared codes (in every lane)
-  auto quantise = [&](const uint4 *row, bool valid, uint4 &codes, float &scale) {
-    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+  // The four rows of a lane are requested before the first is worked on (behind one another, each waited for its load:
+  // B2 S4608 H24 41 us, now 34).
+  uint4 lows[4], highs[4];
+  auto request = [&](int step, const uint4 *row, bool valid) {
+    lows[step] = highs[step] = make_uint4(0, 0, 0, 0);
     if (valid) {
-      lo = __ldg(row + 2 * part);
-      hi = __ldg(row + 2 * part + 1);
+      lows[step] = __ldg(row + 2 * part);
+      highs[step] = __ldg(row + 2 * part + 1);
     }
+  };
+  // codes of this lane's 16 elements of a row and the row's scale (in every lane)
+  auto quantise = [&](int step, uint4 &codes, float &scale) {
+    const uint4 lo = lows[step], hi = highs[step];
     const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     uint64_t v[8];
     float m = 0.0f;
@@ -210,6 +216,11 @@ attention_operands_kernel(const OperandParams p) {
   if (blockIdx.x < p.key_blocks) {
     const uint32_t tiles = p.S_pad / kTile, tile = blockIdx.x % tiles, kvh = (blockIdx.x / tiles) % p.KV,
                    b = blockIdx.x / (tiles * p.KV);
+    auto key_of = [&](int step) { return tile * kTile + step * 32u + warp * 4u + (lane >> 3); };
+    auto row_of = [&](int step) { return ((uint64_t)b * p.S + (key_of(step) < p.S ? key_of(step) : 0)) * p.KV + kvh; };
+#pragma unroll
+    for (int step = 0; step < 4; ++step)
+      request(step, p.k + row_of(step) * 16, key_of(step) < p.S);
     __shared__ uint32_t masked[4]; // whether a segment of 32 keys has masked ones
     if (threadIdx.x < 4)
       masked[threadIdx.x] = 0u;
@@ -219,12 +230,12 @@ attention_operands_kernel(const OperandParams p) {
     uint32_t first_valid = 0; // (thread 0) of the four segments' first keys
 #pragma unroll
     for (int step = 0; step < 4; ++step) {
-      const uint32_t j = tile * kTile + step * 32u + warp * 4u + (lane >> 3);
+      const uint32_t j = key_of(step);
       const bool exists = j < p.S;
-      const uint64_t row = ((uint64_t)b * p.S + (exists ? j : 0)) * p.KV + kvh;
+      const uint64_t row = row_of(step);
       uint4 codes;
       float scale;
-      quantise(p.k + row * 16, exists, codes, scale);
+      quantise(step, codes, scale);
       int n2 = __dp4a((int)codes.x, (int)codes.x, 0);
       n2 = __dp4a((int)codes.y, (int)codes.y, n2);
       n2 = __dp4a((int)codes.z, (int)codes.z, n2);
@@ -266,13 +277,17 @@ attention_operands_kernel(const OperandParams p) {
           t[kTile + 32 * step] = -0.0f;
     }
   } else {
+    auto row_of = [&](int step) { return (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * 32u + warp * 4u + (lane >> 3); };
+#pragma unroll
+    for (int step = 0; step < 4; ++step)
+      request(step, p.q + (row_of(step) < p.q_rows ? row_of(step) : 0) * 16, row_of(step) < p.q_rows);
 #pragma unroll
     for (int step = 0; step < 4; ++step) {
-      const uint64_t row = (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * 32u + warp * 4u + (lane >> 3);
+      const uint64_t row = row_of(step);
       const bool exists = row < p.q_rows;
       uint4 codes;
       float scale;
-      quantise(p.q + (exists ? row : 0) * 16, exists, codes, scale);
+      quantise(step, codes, scale);
       if (exists) {
         reinterpret_cast<uint4 *>(p.q8 + row * kTile)[part] = codes;
         if (part == 0)
