@@ -23,8 +23,8 @@
 // conversion and a byte store per element they kept the quarter-rate unit busy for 256 clocks of a block, and a warp took three
 // blocks at a time to save per-row work. Before -> now, us: 33272 x 3072 83.9 -> 71.8 (4.3 TB/s), 33272 x 8192 220.6 -> 181.7,
 // 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 55.4, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
-// 12288 x 3072 64.7 -> 61.6 (all lanes evaluate samples, in doubles only where candidates are close), with input
-// equalisation 94.5 -> 90.8, RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
+// 12288 x 3072 64.7 -> 56.5 (all lanes evaluate samples, in doubles only where candidates are close), with input
+// equalisation 94.2 -> 72.6, RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
 // copies through shared memory instead of registers gave nothing.
 #include "quant_common.cuh"
 
@@ -115,6 +115,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
         }
       }
     }
+    equalise_fast = __all_sync(0xffffffffu, equalise_fast);
   }
 
   // The 64 bytes of a thread's two runs in block `it` of a row. Widths of concatenated inputs are
@@ -300,12 +301,15 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
                                  act_b ? __ldg(ep + 33) : z};
             const uint32_t ea[8] = {e4[0].x, e4[0].y, e4[0].z, e4[0].w, e4[1].x, e4[1].y, e4[1].z, e4[1].w};
             const uint32_t eb[8] = {e4[2].x, e4[2].y, e4[2].z, e4[2].w, e4[3].x, e4[3].y, e4[3].z, e4[3].w};
+            auto entry = [&](int i, float &e0, float &e1) {
+              e0 = __uint_as_float((i & 1) ? (ea[i >> 1] & 0xffff0000u) : (ea[i >> 1] << 16));
+              e1 = __uint_as_float((i & 1) ? (eb[i >> 1] & 0xffff0000u) : (eb[i >> 1] << 16));
+            };
+            if (equalise_fast) { // (of the warp: a branch for every pair cost packing 12288 x 3072 a tenth)
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float e0 = __uint_as_float((i & 1) ? (ea[i >> 1] & 0xffff0000u) : (ea[i >> 1] << 16));
-              const float e1 = __uint_as_float((i & 1) ? (eb[i >> 1] & 0xffff0000u) : (eb[i >> 1] << 16));
-              if (equalise_fast) {
-                float y0, y1;
+              for (int i = 0; i < 16; ++i) {
+                float e0, e1, y0, y1;
+                entry(i, e0, e1);
                 asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(e0));
                 asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(e1));
                 const uint64_t y2 = pack2(y0, y1), q2 = mul2(P[i], y2);
@@ -313,8 +317,12 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
                 unpack2(q2, q0, q1);
                 unpack2(fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2), x0, x1);
                 P[i] = pack2(x0 == x0 ? x0 : q0, x1 == x1 ? x1 : q1);
-              } else {
-                float w0, w1;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                float e0, e1, w0, w1;
+                entry(i, e0, e1);
                 unpack2(P[i], w0, w1);
                 P[i] = pack2(__fdiv_rn(w0, e0), __fdiv_rn(w1, e1));
               }
@@ -402,37 +410,40 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             e[f] = __fmaf_rn(d1, d1, e[f]);
           }
         }
+        // Halving: with every exchange a lane keeps half of its sums, so that lane l ends with candidate l / 4's (7: none).
+        // 9 exchanges in the place of 35, and what follows is per lane instead of per candidate.
+        float four[4], two[2];
 #pragma unroll
-        for (int f = 0; f < 7; ++f) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1)
-            e[f] += __shfl_xor_sync(0xffffffffu, e[f], o);
-          if (warps_per_row > 1 && lane == 0)
-            sums[f * total_warps + warp] = e[f];
+        for (int f = 0; f < 4; ++f) {
+          const float upper = f < 3 ? e[f + 4] : 0.0f;
+          four[f] = (lane & 16 ? upper : e[f]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? e[f] : upper, 16);
         }
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+          two[f] = (lane & 8 ? four[f + 2] : four[f]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? four[f] : four[f + 2], 8);
+        float own = (lane & 4 ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? two[0] : two[1], 4);
+        own += __shfl_xor_sync(0xffffffffu, own, 2);
+        own += __shfl_xor_sync(0xffffffffu, own, 1);
+        const int mine = lane >> 2;
         if (warps_per_row > 1) {
+          if ((lane & 3) == 0 && mine < 7)
+            sums[mine * total_warps + warp] = own;
           row_barrier();
-#pragma unroll
-          for (int f = 0; f < 7; ++f) {
-            e[f] = 0.0f;
-            for (int w = 0; w < warps_per_row; ++w)
-              e[f] += sums[f * total_warps + slot * warps_per_row + w];
-          }
+          own = 0.0f;
+          for (int v = 0; v < warps_per_row; ++v)
+            own += sums[(mine < 7 ? mine : 0) * total_warps + slot * warps_per_row + v];
         }
-        float best = e[0], worst = e[0];
+        const bool finite = own < INFINITY; // (sums of squares: not negative, or NaN)
+        if (mine == 7 || !finite)
+          own = INFINITY;
+        const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(own)));
+        const uint32_t close = __ballot_sync(0xffffffffu, (lane & 3) == 0 && mine < 7 && own <= best * 1.0001f);
+        const uint32_t all_finite = __ballot_sync(0xffffffffu, finite || mine == 7);
+        const int which = close ? (__ffs((int)close) - 1) >> 2 : 0;
 #pragma unroll
-        for (int f = 1; f < 7; ++f) {
-          best = fminf(best, e[f]);
-          asm("max.NaN.f32 %0, %0, %1;" : "+f"(worst) : "f"(e[f]));
-        }
-        int close = 0;
-#pragma unroll
-        for (int f = 6; f >= 0; --f)
-          if (e[f] <= best * 1.0001f) {
-            ++close;
-            chosen = candidate[f];
-          }
-        decided = close == 1 && best > 1.0e-30f && worst < INFINITY; // the same for every thread of the row
+        for (int f = 1; f < 7; ++f)
+          chosen = which == f ? candidate[f] : chosen;
+        decided = __popc(close) == 1 && best > 1.0e-30f && all_finite == 0xffffffffu; // the same for every thread of the row
       }
       double e[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
       if (!decided) {
@@ -663,12 +674,13 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
   if (norm)
     return launch_single<SIGNED, false, false, kNorm>(p, stream);
   if (pack) {
-    // The scale search is arithmetic per row as well as per element: three blocks per warp where they divide the row
-    // (12288 x 3072 77.5 -> 62.1 us, 3072 x 12288 with equalisation 101.7 -> 94.9; 3072 x 8192 signed, whose last warp
-    // would be a third empty, 69.3 -> 75.2) and the rows are more than the machine holds at once.
+    // The scale search is arithmetic per row as well as per element: three blocks per warp where they divide the row and
+    // the rows are more than the machine holds at once, 16 warps per SM and no prefetch (12288 x 3072 with equalisation: one
+    // block and 24 warps 76.3 us, three with a prefetch and 12 warps 78.7, this 72.6; without 65.1, 61.0, 56.5; 3072 x 8192, whose
+    // last warp would be a third empty, 51.5 / 53.6 / 56.2).
     const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
     return blocks % 3u == 0u && p.rows * blocks > (uint64_t)sm_count() * 24u
-               ? launch_form<SIGNED, false, false, kPack, 3, true, 192, 2>(p, stream)
+               ? launch_form<SIGNED, false, false, kPack, 3, false, 256, 2>(p, stream)
                : launch_single<SIGNED, false, false, kPack>(p, stream);
   }
   return launch_single<SIGNED, false, false, kPlain>(p, stream);
