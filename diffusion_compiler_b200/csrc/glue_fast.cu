@@ -104,23 +104,31 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool v
 }
 
 // acc after the two bf16 elements of a word, low half first. KIND 0: acc + x; 1: acc + x * x (exact
-// square, one rounding); 2: acc + (x - mean)^2 with the roundings of subtract, multiply and add.
+// square, one rounding).
 template <int KIND>
-__device__ __forceinline__ float accumulate_word(uint32_t word, float mean, float acc) {
+__device__ __forceinline__ float accumulate_word(uint32_t word, float acc) {
   if (KIND == 0) {
     asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; add.rn.f32.bf16 %0, lo, %0; add.rn.f32.bf16 %0, hi, %0; }"
         : "+f"(acc) : "r"(word));
-  } else if (KIND == 1) {
+  } else {
     asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; fma.rn.f32.bf16 %0, lo, lo, %0; fma.rn.f32.bf16 %0, hi, hi, %0; }"
         : "+f"(acc) : "r"(word));
-  } else {
-    float d0, d1;
-    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; sub.rn.f32.bf16 %0, lo, %3; sub.rn.f32.bf16 %1, hi, %3; }"
-        : "=f"(d0), "=f"(d1) : "r"(word), "f"(mean));
-    acc = __fadd_rn(acc, __fmul_rn(d0, d0));
-    acc = __fadd_rn(acc, __fmul_rn(d1, d1));
   }
   return acc;
+}
+// The squared deviations of a word's two elements, with the roundings of subtract and multiply. (volatile: stays where
+// it is written, between the dependent sums)
+__device__ __forceinline__ void deviations(uint32_t word, float mean, float &d0, float &d1) {
+  asm volatile("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; sub.rn.f32.bf16 %0, lo, %3; sub.rn.f32.bf16 %1, hi, %3; }"
+               : "=f"(d0), "=f"(d1) : "r"(word), "f"(mean));
+}
+__device__ __forceinline__ float square_in_place(float d) {
+  float q;
+  asm volatile("mul.rn.f32 %0, %1, %1;" : "=f"(q) : "f"(d));
+  return q;
+}
+__device__ __forceinline__ void add_in_place(float &acc, float v) {
+  asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(acc) : "f"(v));
 }
 
 template <bool LAYER, int STAGES>
@@ -157,10 +165,10 @@ k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint
       auto chain = [&](const uint4 (&v)[8]) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          acc = accumulate_word<decltype(kind)::value>(v[c].x, mean, acc);
-          acc = accumulate_word<decltype(kind)::value>(v[c].y, mean, acc);
-          acc = accumulate_word<decltype(kind)::value>(v[c].z, mean, acc);
-          acc = accumulate_word<decltype(kind)::value>(v[c].w, mean, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].x, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].y, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].z, acc);
+          acc = accumulate_word<decltype(kind)::value>(v[c].w, acc);
         }
       };
       // The chunk after the one being summed is already in registers, and the requests sit between the
@@ -190,10 +198,64 @@ k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint
         chain(a);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
+    // The second pass of the layer form, acc + (x - mean)^2: the squares of the next chunk are made between the sums of
+    // this one, which alone depend on one another. (Subtract, multiply and add of an element one behind the other took
+    // 16 us for 3072 columns, the chain of sums takes 7.)
+    auto deviation_pass = [&]() {
+      auto squares_of = [&](const uint4 (&v)[8], int w, float &q0, float &q1) {
+        const uint32_t word = (w & 3) == 0 ? v[w >> 2].x : (w & 3) == 1 ? v[w >> 2].y : (w & 3) == 2 ? v[w >> 2].z : v[w >> 2].w;
+        float d0, d1;
+        deviations(word, mean, d0, d1);
+        q0 = square_in_place(d0);
+        q1 = square_in_place(d1);
+      };
+      auto advance = [&](uint32_t chunk, const float (&q)[64], float (&next)[64]) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 3) : "memory");
+        __syncwarp();
+        uint4 v[8];
+        read(chunk + 1, v);
+        issue(chunk + STAGES - 1);
+#pragma unroll
+        for (int w = 0; w < 32; ++w) {
+          add_in_place(acc, q[2 * w]);
+          if (w >= 4)
+            squares_of(v, w - 4, next[2 * w - 8], next[2 * w - 7]);
+          add_in_place(acc, q[2 * w + 1]);
+        }
+#pragma unroll
+        for (int w = 28; w < 32; ++w)
+          squares_of(v, w, next[2 * w], next[2 * w + 1]);
+      };
+      acc = 0.0f;
+      __syncwarp();
+      for (uint32_t c = 0; c < (uint32_t)STAGES - 1; ++c)
+        issue(c);
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+      __syncwarp();
+      float a[64], b[64];
+      {
+        uint4 v[8];
+        read(0, v);
+#pragma unroll
+        for (int w = 0; w < 32; ++w)
+          squares_of(v, w, a[2 * w], a[2 * w + 1]);
+      }
+      uint32_t chunk = 0;
+#pragma unroll 1
+      for (; chunk + 1 < chunks; chunk += 2) {
+        advance(chunk, a, b);
+        advance(chunk + 1, b, a);
+      }
+      if (chunk < chunks)
+#pragma unroll
+        for (int e = 0; e < 64; ++e)
+          add_in_place(acc, a[e]);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    };
     if (LAYER) {
       pass(std::integral_constant<int, 0>{});
       mean = __fdiv_rn(acc, (float)cols);
-      pass(std::integral_constant<int, 2>{});
+      deviation_pass();
     } else {
       pass(std::integral_constant<int, 1>{});
     }
@@ -431,10 +493,10 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
       const uint4 v = row[c];
-      sum = accumulate_word<1>(v.x, 0.0f, sum);
-      sum = accumulate_word<1>(v.y, 0.0f, sum);
-      sum = accumulate_word<1>(v.z, 0.0f, sum);
-      sum = accumulate_word<1>(v.w, 0.0f, sum);
+      sum = accumulate_word<1>(v.x, sum);
+      sum = accumulate_word<1>(v.y, sum);
+      sum = accumulate_word<1>(v.z, sum);
+      sum = accumulate_word<1>(v.w, sum);
     }
   }
   const float inv_mine = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, 128.0f), p.eps)));
