@@ -185,7 +185,7 @@ attention_operands_kernel(const OperandParams p) {
   grid_dependents_launch(); // (launched plainly)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
   // The four rows of a lane are requested before the first is worked on (behind one another, each waited for its load:
-  // B2 S4608 H24 41 us, now 34).
+  // B2 S4608 H24 41 us against 34).
   uint4 lows[4], highs[4];
   auto request = [&](int step, const uint4 *row, bool valid) {
     lows[step] = highs[step] = make_uint4(0, 0, 0, 0);
@@ -210,7 +210,7 @@ attention_operands_kernel(const OperandParams p) {
       m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     scale = row_scale(m, 1.0f);
     uint32_t out[4];
-    direct_codes(v, scale, out);
+    direct_codes(v, m, scale, out);
     codes = make_uint4(out[0], out[1], out[2], out[3]);
   };
   if (blockIdx.x < p.key_blocks) {

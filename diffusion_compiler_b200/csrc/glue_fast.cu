@@ -581,7 +581,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         n[i] = unpack_bf16_pair(bits[i]);
-      direct_codes(n, scale, words);
+      direct_codes(n, m, scale, words);
       if (exists) {
         *reinterpret_cast<uint2 *>(p.codes + out * 128 + 8 * c0) = make_uint2(words[0], words[1]);
         *reinterpret_cast<uint2 *>(p.codes + out * 128 + 8 * c1) = make_uint2(words[2], words[3]);

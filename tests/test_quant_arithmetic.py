@@ -54,3 +54,24 @@ def test_bf16_quotient_in_two_bf16_parts_for_every_pair_of_significands():
         r2 = bf16(r - r1)
         got = bf16(v * r1 + bf16(v * r2))  # 8 + 8 bits and a term at most 2^9 times smaller: exact in float64
         assert np.array_equal(got, want), step
+
+
+def test_direct_codes_from_one_product_for_every_pair_of_significands():
+    """direct_codes of csrc/quant_common.cuh: the nearest even integer to v y against that to the IEEE quotient
+    RN(v / scale), scale = RN(maximum / 127), for every significand of the maximum, every significand of v (fewer bits
+    too) and every exponent that gives a code, with y up to 2^-22 of itself away from the one computed (the approximate
+    reciprocal, its Newton step and the roundings of the move leave less) unless the scale is a power of two."""
+    f32 = np.float32
+    for M in range(128, 256):
+        scale = f32(np.float64(M) / 127.0)  # no quotient by 127 is near a boundary of fp32
+        apart = 127.0 * np.float64(scale) - M  # exact
+        assert (apart == 0.0) == (M == 254)
+        move = 0.0 if apart == 0.0 else 2.0 ** -21 if apart <= M * 3.0e-8 else -2.0 ** -21
+        y = np.float64(f32(1.0 / np.float64(scale))) * (1.0 + move)
+        for k in range(10):  # beyond, v is below a quarter of the scale
+            v = np.arange(1, 256, dtype=np.float64) * 2.0 ** -k
+            v = v[v <= M]
+            want = np.rint((v / np.float64(scale)).astype(f32))
+            for wobble in (0.0,) if M == 254 else (-2.0 ** -22, 0.0, 2.0 ** -22):
+                got = np.rint((v * np.float64(f32(y * (1.0 + wobble)))).astype(f32))
+                assert np.array_equal(want, got), (M, k, wobble)
