@@ -68,6 +68,21 @@ constexpr float kLeastSum = 1.0f / (1u << 25); // of a running maximum: its larg
 constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
 constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + 256 + kPairBytes;
 
+// Division by a number that a launch fixes, of what is below 2^31: with 2^s the least power of two that is not below the
+// divisor and mul = ceil(2^(31 + s) / by), mul * by exceeds 2^(31 + s) by e < 2^s, so n * e < 2^(31 + s) and the quotient
+// of 2 n * mul and 2^(32 + s) is that of n and by.
+struct Divisor {
+  uint32_t by, mul, shift;
+  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return __umulhi(2u * n, mul) >> shift; }
+};
+Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
+  Divisor d{(uint32_t)by, 0, 0};
+  while ((1ull << d.shift) < by)
+    ++d.shift;
+  d.mul = (uint32_t)(((1ull << (31 + d.shift)) + by - 1) / by);
+  return d;
+}
+
 struct AttnParams {
   const int8_t *q8;      // [B,Sq,H,128]
   const float *qs;       // [B,Sq,H]
@@ -90,6 +105,7 @@ struct AttnParams {
   uint32_t behind_whole; // 1: launched behind the items that are not split, whose operands this launch shares
   uint32_t split_follows; // 1: such a launch comes next
   uint32_t item0, split; // first (batch, head, query block) of this launch; CTAs of a cluster that share its keys
+  Divisor q_blocks, heads, group; // blocks of 256 queries, H, H / KV
 };
 
 __device__ __forceinline__ void report(DeviceStatus *status, uint32_t role, uint32_t detail) {
@@ -309,10 +325,24 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // 32 outputs bf16(o / l) from RN(1 / l) and one Markstein step (the product corrected by its residual, one rounding);
-// where that has no finite value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0.
+// where that has no finite value (o infinite) the product stands. A row without valid keys has l = 0 and gives 0. Both
+// show as a NaN among the results, which a maximum over them carries to one test. (With a test and a choice per result, 64
+// results of each thread and their staging took 3000 of the 13200 clocks of a CTA with one key tile, so 1900.)
 __device__ __forceinline__ void normalise(const uint32_t (&o)[32], float l, uint32_t (&w)[16]) {
   const float y = __frcp_rn(l);
   const uint64_t y2 = pack2(y, y), negl2 = pack2(-l, -l);
+  uint32_t most = 0;
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    const uint64_t o2 = pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1]));
+    const uint64_t q2 = mul2(o2, y2);
+    float x0, x1;
+    unpack2(fma2(fma2(q2, negl2, o2), y2, q2), x0, x1);
+    w[j >> 1] = pack_bf16(x0, x1);
+    asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(most) : "r"(w[j >> 1]));
+  }
+  if ((most & 0x7fffu) <= 0x7f80u && (most >> 16 & 0x7fffu) <= 0x7f80u)
+    return;
 #pragma unroll
   for (int j = 0; j < 32; j += 2) {
     const uint64_t o2 = pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1]));
@@ -329,8 +359,7 @@ __device__ __forceinline__ void normalise(const uint32_t (&o)[32], float l, uint
 template <bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
-               const AttnParams p) {
+               const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -351,13 +380,12 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long wait_ns = p.wait_ns;
-  const uint32_t q_blocks = (p.Sq + 255u) / 256u;
   const uint32_t split = SPLIT ? p.split : 1u, rank = SPLIT ? ptx::cluster_ctarank() : 0u;
   const uint32_t item = SPLIT ? p.item0 + blockIdx.x / split : blockIdx.x;
-  const uint32_t qb = item % q_blocks;
-  const uint32_t head = (item / q_blocks) % p.H;
-  const uint32_t batch = item / (q_blocks * p.H);
-  const uint32_t kvh = head / (p.H / p.KV);
+  // (every warp needs them: with divisions by the parameters it took 1240 clocks to the wait for the operands, so 380)
+  const uint32_t batch_head = p.q_blocks.quotient(item), qb = item - batch_head * p.q_blocks.by;
+  const uint32_t batch = p.heads.quotient(batch_head), head = batch_head - batch * p.H;
+  const uint32_t kvh = p.group.quotient(head);
   const uint32_t q0 = qb * 256u;
   const uint32_t tiles = p.tile_count[0] + p.tile_count[1], first = SPLIT ? tiles * rank / split : 0u;
   const uint32_t n_kv = SPLIT ? tiles * (rank + 1u) / split - first : tiles; // of this CTA (at least one: split <= tiles)
@@ -382,7 +410,6 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                  "r"(kKsBytes), "r"(kv_full + 8 * s)
                  : "memory");
   };
-  const uint32_t early = min(n_kv, 2u); // tiles whose loads thread 0 issues during the set-up (0.6 us of a CTA's 6 us around its steps)
   if (threadIdx.x == 0) {
     ptx::mbar_init(q_full, 8);
     ptx::mbar_init(q_full + 8, 8);
@@ -417,13 +444,14 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ptx::fence_device_and_tma();
     grid_dependents_launch();
   }
+  // Only Q is requested in front of the barrier. The first two tiles are 8 copies more, 700 to 1000 clocks of this one thread
+  // for which all others waited, and the first Q.K^T needs them 2000 clocks later. With this, and the divisions and the
+  // normalisation as they are now, 4096 queries of 24 heads over 77 keys 25.5 -> 22.9 us, over 512 39.4 -> 36.2, B1 S1101
+  // H24 KV8 24.8 -> 24.3, B1 S4608 H24 188.2 -> 187.3.
   if (threadIdx.x == 0) {
     ptx::mbar_expect_tx(q_tma, 2 * kKBytes); // Q codes: staged where the ring is still free
     for (uint32_t t = 0; t < 2; ++t)
       ptx::tma_load_4d(stage_addr + (2u + t) * kStageBytes, &map_q, q_tma, 0, (int32_t)head, (int32_t)(q0 + t * 128u), (int32_t)batch);
-    for (uint32_t i = 0; i < early; ++i)
-      load_tile(i, i);
-    ptx::prefetch_tensormap(&map_o);
   }
   // What the softmax warps need first, requested here and used behind the barrier: the row's scale, the bounds of the
   // first 128 key tiles.
@@ -441,7 +469,6 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *slot_ptr;
-
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
     // The producer and the MMA warps run their loops with all 32 lanes and warp-uniform control
@@ -460,8 +487,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     };
     if (warp == 0) {
       // ---------------- TMA producer ----------------
-      uint32_t s = early, phase = 0;
-      for (uint32_t i = early; i < n_kv; ++i) {
+      uint32_t s = 0, phase = 0;
+      for (uint32_t i = 0; i < n_kv; ++i) {
         if (!ptx::mbar_wait_uniform(kv_empty + 8 * s, phase ^ 1u, abort_ptr, wait_ns) ||
             ((i == 2u || i == 3u) && !ptx::mbar_wait_uniform(q_full + 8 * (i - 2u), 0, abort_ptr, wait_ns))) {
           give_up(0, i);
@@ -1017,32 +1044,31 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
           }
         } else {
-          // Rows leave through shared memory and TMA stores of [32 rows x 64 columns] (rows past Sq are
-          // clipped); a thread's own stores touched 32 lines per instruction.
-          const uint32_t staging = stage_addr + stage * kStageBytes + quarter * (2u * kOutBoxBytes);
-          uint8_t *staging_ptr = base_ptr + (staging - base);
-#pragma unroll 1
-          for (int c = 2 * (int)hf; c < 2 * (int)hf + 2; ++c) {
+          // Rows leave through shared memory, a warp's [32 rows x 64 columns] as four whole lines per store; a thread's
+          // own stores touched 32 lines per instruction. (Tensor stores take the same time: until they have read the staging
+          // the CTA waits 1200 clocks at its end.)
+          uint8_t *box = base_ptr + (stage_addr - base) + stage * kStageBytes + (quarter * 2u + hf) * kOutBoxBytes;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
             uint32_t o[32];
-            ptx::tmem_ld_32x32(o_tmem + 32u * c, o);
+            ptx::tmem_ld_32x32(o_tmem + 64u * hf + 32u * c, o);
             ptx::tmem_ld_wait();
             uint32_t w[16];
             normalise(o, l, w);
-            uint8_t *box = staging_ptr + (c >> 1) * kOutBoxBytes + lane * 128;
 #pragma unroll
             for (int v = 0; v < 4; ++v)
-              *reinterpret_cast<uint4 *>(box + ((((c & 1) * 4 + v) ^ (lane & 7)) << 4)) =
+              *reinterpret_cast<uint4 *>(box + lane * 128 + (((c * 4 + v) ^ (lane & 7)) << 4)) =
                   make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
-            if (c & 1) {
-              ptx::fence_proxy_async();
-              __syncwarp();
-              if (lane == 0 && q0 + t * 128u + quarter * 32u < p.Sq)
-                ptx::tma_store_4d(staging + (c >> 1) * kOutBoxBytes, &map_o, (c >> 1) * 64, (int32_t)head,
-                                  (int32_t)(q0 + t * 128u + quarter * 32u), (int32_t)batch);
-            }
           }
-          if (lane == 0)
-            ptx::tma_store_read_wait();
+          __syncwarp();
+          const uint32_t row0 = qrow - lane + (lane >> 3), part = lane & 7;
+          uint4 *dst = reinterpret_cast<uint4 *>(p.out + (((uint64_t)batch * p.Sq + row0) * p.H + head) * kTile + 64u * hf) + part;
+#pragma unroll
+          for (uint32_t v = 0; v < 8; ++v) {
+            const uint32_t row = 4u * v + (lane >> 3);
+            if (row0 + 4u * v < p.Sq)
+              dst[(uint64_t)(4u * v) * p.H * (kTile / 8)] = *reinterpret_cast<const uint4 *>(box + row * 128u + ((part ^ (row & 7u)) << 4));
+          }
         }
       }
     }
@@ -1178,7 +1204,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       return fail(kInvalidArgument, "Attention(INT8): carried state needs a 16-byte aligned state buffer");
   }
 
-  CUtensorMap map_q, map_k, map_v, map_o;
+  CUtensorMap map_q, map_k, map_v;
   {
     const uint64_t dims[4] = {128, H, Sq, B};
     const uint64_t strides[3] = {128, H * 128, Sq * H * 128};
@@ -1200,14 +1226,6 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     const uint64_t strides[3] = {256, KV * 256, S * KV * 256};
     const uint32_t box[4] = {64, 1, 128, 1};
     if (int rc = encode_tensor_map(&map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, v_bf16, dims, strides, box,
-                                   CU_TENSOR_MAP_SWIZZLE_128B))
-      return rc;
-  }
-  {
-    const uint64_t dims[4] = {128, H, Sq, B};
-    const uint64_t strides[3] = {256, H * 256, Sq * H * 256};
-    const uint32_t box[4] = {64, 1, 32, 1};
-    if (int rc = encode_tensor_map(&map_o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, out_bf16, dims, strides, box,
                                    CU_TENSOR_MAP_SWIZZLE_128B))
       return rc;
   }
@@ -1270,6 +1288,9 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
   p.Sk = (uint32_t)S;
   p.H = (uint32_t)H;
   p.KV = (uint32_t)KV;
+  p.q_blocks = divisor((Sq + 255) / 256);
+  p.heads = divisor(H);
+  p.group = divisor(H / KV);
   p.S_pad = s_pad;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.wait_ns = wait_limit_ns();
@@ -1319,8 +1340,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
       config.attrs = attrs + 1;
       config.numAttrs = 1;
     }
-    return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k, map_v,
-                                       map_o, p),
+    return launched(cudaLaunchKernelEx(&config, ctas > 1 ? attn_i8_kernel<true> : attn_i8_kernel<false>, map_q, map_k, map_v, p),
                     "attn_i8_kernel launch");
   };
   if (whole)

@@ -139,19 +139,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
                "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
-// 4-D tiled TMA store, shared memory -> global, as its own bulk group.
-__device__ __forceinline__ void tma_store_4d(uint32_t src, const CUtensorMap *map, int32_t c0, int32_t c1, int32_t c2,
-                                             int32_t c3) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-// Waits until the sources of all groups have been read (the CTA may go then; the writes end with the kernel).
-__device__ __forceinline__ void tma_store_read_wait() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }

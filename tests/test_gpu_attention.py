@@ -449,3 +449,37 @@ def test_attention_masks_at_the_edges_of_the_tables_segments(ops, q_gain, from_b
     k82, ks2 = ob.orc().quantize_int8_rows([k2.reshape(-1, 128)], 1)
     assert torch.equal(run(k2, v2, k82.reshape(k8.shape), ks2).view(torch.int16), got.view(torch.int16))
     ops.poll_status()
+
+
+@pytest.mark.parametrize("B,Sq,Sk,H,KV", [(1, 1, 77, 1, 1), (3, 513, 130, 6, 2), (2, 31, 5, 15, 5), (2, 257, 260, 7, 7), (5, 33, 128, 3, 1)])
+def test_attention_items_of_every_batch_head_and_query_block(ops, B, Sq, Sk, H, KV):
+    """The items of a launch against calls on one batch and head alone: the same bits. Rows whose sums are infinite, and
+    rows of a batch without valid keys, stand among ordinary ones."""
+    import torch
+    rng = np.random.default_rng(B * Sq + Sk)
+    q, k, v = _qkv(rng, B, Sq, H, KV)[0], *_qkv(rng, B, Sk, KV, KV)[1:]
+    v[0, 0, 0, 5] = 0x7F80   # +infinity: this column of the heads that share it, the same rows' others as they are
+    valid = np.ones((B, Sk), np.uint8)
+    valid[B - 1] = 1 if B == 1 else 0
+    (q8, qs), (k8, ks) = (ops.quantize_int8_rows([to_torch_bf16(x.reshape(-1, 128))], 1) for x in (q, k))
+    q8, qs, k8, ks = q8.view(B, Sq, H, 128), qs.view(B, Sq, H), k8.view(B, Sk, KV, 128), ks.view(B, Sk, KV)
+    tv, tm = to_torch_bf16(v), torch.from_numpy(valid).cuda()
+    got = ops.attention_int8(q8, qs, k8, ks, tv, tm)
+    for b in range(B):
+        for h in range(H):
+            g = h // (H // KV)
+            mine = [x[b:b + 1, :, i:i + 1].contiguous() for x, i in ((q8, h), (qs, h), (k8, g), (ks, g), (tv, g))]
+            alone = ops.attention_int8(*mine, tm[b:b + 1])
+            assert torch.equal(got[b:b + 1, :, h:h + 1].contiguous().view(torch.int16), alone.view(torch.int16)), (b, h)
+    assert torch.isposinf(got[0, :, :H // KV, 5]).all()
+    ordinary = got.float().clone()
+    ordinary[0, :, :H // KV, 5] = 0.0
+    assert torch.isfinite(ordinary).all()
+    if B > 1:
+        assert torch.count_nonzero(got[B - 1]) == 0
+    clean = v.copy()
+    clean[0, 0, 0, 5] = 0
+    rest = ops.attention_int8(q8, qs, k8, ks, to_torch_bf16(clean), tm).float()
+    rest[0, :, :H // KV, 5] = 0.0
+    assert torch.equal(ordinary, rest)
+    ops.poll_status()
