@@ -12,7 +12,7 @@
 // Layout. A warp works on 4 groups (1024 columns) at a time; each thread owns 16 consecutive elements of
 // two neighbouring groups as 16 packed fp32x2 registers (lane 0 of the pair = first group, lane 1 =
 // second group), so every butterfly is one packed add/sub for two groups. Stages 0-1 run on the
-// thread's own 16 elements; a 16x16 transpose through shared memory (XOR-swizzled, conflict-free)
+// thread's own 16 elements; a 16x16 transpose through shared memory (padded rows, conflict-free)
 // gives the thread the 16 elements of stride 16, on which stages 2-3 run.
 //
 // What bounds it: nothing alone. A warp's 1024 elements are about 430 instructions (13.5 per element and lane, 5 of them packed

@@ -421,7 +421,7 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
 // multiply then add): the statistic has the reference's bits. Then 8 lanes share a row, two runs of 8 elements
 // each, chosen so that rotation partners are in the same lane: every access to HBM is a full 128-byte line, and
 // the codes come from direct_codes. HBM-bound by its bytes (3 per element), by its arithmetic in practice:
-// 33272 x 24 rows with rotary 96 and codes take 127 us (230 us as one thread per row with
+// 33272 x 24 rows with rotary 96 and codes take 125 us (230 us as one thread per row with
 // IEEE divisions), 4096 x 24 with rotary 128 in pairs 21 us (37 us). Few rows take 8 per warp, for more warps in flight
 // (256 x 24: 12.6 -> 6.3 us a call).
 struct RowRopeParams {
