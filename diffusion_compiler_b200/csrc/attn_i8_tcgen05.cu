@@ -68,21 +68,6 @@ constexpr float kLeastSum = 1.0f / (1u << 25); // of a running maximum: its larg
 constexpr uint32_t kPairBytes = 4096;          // [2 phases][2 tiles][2 halves][128 rows] fp32
 constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + 256 + kPairBytes;
 
-// Division by a number that a launch fixes, of what is below 2^31: with 2^s the least power of two that is not below the
-// divisor and mul = ceil(2^(31 + s) / by), mul * by exceeds 2^(31 + s) by e < 2^s, so n * e < 2^(31 + s) and the quotient
-// of 2 n * mul and 2^(32 + s) is that of n and by.
-struct Divisor {
-  uint32_t by, mul, shift;
-  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return __umulhi(2u * n, mul) >> shift; }
-};
-Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
-  Divisor d{(uint32_t)by, 0, 0};
-  while ((1ull << d.shift) < by)
-    ++d.shift;
-  d.mul = (uint32_t)(((1ull << (31 + d.shift)) + by - 1) / by);
-  return d;
-}
-
 struct AttnParams {
   const int8_t *q8;      // [B,Sq,H,128]
   const float *qs;       // [B,Sq,H]

@@ -78,6 +78,21 @@ int poll_device_status(const char *what); // copies back, clears, maps to kExecu
 
 #ifdef __CUDACC__
 
+// Division by a number that a launch fixes, of what is below 2^31: with 2^s the least power of two that is not below the
+// divisor and mul = ceil(2^(31 + s) / by), mul * by exceeds 2^(31 + s) by e < 2^s, so n * e < 2^(31 + s) and the quotient
+// of 2 n * mul and 2^(32 + s) is that of n and by.
+struct Divisor {
+  uint32_t by, mul, shift;
+  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return __umulhi(2u * n, mul) >> shift; }
+};
+inline Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
+  Divisor d{(uint32_t)by, 0, 0};
+  while ((1ull << d.shift) < by)
+    ++d.shift;
+  d.mul = (uint32_t)(((1ull << (31 + d.shift)) + by - 1) / by);
+  return d;
+}
+
 // ---- programmatic dependent launch ----
 // A kernel launched with dependent_launch() may start while the one in front of it on the stream still runs: as soon as
 // all CTAs of that one have called grid_dependents_launch() (or ended) and there is room. Its set-up runs then; what

@@ -62,11 +62,19 @@ k_residual_gate_bf16(const uint4 *res, const uint4 *branch, const uint4 *gate, u
 }
 
 // ---- SwiGlu (cpu_executor.cpp:1267-1286): out = value * (gate / (1 + exp(-gate))) ----
+// Near HBM's rate, with the issue slots next (an exponential and a division per element), of which a 64-bit division per
+// group of 8 elements took its share: 33272 x 8192 296 us, so 272 = 6.0 TB/s; 4608 x 12288 67 -> 61. The launch makes a
+// reciprocal where that holds, for less than 2^31 groups. (ResidualGate, whose time is its bytes, gains nothing by it.)
+struct Wide {
+  uint64_t by;
+  __device__ __forceinline__ uint64_t quotient(uint64_t n) const { return n / by; }
+};
+template <class D>
 __global__ void __launch_bounds__(256)
-k_swiglu_bf16(const uint4 *x, uint4 *o, uint64_t rows, uint64_t width8, uint64_t in_width8, uint64_t start8,
-              int gate_first) {
-  GRID_STRIDE(i, rows * width8) {
-    const uint64_t row = i / width8, col = i - row * width8, base = row * in_width8 + start8 + col;
+k_swiglu_bf16(const uint4 *x, uint4 *o, uint64_t groups, const D width, uint64_t in_width8, uint64_t start8, int gate_first) {
+  const uint64_t width8 = width.by;
+  GRID_STRIDE(i, groups) {
+    const uint64_t row = width.quotient(i), col = i - row * width8, base = row * in_width8 + start8 + col;
     float value[8], gate[8], y[8];
     unpack8(__ldg(x + base + (gate_first ? width8 : 0)), value);
     unpack8(__ldg(x + base + (gate_first ? 0 : width8)), gate);
@@ -653,9 +661,15 @@ bool swiglu_fast(const void *x, void *o, uint32_t dt, uint64_t rows, uint64_t wi
                  uint64_t start, bool gate_first, cudaStream_t s, int *rc) {
   if (dt != 2 || width % 8 != 0 || in_width % 8 != 0 || start % 8 != 0 || !aligned16(x) || !aligned16(o))
     return false;
-  k_swiglu_bf16<<<blocks_for(rows * (width / 8), 256), 256, 0, s>>>(
-      static_cast<const uint4 *>(x), static_cast<uint4 *>(o), rows, width / 8, in_width / 8, start / 8,
-      gate_first ? 1 : 0);
+  const uint64_t groups = rows * (width / 8);
+  auto launch = [&](auto kernel, auto by) {
+    kernel<<<blocks_for(groups, 256), 256, 0, s>>>(static_cast<const uint4 *>(x), static_cast<uint4 *>(o), groups, by,
+                                                   in_width / 8, start / 8, gate_first ? 1 : 0);
+  };
+  if (groups != 0 && groups < (1ull << 31))
+    launch(k_swiglu_bf16<Divisor>, divisor(width / 8));
+  else
+    launch(k_swiglu_bf16<Wide>, Wide{width / 8});
   *rc = done("k_swiglu_bf16");
   return true;
 }

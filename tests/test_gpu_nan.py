@@ -83,3 +83,27 @@ def test_qk_norm_rope(dim):
     c, s = angle.cos()[:, None], angle.sin()[:, None]
     half = torch.cat([-n[..., dim // 2:], n[..., :dim // 2]], -1)
     _same_nan(out.view(9, 3, dim), n * c + half * s)
+
+
+@pytest.mark.parametrize("rows,width,start,gate_first", [(1, 8, 0, 0), (5, 24, 8, 1), (300, 3072, 0, 1), (77, 8192, 16, 0), (1101, 136, 0, 0)])
+def test_swiglu_rows_and_columns_of_the_fast_form(rows, width, start, gate_first):
+    """The form that takes 16 bytes at a time finds rows and columns by a reciprocal of the width; the general form, which
+    operands that start on two bytes take, divides. The same bits, and nothing written behind the last row."""
+    import ctypes as C
+    import torch
+    from diffusion_compiler_b200 import _lib
+    in_width = start + 2 * width + 8
+    n, m = rows * in_width, rows * width
+    x = torch.randn(n + 8, generator=torch.Generator().manual_seed(rows + width)).to(torch.bfloat16).cuda()
+    moved = torch.cat([x[:1], x[:n]])
+    fast, general = (torch.full((m + 16,), 3.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+
+    def call(src, dst):
+        _lib.check(_lib.lib().difb200_swiglu(C.c_void_p(src.data_ptr()), C.c_void_p(dst.data_ptr()), 2, C.c_uint64(rows), C.c_uint64(width),
+                                             C.c_uint64(in_width), C.c_uint64(start), gate_first, None))
+        torch.cuda.synchronize()
+
+    call(x, fast)
+    call(moved[1:], general[1:])
+    assert torch.equal(fast[:m].view(torch.int16), general[1:m + 1].view(torch.int16))
+    assert bool((fast[m:] == 3.0).all()) and bool((general[m + 1:] == 3.0).all()) and bool(general[0] == 3.0)
