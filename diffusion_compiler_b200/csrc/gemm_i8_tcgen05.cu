@@ -376,8 +376,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t row = m0 + quarter * 32u + lane;
       const bool row_ok = row < p.M;
       const float rs = row_ok ? load_produced(p.row_scales + row) : 0.0f;
+      // A warp whose 32 rows lie behind the last one has nothing to convert. Nor may it fill a box: the wait for a box counts
+      // the groups committed behind its last store, so that a fill without a store and commit of its own would let the next
+      // fill overwrite a box that an earlier tile's store still reads.
+      const uint32_t subs = m0 + quarter * 32u < p.M ? BN / 64 : 0u;
 #pragma unroll 1
-      for (uint32_t sub = 0; sub < BN / 64; ++sub) {
+      for (uint32_t sub = 0; sub < subs; ++sub) {
         const uint32_t chunk = col_half * (BN / 64) + sub; // 32-column chunk of the tile
         uint32_t r[32];
         ptx::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + acc * BN + chunk * 32u, r);
@@ -450,7 +454,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
           ptx::fence_proxy_async();
           __syncwarp();
-          if (lane == 0 && m0 + quarter * 32u < p.M) {
+          if (lane == 0) {
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                              reinterpret_cast<uint64_t>(&map_c)),
                          "r"(my_staging + store_buf * kStoreBoxBytes), "r"((int32_t)n_base),

@@ -181,6 +181,31 @@ def test_linear_int8_scaled_narrow_and_split_tiles(ops, monkeypatch, form, M, K,
     ops.poll_status()
 
 
+@pytest.mark.parametrize("form", ["2,256,1", "2,192,1", "2,128,1", "1,256,1", "1,128,1"])
+@pytest.mark.parametrize("K", [256, 512])
+def test_linear_int8_scaled_warps_without_rows_behind_full_tiles(ops, monkeypatch, form, K):
+    """Three and more tiles per CTA, of which the last ones end with the rows in every quarter of a 128-row tile: a warp
+    without rows there has just stored boxes of full tiles, which must not be filled again while they are read. Few
+    k-blocks, so that the next accumulator is complete when a tile's epilogue ends. The bias would show in the full tiles."""
+    import torch
+    monkeypatch.setenv("DIFB200_GEMM_FORM", form)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    N, rest = 74 * 256 + 8, (1, 33, 97, 129, 193, 224)
+    x8, w8 = (torch.randint(-127, 128, s, generator=g, device="cuda", dtype=torch.int8) for s in ((512 + max(rest), K), (N, K)))
+    xs, ws = torch.rand(len(x8), generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+    bias = torch.randn(N, generator=g, device="cuda").to(torch.bfloat16) * 1000
+    acc = (x8.double() @ w8.double().T).float()  # exact: |sum| < 2^24
+    want = ((((acc * xs[:, None]) * ws[None]).to(torch.bfloat16)).float() + bias.float()[None]).to(torch.bfloat16)
+    for M in (512 + r for r in rest):
+        outs = [torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+        for out in outs:
+            ops.linear_int8_scaled(x8[:M], w8, xs[:M], ws, bias=bias, out=out[:M])
+        for out in outs:
+            assert torch.equal(out[:M].view(torch.int16), want[:M].view(torch.int16)), M
+            assert bool((out[M] == 7.0).all())
+    ops.poll_status()
+
+
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32, 33])  # 8, 16 and 32 rows per form; 33 is the tile kernel's
 @pytest.mark.parametrize("K,N", [(16, 16), (48, 1), (80, 131), (3072, 40), (3136, 24), (12288, 17), (16, 3000)])
 def test_linear_of_few_rows_bit_exact(ops, M, K, N):
