@@ -230,6 +230,42 @@ def test_linear_of_few_rows_bit_exact(ops, M, K, N):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("packer", ["quantize", "pack"])
+@pytest.mark.parametrize("rows", [1, 9, 30])
+def test_linear_of_few_rows_directly_behind_the_kernel_that_writes_its_weights(ops, rows, packer):
+    """The weights' codes are written into the same buffer again and again, by kernels that let the linear start early, with no
+    synchronisation in between: every linear reads the codes written directly in front of it."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    weights = [torch.randn((3000, 2048), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    codes, scales = torch.empty((3000, 2048), dtype=torch.int8, device="cuda"), torch.empty(3000, device="cuda")
+    x8 = torch.randint(-127, 128, (rows, 2048), generator=g, device="cuda", dtype=torch.int8)
+    xs = torch.rand(rows, generator=g, device="cuda")
+    from diffusion_compiler_b200 import _lib
+
+    def write(w):
+        if packer == "quantize":
+            ops.quantize_int8_rows([w], 2, out=(codes, scales))
+        else:
+            ops._call(_lib.lib().difb200_quantize_weight_rows, 0, w.data_ptr(), None, 3000, 2048, 2, 0, codes.data_ptr(),
+                      scales.data_ptr())
+
+    want = []
+    for w in weights:
+        write(w)
+        torch.cuda.synchronize()
+        want.append(((x8.double() @ codes.double().T).float() * xs[:, None] * scales[None]).to(torch.bfloat16))  # exact sums
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(4):
+        for w in weights:
+            write(w)
+            got.append(ops.linear_int8_scaled(x8, codes, xs, scales))
+    for i, out in enumerate(got):
+        assert torch.equal(out.view(torch.int16), want[i % 3].view(torch.int16)), i
+    ops.poll_status()
+
+
 @pytest.mark.parametrize("rows", [1, 16, 30])
 def test_w8a8_linear_of_few_rows_matches_two_calls(ops, rows):
     """The single call, whose weights are requested before the quantiser in front is complete, back to back."""
