@@ -25,7 +25,7 @@ struct GemmParams {
 };
 
 // Whether the kernels of few rows take a problem, and their launch (weights and codes start on 16 bytes, K % 16 == 0).
-bool few_rows(uint64_t M, uint64_t N, uint64_t K);
+bool few_rows(uint64_t M, uint64_t N, uint64_t K, bool weights_first);
 int launch_few_rows(const int8_t *x, const int8_t *w, const GemmParams &p, cudaStream_t stream);
 
 #ifdef __CUDACC__

@@ -646,7 +646,7 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   p.weights_first = weights_ready && p.withhold_kb == 0xffffffffu ? 1u : 0u;
   p.wait_ns = wait_limit_ns();
   p.status = status;
-  if (p.withhold_kb == 0xffffffffu && few_rows(M, N, K))
+  if (p.withhold_kb == 0xffffffffu && few_rows(M, N, K, p.weights_first != 0u))
     return launch_few_rows(x, w, p, stream);
 
   const Form form = choose_form(M, N, K);

@@ -308,17 +308,47 @@ int launch_groups(const FewParams &f, cudaStream_t stream) {
                   "gemm_i8_few_rows_kernel launch");
 }
 
+// Waves of the few-rows kernels: two CTAs of 16 columns per SM.
+uint64_t few_waves(uint64_t N) {
+  const uint64_t columns = 32ull * (uint64_t)sm_count();
+  return (N + columns - 1) / columns;
+}
+bool tile_form_is_forced() { return std::getenv("DIFB200_GEMM_FORM") || std::getenv("DIFB200_GEMM_CTAS"); }
+
 } // namespace
 
-// Whether the few-rows kernels take a problem. Every CTA reads all rows' codes, which come from the same few lines of L2, so
-// the time grows with the rows and, the more of them, with the weights. us of a linear, tile kernel / this (K x N): 8 rows
-// 3072 x 3072 10.4 / 5.3, 3072 x 9216 10.2 / 7.9, 3072 x 16384 11.5 / 11.9, 12288 x 3072 14.4 / 11.4; 16 rows 10.4 / 6.3, 10.2 / 10.5,
-// 11.5 / 15.2, 14.4 / 13.2, 3072 x 12288 12.9 / 12.8; 32 rows 10.4 / 8.3, 10.4 / 14.5.
-bool few_rows(uint64_t M, uint64_t N, uint64_t K) {
-  if (std::getenv("DIFB200_GEMM_FORM") || std::getenv("DIFB200_GEMM_CTAS"))
-    return false; // a tile form is forced
-  return M <= 8 || (M <= 16 && N * K <= (5ull << 23)) || (M <= 32 && N * K <= (1ull << 24));
+// Whether the few-rows kernel takes a linear from the tile kernel. Every CTA reads all rows' codes and pays its start, its sums
+// and its outputs for 16 columns: the time grows with the waves of CTAs, and with 9 and 17 rows by an MMA per chunk, where the
+// tile kernel's hardly does. So the line is one of waves (4736 columns each on 148 SMs), and of K where both come close. Tile
+// kernel / this one, us, weights not in L2:
+//   1 to 8 rows    two waves   8 x 128 x 9216 3.9 / 3.7, 8 x 3072 x 9216 10.4 / 9.1, 8 x 8192 x 9216 18.3 / 18.6
+//                  three       8 x 3072 x 12288 11.4 / 11.8, 4 x 8192 x 12288 24.1 / 23.7; 8 x 512 x 16384 5.8 / 7.8; with a
+//                              quantiser in front, behind which this one has its first weights already, 8 x 512 x 12288 8.0 / 9.0,
+//                              8 x 2048 x 12288 11.9 / 11.7, 4 x 3072 x 12288 13.8 / 13.2
+//   9 to 16 rows   one wave    16 x 128 x 4736 3.9 / 2.7, 16 x 12288 x 3072 13.9 / 12.7
+//                  two         16 x 3072 x 9216 10.5 / 10.4, 16 x 128 x 9216 3.9 / 4.4, 16 x 4096 x 9216 12.3 / 14.0
+//   17 to 32 rows  one wave    32 x 256 x 4736 4.1 / 4.0, 32 x 3072 x 4736 8.8 / 7.8, 32 x 12288 x 1024 11.5 / 11.2
+//                  two         32 x 512 x 5120 6.0 / 6.1, 17 x 512 x 12288 5.4 / 10.5
+// The limits on N K end what was measured: beyond them the two are within a few percent.
+bool few_rows(uint64_t M, uint64_t N, uint64_t K, bool weights_first) {
+  if (M > 32 || tile_form_is_forced())
+    return false;
+  const uint64_t waves = few_waves(N);
+  if (M <= 8)
+    return waves <= 2 || (waves == 3 && K >= (weights_first ? 2048u : 8192u));
+  if (M <= 16)
+    return waves == 1 ? N * K <= (5ull << 23) : waves == 2 && K >= 256 && K <= 3072;
+  return waves == 1 && N * K <= (1ull << 24);
 }
+
+namespace {
+// The same for the whole linear in one launch, which has the quantiser's launch to save and stays for further tiles. Quantiser and
+// tile kernel / this one, us: 8 x 1024 x 16384 10.0 / 9.8, 2 x 3072 x 16384 15.6 / 13.3, 2 x 3072 x 32768 24.5 / 19.8; but
+// 8 x 256 x 32768 9.7 / 11.5, 8 x 1024 x 32768 13.1 / 14.8.
+bool few_rows_in_one_launch(uint64_t M, uint64_t N, uint64_t K) {
+  return M <= kFusedRows && !tile_form_is_forced() && (few_waves(N) <= 4 || K >= 2048);
+}
+} // namespace
 
 int launch_few_rows(const int8_t *x, const int8_t *w, const GemmParams &p, cudaStream_t stream) {
   const FewParams f{x, w, p};
@@ -330,10 +360,10 @@ bool w8a8_few_rows(const void *x_bf16, const int8_t *w, const float *col_scales,
                    void *out_bf16, cudaStream_t stream, int *rc) {
   const uint64_t row_blocks = (K + 1023) / 1024;
   const uintptr_t aligned = reinterpret_cast<uintptr_t>(x_bf16) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(codes);
-  if (implementation != 2 || M == 0 || M > kFusedRows || N == 0 || N > 0x7fffffffull || K == 0 || K % 256 != 0 ||
+  if (implementation != 2 || M == 0 || N == 0 || N > 0x7fffffffull || K == 0 || K % 256 != 0 ||
       M * row_blocks > kFusedBlocks || !(clip > 0.0f) || !x_bf16 || !w || !col_scales || !codes || !scales || !out_bf16 ||
-      (epilogue & ~(kEpiBias | kEpiGeluTanh)) || ((epilogue & kEpiBias) && !bias_bf16) || (aligned & 15) || !few_rows(M, N, K) ||
-      gemm_load_is_withheld())
+      (epilogue & ~(kEpiBias | kEpiGeluTanh)) || ((epilogue & kEpiBias) && !bias_bf16) || (aligned & 15) ||
+      gemm_load_is_withheld() || !few_rows_in_one_launch(M, N, K))
     return false;
   // Every CTA reads all of x, and other CTAs write meanwhile: not where a call is in place.
   const uintptr_t begin = reinterpret_cast<uintptr_t>(x_bf16), end = begin + M * K * 2;

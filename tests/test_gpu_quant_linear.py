@@ -230,6 +230,55 @@ def test_linear_of_few_rows_bit_exact(ops, M, K, N):
     ops.poll_status()
 
 
+@pytest.mark.parametrize("M", [8, 9, 16, 17, 32])
+@pytest.mark.parametrize("K,N", [(16, 4736), (240, 4752), (256, 4752), (528, 9472), (528, 9488), (3072, 9472), (3088, 9472), (3088, 4736),
+                                 (3856, 4352), (8176, 9488), (8192, 14208), (8192, 14224), (10240, 4096), (10240, 4100)])
+def test_linear_on_both_sides_of_the_lines_of_few_rows(ops, monkeypatch, M, K, N):
+    """Numbers of rows, columns (waves of 4736 on 148 SMs) and k at which the dispatch goes from the few-rows kernel to the tile
+    kernel: the same bits from both, and never one that takes half as long again as the other would."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x8, w8 = (torch.randint(-128, 128, s, generator=g, device="cuda", dtype=torch.int8) for s in ((M, K), (N, K)))
+    xs, ws = torch.rand(M, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+
+    def run():
+        out = ops.linear_int8_scaled(x8, w8, xs, ws)
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            for _ in range(10):
+                ops.linear_int8_scaled(x8, w8, xs, ws, out=out)
+        times = []
+        for _ in range(20):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return out, min(times)
+
+    got, time = run()
+    monkeypatch.setenv("DIFB200_GEMM_FORM", "0,0,0")  # no such form: the tile kernel's own choice
+    want, tile_time = run()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert time <= 1.5 * tile_time, (time, tile_time)
+    ops.poll_status()
+
+
+@pytest.mark.parametrize("M,K,N", [(8, 256, 18944), (8, 256, 18960), (8, 1024, 32768), (4, 2048, 32768), (2, 3072, 20000), (3, 3072, 14208), (3, 3072, 14224), (16, 512, 12288), (32, 256, 16384)])
+def test_w8a8_linear_on_both_sides_of_the_lines_of_few_rows(ops, monkeypatch, M, K, N):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    w8 = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(N, generator=g, device="cuda") * 0.01
+    got = ops.w8a8_linear(x, w8, ws)
+    monkeypatch.setenv("DIFB200_GEMM_FORM", "0,0,0")
+    assert torch.equal(got.view(torch.int16), ops.w8a8_linear(x, w8, ws).view(torch.int16))
+    ops.poll_status()
+
+
 @pytest.mark.parametrize("packer", ["quantize", "pack"])
 @pytest.mark.parametrize("rows", [1, 9, 30])
 def test_linear_of_few_rows_directly_behind_the_kernel_that_writes_its_weights(ops, rows, packer):
