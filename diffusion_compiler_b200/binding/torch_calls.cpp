@@ -92,6 +92,8 @@ PyObject *w8a8_linear(PyObject *, Args args, Py_ssize_t n) {
     if (args[3] != Py_None && !(bias = dense(args[3], at::kBFloat16, device)))
       return none();
     const int64_t K = x->size(-1), M = x->numel() / K, N = w->size(0);
+    if (w->size(1) != K || ws->numel() != N || (bias && bias->numel() != N))
+      return none();
     const int gelu = PyObject_IsTrue(args[4]);
     const long implementation = PyLong_AsLong(args[5]);
     const double clip = PyFloat_AsDouble(args[6]);
@@ -177,6 +179,8 @@ PyObject *norm_modulate_quant(PyObject *, Args args, Py_ssize_t n) {
     if ((layer || args[1] != Py_None) && !(weight = dense(args[1], at::kBFloat16, device)))
       return none();
     if (layer && !(bias = dense(args[2], at::kBFloat16, device)))
+      return none();
+    if ((weight && weight->numel() != x->size(1)) || (bias && bias->numel() != x->size(1)))
       return none();
     const double epsilon = PyFloat_AsDouble(args[5]), clip = PyFloat_AsDouble(args[7]);
     const long implementation = PyLong_AsLong(args[6]);

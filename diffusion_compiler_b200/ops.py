@@ -55,6 +55,12 @@ def _require(t: torch.Tensor, dtype: torch.dtype, name: str) -> torch.Tensor:
     return t.contiguous()
 
 
+def _require_elements(t: Optional[torch.Tensor], count: int, name: str) -> None:
+    """The kernels read ``count`` elements behind the pointer they are given."""
+    if t is not None and t.numel() < count:
+        raise ValueError("%s has %d elements, %d are needed" % (name, t.numel(), count))
+
+
 def quantize_int8_rows(parts: Sequence[torch.Tensor], implementation: int = 2, clip: float = 1.0,
                        clip_tensor: Optional[torch.Tensor] = None, residual: bool = False,
                        out: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> Tuple[torch.Tensor, ...]:
@@ -113,6 +119,7 @@ def rms_norm_modulate_quant(x: torch.Tensor, weight: Optional[torch.Tensor], sca
     M, K = x.shape
     if scale.shape != x.shape or shift.shape != x.shape:
         raise ValueError("scale and shift must have the shape of x")
+    _require_elements(weight, K, "weight")
     codes = torch.empty((M, K), dtype=torch.int8, device=x.device)
     scales = torch.empty((M,), dtype=torch.float32, device=x.device)
     _call(_lib.lib().difb200_rms_norm_modulate_quant, x.device.index, x.data_ptr(), _ptr(weight), scale.data_ptr(),
@@ -135,6 +142,8 @@ def layer_norm_modulate_quant(x: torch.Tensor, weight: torch.Tensor, bias: torch
     M, K = x.shape
     if scale.shape != shift.shape or scale.shape[-1] != K or M % scale.shape[0] != 0:
         raise ValueError("scale and shift must be [M / r, K]")
+    _require_elements(weight, K, "weight")
+    _require_elements(bias, K, "bias")
     codes = torch.empty((M, K), dtype=torch.int8, device=x.device)
     scales = torch.empty((M,), dtype=torch.float32, device=x.device)
     _call(_lib.lib().difb200_layer_norm_modulate_quant, x.device.index, x.data_ptr(), weight.data_ptr(),
@@ -193,6 +202,7 @@ def linear_int8_scaled(x8: torch.Tensor, w8: torch.Tensor, row_scales: torch.Ten
     flags = 0
     if bias is not None:
         bias = _require(bias, torch.bfloat16, "bias")
+        _require_elements(bias, N, "bias")
         flags |= EPILOGUE_BIAS
     if gelu:
         flags |= EPILOGUE_GELU_TANH
@@ -220,9 +230,13 @@ def w8a8_linear(x: torch.Tensor, w8: torch.Tensor, col_scales: torch.Tensor,
     K = x.shape[-1]
     M = x.numel() // K
     N = w8.shape[0]
+    if w8.numel() != N * K:
+        raise ValueError("w8 must be [N,K] for an x of K columns")
+    _require_elements(col_scales, N, "col_scales")
     flags = 0
     if bias is not None:
         bias = _require(bias, torch.bfloat16, "bias")
+        _require_elements(bias, N, "bias")
         flags |= EPILOGUE_BIAS
     if gelu:
         flags |= EPILOGUE_GELU_TANH
@@ -325,10 +339,13 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key_valid: Opti
     v = _require(v, torch.bfloat16, "v")
     B, S, H, D = q.shape
     KV = k.shape[2]
+    _require_elements(k, B * S * KV * D, "k")
+    _require_elements(v, B * S * KV * D, "v")
     if key_valid is not None:
         if key_valid.dtype != torch.uint8:
             key_valid = key_valid.to(torch.uint8)
         key_valid = key_valid.contiguous()
+        _require_elements(key_valid, B * S, "key_valid")
     if scale is None:
         scale = 1.0 / (D ** 0.5)
     if out is None:

@@ -61,6 +61,9 @@ def test_native_calls_equal_the_general_way(both):
     for i, call in enumerate(calls):
         native, general = both(call)
         assert _same(native, general), i
+    wide = n(64)  # more entries than are read
+    native, general = both(lambda: ops.w8a8_linear(x, w8, torch.cat([ws, ws]), bias=wide))
+    assert _same(native, ops.w8a8_linear(x, w8, ws, bias=wide[:48])) and _same(native, general)
     stream = torch.cuda.Stream()  # the current stream's, whichever it is
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
@@ -76,3 +79,31 @@ def test_native_calls_equal_the_general_way(both):
         with pytest.raises(ValueError):
             bad()
     ops.poll_status()
+
+
+def test_operands_of_too_few_elements_are_refused():
+    """Refused on the host, before a launch, natively and the general way: weights of another width, vectors that end early,
+    keys of fewer tokens than the queries."""
+    import torch
+    from diffusion_compiler_b200 import _lib, ops
+    z = lambda *s, dtype=torch.bfloat16: torch.zeros(s, dtype=dtype, device="cuda")  # noqa: E731
+    x, w8, ws = z(2, 512), z(48, 512, dtype=torch.int8), z(48, dtype=torch.float32)
+    x8, xs = z(2, 512, dtype=torch.int8), z(2, dtype=torch.float32)
+    q, k = z(1, 70, 4, 128), z(1, 70, 2, 128)
+    launches = _lib.lib().difb200_launch_count()
+    for bad in (lambda **o: ops.w8a8_linear(x, w8[:, :256].contiguous(), ws, **o), lambda **o: ops.w8a8_linear(x, w8[:, :496], ws, **o),
+                lambda **o: ops.w8a8_linear(x, z(48, 768, dtype=torch.int8), ws, **o), lambda **o: ops.w8a8_linear(x, w8, ws[:47], **o),
+                lambda **o: ops.w8a8_linear(x, w8, ws, bias=x[0, :47], **o)):
+        for kwargs in ({}, {"out": z(2, 48)}):  # with `out` the general way takes the call
+            with pytest.raises(ValueError):
+                bad(**kwargs)
+    for bad in (lambda: ops.linear_int8_scaled(x8, w8, xs, ws, bias=x[0, :47]),
+                lambda: ops.rms_norm_modulate_quant(x, x[0, :511], x, x),
+                lambda: ops.layer_norm_modulate_quant(x, x[0, :511], x[0], x, x),
+                lambda: ops.layer_norm_modulate_quant(x, x[0], x[0, :511], x, x),
+                lambda: ops.attention(q, k[:, :69], k), lambda: ops.attention(q, k, k[:, :69]),
+                lambda: ops.attention(q, k, k, key_valid=z(1, 69, dtype=torch.uint8)),
+                lambda: ops.attention(q, k, k[:, :, :1], out=z(1, 70, 4, 128))):
+        with pytest.raises(ValueError):
+            bad()
+    assert _lib.lib().difb200_launch_count() == launches
