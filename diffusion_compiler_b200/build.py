@@ -9,6 +9,7 @@ that ops.py calls it through on torch tensors.
 """
 from __future__ import annotations
 
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -22,6 +23,7 @@ OBJ_DIR = os.path.join(HERE, "_obj")
 LIB_PATH = os.path.join(HERE, "libdifb200.so")
 CALLS_SOURCE = os.path.join(HERE, "binding", "torch_calls.cpp")
 CALLS_PATH = os.path.join(HERE, "_torch_calls.so")
+CALLS_STAMP = os.path.join(OBJ_DIR, "torch_calls.stamp")  # what _torch_calls.so was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -68,9 +70,23 @@ def build(force: bool = False, verbose: bool = False) -> str:
         list(pool.map(run, jobs))
     if jobs or force or _stale(LIB_PATH, objs):
         run([nvcc, "-shared", "-o", LIB_PATH] + objs + ["-Xlinker", "--no-undefined", "-ldl", "-lpthread"])
-    if force or _stale(CALLS_PATH, [CALLS_SOURCE] + headers):
+    if force or _calls_stale([CALLS_SOURCE] + headers):
         run(_calls_command())
+        with open(CALLS_STAMP, "w") as f:
+            f.write(_calls_target())
     return LIB_PATH
+
+
+def _calls_target() -> str:
+    """The interpreter and the torch that a binding built now is for: it loads with no others."""
+    return "Python %s, torch %s" % (sys.version, importlib.metadata.version("torch"))
+
+
+def _calls_stale(deps) -> bool:
+    if _stale(CALLS_PATH, deps) or not os.path.exists(CALLS_STAMP):
+        return True
+    with open(CALLS_STAMP) as f:
+        return f.read() != _calls_target()
 
 
 def _calls_command():

@@ -137,3 +137,17 @@ def test_abi_layout_matches_reference(tmp_path):
     path.write_text("\n".join(src))
     res = subprocess.run(["gcc", "-std=c11", "-fsyntax-only", str(path)], capture_output=True, text=True)
     assert res.returncode == 0, res.stderr
+
+
+def test_binding_is_built_again_for_another_torch_or_python(monkeypatch, tmp_path):
+    from diffusion_compiler_b200 import build
+    binding, stamp = tmp_path / "binding.so", tmp_path / "stamp"
+    monkeypatch.setattr(build, "CALLS_PATH", str(binding))
+    monkeypatch.setattr(build, "CALLS_STAMP", str(stamp))
+    assert build._calls_stale([])
+    binding.write_text("")
+    assert build._calls_stale([])  # not known for what
+    stamp.write_text(build._calls_target())
+    assert not build._calls_stale([])
+    monkeypatch.setattr(build.importlib.metadata, "version", lambda name: "0.1")
+    assert build._calls_stale([])
