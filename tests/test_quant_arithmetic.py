@@ -38,22 +38,28 @@ def test_bf16_quotient_for_every_pair_of_significands():
 
 
 def test_bf16_quotient_in_two_bf16_parts_for_every_pair_of_significands():
-    """bf16(v / s) as fma(v, r1, bf16(v r2)) rounded once to bf16, with r1 = bf16(r), r2 = bf16(r - r1), as the 256-wide
-    quantiser forms it, for all 128 x 128 pairs. r is 1 + 6 / 2^23 times an approximate reciprocal that is within 2^-23
-    of the exact one: every r between 1 + 18 / 2^25 and 1 + 30 / 2^25 times the exact reciprocal has to do (steps of 2^-25)."""
+    """bf16(v / s) as fma(v, r1, bf16(v r2)) rounded once to bf16, with r1 = bf16(r), r2 = bf16(r - r1), as SplitReciprocal of
+    csrc/quant_common.cuh forms it, for all 128 x 128 pairs and every fp32 r between 1 + 2^-25 and 1 + 43 / 2^25 times the
+    exact reciprocal. The kernel's r is 1 + 6 / 2^23 times an approximate one within 2^-23 of the exact one, rounded once
+    more: between 1 + 18 / 2^25 and 1 + 30 / 2^25 times."""
     def bf16(x):  # nearest even, 8 significant bits; x exact in float64
         m, e = np.frexp(x)
         return np.ldexp(np.rint(m * 256.0), e - 8)
 
-    v = np.arange(128, 256, dtype=np.float64)[:, None]
-    s = np.arange(128, 256, dtype=np.float64)[None, :]
-    want = bf16(v / s)  # no quotient is within 2^-17 of a rounding boundary
-    for step in range(16, 33):
-        r = (1.0 / s) * (1.0 + step * 2.0 ** -25)
+    v = np.arange(128, 256, dtype=np.float64)
+    seen = 0
+    for s in range(128, 256):
+        want = bf16(v / s)  # no quotient is within 2^-17 of a rounding boundary
+        least, most = ((1.0 + step * 2.0 ** -25) / s for step in (1, 43))
+        bits = np.float32([least, most]).view(np.uint32)
+        r = np.arange(bits[0] - 1, bits[1] + 2, dtype=np.uint32).view(np.float32).astype(np.float64)
+        r = r[(r >= least) & (r <= most)]
+        seen += len(r)
         r1 = bf16(r)
-        r2 = bf16(r - r1)
-        got = bf16(v * r1 + bf16(v * r2))  # 8 + 8 bits and a term at most 2^9 times smaller: exact in float64
-        assert np.array_equal(got, want), step
+        r2 = bf16(r - r1)  # the difference is exact
+        got = bf16(v[:, None] * r1 + bf16(v[:, None] * r2))  # 8 + 8 bits and a term at most 2^9 times smaller: exact in float64
+        assert np.array_equal(got, np.broadcast_to(want[:, None], got.shape)), s
+    assert seen >= 128 * 10  # an fp32 step is 2^-24 to 2^-23 of the reciprocal
 
 
 def test_direct_codes_from_one_product_for_every_pair_of_significands():
