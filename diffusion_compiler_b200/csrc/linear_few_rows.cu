@@ -9,8 +9,9 @@
 // tile kernel, whose epilogue arithmetic this one shares.
 //
 // The smallest problems are one launch: every CTA rotates and quantises the rows itself, while its weights are on their way.
-// That costs a CTA about 1.5 us and saves the quantiser's launch, 2.5 us of the GPU and as much of the host (2 x 3072 x 3072: a
-// call 8.1 -> 5.0 us, which the host's part bounds; 10.8 of the GPU with the tile kernel).
+// That costs a CTA about 1.5 us and saves a launch, 3 us of the host. 2 x 3072 x 3072, one launch / two / the tile kernel and a
+// quantiser, us per call of calls one behind the other: weights in L2 6.7 / 8.0 / 12.3, not in L2 8.2 / 8.0 / 12.3, of these the
+// host 5.1 / 8.0 / 8.5; from a graph, not in L2, 6.2 / 5.4 / 11.0.
 #include "gemm_common.cuh"
 #include "ops.h"
 #include "quant_common.cuh"
@@ -54,79 +55,6 @@ __device__ __forceinline__ void write_output(const GemmParams &p, uint32_t row, 
   p.out[(size_t)row * p.N + n] = (uint16_t)bits;
 }
 
-// GROUPS: of 8 rows. READY: no kernel that may still run writes the weights (GemmParams::weights_first). Otherwise they are
-// read like everything that the kernel in front produces: the non-coherent path is for what nobody writes meanwhile. (It is
-// the faster one: 8 x 12288 x 3072, weights not in L2, 11.0 us against 11.2.)
-template <int GROUPS, bool READY>
-__global__ void __launch_bounds__(32 * kFewWarps, 2)
-gemm_i8_few_rows_kernel(const FewParams f) {
-  const GemmParams &p = f.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint32_t n0 = blockIdx.x * 16u;
-  const bool low_ok = n0 + g < p.N, high_ok = n0 + 8u + g < p.N;
-  const int8_t *low = f.w + (size_t)(low_ok ? n0 + g : 0) * p.K, *high = f.w + (size_t)(high_ok ? n0 + 8u + g : 0) * p.K;
-  const uint32_t chunks = (p.K + 63u) / 64u;
-  uint4 wl[kFewBatch], wh[kFewBatch];
-  auto at = [&](uint32_t first, int u) { return (first + warp + kFewWarps * u) * 64u + 16u * t; }; // this lane's k of a chunk
-  auto load = [](const int8_t *from) { return READY ? load_streamed(from) : load_produced(reinterpret_cast<const uint4 *>(from)); };
-  auto load_weights = [&](uint32_t first) {
-#pragma unroll
-    for (int u = 0; u < kFewBatch; ++u) {
-      const uint32_t k = at(first, u);
-      wl[u] = wh[u] = make_uint4(0, 0, 0, 0);
-      if (k < p.K) {
-        if (low_ok)
-          wl[u] = load(low + k);
-        if (high_ok)
-          wh[u] = load(high + k);
-      }
-    }
-  };
-  if (READY)
-    load_weights(0);
-  grid_dependency_wait();
-  grid_dependents_launch();
-  if (!READY)
-    load_weights(0);
-  int32_t c[GROUPS][4] = {};
-  for (uint32_t first = 0; first < chunks; first += kFewWarps * kFewBatch) {
-    if (first != 0u)
-      load_weights(first);
-#pragma unroll
-    for (int q = 0; q < GROUPS; ++q) {
-      const uint32_t row = 8u * q + g;
-      uint4 x[kFewBatch];
-#pragma unroll
-      for (int u = 0; u < kFewBatch; ++u) {
-        const uint32_t k = at(first, u);
-        x[u] = make_uint4(0, 0, 0, 0);
-        if (k < p.K && row < p.M)
-          x[u] = load_produced(reinterpret_cast<const uint4 *>(f.x + (size_t)row * p.K + k));
-      }
-#pragma unroll
-      for (int u = 0; u < kFewBatch; ++u) {
-        mma_s8_16x8x32(c[q], wl[u].x, wh[u].x, wl[u].y, wh[u].y, x[u].x, x[u].y);
-        mma_s8_16x8x32(c[q], wl[u].z, wh[u].z, wl[u].w, wh[u].w, x[u].z, x[u].w);
-      }
-    }
-  }
-  __shared__ int32_t sums[kFewWarps][GROUPS * 8][16]; // [warp][row][column]
-#pragma unroll
-  for (int q = 0; q < GROUPS; ++q)
-    store_sums(&sums[warp][8 * q][0], c[q]);
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < 16u * p.M; i += 32 * kFewWarps) {
-    const uint32_t row = i >> 4, n = n0 + (i & 15u);
-    if (n >= p.N)
-      continue;
-    int32_t acc = 0;
-#pragma unroll
-    for (int w = 0; w < kFewWarps; ++w)
-      acc += sums[w][row][i & 15u];
-    write_output(p, row, n, acc, load_produced(p.row_scales + row));
-  }
-}
-
 // The 16 columns from n0 on: lane (g, t) has columns g and g + 8.
 struct Columns {
   const int8_t *low, *high;
@@ -148,16 +76,18 @@ __device__ __forceinline__ uint32_t k_of(uint32_t first, int u) {
 // A batch of this warp's chunks of 16 columns' weights.
 struct Weights {
   uint4 low[kFewBatch], high[kFewBatch];
+  template <bool READY>
   __device__ __forceinline__ void load(const Columns &columns, uint32_t K, uint32_t first) {
+    auto from = [](const int8_t *at) { return READY ? load_streamed(at) : load_produced(reinterpret_cast<const uint4 *>(at)); };
 #pragma unroll
     for (int u = 0; u < kFewBatch; ++u) {
       const uint32_t k = k_of(first, u);
       low[u] = high[u] = make_uint4(0, 0, 0, 0);
       if (k < K) {
         if (columns.low_ok)
-          low[u] = load_streamed(columns.low + k);
+          low[u] = from(columns.low + k);
         if (columns.high_ok)
-          high[u] = load_streamed(columns.high + k);
+          high[u] = from(columns.high + k);
       }
     }
   }
@@ -170,9 +100,62 @@ struct Weights {
   }
 };
 
+// GROUPS: of 8 rows. READY: no kernel that may still run writes the weights (GemmParams::weights_first). Otherwise they are
+// read like everything that the kernel in front produces: the non-coherent path is for what nobody writes meanwhile. (It is
+// the faster one: 8 x 12288 x 3072, weights not in L2, 11.0 us against 11.2.)
+template <int GROUPS, bool READY>
+__global__ void __launch_bounds__(32 * kFewWarps, 2)
+gemm_i8_few_rows_kernel(const FewParams f) {
+  const GemmParams &p = f.g;
+  const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2;
+  const uint32_t n0 = blockIdx.x * 16u, chunks = (p.K + 63u) / 64u;
+  const Columns columns(f.w, n0, p.N, p.K);
+  Weights w;
+  if (READY)
+    w.load<READY>(columns, p.K, 0);
+  grid_dependency_wait();
+  grid_dependents_launch();
+  if (!READY)
+    w.load<READY>(columns, p.K, 0);
+  int32_t c[GROUPS][4] = {};
+  for (uint32_t first = 0; first < chunks; first += kFewWarps * kFewBatch) {
+    if (first != 0u)
+      w.load<READY>(columns, p.K, first);
+#pragma unroll
+    for (int q = 0; q < GROUPS; ++q) {
+      const uint32_t row = 8u * q + g;
+      uint4 x[kFewBatch];
+#pragma unroll
+      for (int u = 0; u < kFewBatch; ++u) {
+        const uint32_t k = k_of(first, u);
+        x[u] = make_uint4(0, 0, 0, 0);
+        if (k < p.K && row < p.M)
+          x[u] = load_produced(reinterpret_cast<const uint4 *>(f.x + (size_t)row * p.K + k));
+      }
+      w.multiply(c[q], x);
+    }
+  }
+  __shared__ int32_t sums[kFewWarps][GROUPS * 8][16]; // [warp][row][column]
+#pragma unroll
+  for (int q = 0; q < GROUPS; ++q)
+    store_sums(&sums[warp][8 * q][0], c[q]);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < 16u * p.M; i += 32 * kFewWarps) {
+    const uint32_t row = i >> 4, n = n0 + (i & 15u);
+    if (n >= p.N)
+      continue;
+    int32_t acc = 0;
+#pragma unroll
+    for (int v = 0; v < kFewWarps; ++v)
+      acc += sums[v][row][i & 15u];
+    write_output(p, row, n, acc, load_produced(p.row_scales + row));
+  }
+}
+
 // QuantizeInt8Rows (the unsigned 256-wide rotation on bf16) and the linear in one launch: rows of at most 8 blocks of 1024
-// columns in all, one for each warp (two for each take longer than a quantiser in front: 5 x 3072 x 3072 7.9 and 5.1 us). Every CTA makes the same codes; the first one also writes them and the row
-// scales to the caller's scratch. A CTA then takes every gridDim.x-th tile of 16 columns.
+// columns in all, one for each warp (two for each take longer than a quantiser in front: 5 x 3072 x 3072 7.9 and 5.1 us). Every
+// CTA makes the same codes; the first one also writes them and the row scales to the caller's scratch. A CTA then takes every
+// gridDim.x-th tile of 16 columns.
 struct FusedParams {
   const uint16_t *x;
   const int8_t *w;
@@ -194,7 +177,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t K = p.K, tiles = (p.N + 15u) / 16u, chunks = (K + 63u) / 64u, pitch = K + 16u;
   Weights w;
-  w.load(Columns(f.w, blockIdx.x * 16u, p.N, K), K, 0); // (the grid has no more CTAs than tiles)
+  w.load<true>(Columns(f.w, blockIdx.x * 16u, p.N, K), K, 0); // (the grid has no more CTAs than tiles)
 
   uint8_t *codes = few_smem + kFewWarps * kWarpBytes256;
   float *maxima = reinterpret_cast<float *>(codes + p.M * pitch), *scales = maxima + kFusedBlocks;
@@ -270,7 +253,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
     int32_t c[4] = {};
     for (uint32_t first = 0; first < chunks; first += kFewWarps * kFewBatch) {
       if (first != 0u)
-        w.load(Columns(f.w, tile * 16u, p.N, K), K, first);
+        w.load<true>(Columns(f.w, tile * 16u, p.N, K), K, first);
       uint4 x[kFewBatch];
 #pragma unroll
       for (int u = 0; u < kFewBatch; ++u) {
@@ -280,7 +263,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
       w.multiply(c, x);
     }
     if (tile + gridDim.x < tiles)
-      w.load(Columns(f.w, (tile + gridDim.x) * 16u, p.N, K), K, 0);
+      w.load<true>(Columns(f.w, (tile + gridDim.x) * 16u, p.N, K), K, 0);
     store_sums(sums + warp * 128, c);
     __syncthreads();
     const uint32_t row = threadIdx.x >> 4, n = tile * 16u + (threadIdx.x & 15u);
