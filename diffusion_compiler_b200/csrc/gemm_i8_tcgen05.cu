@@ -508,11 +508,12 @@ struct Form {
 // The form with the least modelled time: waves of tiles x k-blocks per CTA x time of a k-block, plus what a
 // launch pays once (first loads, the last tile's epilogue, the exchange of a split). The figures, in ns, are
 // fitted to event times of every form at N 3072 / 9216 / 12288 / 16384, K 3072 / 8192 / 12288 and 17 to 12000 rows; over 160
-// such problems the form chosen is within 5 % of the best one, and within 2 % of it for all but 20. Large problems go to the 256 x 256 pair (fewest bytes per MAC). The narrower tiles and the
-// splits are for problems that leave SMs idle, where time is one CTA's serial chain of k-blocks: 2 rows,
-// K 12288, N 3072 45 -> 22.5 us (12 CTAs of 96 k-blocks -> 96 of 24), K 3072 20.5 -> 14.3 us; 512 rows, K 12288
-// 43 -> 31 us; 1600 rows, K 8192 53 -> 49 us; 1101 rows, N 12288 47 -> 43 us. A split costs more than it gives
-// once its clusters need a second wave (512 rows, N 3072, K 3072, split 4: 31 us), hence `resident`. Pairs of 192 columns
+// such problems the form chosen is within 5 % of the best one, and within 2 % of it for all but 20. Large problems go to the
+// 256 x 256 pair (fewest bytes per MAC). The narrower tiles and the splits are for problems that leave SMs idle, where time is
+// one CTA's serial chain of k-blocks: 64 rows, K 12288, N 3072 take 37.7 us with 128 x 256 tiles (12 CTAs of 96 k-blocks), 26.0
+// with 128 x 128, 17.3 shared by two CTAs and 13.9 by four (96 of 24), K 3072 13.7, 9.8, 8.6, 8.7; 512 rows, K 12288 37.3, 26.9
+// and 23.2 with pairs of 256 x 128. A split costs more than it gives once its clusters need a second wave (512 rows, N 3072,
+// K 3072: by four 25.4 us, not split 10.4), hence `resident`. Pairs of 192 columns
 // fill waves that the others leave half empty (the GEMM alone, best of the others -> 192: 512 rows, N 12288, K 3072
 // 21.9 -> 19.8 us; 900 rows, K 8192 26 -> 21; 1024 rows, K 12288 36 -> 29; 2048 rows, K 8192 41 -> 35).
 Form choose_form(uint64_t M, uint64_t N, uint64_t K) {
@@ -654,7 +655,7 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
   const uint64_t dims_a[2] = {K, M}, dims_b[2] = {K, N};
   const uint64_t strides[1] = {K};
   // Where all rows are one tile of a CTA, loads end with them (a multiple of 8 rows, the swizzle's period): rows beyond
-  // the tensor are not free, 17 x 3072 x 16384 took 16.6 us with boxes of 128 rows and 9.9 with boxes of 32. What stands in the
+  // the tensor are not free, 17 x 3072 x 16384 took 15.3 us with boxes of 128 rows and takes 9.4 with boxes of 24. What stands in the
   // others' place meets only rows of the accumulator that are never read.
   p.a_rows = form.ctas == 1 && M < (uint64_t)kBM ? (uint32_t)(M + 7) / 8 * 8 : (uint32_t)kBM;
   const uint32_t box_a[2] = {(uint32_t)kBK, p.a_rows}, box_b[2] = {(uint32_t)kBK, (uint32_t)(form.tile_n / form.ctas)};
