@@ -130,13 +130,15 @@ PyObject *quantize_int8_rows(PyObject *, Args args, Py_ssize_t n) {
       return none();
     const void *parts[8];
     uint64_t widths[8], total = 0;
+    at::Tensor held[8]; // the list may change while arguments are converted and while the lock is given up
     const at::Tensor *first = nullptr;
     for (Py_ssize_t i = 0; i < count; ++i) {
       const at::Tensor *t = dense(PyList_GET_ITEM(args[0], i), at::kBFloat16, device);
       if (!t || t->dim() < 1 || t->numel() == 0)
         return none();
+      held[i] = *t;
       if (i == 0)
-        first = t;
+        first = &held[0];
       else if (t->dim() != first->dim() || t->sizes().slice(0, t->dim() - 1) != first->sizes().slice(0, t->dim() - 1))
         return none();
       parts[i] = in(t);

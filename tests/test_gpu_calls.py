@@ -81,6 +81,30 @@ def test_native_calls_equal_the_general_way(both):
     ops.poll_status()
 
 
+def test_inputs_live_as_long_as_the_call(both):
+    """A list of inputs that loses them while the arguments are converted."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    x, y = (torch.randn(5, k, device="cuda").to(torch.bfloat16) for k in (512, 256))
+    want = ops.quantize_int8_rows([x, y], 2, clip=0.75)
+
+    class Clip:
+        def __init__(self, parts):
+            self.parts = parts
+
+        def __float__(self):
+            self.parts.clear()
+            return 0.75
+
+    def call():
+        parts = [x.clone(), y.clone()]
+        return ops.quantize_int8_rows(parts, 2, clip=Clip(parts))
+
+    native, general = both(call)
+    assert _same(native, want) and _same(general, want)
+    ops.poll_status()
+
+
 def test_operands_of_too_few_elements_are_refused():
     """Refused on the host, before a launch, natively and the general way: weights of another width, vectors that end early,
     keys of fewer tokens than the queries."""
