@@ -650,6 +650,19 @@ int launch_single(const QuantParams &p, cudaStream_t stream) {
   if constexpr (!kArithmetic && F32 && !SIGNED)
     if (blocks <= 3u)
       return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 3>(p, stream);
+  // Rows of 7 and 8 blocks are a CTA each: from as many as three CTAs per SM hold up to five for each SM the second round is
+  // short, and its few CTAs want the shortest path. us with three / as here: 700 rows of 8192 columns 7.6 / 6.8, fp32 8.2 / 7.3,
+  // signed 9.4 / 8.2, both 10.0 / 8.6; 592 of 7168 6.2 / 5.6, 6.8 / 5.9, 7.8 / 7.1, 8.6 / 7.4; 740 of 8192 7.4 / 7.2, 8.2 / 7.8,
+  // 9.4 / 9.1, 10.2 / 9.8; at 445 within 3 %. Beyond, three hide more (4159 x 8192 26.6, four 28.0).
+  if constexpr (!kArithmetic) {
+    const uint64_t sms = (uint64_t)sm_count();
+    if (blocks > 6u && p.rows > 3u * sms && p.rows <= 5u * sms) {
+      if constexpr (SIGNED)
+        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 256, 2>(p, stream);
+      else
+        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, false, 256, 4>(p, stream);
+    }
+  }
   return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, !kArithmetic, 256, 3>(p, stream);
 }
 

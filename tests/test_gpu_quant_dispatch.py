@@ -1,5 +1,5 @@
-"""The forms of the 256-wide ConvRot quantiser at the edges of their dispatch: one or three blocks of 1024
-columns per warp, partial blocks, several warps per row, rows that only start on 16 bytes, and the
+"""The forms of the 256-wide ConvRot quantiser at the edges of their dispatch: one block of 1024 columns per warp
+(packing: or three), partial blocks, several warps per row, rows that only start on 16 bytes, and the
 norm prologue. Codes and scales are whole numbers and exact fp32 values: every bit must agree."""
 import numpy as np
 import pytest
@@ -16,13 +16,13 @@ def _bits_equal(want, got):
 
 
 @pytest.mark.parametrize("impl,rows,widths,clip,residual", [
-    (2, 1200, [3072], 1.0, False),        # three blocks per warp, more rows than resident warps
+    (2, 1200, [3072], 1.0, False),        # several rows per CTA, more than are resident at once
     (3, 1190, [3072], 0.97, False),       # the same with sign masks and clipped codes
     (2, 1301, [2816], 1.0, False),        # the row's last block holds three of four groups
-    (2, 800, [3072, 12288], 1.0, False),  # five warps per row, two inputs
-    (2, 3, [3072, 12288], 1.0, False),    # the same width with few rows: one block per warp
-    (2, 330, [10496], 1.0, False),        # eleven blocks: the last warp has an empty one
-    (2, 500, [8192], 1.0, False),         # eight blocks: one per warp although the rows are many
+    (2, 800, [3072, 12288], 1.0, False),  # fifteen warps per row, two inputs
+    (2, 3, [3072, 12288], 1.0, False),    # the same width with few rows
+    (2, 330, [10496], 1.0, False),        # eleven blocks, the last of one group
+    (2, 500, [8192], 1.0, False),         # eight blocks: a CTA each
     (5, 130, [8192], 1.0, False),         # fp32 division
     (6, 40, [256], 1.0, True),            # the narrowest row, residual pair
     (2, 7, [16384], 1.0, True),           # the widest row, residual pair
@@ -45,6 +45,18 @@ def test_forms_bit_exact(impl, rows, widths, clip, residual):
         got = ops.quantize_int8_rows(tensors, impl, clip, residual=residual)
         for name, w, g in zip(("codes", "scales", "rcodes", "rscales"), want, got):
             assert _bits_equal(w, g), (name, shift)
+
+
+@pytest.mark.parametrize("rows,K", [(444, 8192), (445, 6400), (445, 8192), (740, 7168), (740, 6144), (741, 8192)])
+@pytest.mark.parametrize("impl", [2, 3, 5, 6])
+def test_rows_of_a_cta_each_around_the_second_round(impl, rows, K):
+    """Rows of 7 and 8 blocks, from as many as three CTAs per SM hold (444 on 148 SMs) to five for each SM, and 6 blocks."""
+    from diffusion_compiler_b200 import ops
+    x = activations(np.random.default_rng(rows + K + impl), rows, K)
+    x[1] = 0
+    want = ob.orc().quantize_int8_rows([x], impl, 1.0, False)
+    got = ops.quantize_int8_rows([to_torch_bf16(x)], impl)
+    assert _bits_equal(want[0], got[0]) and _bits_equal(want[1], got[1])
 
 
 @pytest.mark.parametrize("N,K,impl", [(1300, 3072, 2), (450, 8192, 3), (9, 8192, 2), (20, 10496, 5)])
