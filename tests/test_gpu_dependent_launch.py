@@ -168,3 +168,42 @@ def test_gemm_directly_behind_an_attention(tokens):
     assert bool(torch.isfinite(want.float()).all()) and bool(want.float().any())
     for i, o in enumerate(got):
         assert torch.equal(_bits(o), _bits(want)), i
+
+
+@pytest.mark.parametrize("rows,K", [(1, 256), (2, 3072), (8, 1024)])  # with the quantiser in the same launch: at most 8 blocks of 1024 columns
+def test_linears_of_few_rows_one_behind_the_other(rows, K):
+    """Single-call linears in one launch each, which starts while the one in front of it still runs: every one reads what the
+    last one wrote and writes the buffer that the last one read, on the stream and from a graph."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows * K)
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, weights = normal(rows, K), [ops.quantize_weight_rows(normal(K, K), 2) for _ in range(4)]
+    want = x
+    for i in range(12):
+        want = ops.w8a8_linear(want, *weights[i % 4]).clone()
+        torch.cuda.synchronize()
+    assert bool(torch.isfinite(want.float()).all()) and bool(want.float().any())
+    a, b = x.clone(), torch.empty_like(x)
+
+    def chain():
+        for i in range(6):
+            ops.w8a8_linear(a, *weights[2 * i % 4], out=b)
+            ops.w8a8_linear(b, *weights[(2 * i + 1) % 4], out=a)
+
+    got = []
+    for _ in range(3):
+        a.copy_(x)
+        chain()
+        got.append(a.clone())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for _ in range(3):
+        a.copy_(x)
+        graph.replay()
+        got.append(a.clone())
+    torch.cuda.synchronize()
+    ops.poll_status()
+    for i, o in enumerate(got):
+        assert torch.equal(_bits(o), _bits(want)), i
