@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(128)
 key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, float *table,
                  float *tile_bound, uint32_t S, uint32_t KV, uint32_t S_pad, uint32_t begin0, uint32_t count0,
                  uint32_t begin1, uint32_t count1) {
-  grid_dependents_launch(); // (launched plainly)
+  const uint64_t after = grid_dependency_wait_zero();
+  grid_dependents_launch();
   const uint32_t tiles = S_pad / kTile;     // tiles of the whole key axis (table layout)
   const uint32_t mine = count0 + count1;    // tiles this launch covers
   const uint32_t local = blockIdx.x % mine;
@@ -136,7 +137,7 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
   const uint32_t j = tile * kTile + threadIdx.x;
   float k22 = 0.0f, mask = -INFINITY, bound = 0.0f;
   if (j < S && (key_valid == nullptr || key_valid[(uint64_t)b * S + j] != 0)) {
-    const uint4 *row = reinterpret_cast<const uint4 *>(k8 + (((uint64_t)b * S + j) * KV + kvh) * kTile);
+    const uint4 *row = reinterpret_cast<const uint4 *>(k8 + after + (((uint64_t)b * S + j) * KV + kvh) * kTile);
     int n2 = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -183,7 +184,8 @@ struct OperandParams {
 };
 __global__ void __launch_bounds__(256)
 attention_operands_kernel(const OperandParams p) {
-  grid_dependents_launch(); // (launched plainly)
+  const uint64_t after = grid_dependency_wait_zero();
+  grid_dependents_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
   // The four rows of a lane are requested before the first is worked on (behind one another, each waited for its load:
   // B2 S4608 H24 41 us against 34).
@@ -221,7 +223,7 @@ attention_operands_kernel(const OperandParams p) {
     auto row_of = [&](int step) { return ((uint64_t)b * p.S + (key_of(step) < p.S ? key_of(step) : 0)) * p.KV + kvh; };
 #pragma unroll
     for (int step = 0; step < 4; ++step)
-      request(step, p.k + row_of(step) * 16, key_of(step) < p.S);
+      request(step, p.k + after + row_of(step) * 16, key_of(step) < p.S);
     __shared__ uint32_t masked[4]; // whether a segment of 32 keys has masked ones
     if (threadIdx.x < 4)
       masked[threadIdx.x] = 0u;
@@ -281,7 +283,7 @@ attention_operands_kernel(const OperandParams p) {
     auto row_of = [&](int step) { return (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * 32u + warp * 4u + (lane >> 3); };
 #pragma unroll
     for (int step = 0; step < 4; ++step)
-      request(step, p.q + (row_of(step) < p.q_rows ? row_of(step) : 0) * 16, row_of(step) < p.q_rows);
+      request(step, p.q + after + (row_of(step) < p.q_rows ? row_of(step) : 0) * 16, row_of(step) < p.q_rows);
 #pragma unroll
     for (int step = 0; step < 4; ++step) {
       const uint64_t row = row_of(step);
@@ -424,9 +426,8 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     grid_dependency_wait();
   else
     ptx::fence_device_and_tma();
-  if (!SPLIT && warp == 3) { // (the idle one)
-    if (p.split_follows)
-      ptx::fence_device_and_tma();
+  if (!SPLIT && warp == 3 && p.split_follows) { // (the idle one)
+    ptx::fence_device_and_tma();
     grid_dependents_launch();
   }
   // Only Q is requested in front of the barrier. The first two tiles are 8 copies more, 700 to 1000 clocks of this one thread
@@ -1249,17 +1250,15 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     if (blocks > 0x7fffffffull)
       return fail(kUnsupported, "Attention(INT8): problem too large");
     o.key_blocks = (uint32_t)key_blocks;
-    attention_operands_kernel<<<(unsigned)blocks, 256, 0, stream>>>(o);
-    if (int rc = launched(cudaGetLastError(), "attention_operands_kernel launch"))
+    if (int rc = launch_ahead("attention_operands_kernel launch", attention_operands_kernel, blocks, 256, 0, stream, o))
       return rc;
   }
   if (!(source && source->k)) {
     const uint64_t blocks = B * KV * (count[0] + count[1]);
     if (blocks > 0x7fffffffull)
       return fail(kUnsupported, "Attention(INT8): problem too large");
-    key_table_kernel<<<(unsigned)blocks, 128, 0, stream>>>(k8, ks, key_valid, table, tile_bound, (uint32_t)S, (uint32_t)KV, s_pad, begin[0],
-                                                           count[0], begin[1], count[1]);
-    if (int rc = launched(cudaGetLastError(), "key_table_kernel launch"))
+    if (int rc = launch_ahead("key_table_kernel launch", key_table_kernel, blocks, 128, 0, stream, k8, ks, key_valid, table, tile_bound,
+                              (uint32_t)S, (uint32_t)KV, s_pad, begin[0], count[0], begin[1], count[1]))
       return rc;
   }
   AttnParams p{};

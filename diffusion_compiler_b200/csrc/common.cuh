@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 namespace difb200 {
 
@@ -97,14 +98,24 @@ inline Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
 // A kernel launched with dependent_launch() may start while the one in front of it on the stream still runs: as soon as
 // all CTAs of that one have called grid_dependents_launch() (or ended) and there is room. Its set-up runs then; what
 // the kernel in front wrote is read behind grid_dependency_wait(), which every thread passes that touches global
-// memory, and through loads that the compiler cannot move up (load_produced or TMA). A kernel that lets dependents
-// start and is itself launched so waits first: when a kernel starts, the one two in front is complete.
+// memory, and through loads that the compiler cannot move up: load_produced, TMA, or addresses that the wait is a part of
+// (grid_dependency_wait_zero). A kernel that lets dependents start waits first: when a kernel starts, the one two in front
+// is complete.
 // Two reads are not behind such a wait. Both are of what a kernel further in front wrote, and both hold only because
-// the kernel in between was launched plainly or waited before it let anything start (then that kernel is complete):
-// * the first weights of a GEMM, requested ahead in w8a8_linear, whose quantiser, the kernel in between, is launched plainly;
+// the kernel in between waited before it let anything start (then that kernel is complete):
+// * the first weights of a GEMM, requested ahead in w8a8_linear, whose quantiser is the kernel in between;
 // * the operands of the attention's split launch: the unsplit one waits for their kernel, then fences, then lets it start.
-// Every kernel that calls grid_dependents_launch() in its first lines is launched plainly, and has to stay so.
+// Launched plainly, a kernel starts 1 to 2.5 us after the end of the one in front; ahead, with a wait as the first thing
+// it does, within half of one, whether or not that one says that dependents may start (calls of 2 x 3072 x 3072, one behind the
+// other: 8.2 us, 5.9, and 5.8 where it says so at its start or its end). So it says so only where the next one has work to do
+// meanwhile: CTAs that only wait would gather on the SMs that happen to be free.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The wait and a zero behind it: addresses of loads that could otherwise be moved in front of the wait (__ldg) contain it.
+__device__ __forceinline__ uint64_t grid_dependency_wait_zero() {
+  uint64_t zero;
+  asm volatile("griddepcontrol.wait;\nmov.u64 %0, 0;" : "=l"(zero)::"memory");
+  return zero;
+}
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ float load_produced(const float *p) {
   float v;
@@ -132,6 +143,19 @@ inline cudaLaunchAttribute dependent_launch() {
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   return attr;
+}
+// Launches a kernel that begins with its wait.
+template <class... P, class... A>
+int launch_ahead(const char *what, void (*kernel)(P...), uint64_t grid, int threads, size_t smem, cudaStream_t stream, A &&...args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)grid);
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attr = dependent_launch();
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return launched(cudaLaunchKernelEx(&config, kernel, std::forward<A>(args)...), what);
 }
 
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t bits16) {

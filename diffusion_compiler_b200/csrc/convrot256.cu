@@ -56,7 +56,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   static_assert(EXTRA != kNorm || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
-  grid_dependents_launch(); // (launched plainly)
+  const uint64_t after = grid_dependency_wait_zero(); // in the address of every load
+  grid_dependents_launch();
   constexpr bool kWeights = EXTRA == kPack || EXTRA == kEqualise;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = warp / warps_per_row;         // which row of this CTA's batch
@@ -66,7 +67,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   const uint32_t smem_addr = smem_u32(smem);
   const uint32_t warp_addr = smem_addr + warp * kWarpBytes;
   float *red = reinterpret_cast<float *>(smem + total_warps * (kWarpBytes / 4)); // [2][2][total_warps]
-  const float clip = p.clip_device ? __ldg(p.clip_device) : p.clip;
+  const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
   constexpr float kCarry = 16.0f; // the values carried through the rotation are scaled by 2^stages
   const uint32_t columns = p.columns;
   const uint32_t col_warp = (uint32_t)wrow * (NIT * 1024u);
@@ -105,7 +106,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     for (int q = 0; q < 2 * NIT; ++q) {
       const uint32_t c = col0 + (uint32_t)(q >> 1) * 1024u + (uint32_t)(q & 1) * 256u;
       if (c < columns) {
-        const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + c);
+        const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
         const uint4 e0 = __ldg(ep), e1 = __ldg(ep + 1);
         const uint32_t w[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
@@ -122,23 +123,23 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   // multiples of 16, so a run never straddles two of them.
   auto run_of = [&](uint64_t row, uint32_t c) {
     if (p.part_count == 1)
-      return reinterpret_cast<const uint4 *>(p.part[0] + row * columns + c);
+      return reinterpret_cast<const uint4 *>(p.part[0] + after + row * columns + c);
     uint32_t i = 0;
     while (c >= p.width[i])
       c -= p.width[i++];
-    return reinterpret_cast<const uint4 *>(p.part[i] + row * p.width[i] + c);
+    return reinterpret_cast<const uint4 *>(p.part[i] + after + row * p.width[i] + c);
   };
   // With one block per warp the runs of a thread are in the same place of every row: looked up once. (Not where
   // registers are short: the fp32 form with 64 of them spills, 9216 x 15360 147 -> 156 us.)
   constexpr bool kPlaced = NIT == 1 && EXTRA == kPlain && !RESIDUAL && !(F32 && !SIGNED && MAXT * MINB > 768);
-  const uint16_t *src_a = p.part[0] + col0, *src_b = src_a + 256;
+  const uint16_t *src_a = p.part[0] + after + col0, *src_b = src_a + 256;
   uint32_t pitch_a = columns, pitch_b = columns;
   if (kPlaced && p.part_count > 1) {
     auto place = [&](uint32_t c, const uint16_t *&src, uint32_t &pitch) {
       uint32_t i = 0;
       while (c >= p.width[i])
         c -= p.width[i++];
-      src = p.part[i] + c;
+      src = p.part[i] + after + c;
       pitch = p.width[i];
     };
     if (col0 < columns)
@@ -204,7 +205,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
           // The norm in front (reference cpu_executor.cpp:1241-1264 RmsNormModulate, :1108-1148
           // LayerNormModulate): the words are replaced by the bf16 result the unfused op would have
           // stored, rounding for rounding, two groups per packed operation.
-          const uint64_t at = (row / p.norm_rows_per_mod) * (uint64_t)columns + c;
+          const uint64_t at = (row / p.norm_rows_per_mod) * (uint64_t)columns + c + after;
           const bool layer = p.norm_bias != nullptr, weighted = p.norm_weight != nullptr;
           auto product = [&](uint64_t u, uint64_t v) { return fma2(u, v, p.minus_zero2); };
           const uint64_t inv2 = pack2(inv, inv), mean2 = pack2(mean, mean), one2 = pack2(1.0f, 1.0f);
@@ -216,10 +217,10 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             };
             const uint4 sa4 = pick(p.norm_scale, at, act_a, zero), sb4 = pick(p.norm_scale, at + 256u, act_b, zero);
             const uint4 ha4 = pick(p.norm_shift, at, act_a, zero), hb4 = pick(p.norm_shift, at + 256u, act_b, zero);
-            const uint4 ga4 = pick(p.norm_weight, c, act_a && weighted, one),
-                        gb4 = pick(p.norm_weight, c + 256u, act_b && weighted, one);
-            const uint4 ba4 = pick(p.norm_bias, c, act_a && layer, zero),
-                        bb4 = pick(p.norm_bias, c + 256u, act_b && layer, zero);
+            const uint4 ga4 = pick(p.norm_weight, c + after, act_a && weighted, one),
+                        gb4 = pick(p.norm_weight, c + 256u + after, act_b && weighted, one);
+            const uint4 ba4 = pick(p.norm_bias, c + after, act_a && layer, zero),
+                        bb4 = pick(p.norm_bias, c + 256u + after, act_b && layer, zero);
             const uint32_t sa[4] = {sa4.x, sa4.y, sa4.z, sa4.w}, sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
             const uint32_t ha[4] = {ha4.x, ha4.y, ha4.z, ha4.w}, hb[4] = {hb4.x, hb4.y, hb4.z, hb4.w};
             const uint32_t ga[4] = {ga4.x, ga4.y, ga4.z, ga4.w}, gb[4] = {gb4.x, gb4.y, gb4.z, gb4.w};
@@ -296,7 +297,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             // which then is the quotient, stands. Subnormal quotients may be off by 2^-149: the row scale
             // is at least 1e-30.
             const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
-            const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + c);
+            const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
             const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z,
                                  act_b ? __ldg(ep + 33) : z};
             const uint32_t ea[8] = {e4[0].x, e4[0].y, e4[0].z, e4[0].w, e4[1].x, e4[1].y, e4[1].z, e4[1].w};
@@ -621,8 +622,7 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   const uint64_t batches = (p.rows + rows_per_cta - 1) / rows_per_cta;
   uint64_t grid = (uint64_t)sm_count() * resident; // persistent: as many CTAs as are resident at once
   grid = grid > batches ? batches : grid;
-  kernel<<<(unsigned)grid, threads, smem, stream>>>(p, warps_per_row, rows_per_cta);
-  return launched(cudaGetLastError(), "convrot256_kernel launch");
+  return launch_ahead("convrot256_kernel launch", kernel, grid, threads, smem, stream, p, warps_per_row, rows_per_cta);
 }
 
 // The form of a row of `blocks` blocks of 1024 columns, one per warp: threads and CTAs per SM, and whether a warp requests

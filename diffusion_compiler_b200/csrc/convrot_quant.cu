@@ -23,13 +23,14 @@ template <bool F32, bool RESIDUAL, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : (MAXT == 384 ? 2 : 1))
 convrot4096_kernel(const QuantParams p) {
   extern __shared__ __align__(128) uint32_t smem[];
-  grid_dependents_launch(); // (launched plainly)
+  const uint64_t after = grid_dependency_wait_zero();
+  grid_dependents_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = lane >> 4, a = lane & 15;
   const int warps = blockDim.x >> 5;
   const uint32_t smem_addr = smem_u32(smem), warp_addr = smem_addr + warp * kWarpBytes;
   float *red = reinterpret_cast<float *>(smem + warps * (kWarpBytes / 4)); // [2][2][warps]
-  const float clip = p.clip_device ? __ldg(p.clip_device) : p.clip;
+  const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
   constexpr float kCarry = 64.0f; // the values carried through the rotation are scaled by 2^stages
   const uint32_t columns = p.columns, col0 = 1024u * warp + 512u * h + 16u * a;
 
@@ -67,7 +68,7 @@ convrot4096_kernel(const QuantParams p) {
         uint32_t c = col0 + 256u * g, i = 0;
         while (c >= p.width[i])
           c -= p.width[i++];
-        const uint4 *src = reinterpret_cast<const uint4 *>(p.part[i] + row * p.width[i] + c);
+        const uint4 *src = reinterpret_cast<const uint4 *>(p.part[i] + after + row * p.width[i] + c);
         v[2 * g] = __ldg(src);
         v[2 * g + 1] = __ldg(src + 1);
       }
@@ -260,8 +261,7 @@ int launch_convrot4096(const QuantParams &p, cudaStream_t stream) {
     return rc;
   uint64_t grid = (uint64_t)sm_count() * resident;
   grid = grid > p.rows ? p.rows : grid;
-  kernel<<<(unsigned)grid, threads, smem, stream>>>(p);
-  return launched(cudaGetLastError(), "convrot4096_kernel launch");
+  return launch_ahead("convrot4096_kernel launch", kernel, grid, threads, smem, stream, p);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -269,11 +269,11 @@ int launch_convrot4096(const QuantParams &p, cudaStream_t stream) {
 // width. Used for activations of plain W8A8 linears and for the per-token-per-head
 // quantisation of attention Q/K (rows of width 128).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float load_logical(const QuantParams &p, uint64_t row, uint32_t column) {
+__device__ __forceinline__ float load_logical(const QuantParams &p, uint64_t after, uint64_t row, uint32_t column) {
   uint32_t c = column;
   for (uint32_t i = 0; i < p.part_count; ++i) {
     if (c < p.width[i])
-      return bf16_bits_to_f32(__ldg(p.part[i] + row * p.width[i] + c));
+      return bf16_bits_to_f32(__ldg(p.part[i] + after + row * p.width[i] + c));
     c -= p.width[i];
   }
   return 0.0f;
@@ -282,16 +282,17 @@ __device__ __forceinline__ float load_logical(const QuantParams &p, uint64_t row
 template <bool VEC8>
 __global__ void __launch_bounds__(256)
 direct_quant_kernel(const QuantParams p) {
-  grid_dependents_launch(); // (launched plainly)
+  const uint64_t after = grid_dependency_wait_zero();
+  grid_dependents_launch();
   const int lane = threadIdx.x & 31;
   const uint64_t warp_global = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t warp_count = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const float clip = p.clip_device ? __ldg(p.clip_device) : p.clip;
+  const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
   const uint32_t K = p.columns;
   for (uint64_t row = warp_global; row < p.rows; row += warp_count) {
     float m = 0.0f;
     if (VEC8) { // single part, width % 8 == 0, 16-byte aligned rows
-      const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + row * K);
+      const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + after + row * K);
       for (uint32_t c = lane; c < (K >> 3); c += 32) {
         const uint4 v = __ldg(src + c);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -303,7 +304,7 @@ direct_quant_kernel(const QuantParams p) {
       }
     } else {
       for (uint32_t c = lane; c < K; c += 32)
-        m = fmaxf(m, fabsf(load_logical(p, row, c)));
+        m = fmaxf(m, fabsf(load_logical(p, after, row, c)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -314,7 +315,7 @@ direct_quant_kernel(const QuantParams p) {
     const bool residual = p.rcodes != nullptr;
     float rm = 0.0f;
     if (VEC8) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + row * K);
+      const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + after + row * K);
       uint2 *dst = reinterpret_cast<uint2 *>(p.codes + row * K);
       for (uint32_t c = lane; c < (K >> 3); c += 32) {
         const uint4 v = __ldg(src + c);
@@ -336,7 +337,7 @@ direct_quant_kernel(const QuantParams p) {
       }
     } else {
       for (uint32_t c = lane; c < K; c += 32) {
-        const float x = load_logical(p, row, c);
+        const float x = load_logical(p, after, row, c);
         const int code = max(sat_s8(__fdiv_rn(x, scale)), -127);
         p.codes[row * K + c] = (int8_t)code;
         if (residual)
@@ -352,7 +353,7 @@ direct_quant_kernel(const QuantParams p) {
         p.rscales[row] = rscale;
       __syncwarp();
       for (uint32_t c = lane; c < K; c += 32) {
-        const float x = load_logical(p, row, c);
+        const float x = load_logical(p, after, row, c);
         const float r = __fmaf_rn(-(float)p.codes[row * K + c], scale, x);
         p.rcodes[row * K + c] = (int8_t)max(sat_s8(__fdiv_rn(r, rscale)), -127);
       }
@@ -435,11 +436,7 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
         return rc;
     }
     const bool vec = part_count == 1 && aligned8 && (reinterpret_cast<uintptr_t>(codes) & 7) == 0;
-    if (vec)
-      direct_quant_kernel<true><<<(unsigned)blocks, threads, 0, stream>>>(p);
-    else
-      direct_quant_kernel<false><<<(unsigned)blocks, threads, 0, stream>>>(p);
-    return launched(cudaGetLastError(), "direct_quant_kernel launch");
+    return launch_ahead("direct_quant_kernel launch", vec ? direct_quant_kernel<true> : direct_quant_kernel<false>, blocks, threads, 0, stream, p);
   }
   if (implementation < 2 || implementation > 7)
     return fail(kInvalidArgument, "QuantizeInt8Rows: unknown implementation");

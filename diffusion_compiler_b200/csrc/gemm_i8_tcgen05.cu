@@ -221,7 +221,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         load(&map_b, smem_base + i * kStageBytes + kABytes, full_bar + 8 * i, kb_first + i, columns_of(unit));
       }
     grid_dependency_wait();
-    grid_dependents_launch();
     if (early != 0u && ptx::elect_one())
       for (uint32_t i = 0; i < early; ++i)
         load(&map_a, smem_base + i * kStageBytes, full_bar + 8 * i, kb_first + i, rows_of(unit));

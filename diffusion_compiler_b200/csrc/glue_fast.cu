@@ -48,6 +48,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 __global__ void __launch_bounds__(256)
 k_residual_gate_bf16(const uint4 *res, const uint4 *branch, const uint4 *gate, uint4 *o, uint64_t groups,
                      uint64_t width8, uint64_t rows_per_gate) {
+  const uint64_t after = grid_dependency_wait_zero();
+  res += after;
+  branch += after;
+  gate += after;
   GRID_STRIDE(i, groups) {
     const uint64_t row = i / width8, col = i - row * width8;
     float r[8], b[8], g[8], y[8];
@@ -72,6 +76,7 @@ struct Wide {
 template <class D>
 __global__ void __launch_bounds__(256)
 k_swiglu_bf16(const uint4 *x, uint4 *o, uint64_t groups, const D width, uint64_t in_width8, uint64_t start8, int gate_first) {
+  x += grid_dependency_wait_zero();
   const uint64_t width8 = width.by;
   GRID_STRIDE(i, groups) {
     const uint64_t row = width.quotient(i), col = i - row * width8, base = row * in_width8 + start8 + col;
@@ -143,6 +148,7 @@ template <bool LAYER, int STAGES>
 __global__ void __launch_bounds__(32 * kStatWarps)
 k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps) {
   extern __shared__ uint4 stat_smem[];
+  grid_dependency_wait(); // (every load is an asynchronous copy)
   auto tile = reinterpret_cast<uint4 (*)[STAGES][32 * kStatPitch]>(stat_smem); // [kStatWarps]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t cols8 = cols >> 3, chunks = cols / kStatCols;
@@ -276,6 +282,7 @@ k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint
 // The statistics as parallel sums, one warp per row.
 __global__ void __launch_bounds__(256)
 k_row_stats_parallel(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps, int layer) {
+  x += grid_dependency_wait_zero();
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t cols8 = cols >> 3;
@@ -314,6 +321,11 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(256)
 k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const uint4 *b, uint4 *o, uint64_t rows,
                          uint32_t cols, float eps, const RowStats stats) {
+  const uint64_t after = grid_dependency_wait_zero();
+  x += after;
+  w += after;
+  a += after;
+  b += after;
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -365,6 +377,12 @@ __global__ void __launch_bounds__(256)
 k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const uint4 *scale, const uint4 *shift,
                            uint4 *o, uint64_t rows, uint32_t cols, uint64_t rows_per_mod, float eps,
                            const RowStats stats) {
+  const uint64_t after = grid_dependency_wait_zero();
+  x += after;
+  w += after;
+  b += after;
+  scale += after;
+  shift += after;
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -462,6 +480,7 @@ template <int ROTARY, bool V2, int ROWS>
 __global__ void __launch_bounds__(32 * kRopeWarps)
 k_qk_norm_rope_row128(const RowRopeParams p) {
   __shared__ uint4 tile[kRopeWarps][ROWS * kRopePitch];
+  const uint64_t after = grid_dependency_wait_zero();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t row0 = ((uint64_t)blockIdx.x * kRopeWarps + warp) * ROWS;
   if (row0 >= p.rows)
@@ -472,7 +491,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
   const uint64_t in_sequence = token - sequence * p.input_seq;
   const uint64_t src = token * p.in_token_stride16 + p.in_offset16 + head * 16;
   const uint64_t out_row = (sequence * p.out_seq + p.out_start + in_sequence) * p.heads + head;
-  const uint64_t trow = (sequence * p.table_seq + p.table_start + in_sequence) * p.table_width;
+  const uint64_t trow = (sequence * p.table_seq + p.table_start + in_sequence) * p.table_width + after;
 #pragma unroll
   for (int i = 0; i < ROWS; i += 2) { // half a warp copies a row
     const int r = i + (lane >> 4);
@@ -487,7 +506,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
   const int c1 = V2 || !rotates ? c0 + 1 : j + kRun / 2;
   uint64_t w[8];
   {
-    const uint4 a = __ldg(p.w + c0), b = __ldg(p.w + c1);
+    const uint4 a = __ldg(p.w + after + c0), b = __ldg(p.w + after + c1);
     const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -604,6 +623,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
 // warp-per-row kernel in convrot_quant.cu) ----
 __global__ void __launch_bounds__(128)
 k_direct_quant_row128(const uint4 *x, int8_t *codes, float *scales, uint64_t rows, float clip) {
+  x += grid_dependency_wait_zero();
   const uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= rows)
     return;
@@ -642,7 +662,6 @@ inline unsigned blocks_for(uint64_t n, int threads) {
   const uint64_t cap = (uint64_t)sm_count() * 32;
   return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
-int done(const char *what) { return launched(cudaGetLastError(), what); }
 
 } // namespace
 
@@ -650,10 +669,9 @@ bool residual_gate_fast(const void *res, const void *branch, const void *gate, v
                         uint64_t width, uint64_t rows_per_gate, cudaStream_t s, int *rc) {
   if (dt != 2 || width % 8 != 0 || !aligned16(res) || !aligned16(branch) || !aligned16(gate) || !aligned16(o))
     return false;
-  k_residual_gate_bf16<<<blocks_for(n / 8, 256), 256, 0, s>>>(
-      static_cast<const uint4 *>(res), static_cast<const uint4 *>(branch), static_cast<const uint4 *>(gate),
-      static_cast<uint4 *>(o), n / 8, width / 8, rows_per_gate);
-  *rc = done("k_residual_gate_bf16");
+  *rc = launch_ahead("k_residual_gate_bf16", k_residual_gate_bf16, blocks_for(n / 8, 256), 256, 0, s,
+                     static_cast<const uint4 *>(res), static_cast<const uint4 *>(branch), static_cast<const uint4 *>(gate),
+                     static_cast<uint4 *>(o), n / 8, width / 8, rows_per_gate);
   return true;
 }
 
@@ -663,14 +681,13 @@ bool swiglu_fast(const void *x, void *o, uint32_t dt, uint64_t rows, uint64_t wi
     return false;
   const uint64_t groups = rows * (width / 8);
   auto launch = [&](auto kernel, auto by) {
-    kernel<<<blocks_for(groups, 256), 256, 0, s>>>(static_cast<const uint4 *>(x), static_cast<uint4 *>(o), groups, by,
-                                                   in_width / 8, start / 8, gate_first ? 1 : 0);
+    *rc = launch_ahead("k_swiglu_bf16", kernel, blocks_for(groups, 256), 256, 0, s, static_cast<const uint4 *>(x),
+                       static_cast<uint4 *>(o), groups, by, in_width / 8, start / 8, gate_first ? 1 : 0);
   };
   if (groups != 0 && groups < (1ull << 31))
     launch(k_swiglu_bf16<Divisor>, divisor(width / 8));
   else
     launch(k_swiglu_bf16<Wide>, Wide{width / 8});
-  *rc = done("k_swiglu_bf16");
   return true;
 }
 
@@ -705,8 +722,7 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
     uint64_t blocks = (rows + 7) / 8;
     const uint64_t cap = (uint64_t)sm_count() * 8;
     blocks = blocks > cap ? cap : blocks;
-    k_row_stats_parallel<<<(unsigned)blocks, 256, 0, s>>>(X, *stats, rows, (uint32_t)cols, eps, layer ? 1 : 0);
-    return done("k_row_stats_parallel");
+    return launch_ahead("k_row_stats_parallel", k_row_stats_parallel, blocks, 256, 0, s, X, *stats, rows, (uint32_t)cols, eps, layer ? 1 : 0);
   }
   // Eight chunks in flight where a few warps per SM have to cover the latency alone, four where the rows
   // give an SM more than six warps (33272 x 3072: one wave of resident CTAs instead of two).
@@ -721,8 +737,7 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
   uint64_t blocks = (warps + kStatWarps - 1) / kStatWarps;
   const uint64_t cap = (uint64_t)sm_count() * resident;
   blocks = blocks > cap ? cap : blocks;
-  kernel<<<(unsigned)blocks, 32 * kStatWarps, smem, s>>>(X, *stats, rows, (uint32_t)cols, eps);
-  return done("k_row_stats_sequential");
+  return launch_ahead("k_row_stats_sequential", kernel, blocks, 32 * kStatWarps, smem, s, X, *stats, rows, (uint32_t)cols, eps);
 }
 
 bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const void *b, void *o, uint32_t dt,
@@ -741,13 +756,8 @@ bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const v
   if ((*rc = row_stats(x, rows, cols, eps, false, false, o, row_bytes, {{w, row_bytes}, {a, rows * row_bytes}, {b, rows * row_bytes}},
                        scratch, &stats, s)))
     return true;
-  if (cols == 3072)
-    k_rms_norm_modulate_bf16<12><<<(unsigned)blocks, 256, 0, s>>>(X, W, A, B, static_cast<uint4 *>(o), rows,
-                                                                  (uint32_t)cols, eps, stats);
-  else
-    k_rms_norm_modulate_bf16<0><<<(unsigned)blocks, 256, 0, s>>>(X, W, A, B, static_cast<uint4 *>(o), rows,
-                                                                 (uint32_t)cols, eps, stats);
-  *rc = done("k_rms_norm_modulate_bf16");
+  *rc = launch_ahead("k_rms_norm_modulate_bf16", cols == 3072 ? k_rms_norm_modulate_bf16<12> : k_rms_norm_modulate_bf16<0>, blocks, 256, 0,
+                     s, X, W, A, B, static_cast<uint4 *>(o), rows, (uint32_t)cols, eps, stats);
   return true;
 }
 
@@ -768,13 +778,8 @@ bool layer_norm_modulate_fast(const void *x, const void *w, const void *b, const
   if ((*rc = row_stats(x, rows, cols, eps, true, false, o, row_bytes,
                        {{w, row_bytes}, {b, row_bytes}, {scale, mod_bytes}, {shift, mod_bytes}}, scratch, &stats, s)))
     return true;
-  if (cols == 3072)
-    k_layer_norm_modulate_bf16<12><<<(unsigned)blocks, 256, 0, s>>>(X, W, B, SC, SH, static_cast<uint4 *>(o), rows,
-                                                                    (uint32_t)cols, rows_per_mod, eps, stats);
-  else
-    k_layer_norm_modulate_bf16<0><<<(unsigned)blocks, 256, 0, s>>>(X, W, B, SC, SH, static_cast<uint4 *>(o), rows,
-                                                                   (uint32_t)cols, rows_per_mod, eps, stats);
-  *rc = done("k_layer_norm_modulate_bf16");
+  *rc = launch_ahead("k_layer_norm_modulate_bf16", cols == 3072 ? k_layer_norm_modulate_bf16<12> : k_layer_norm_modulate_bf16<0>, blocks,
+                     256, 0, s, X, W, B, SC, SH, static_cast<uint4 *>(o), rows, (uint32_t)cols, rows_per_mod, eps, stats);
   return true;
 }
 
@@ -813,11 +818,8 @@ bool qk_norm_rope_fast(const void *x, const void *w, const void *cosv, const voi
     return false;
 #define DIFB200_ROPE_CASE(R, V)                                                                   \
   if (rotary == R && interleaved_v2 == V) {                                                       \
-    if (few)                                                                                      \
-      k_qk_norm_rope_row128<R, V, 8><<<(unsigned)blocks, 32 * kRopeWarps, 0, s>>>(p);             \
-    else                                                                                          \
-      k_qk_norm_rope_row128<R, V, 32><<<(unsigned)blocks, 32 * kRopeWarps, 0, s>>>(p);            \
-    *rc = done("k_qk_norm_rope_row128");                                                          \
+    *rc = launch_ahead("k_qk_norm_rope_row128", few ? k_qk_norm_rope_row128<R, V, 8> : k_qk_norm_rope_row128<R, V, 32>, blocks, \
+                       32 * kRopeWarps, 0, s, p);                                                 \
     return true;                                                                                  \
   }
   DIFB200_ROPE_CASE(64, false)
@@ -834,9 +836,8 @@ bool direct_quant_rows128(const void *x, int8_t *codes, float *scales, uint64_t 
                           int *rc) {
   if (!aligned16(x) || !aligned16(codes) || rows + 127 > 0x7fffffffull * 128ull)
     return false;
-  k_direct_quant_row128<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(static_cast<const uint4 *>(x), codes, scales,
-                                                                      rows, clip);
-  *rc = done("k_direct_quant_row128");
+  *rc = launch_ahead("k_direct_quant_row128", k_direct_quant_row128, (rows + 127) / 128, 128, 0, s, static_cast<const uint4 *>(x), codes,
+                     scales, rows, clip);
   return true;
 }
 

@@ -10,7 +10,7 @@
 //
 // The smallest problems are one launch: every CTA rotates and quantises the rows itself, while its weights are on their way. It
 // is launched ahead and waits at its start: the time between two kernels, not their work, was a third of a call (2 x 3072 x 3072,
-// calls one behind the other, weights not in L2: 8.0 us launched plainly, 5.6 so).
+// calls one behind the other, weights not in L2: 8.0 us launched plainly, 5.4 so).
 // That costs a CTA about 1.5 us and saves a launch, 3 us of the host. 2 x 3072 x 3072, one launch / two / the tile kernel and a
 // quantiser, us per call of calls one behind the other: weights in L2 6.7 / 8.0 / 12.3, not in L2 8.2 / 8.0 / 12.3, of these the
 // host 5.1 / 8.0 / 8.5; from a graph, not in L2, 6.2 / 5.4 / 11.0.
@@ -116,7 +116,6 @@ gemm_i8_few_rows_kernel(const FewParams f) {
   if (READY)
     w.load<READY>(columns, p.K, 0);
   grid_dependency_wait();
-  grid_dependents_launch();
   if (!READY)
     w.load<READY>(columns, p.K, 0);
   int32_t c[GROUPS][4] = {};
@@ -175,8 +174,7 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2)
 w8a8_few_rows_kernel(const FusedParams f) {
   const GemmParams &p = f.g;
   extern __shared__ __align__(128) uint8_t few_smem[];
-  grid_dependency_wait();
-  grid_dependents_launch();
+  const uint64_t after = grid_dependency_wait_zero();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t K = p.K, tiles = (p.N + 15u) / 16u, chunks = (K + 63u) / 64u, pitch = K + 16u;
   Weights w;
@@ -192,7 +190,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
     uint32_t V[16];
     {
       const uint4 zero = make_uint4(0, 0, 0, 0);
-      const uint4 *src = reinterpret_cast<const uint4 *>(f.x + (size_t)row * K + column + 16u * a);
+      const uint4 *src = reinterpret_cast<const uint4 *>(f.x + after + (size_t)row * K + column + 16u * a);
       const uint4 v[4] = {act_a ? __ldg(src) : zero, act_a ? __ldg(src + 1) : zero, act_b ? __ldg(src + 32) : zero,
                           act_b ? __ldg(src + 33) : zero};
       const uint32_t wa[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
@@ -283,15 +281,9 @@ w8a8_few_rows_kernel(const FusedParams f) {
 
 template <int GROUPS>
 int launch_groups(const FewParams &f, cudaStream_t stream) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3((f.g.N + 15u) / 16u);
-  config.blockDim = dim3(32 * kFewWarps);
-  config.stream = stream;
-  cudaLaunchAttribute attr = dependent_launch();
-  config.attrs = &attr;
-  config.numAttrs = 1;
-  return launched(cudaLaunchKernelEx(&config, f.g.weights_first ? gemm_i8_few_rows_kernel<GROUPS, true> : gemm_i8_few_rows_kernel<GROUPS, false>, f),
-                  "gemm_i8_few_rows_kernel launch");
+  return launch_ahead("gemm_i8_few_rows_kernel launch",
+                      f.g.weights_first ? gemm_i8_few_rows_kernel<GROUPS, true> : gemm_i8_few_rows_kernel<GROUPS, false>,
+                      (f.g.N + 15u) / 16u, 32 * kFewWarps, 0, stream, f);
 }
 
 // Waves of the few-rows kernels: two CTAs of 16 columns per SM.
@@ -378,15 +370,7 @@ bool w8a8_few_rows(const void *x_bf16, const int8_t *w, const float *col_scales,
   if ((*rc = resident_blocks(reinterpret_cast<const void *>(w8a8_few_rows_kernel), 32 * kFewWarps, smem, &resident)))
     return true;
   const uint64_t tiles = (N + 15) / 16, most = (uint64_t)sm_count() * resident;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3((unsigned)(tiles < most ? tiles : most));
-  config.blockDim = dim3(32 * kFewWarps);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attr = dependent_launch();
-  config.attrs = &attr;
-  config.numAttrs = 1;
-  *rc = launched(cudaLaunchKernelEx(&config, w8a8_few_rows_kernel, f), "w8a8_few_rows_kernel launch");
+  *rc = launch_ahead("w8a8_few_rows_kernel launch", w8a8_few_rows_kernel, tiles < most ? tiles : most, 32 * kFewWarps, smem, stream, f);
   return true;
 }
 

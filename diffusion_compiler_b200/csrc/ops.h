@@ -32,8 +32,8 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
                        const float *col_scales, const void *bias_bf16, uint32_t epilogue, uint64_t M,
                        uint64_t N, uint64_t K, void *out_bf16, int32_t *acc_out, cudaStream_t stream,
                        DeviceStatus *status_words = nullptr, bool weights_ready = false);
-// weights_ready: the kernel launched last on the stream does not write w, and was launched plainly or waits for the
-// one before it: the first blocks of w are requested while that kernel still runs.
+// weights_ready: the kernel launched last on the stream does not write w, and waits for the one before it before it lets this
+// one start: the first blocks of w are requested while that kernel still runs.
 
 // The same pair for the fewest rows in one launch; false: not a problem for it (or a call that the general way refuses).
 bool w8a8_few_rows(const void *x_bf16, const int8_t *w, const float *col_scales, const void *bias_bf16, uint32_t epilogue,

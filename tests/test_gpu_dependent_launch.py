@@ -207,3 +207,78 @@ def test_linears_of_few_rows_one_behind_the_other(rows, K):
     ops.poll_status()
     for i, o in enumerate(got):
         assert torch.equal(_bits(o), _bits(want)), i
+
+
+def _readers():
+    """name -> a call that reads bf16 rows [rows, 1024] (8 heads of 128) first of all."""
+    import ctypes as C
+
+    import torch
+    from diffusion_compiler_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(7)
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    K = 1024
+    vector, table = normal(K), normal(1200, 96)
+    w8, ws = ops.quantize_weight_rows(normal(1536, K), 2)
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    stream = lambda: C.c_void_p(torch.cuda.current_stream().cuda_stream)  # noqa: E731
+
+    def glue(name, x, columns, *args):
+        o = torch.zeros((x.shape[0], columns), dtype=torch.bfloat16, device="cuda")
+        _lib.check(getattr(_lib.lib(), name)(*(ptr(a) if torch.is_tensor(a) else ptr(o) if a is None else a for a in args), stream()))
+        return o
+
+    def rope(x):
+        codes, scales = torch.zeros_like(x, dtype=torch.int8), torch.zeros(8 * x.shape[0], device="cuda")
+        _lib.check(_lib.lib().difb200_qk_norm_rope_quant(ptr(x), ptr(vector), ptr(table), ptr(table), None, ptr(codes), ptr(scales), 2,
+                                                         x.shape[0], 8, 96, 96, x.shape[0], 1200, 0, 1e-5, 0, stream()))
+        return codes, scales
+
+    heads = lambda x: x.view(1, x.shape[0], 8, 128)  # noqa: E731
+    calls = {"variant %d" % i: (lambda x, i=i: ops.quantize_int8_rows([x if i not in (4, 7) else x.view(-1, 4096)], i)) for i in range(1, 8)}
+    calls.update({
+        "residual": lambda x: ops.quantize_int8_rows([x], 3, residual=True),
+        "two inputs": lambda x: ops.quantize_int8_rows([x, x], 2),
+        "direct heads": lambda x: ops.quantize_int8_rows([x.view(-1, 128)], 1),
+        "packing": lambda x: ops.quantize_weight_rows(x, 2, mse_scale=True, input_scale=x[0].clamp(0.5, 2.0)),
+        "rms norm": lambda x: ops.rms_norm_modulate_quant(x, vector, x, x),
+        "layer norm": lambda x: ops.layer_norm_modulate_quant(x, vector, vector, x, x),
+        "linear": lambda x: ops.w8a8_linear(x, w8, ws),
+        "attention": lambda x: ops.attention(heads(x), heads(x), heads(x)),
+        "gate": lambda x: glue("difb200_residual_gate", x, K, x, x, x, None, 2, x.shape[0], K, x.shape[0]),
+        "swiglu": lambda x: glue("difb200_swiglu", x, K // 2, x, None, 2, x.shape[0], K // 2, K, 0, 0),
+        "rope": rope,
+    })
+    return calls
+
+
+@pytest.mark.parametrize("rows", [4, 332, 1200])
+def test_kernels_launched_ahead_read_what_the_kernel_in_front_writes(rows):
+    """Every kernel that is launched ahead, behind a quantiser that lets it start at once and whose codes (as the bits of bf16
+    numbers) are what it reads: the buffer holds other numbers until that quantiser is done."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    sources = [0.55 + 0.2 * torch.rand((rows, 2048), generator=g, device="cuda") for _ in range(2)]
+    for s in sources:
+        s[:, 5] = 1.0  # the largest of a row: its code with clip 2 is 64, the others' are 35 to 48
+    sources = [s.to(torch.bfloat16) for s in sources]
+    codes, scales = torch.zeros((rows, 2048), dtype=torch.int8, device="cuda"), torch.zeros(rows, device="cuda")
+    x = codes.view(torch.bfloat16)
+    write = lambda i: ops.quantize_int8_rows([sources[i]], 1, clip=2.0, out=(codes, scales))  # noqa: E731
+    tensors = lambda r: [r] if torch.is_tensor(r) else list(r)  # noqa: E731
+    for name, call in _readers().items():
+        want = []
+        for i in range(2):
+            write(i)
+            torch.cuda.synchronize()
+            want.append([t.clone() for t in tensors(call(x))])
+            torch.cuda.synchronize()
+        assert any(not torch.equal(a, b) for a, b in zip(*want)), name
+        for i in range(6):
+            write(i % 2)
+            got = tensors(call(x))
+            torch.cuda.synchronize()
+            for a, b in zip(got, want[i % 2]):
+                assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), (name, i)
+    ops.poll_status()
