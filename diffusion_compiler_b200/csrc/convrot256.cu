@@ -24,7 +24,7 @@
 // blocks at a time to save per-row work. Before -> now, us: 33272 x 3072 83.9 -> 71.8 (4.3 TB/s), 33272 x 8192 220.6 -> 181.7,
 // 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 55.4, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
 // 12288 x 3072 64.7 -> 56.5 (all lanes evaluate samples, in doubles only where candidates are close), with input
-// equalisation 94.2 -> 72.6, RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
+// equalisation 94.2 -> 62.6 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
 // copies through shared memory instead of registers gave nothing.
 #include "quant_common.cuh"
 
@@ -35,8 +35,23 @@ namespace {
 constexpr int kWarpBytes = kWarpBytes256;
 constexpr uint32_t kCodeHalfBytes = 544, kCodeBytes = 2 * kCodeHalfBytes; // code pairs of a half-warp's two groups, of a block
 
-// kPack: weight rows with the scale search (and input equalisation where given), kEqualise: without the search.
-enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3 };
+// kPack: weight rows with the scale search, kEqualise: with input equalisation, kPackEqualise: with both, kPackTable: with both
+// and a table of the equalisation's reciprocals.
+enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3, kPackEqualise = 4, kPackTable = 5 };
+__host__ __device__ constexpr bool searches(int extra) { return extra == kPack || extra == kPackEqualise || extra == kPackTable; }
+__host__ __device__ constexpr bool equalises(int extra) { return extra == kEqualise || extra == kPackEqualise || extra == kPackTable; }
+
+// Shared memory of a CTA: per warp the transpose / staging area and the row maxima; for the signed variants 16 XOR masks per
+// thread and block (with input equalisation the signs are in its table); the sums of the scale search; that table.
+template <bool SIGNED, int EXTRA, int NIT>
+__host__ __device__ constexpr uint32_t sums_offset(uint32_t warps) {
+  return warps * kWarpBytes + warps * 16u + 64u + (SIGNED && EXTRA != kPackTable ? warps * 32u * 64u * NIT : 0u);
+}
+template <bool SIGNED, int EXTRA, int NIT>
+__host__ __device__ constexpr uint32_t table_offset(uint32_t warps) {
+  return (sums_offset<SIGNED, EXTRA, NIT>(warps) + (searches(EXTRA) ? warps * 7u * (uint32_t)(sizeof(double) + sizeof(float)) : 0u) + 15u) & ~15u;
+}
+constexpr uint32_t kTableBlockBytes = 8192; // of 1024 columns: [16][32 lanes] x 16 bytes, pairs of high parts, then of low parts
 
 // 32 bytes of one thread: one 256-bit load where every run starts on 32 bytes, else two of 128 bits.
 __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, uint4 &b) {
@@ -58,7 +73,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   extern __shared__ __align__(128) uint32_t smem[];
   const uint64_t after = grid_dependency_wait_zero(); // in the address of every load
   grid_dependents_launch();
-  constexpr bool kWeights = EXTRA == kPack || EXTRA == kEqualise;
+  constexpr bool kEqualised = equalises(EXTRA), kTable = EXTRA == kPackTable, kFlips = SIGNED && !kTable;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = warp / warps_per_row;         // which row of this CTA's batch
   const int wrow = warp - slot * warps_per_row;  // warp index inside the row
@@ -86,7 +101,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   // (two per group), vector q of all threads contiguous.
   const uint32_t mask_step = blockDim.x * 16u;
   const uint32_t mask_addr = smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u) + 64u + threadIdx.x * 16u;
-  if (SIGNED) {
+  if (kFlips) {
 #pragma unroll 1
     for (int q = 0; q < 4 * NIT; ++q) {
       const uint32_t c = col0 + (uint32_t)(q >> 2) * 1024u + (uint32_t)((q >> 1) & 1) * 256u + 8u * (q & 1);
@@ -99,9 +114,51 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
                    : "memory");
     }
   }
-  // Weight packing: may the fast quotient be used for every entry of this thread's columns?
-  bool equalise_fast = true;
-  if (kWeights && p.equalise) {
+  // Input equalisation divides every row by the same vector e: the CTA's rows share a table of 1 / e as the sum of two fp32 numbers,
+  // good to 2^-48, so that w / e is a product and a fused sum. (The quotient of two 8-bit significands is never within 2^-33 of a
+  // rounding boundary of fp32.) Reciprocal, residual and correction in every row: packing 12288 x 3072 with
+  // the search 71.6 us, with the table and the prefetch that its registers allow 65.2 (16384 rows, seven full rounds, 94.8 and 79.0).
+  const uint32_t table_addr = smem_addr + table_offset<SIGNED, EXTRA, NIT>((uint32_t)total_warps);
+  bool equalise_fast = true; // this warp's entries are of ordinary magnitude
+  if (kTable) {
+    for (uint32_t i = threadIdx.x; i < ((columns + 1023u) >> 10) * 32u; i += blockDim.x) { // one lane's runs of one block
+      const uint32_t c = (i >> 5) * 1024u + 512u * ((i >> 4) & 1u) + 16u * (i & 15u), to = table_addr + (i >> 5) * kTableBlockBytes + (i & 31u) * 16u;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint4 one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+        const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c) + half;
+        const uint4 ea4 = c < columns ? __ldg(ep) : one, eb4 = c + 256u < columns ? __ldg(ep + 32) : one;
+        const uint32_t ea[4] = {ea4.x, ea4.y, ea4.z, ea4.w}, eb[4] = {eb4.x, eb4.y, eb4.z, eb4.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float e[4] = {__uint_as_float(ea[k] << 16), __uint_as_float(eb[k] << 16), __uint_as_float(ea[k] & 0xffff0000u),
+                              __uint_as_float(eb[k] & 0xffff0000u)};
+          float high[4], low[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (SIGNED && sign_bit(c + 256u * (j & 1u) + 8u * half + 2u * k + (j >> 1)))
+              e[j] = -e[j];
+            high[j] = __frcp_rn(e[j]);
+            low[j] = __fmul_rn(__fmaf_rn(-e[j], high[j], 1.0f), high[j]);
+          }
+          sts128(to + (4u * half + k) * 512u, high[0], high[1], high[2], high[3]);
+          sts128(to + (8u + 4u * half + k) * 512u, low[0], low[1], low[2], low[3]);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8 * NIT; ++q) {
+      if (col0 + 1024u * (q >> 3) < columns) {
+        const uint4 h = lds128(table_addr + ((uint32_t)wrow * NIT + (q >> 3)) * kTableBlockBytes + (q & 7u) * 512u + lane * 16u);
+        const uint32_t high[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          equalise_fast = equalise_fast && fabsf(__uint_as_float(high[i])) > 1.0e-9f && fabsf(__uint_as_float(high[i])) < 1.0e9f;
+      }
+    }
+    equalise_fast = __all_sync(0xffffffffu, equalise_fast);
+  } else if (kEqualised) {
 #pragma unroll
     for (int q = 0; q < 2 * NIT; ++q) {
       const uint32_t c = col0 + (uint32_t)(q >> 1) * 1024u + (uint32_t)(q & 1) * 256u;
@@ -163,12 +220,16 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     }
   };
   auto row_barrier = [&]() { // the warps of one row only; rows in flight do not wait for each other
-    if (NIT == 1 || warps_per_row > 1)
+    if (kTable && warps_per_row == 1)
+      __syncwarp();
+    else if (NIT == 1 || warps_per_row > 1)
       asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(warps_per_row * 32) : "memory");
   };
 
   const uint64_t row_step = (uint64_t)gridDim.x * rows_per_cta;
-  uint64_t row = (uint64_t)blockIdx.x * rows_per_cta + slot;
+  // Where a CTA has all rows of an SM, those of a last round are spread over the SMs (12288 x 3072 with the table 71.0 -> 67.0 us);
+  // of smaller CTAs every SM gets its share of a last round anyway.
+  uint64_t row = kTable ? (uint64_t)slot * gridDim.x + blockIdx.x : (uint64_t)blockIdx.x * rows_per_cta + slot;
   uint4 next[4];
   if (PREFETCH)
     fetch(row, 0, next);
@@ -271,7 +332,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             }
           }
         } else {
-          if (SIGNED) {
+          if (kFlips) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
               const uint4 ma4 = lds128(mask_addr + (4 * it + q) * mask_step), mb4 = lds128(mask_addr + (4 * it + 2 + q) * mask_step);
@@ -288,44 +349,77 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             P[2 * i] = pack2(__uint_as_float(wa[i] << 16), __uint_as_float(wb[i] << 16));
             P[2 * i + 1] = pack2(__uint_as_float(wa[i] & 0xffff0000u), __uint_as_float(wb[i] & 0xffff0000u));
           }
-          if (kWeights && p.equalise) {
+          if (kEqualised) {
             // weight rows with input equalisation: w / e in fp32 before anything else (reference
-            // tools/difflux2sample.cpp:3005-3014; the sign flip commutes with the division).
-            // One Markstein step from the approximate reciprocal: the quotient of two 8-bit
-            // significands is never within 2^-33 of a rounding boundary of fp32, far outside the
-            // 2^-44 error of fma(r, y, q). Where w or the quotient is not finite the step gives NaN and the product,
-            // which then is the quotient, stands. Subnormal quotients may be off by 2^-149: the row scale
-            // is at least 1e-30.
-            const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
-            const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
-            const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z,
-                                 act_b ? __ldg(ep + 33) : z};
-            const uint32_t ea[8] = {e4[0].x, e4[0].y, e4[0].z, e4[0].w, e4[1].x, e4[1].y, e4[1].z, e4[1].w};
-            const uint32_t eb[8] = {e4[2].x, e4[2].y, e4[2].z, e4[2].w, e4[3].x, e4[3].y, e4[3].z, e4[3].w};
-            auto entry = [&](int i, float &e0, float &e1) {
-              e0 = __uint_as_float((i & 1) ? (ea[i >> 1] & 0xffff0000u) : (ea[i >> 1] << 16));
-              e1 = __uint_as_float((i & 1) ? (eb[i >> 1] & 0xffff0000u) : (eb[i >> 1] << 16));
-            };
-            if (equalise_fast) { // (of the warp: a branch for every pair cost packing 12288 x 3072 a tenth)
+            // tools/difflux2sample.cpp:3005-3014; the sign flip commutes with the division). Where a result is not finite
+            // the division decides. Results below 2^-100 may be off by 2^-149: the row scale is at least 1e-30.
+            auto number = [](const uint32_t(&w)[8], int i) { return __uint_as_float((i & 1) ? (w[i >> 1] & 0xffff0000u) : (w[i >> 1] << 16)); };
+            auto entries = [&](uint32_t(&ea)[8], uint32_t(&eb)[8]) {
+              const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
+              const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
+              const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z, act_b ? __ldg(ep + 33) : z};
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                float e0, e1, y0, y1;
-                entry(i, e0, e1);
-                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(e0));
-                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(e1));
-                const uint64_t y2 = pack2(y0, y1), q2 = mul2(P[i], y2);
-                float q0, q1, x0, x1;
-                unpack2(q2, q0, q1);
-                unpack2(fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2), x0, x1);
-                P[i] = pack2(x0 == x0 ? x0 : q0, x1 == x1 ? x1 : q1);
+              for (int i = 0; i < 8; ++i) {
+                const uint4 &va = e4[i >> 2], &vb = e4[2 + (i >> 2)];
+                ea[i] = (i & 3) == 0 ? va.x : (i & 3) == 1 ? va.y : (i & 3) == 2 ? va.z : va.w;
+                eb[i] = (i & 3) == 0 ? vb.x : (i & 3) == 1 ? vb.y : (i & 3) == 2 ? vb.z : vb.w;
+              }
+            };
+            uint32_t ea[8], eb[8];
+            if constexpr (kTable) {
+              float most = 0.0f;
+              if (equalise_fast) { // (of the warp)
+                const uint32_t at = table_addr + ((uint32_t)wrow * NIT + it) * kTableBlockBytes + lane * 16u;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                  const uint4 h = lds128(at + q * 512u), l = lds128(at + (8u + q) * 512u);
+                  auto of = [](uint32_t a_, uint32_t b_) { return pack2(__uint_as_float(a_), __uint_as_float(b_)); };
+                  P[2 * q] = fma2(P[2 * q], of(h.x, h.y), mul2(P[2 * q], of(l.x, l.y)));
+                  P[2 * q + 1] = fma2(P[2 * q + 1], of(h.z, h.w), mul2(P[2 * q + 1], of(l.z, l.w)));
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  float lo, hi;
+                  unpack2(P[i], lo, hi);
+                  asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(fabsf(lo)), "f"(fabsf(hi)));
+                }
+              }
+              if (!equalise_fast || !(most < INFINITY)) { // the words once more: they are not kept for this
+                uint4 again[4];
+                fetch(row, it, again);
+                const uint32_t xa[8] = {again[0].x, again[0].y, again[0].z, again[0].w, again[1].x, again[1].y, again[1].z, again[1].w};
+                const uint32_t xb[8] = {again[2].x, again[2].y, again[2].z, again[2].w, again[3].x, again[3].y, again[3].z, again[3].w};
+                entries(ea, eb);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  P[i] = pack2(__fdiv_rn(number(xa, i), number(ea, i)), __fdiv_rn(number(xb, i), number(eb, i)));
+                  if (SIGNED)
+                    P[i] ^= (uint64_t)sign_bit(c + i) << 31 | (uint64_t)sign_bit(c + 256u + i) << 63;
+                }
               }
             } else {
+              // without a table: a reciprocal and one Markstein step, 2^-44 at most off, and a choice per result instead of a test of all
+              entries(ea, eb);
+              if (equalise_fast) { // (of the warp: a branch for every pair cost packing 12288 x 3072 a tenth)
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                float e0, e1, w0, w1;
-                entry(i, e0, e1);
-                unpack2(P[i], w0, w1);
-                P[i] = pack2(__fdiv_rn(w0, e0), __fdiv_rn(w1, e1));
+                for (int i = 0; i < 16; ++i) {
+                  const float e0 = number(ea, i), e1 = number(eb, i);
+                  float y0, y1;
+                  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(e0));
+                  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(e1));
+                  const uint64_t y2 = pack2(y0, y1), q2 = mul2(P[i], y2);
+                  float q0, q1, x0, x1;
+                  unpack2(q2, q0, q1);
+                  unpack2(fma2(fma2(pack2(-e0, -e1), q2, P[i]), y2, q2), x0, x1);
+                  P[i] = pack2(x0 == x0 ? x0 : q0, x1 == x1 ? x1 : q1);
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  float w0, w1;
+                  unpack2(P[i], w0, w1);
+                  P[i] = pack2(__fdiv_rn(w0, number(ea, i)), __fdiv_rn(w1, number(eb, i)));
+                }
               }
             }
           }
@@ -354,7 +448,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     }
     const float maximum = m * (1.0f / kCarry);
     float scale = row_scale(maximum, clip);
-    if (EXTRA == kPack && p.mse) {
+    if (searches(EXTRA)) {
       // The scale is the one of seven clipped candidates with the lowest squared error over every
       // fourth rotated element, the offline packer's rule (reference tools/difflux2sample.cpp:
       // 1225-1259). Those elements sit in the lanes with a % 4 == 0; they go through shared memory
@@ -380,8 +474,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       }
       // sums of the row's warps: doubles, then floats in an area of their own (rows of a CTA are not in step)
       double *errors = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(smem) +
-                                                  (size_t)total_warps * (kWarpBytes + 16) + 64 +
-                                                  (SIGNED ? (size_t)total_warps * 32 * 64 * NIT : 0));
+                                                  sums_offset<SIGNED, EXTRA, NIT>((uint32_t)total_warps));
       float *sums = reinterpret_cast<float *>(errors + 7 * total_warps);
       auto sample = [&](int i) {
         uint32_t pair;
@@ -395,21 +488,26 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       float chosen = candidate[0];
       bool decided;
       {
-        float e[7] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        uint64_t e2[7] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
+        const uint64_t bias2 = pack2(kCodeBias, kCodeBias);
 #pragma unroll 1
         for (int i = lane; i < 8 * samples; i += 32) {
           const uint64_t v2 = unpack_bf16_pair(sample(i));
-          float v0, v1;
-          unpack2(v2, v0, v1);
 #pragma unroll
           for (int f = 0; f < 7; ++f) {
             uint32_t t0, t1;
             code_words(pack_bf16_pair(mul2(v2, pack2(reciprocal[f], reciprocal[f]))), t0, t1);
-            const float d0 = __fmaf_rn(kCodeBias - __uint_as_float(t0), candidate[f], v0);
-            const float d1 = __fmaf_rn(kCodeBias - __uint_as_float(t1), candidate[f], v1);
-            e[f] = __fmaf_rn(d0, d0, e[f]);
-            e[f] = __fmaf_rn(d1, d1, e[f]);
+            const uint64_t minus2 = sub2(bias2, pack2(__uint_as_float(t0), __uint_as_float(t1)));
+            const uint64_t d2 = fma2(minus2, pack2(candidate[f], candidate[f]), v2);
+            e2[f] = fma2(d2, d2, e2[f]);
           }
+        }
+        float e[7];
+#pragma unroll
+        for (int f = 0; f < 7; ++f) {
+          float lo, hi;
+          unpack2(e2[f], lo, hi);
+          e[f] = lo + hi;
         }
         // Halving: with every exchange a lane keeps half of its sums, so that lane l ends with candidate l / 4's (7: none).
         // 9 exchanges in the place of 35, and what follows is per lane instead of per candidate.
@@ -497,7 +595,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       __syncwarp(); // the samples are read before the codes overwrite them
     }
     const float scale_bf16 = round_bf16_number(scale);
-    const float stored = ((SIGNED || (EXTRA == kPack && p.mse)) && !F32) ? scale_bf16 : scale;
+    const float stored = ((SIGNED || searches(EXTRA)) && !F32) ? scale_bf16 : scale;
     const float divisor = (F32 ? scale : scale_bf16) * kCarry;
     if (wrow == 0 && lane == 0)
       p.scales[row] = stored;
@@ -606,15 +704,17 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   const int warps_per_row = (int)((groups + 4u * NIT - 1u) / (4u * NIT));
   if (warps_per_row > MAXT / 32)
     return fail(kInternalError, "QuantizeInt8Rows: row too wide for this form");
-  constexpr int kWarps = MAXT / 32 < 8 ? MAXT / 32 : 8;
-  int rows_per_cta = kWarps / warps_per_row;
+  int rows_per_cta = (MAXT / 32 < 8 || EXTRA == kPackTable ? MAXT / 32 : 8) / warps_per_row;
   rows_per_cta = rows_per_cta < 1 ? 1 : rows_per_cta;
   if ((uint64_t)rows_per_cta > p.rows)
     rows_per_cta = (int)p.rows;
+  if (EXTRA == kPackTable) { // all rows in flight on an SM share its table, as far as the rows go round
+    const uint64_t share = (p.rows + sm_count() - 1) / sm_count();
+    rows_per_cta = (uint64_t)rows_per_cta > share ? (int)share : rows_per_cta;
+  }
   const int warps = warps_per_row * rows_per_cta, threads = warps * 32;
-  // per warp: transpose / staging area; row maxima; for the signed variants 16 XOR masks per thread and block
-  const size_t smem = (size_t)warps * kWarpBytes + (size_t)warps * 4 * sizeof(float) + 64 +
-                      (SIGNED ? (size_t)warps * 32 * 64 * NIT : 0) + (EXTRA == kPack ? (size_t)warps * 7 * (sizeof(double) + sizeof(float)) : 0);
+  const size_t smem = table_offset<SIGNED, EXTRA, NIT>((uint32_t)warps) +
+                      (EXTRA == kPackTable ? (size_t)((p.columns + 1023u) >> 10) * kTableBlockBytes : 0);
   auto kernel = convrot256_kernel<SIGNED, F32, RESIDUAL, EXTRA, NIT, PREFETCH, MAXT, MINB>;
   int resident = 1;
   if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), threads, smem, &resident))
@@ -674,6 +774,25 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
                               "the 256-wide variants without residual outputs");
   if (pack && !p.mse)
     return f32 ? launch_single<SIGNED, true, false, kEqualise>(p, stream) : launch_single<SIGNED, false, false, kEqualise>(p, stream);
+  // The scale search is arithmetic per row as well as per element: three blocks per warp where they divide the row and
+  // the rows are more than the machine holds at once, 16 warps per SM (12288 x 3072 one block and 24 warps 65.1 us, three with a
+  // prefetch and 12 warps 61.0, this without a prefetch 56.3; 3072 x 8192, whose last warp would be a third empty, 51.5 / 53.6 / 56.2).
+  const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+  const bool three = blocks % 3u == 0u && p.rows * blocks > (uint64_t)sm_count() * 24u;
+  if (pack && p.equalise) {
+    // With input equalisation one CTA per SM, whose rows share the table: 16 warps of three blocks with a prefetch, or 24 of one. The
+    // table takes 1.5 us, so from three rounds of 24 warps per SM on, and not where rows of more than 8 blocks leave warps idle. Every
+    // row its own reciprocals / table: 16384 x 3072 94.8 / 79.0, 12288 x 3072 71.6 / 65.2, 3072 x 12288 72.6 / 69.2, 3072 x 8192
+    // 53.9 / 52.1, fp32 112.3 / 94.5, 86.0 / 74.2, 88.7 / 84.3, 58.2 / 54.5; but 1500 x 10240 39.4 / 41.6, 3000 x 2304 25.8 / 26.9,
+    // 3000 x 512 12.3 / 13.9.
+    if (p.rows * blocks >= (uint64_t)sm_count() * 72u && (blocks % 3u == 0u || blocks <= 8u))
+      return f32     ? launch_form<SIGNED, true, false, kPackTable, 1, false, 768, 1>(p, stream)
+             : three ? launch_form<SIGNED, false, false, kPackTable, 3, true, 512, 1>(p, stream)
+                     : launch_form<SIGNED, false, false, kPackTable, 1, false, 768, 1>(p, stream);
+    return f32     ? launch_single<SIGNED, true, false, kPackEqualise>(p, stream)
+           : three ? launch_form<SIGNED, false, false, kPackEqualise, 3, false, 256, 2>(p, stream)
+                   : launch_single<SIGNED, false, false, kPackEqualise>(p, stream);
+  }
   if (f32) {
     if (pack)
       return launch_single<SIGNED, true, false, kPack>(p, stream);
@@ -686,16 +805,8 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     return launch_single<SIGNED, false, true, kPlain>(p, stream);
   if (norm)
     return launch_single<SIGNED, false, false, kNorm>(p, stream);
-  if (pack) {
-    // The scale search is arithmetic per row as well as per element: three blocks per warp where they divide the row and
-    // the rows are more than the machine holds at once, 16 warps per SM and no prefetch (12288 x 3072 with equalisation: one
-    // block and 24 warps 76.3 us, three with a prefetch and 12 warps 78.7, this 72.6; without 65.1, 61.0, 56.5; 3072 x 8192, whose
-    // last warp would be a third empty, 51.5 / 53.6 / 56.2).
-    const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
-    return blocks % 3u == 0u && p.rows * blocks > (uint64_t)sm_count() * 24u
-               ? launch_form<SIGNED, false, false, kPack, 3, false, 256, 2>(p, stream)
-               : launch_single<SIGNED, false, false, kPack>(p, stream);
-  }
+  if (pack)
+    return three ? launch_form<SIGNED, false, false, kPack, 3, false, 256, 2>(p, stream) : launch_single<SIGNED, false, false, kPack>(p, stream);
   return launch_single<SIGNED, false, false, kPlain>(p, stream);
 }
 

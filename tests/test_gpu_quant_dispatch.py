@@ -196,3 +196,30 @@ def test_quotients_out_of_the_two_part_products_range(impl, K):
     for clip in (1.0e-12, 1.0e-30):  # beyond the integers the reference converts to: saturated by sign
         codes = ops.quantize_int8_rows([to_torch_bf16(x)], impl, clip)[0].cpu().numpy()
         assert np.all(codes[want[0] > 0] == 127) and np.all(codes[want[0] < 0] == -128), clip
+
+
+@pytest.mark.parametrize("impl", [2, 3, 5, 6])
+@pytest.mark.parametrize("rows,width", [
+    (10656, 256),   # one warp per row: as many rows as the table of reciprocals is made for
+    (3553, 3072),   # three blocks per warp, a last round of one row
+    (4000, 2816),   # the same with a partial third block
+    (5400, 1280),   # two blocks, the second of one group
+    (1340, 8192),   # eight blocks
+    (900, 12288),   # twelve
+])
+def test_packing_with_a_table_of_reciprocals(impl, rows, width):
+    """Rows are packed one by one: all at once, where a CTA's rows share a table of the equalisation's reciprocals, and a few hundred
+    at a time, where every row makes its own. Entries beyond the table's range, infinities and NaN among them."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(rows + impl)
+    w = to_torch_bf16(bf16_normal(rng, (rows, width), std=0.02))
+    eq = to_torch_bf16(ob.f32_to_bf16(np.exp(0.7 * rng.standard_normal(width)).astype(np.float32)))
+    w[1], w[2, 3], w[3, 5], w[4] = 0, float("inf"), float("nan"), w[4] * 2.0**-110
+    for wild in (False, True):
+        if wild:
+            eq[7], eq[255], eq[100] = 2.0**-60, -eq[255], 2.0**70
+        codes, scales = ops.quantize_weight_rows(w, impl, mse_scale=True, input_scale=eq)
+        parts = [ops.quantize_weight_rows(w[i:i + 400], impl, mse_scale=True, input_scale=eq) for i in range(0, rows, 400)]
+        assert torch.equal(codes, torch.cat([p[0] for p in parts]))
+        assert torch.equal(scales.view(torch.int32), torch.cat([p[1] for p in parts]).view(torch.int32))
