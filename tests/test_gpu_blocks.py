@@ -59,6 +59,35 @@ def test_video_block_replayed_from_cuda_graphs_keeps_the_bits():
     ops.poll_status()
 
 
+@pytest.mark.parametrize("tokens", [2000, 4100, 8301])  # the last step as a whole, in two and in four blocks of rows
+def test_video_block_with_page_locked_arrays_keeps_the_bits(tokens):
+    """With page-locked arrays on both sides the gate of the last step comes in, and the output leaves, a block of rows at a
+    time; with ordinary arrays, or only one side page-locked, as a whole. The same bits, for every input."""
+    import torch
+    from diffusion_compiler_b200 import plugin
+    rng = np.random.default_rng(tokens)
+    p, ids, consts, inputs = blocks.synth_video_block(rng, tokens, 1024, 8, 128, 256, 96, _cpu_quantize)
+    ex = plugin.PluginExecutor(0)
+    prepared = ex.prepare(p, consts)
+
+    def locked(a):
+        host = torch.empty(a.shape, dtype=torch.int16, pin_memory=True)
+        host.numpy()[...] = a.view(np.int16)
+        return host.numpy().view(np.uint16)
+
+    for trial in range(3):
+        want, _ = prepared.run(inputs)
+        gate, want = inputs[ids["mods"][5]], want[ids["out"]]
+        pinned = {t: locked(a) if a.dtype == np.uint16 else a for t, a in inputs.items()}
+        for given, out in ((pinned, locked(np.full_like(want, 0x4000 + trial))), (pinned, np.zeros_like(want)), (inputs, locked(np.zeros_like(want)))):
+            prepared.run(given, outputs={ids["out"]: out})
+            assert np.array_equal(out, want)
+        inputs = dict(inputs)
+        inputs[ids["mods"][5]] = np.ascontiguousarray(gate[::-1])
+        inputs[ids["x"]] = np.ascontiguousarray(inputs[ids["x"]][::-1])
+    ex.close()
+
+
 def test_plugin_rope_fusions_keep_the_bits(monkeypatch):
     """The planner reads last-axis slices in place from QkNormPartialRope and lets that op write
     the attention kernel's INT8 q / k directly (through a Concat along tokens too). Same arithmetic,
