@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "quant_common.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -144,7 +145,12 @@ __device__ __forceinline__ void add_in_place(float &acc, float v) {
   asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(acc) : "f"(v));
 }
 
-template <bool LAYER, int STAGES>
+// What the sequential kernel computes: the RMS statistic, the layer form's two, or of these the mean alone.
+enum RowSums { kRms, kLayer, kMean };
+__device__ __forceinline__ float inverse_deviation(float sum, uint32_t cols, float eps) {
+  return __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps)));
+}
+template <int SUMS, int STAGES>
 __global__ void __launch_bounds__(32 * kStatWarps)
 k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps) {
   extern __shared__ uint4 stat_smem[];
@@ -266,16 +272,209 @@ k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint
           add_in_place(acc, a[e]);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
-    if (LAYER) {
+    if (SUMS != kRms) {
       pass(std::integral_constant<int, 0>{});
       mean = __fdiv_rn(acc, (float)cols);
-      deviation_pass();
+      if (SUMS == kLayer)
+        deviation_pass();
     } else {
       pass(std::integral_constant<int, 1>{});
     }
     if (row < rows)
-      *reinterpret_cast<float2 *>(stats.at + row * stats.pitch) =
-          make_float2(mean, __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(acc, (float)cols), eps))));
+      *reinterpret_cast<float2 *>(stats.at + row * stats.pitch) = make_float2(mean, SUMS == kMean ? 0.0f : inverse_deviation(acc, cols, eps));
+  }
+}
+
+// ---- the same sums of squares in 16 parts per row, for few rows ----
+// A chain of cols dependent additions takes 7 us for 3072, however few rows there are. Its terms are not negative, so that
+// it can be cut: of two chains of the same terms that start at t and r, in one binade and a multiple of four units of its last place
+// apart, each step adds the same number to both, by round to nearest even on the same grid, and one crossing into the next
+// binade changes nothing as long as both cross it in the same step, since the grid there is twice as wide. So every lane runs the
+// chain of its part of the row from a guess r of where the row's chain will arrive (the sum of what lies in front), for each value
+// of the guess's last two bits, and the row's chain t then steps from lane to lane: it takes the chain with its own last two
+// bits and adds the distance t - r that it has from that one's start. Every lane says between which distances that holds (the
+// same binade at the start, at most one crossing, in a step whose sums on either side are further from the boundary than t and r from
+// one another); where it does not, in one row of ten as a part's numbers cross several binades at once, or where numbers are not
+// finite, the part's terms are added one by one. Compared with the sequential chain on a CPU: 60000 rows of nine kinds of
+// numbers, some of them built to meet boundaries and ties, same bits.
+// It is bound by the operations of five chains (about 750 per row and warp at IPC 0.5), so that many rows are better off with the
+// sequential kernel, whose lanes have a row each: row_stats has the line. 32 parts per row took the same time for few rows and
+// a fifth more for many, 8 more for few; rows kept for a second pass in registers (unrolled: 168 of them) the same.
+constexpr int kSquareWarps = 4, kSquareParts = 16; // warps of a CTA, parts of a row
+struct SquareParams {
+  const uint4 *x;
+  RowStats stats; // the layer form's mean stands there
+  uint64_t rows;
+  uint32_t cols, groups; // groups of 8 columns in a part of a row
+  float eps;
+  Divisor by_groups;
+};
+__host__ __device__ constexpr uint32_t square_pitch(uint32_t groups) { return (groups | 1u) * 16u; } // of a part in shared memory
+
+// The terms of a word's two elements, and a step of the chain.
+__device__ __forceinline__ void square_terms(uint32_t word, float mean, float &q0, float &q1) {
+  float d0, d1;
+  asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; sub.rn.f32.bf16 %0, lo, %3; sub.rn.f32.bf16 %1, hi, %3; }"
+      : "=f"(d0), "=f"(d1) : "r"(word), "f"(mean));
+  q0 = __fmul_rn(d0, d0);
+  q1 = __fmul_rn(d1, d1);
+}
+// CHAINS sums after the eight elements of a group; `after` sees each of them.
+template <bool LAYER, int CHAINS, class F>
+__device__ __forceinline__ void square_chain(const uint4 &v, float mean, float (&acc)[CHAINS], F &&after) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (LAYER) {
+      float q0, q1;
+      square_terms(w[i], mean, q0, q1);
+#pragma unroll
+      for (int c = 0; c < CHAINS; ++c)
+        acc[c] = __fadd_rn(acc[c], q0);
+      after();
+#pragma unroll
+      for (int c = 0; c < CHAINS; ++c)
+        acc[c] = __fadd_rn(acc[c], q1);
+      after();
+    } else {
+#pragma unroll
+      for (int c = 0; c < CHAINS; ++c)
+        asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; fma.rn.f32.bf16 %0, lo, lo, %0; }" : "+f"(acc[c]) : "r"(w[i]));
+      after();
+#pragma unroll
+      for (int c = 0; c < CHAINS; ++c)
+        asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; fma.rn.f32.bf16 %0, hi, hi, %0; }" : "+f"(acc[c]) : "r"(w[i]));
+      after();
+    }
+  }
+}
+
+// A lane per part, two rows per warp at a time. GROUPS: p.groups as a constant, or 0.
+template <bool LAYER, int GROUPS>
+__global__ void __launch_bounds__(32 * kSquareWarps)
+k_row_squares(const SquareParams p) {
+  extern __shared__ uint4 square_smem[];
+  const uint64_t after = grid_dependency_wait_zero();
+  constexpr uint32_t kParts = kSquareParts, kRows = 32 / kParts;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, part = lane % kParts, groups = GROUPS ? GROUPS : p.groups;
+  const uint32_t pitch = square_pitch(groups), cols8 = groups * kParts;
+  unsigned char *buffer = reinterpret_cast<unsigned char *>(square_smem) + warp * 32u * pitch;
+  const uint4 *mine = reinterpret_cast<const uint4 *>(buffer + lane * pitch);
+  const uint32_t to = smem_u32(buffer);
+  for (uint64_t row0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + warp) * kRows; row0 < p.rows; row0 += (uint64_t)gridDim.x * (blockDim.x >> 5) * kRows) {
+    const uint64_t row = row0 + lane / kParts;
+    { // the rows are neighbours: 32 parts one behind the other
+      const uint32_t valid = (uint32_t)min((uint64_t)kRows, p.rows - row0) * cols8;
+      const uint4 *from = p.x + row0 * cols8;
+#pragma unroll
+      for (uint32_t k = 0; k < groups; ++k) {
+        const uint32_t c = lane + 32u * k, of = GROUPS ? c / groups : p.by_groups.quotient(c);
+        cp_async16(to + of * pitch + (c - of * groups) * 16u, c < valid ? from + c : p.x, c < valid);
+      }
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+    }
+    const float mean = LAYER && row < p.rows ? row_stat(p.stats, row).x : 0.0f;
+    // the guess: the sum of the parts in front (each in order, so that the second part starts from the row's very chain: it
+    // is the one that most often crosses several binades)
+    float sum[1] = {0.0f};
+#pragma unroll 4
+    for (uint32_t k = 0; k < groups; ++k)
+      square_chain<LAYER>(mine[k], mean, sum, [] {});
+    float front = sum[0];
+#pragma unroll
+    for (int o = 1; o < (int)kParts; o <<= 1) {
+      const float other = __shfl_up_sync(0xffffffffu, front, o, kParts);
+      if (part >= (uint32_t)o)
+        front += other;
+    }
+    front = __shfl_up_sync(0xffffffffu, front, 1, kParts);
+    const uint32_t start = part == 0u ? 0u : __float_as_uint(front) & ~3u;
+    const float bound = __uint_as_float(((start >> 23) + 1u) << 23);
+    // the four chains, and the group in which the first of them crosses into the next binade
+    float acc[4], before = 0.0f, behind = 0.0f;
+    uint32_t crossing = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      acc[c] = __uint_as_float(start + c);
+#pragma unroll 4
+    for (uint32_t k = 0; k < groups; ++k) {
+      if (acc[0] < bound) {
+        before = acc[0];
+        crossing = k;
+      }
+      square_chain<LAYER>(mine[k], mean, acc, [] {});
+    }
+    if (acc[0] >= bound) { // (also where the chain has crossed more than once: the ends will tell)
+      float one[1] = {before}, sums[8];
+      int at = 0;
+      square_chain<LAYER>(mine[crossing], mean, one, [&] { sums[at++] = one[0]; });
+      behind = INFINITY;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        before = fmaxf(before, sums[i] < bound ? sums[i] : 0.0f);
+        behind = fminf(behind, sums[i] < bound ? INFINITY : sums[i]);
+      }
+    }
+    // Distances t - r with which the row's chain goes the way of these: it stays below the boundary where they do; where they
+    // cross it, it is below it in front of the same step and above it behind, and meets no other.
+    float above = INFINITY, below = -INFINITY; // none
+    {
+      const uint32_t binade = start >> 23;
+      const float four_units = __uint_as_float((binade - 21u) << 23), room = bound - before - four_units;
+      if (binade >= 25u && binade < 253u) {
+        if (acc[3] < bound) {
+          above = -INFINITY;
+          below = bound - acc[3];
+        } else if (acc[0] >= bound && acc[3] < 2.0f * bound && room > 0.0f && behind > bound && behind < INFINITY) {
+          above = bound - behind;
+          below = fminf(room, 2.0f * bound - acc[3]);
+        }
+      }
+    }
+    // the row's chain from part to part
+    bool done = false; // this part's end is known
+    float total = 0.0f;
+    for (;;) {
+      bool open = false;
+#pragma unroll
+      for (uint32_t s = 0; s < kParts; ++s) {
+        const float in = s == 0u ? 0.0f : __shfl_sync(0xffffffffu, total, s - 1u, kParts);
+        const uint32_t t = __float_as_uint(in), last = t & 3u, from = start | last;
+        const float end = last & 2u ? (last & 1u ? acc[3] : acc[2]) : (last & 1u ? acc[1] : acc[0]);
+        const float apart = in - __uint_as_float(from); // where they hold, a multiple of four units
+        const bool holds = t == from || ((t ^ from) < 0x800000u && apart > above && apart < below);
+        if (part == s && !done) {
+          total = t == from ? end : end + apart; // (infinite ones have no distance)
+          open = !holds;
+        }
+      }
+      uint32_t all_open = __ballot_sync(0xffffffffu, open && row < p.rows);
+      if (all_open == 0u)
+        break;
+      // The first open part of every row, term by term and by all lanes; what is in front of it is final.
+      constexpr uint32_t kPartsMask = (1u << kParts) - 1u;
+#pragma unroll 1
+      for (uint32_t r = 0; r < kRows; ++r) {
+        const uint32_t of_row = all_open >> (r * kParts) & kPartsMask;
+        if (of_row == 0u)
+          continue;
+        const uint32_t at = r * kParts + (uint32_t)__ffs((int)of_row) - 1u;
+        const float in = __shfl_sync(0xffffffffu, total, at == 0u ? 0u : at - 1u);
+        float one[1] = {at % kParts == 0u ? 0.0f : in};
+        const float row_mean = __shfl_sync(0xffffffffu, mean, at);
+        const uint4 *terms = reinterpret_cast<const uint4 *>(buffer + at * pitch);
+        for (uint32_t k = 0; k < groups; ++k)
+          square_chain<LAYER>(terms[k], row_mean, one, [] {});
+        if (lane == at)
+          total = one[0];
+        if (lane / kParts == r && lane <= at)
+          done = true;
+      }
+    }
+    if (part == kParts - 1u && row < p.rows)
+      *reinterpret_cast<float2 *>(p.stats.at + row * p.stats.pitch) = make_float2(mean, inverse_deviation(total, p.cols, p.eps));
+    __syncwarp(); // the rows are read: the next ones may come
   }
 }
 
@@ -724,12 +923,34 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
     blocks = blocks > cap ? cap : blocks;
     return launch_ahead("k_row_stats_parallel", k_row_stats_parallel, blocks, 256, 0, s, X, *stats, rows, (uint32_t)cols, eps, layer ? 1 : 0);
   }
+  auto squares = [&]() {
+    constexpr int kGroups3072 = 3072 / (8 * kSquareParts);
+    const uint32_t groups = (uint32_t)(cols / (8 * kSquareParts)), warp_bytes = 32u * square_pitch(groups);
+    const SquareParams p{X, *stats, rows, (uint32_t)cols, groups, eps, divisor(groups)};
+    const uint64_t sms = (uint64_t)sm_count(), wanted = (rows + 32 / kSquareParts - 1) / (32 / kSquareParts);
+    const uint32_t warps = (uint32_t)std::min<uint64_t>(kSquareWarps, (wanted + sms - 1) / sms);
+    auto kernel = groups == kGroups3072 ? (layer ? k_row_squares<true, kGroups3072> : k_row_squares<false, kGroups3072>)
+                                        : (layer ? k_row_squares<true, 0> : k_row_squares<false, 0>);
+    int resident = 1;
+    if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * (int)warps, warps * warp_bytes, &resident))
+      return rc;
+    const uint64_t blocks = std::min<uint64_t>((wanted + warps - 1) / warps, sms * resident);
+    return launch_ahead("k_row_squares", kernel, blocks, 32 * (int)warps, warps * warp_bytes, s, p);
+  };
+  // Norm and quantiser, us, sequential / in parts: RMS, 3072 columns, 1 row 12.8 / 6.3, 150 13.2 / 7.7, 1500 23.6 / 16.9, 4700 36.8 / 32.8,
+  // 8318 51.6 / 53.5; 8192 columns, 150 35.4 / 14.9, 4700 92.5 / 88.3, 8318 132 / 151; 4096 columns, 4700 47.9 / 47.5; 1024 columns,
+  // 150 7.8 / 6.8, 600 7.9 / 7.8, 1500 11.7 / 15.6. Of the layer form, whose mean stays a chain, the deviations: 3072 columns, 150
+  // 25.0 / 19.6, 1500 44.1 / 32.4, 4700 59.1 / 52.8, 8318 75.7 / 75.5; 1024 columns, 600 12.5 / 12.5.
+  const bool in_parts = cols % (8 * kSquareParts) == 0 && cols >= 1024 && cols <= 8192 && rows <= (cols >= 2048 ? 32ull : 4ull) * (uint64_t)sm_count();
+  if (in_parts && !layer)
+    return squares();
   // Eight chunks in flight where a few warps per SM have to cover the latency alone, four where the rows
   // give an SM more than six warps (33272 x 3072: one wave of resident CTAs instead of two).
   const uint64_t warps = (rows + 31) / 32;
   const bool deep = warps <= (uint64_t)sm_count() * 6;
-  auto kernel = deep ? (layer ? k_row_stats_sequential<true, 8> : k_row_stats_sequential<false, 8>)
-                     : (layer ? k_row_stats_sequential<true, 4> : k_row_stats_sequential<false, 4>);
+  auto kernel = !layer     ? (deep ? k_row_stats_sequential<kRms, 8> : k_row_stats_sequential<kRms, 4>)
+                : in_parts ? (deep ? k_row_stats_sequential<kMean, 8> : k_row_stats_sequential<kMean, 4>)
+                           : (deep ? k_row_stats_sequential<kLayer, 8> : k_row_stats_sequential<kLayer, 4>);
   const size_t smem = sizeof(uint4) * kStatWarps * (deep ? 8 : 4) * 32 * kStatPitch;
   int resident = 1;
   if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * kStatWarps, smem, &resident))
@@ -737,7 +958,9 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
   uint64_t blocks = (warps + kStatWarps - 1) / kStatWarps;
   const uint64_t cap = (uint64_t)sm_count() * resident;
   blocks = blocks > cap ? cap : blocks;
-  return launch_ahead("k_row_stats_sequential", kernel, blocks, 32 * kStatWarps, smem, s, X, *stats, rows, (uint32_t)cols, eps);
+  if (int rc = launch_ahead("k_row_stats_sequential", kernel, blocks, 32 * kStatWarps, smem, s, X, *stats, rows, (uint32_t)cols, eps))
+    return rc;
+  return in_parts ? squares() : kOk;
 }
 
 bool rms_norm_modulate_fast(const void *x, const void *w, const void *a, const void *b, void *o, uint32_t dt,

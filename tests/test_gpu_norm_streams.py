@@ -114,3 +114,31 @@ def test_norm_ops_in_place(K, over):
         got = run(layer, own[over], own["x"], own["scale"], own["shift"])
         torch.cuda.synchronize()
         assert torch.equal(want.view(torch.int16), got.view(torch.int16)), layer
+
+
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("cols", [1024, 2048, 2816, 3072, 8192])
+def test_statistics_of_few_rows_are_those_of_many(layer, cols):
+    """Few rows have their sums of squares from a kernel that cuts the sequential chain in 16 parts; many from the chain itself. Rows are
+    independent, so any slice of a tensor gives the bits of the whole: with outliers, equal numbers (ties in every step), rows whose
+    sums meet powers of two, zeros, steps over many binades, infinities and NaN."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    rows = 32 * torch.cuda.get_device_properties(0).multi_processor_count + 5
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = torch.randn((rows, cols), generator=g, device="cuda")
+    x[:, :: cols // 32] *= 16.0  # (and so that single parts cross several binades)
+    x[100:400] = x[100:400].round()
+    x[400:500] = torch.exp2(torch.arange(100, device="cuda").remainder(12).float() - 6.0)[:, None]
+    x[500:600] *= torch.exp(4.0 * torch.randn((100, cols), generator=g, device="cuda"))
+    x[600:650, : cols // 2] = 0.0
+    x[650], x[651, 7], x[652, 9], x[653] = 0.0, float("inf"), float("nan"), x[653] * 2.0**-40
+    x[654:700] *= 2.0 ** torch.arange(-23, 23, device="cuda").float()[:, None]
+    x = x.to(torch.bfloat16)
+    normal = lambda *s: (0.1 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)  # noqa: E731
+    w, b, s, h = normal(cols) + 1, normal(cols), normal(rows, cols), normal(rows, cols)
+    want = _call(ops, layer, x, w, b, s, h)
+    for first, count in ((0, 1), (3, 40), (90, 502), (600, 149), (0, rows - 5), (5, rows - 5)):
+        at = slice(first, first + count)
+        got = _call(ops, layer, x[at].contiguous(), w, b, s[at].contiguous(), h[at].contiguous())
+        assert torch.equal(got[0], want[0][at]) and torch.equal(got[1].view(torch.int32), want[1][at].view(torch.int32)), (first, count)
