@@ -63,7 +63,8 @@ struct Step {
   int out_tensor = -1;              // index of the tensor the (fused) step writes
   int mask_tensor = -1;             // Attention: index of the fused Bool key mask
   bool skip = false;                // op absorbed by a neighbour, or a Reshape served by aliasing
-  bool alias = false;               // Reshape: the output shares the input's buffer
+  bool alias = false;               // Reshape, or a Slice of neighbouring elements: the output shares the input's buffer,
+  uint64_t alias_offset = 0;        // from this byte on
   // QkNormPartialRope fused with its neighbours
   int rope_source = -1;             // tensor read in place (an absorbed last-axis Slice), else in[0]
   uint64_t rope_in_stride = 0, rope_in_offset = 0;
@@ -413,6 +414,23 @@ void plan(Executable &exe) {
       (role == 0 ? exe.steps[a].q_quantised : exe.steps[a].k_quantised) = true;
     }
   }
+  // A Slice whose elements are neighbours (nothing in front of its axis is repeated) is a part of its input's buffer, where
+  // that starts as kernels expect (16 bytes). At batch 1 the modulation vectors of a block, its streams' rows of the joint
+  // sequence: MMDiT block of 256 + 77 tokens, 16 of 51 launches. (Not token-sharded: there V's buffer is placed by its chain of aliases.)
+  for (Step &st : exe.steps) {
+    if (st.op->opcode != ir::Slice || st.skip || exe.ctx->world)
+      continue;
+    const ir::Tensor &o = *p.tensor(st.op->out[0]);
+    const uint64_t axis = st.op->u64(ir::Axis, 0);
+    uint64_t outer = 1, inner = ir::dtype_size(o.dtype);
+    for (size_t a = 0; a < o.dims.size(); ++a)
+      (a < axis ? outer : inner) *= a == axis ? 1 : o.dims[a];
+    const uint64_t offset = st.op->u64(ir::Start, 0) * inner;
+    if (outer == 1 && offset % 16 == 0) {
+      st.alias = st.skip = true;
+      st.alias_offset = offset;
+    }
+  }
 }
 
 
@@ -575,7 +593,7 @@ void allocate(Executable &exe) {
   const ir::Program &p = exe.program;
   const size_t n = p.tensors.size();
   exe.dev.assign(n, nullptr);
-  // Reshape outputs share the buffer of their input: every tensor belongs to the group of its root
+  // Outputs of aliasing steps share the buffer of their input: every tensor belongs to the group of its root
   std::vector<size_t> root(n);
   for (size_t i = 0; i < n; ++i)
     root[i] = i;
@@ -704,7 +722,7 @@ void allocate(Executable &exe) {
   for (const Step &st : exe.steps) // program order: a chain of reshapes resolves front to back
     if (st.alias) {
       const size_t out = (size_t)p.index_of(st.op->out[0]);
-      exe.dev[out] = exe.dev[(size_t)p.index_of(st.op->in[0])];
+      exe.dev[out] = static_cast<unsigned char *>(exe.dev[(size_t)p.index_of(st.op->in[0])]) + st.alias_offset;
       exe.owned[out] = 0;
     }
   size_t scratch = 0;

@@ -171,6 +171,31 @@ def test_mmdit_double_stream_block_through_plugin_matches_reference_executor():
     ex.close()
 
 
+def test_mmdit_block_at_batch_one_has_the_bits_of_batch_two():
+    """At batch 1 the slices of the modulations and of the joint sequence are parts of their inputs' buffers, at batch 2 copies: the
+    same image twice gives the same bits, also after other inputs."""
+    from diffusion_compiler_b200 import plugin
+    results = []
+    for batch in (1, 2):
+        rng = np.random.default_rng(15)
+        p, ids, consts, inputs = blocks.synth_mmdit_block(rng, batch=batch, grid=(8, 6), text_tokens=19, hidden=512, heads=4, mlp=1024,
+                                                         quantize=_cpu_quantize)
+        if batch == 1:
+            first_consts, first = consts, [inputs, {t: np.ascontiguousarray(a[..., ::-1]) if a.dtype == np.uint16 else a for t, a in inputs.items()}]
+        names = ids
+        ex = plugin.PluginExecutor(0)
+        prepared = ex.prepare(p, {t: first_consts[t] for t in consts})
+        for given in first:
+            twice = {t: a if a.shape == tuple(inputs[t].shape) else np.concatenate([a] * 2, axis=0) for t, a in given.items()}
+            got, _ = prepared.run(twice)
+            results.append([got[names[key]] for key in ("image_out", "text_out")])
+        ex.close()
+    for one, two in zip(results[:2], results[2:]):
+        for a, b in zip(one, two):
+            assert np.array_equal(a[0], b[0]) and np.array_equal(a[0], b[1])
+    assert not np.array_equal(results[0][0], results[1][0])
+
+
 @pytest.mark.parametrize("S,world", [(512, 4), (437, 4)])
 def test_token_sharded_video_block_matches_unsharded(S, world):
     """Ranks are emulated sequentially on one GPU: every rank runs its row-local part, the gather
