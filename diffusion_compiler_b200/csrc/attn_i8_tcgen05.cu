@@ -182,14 +182,19 @@ struct OperandParams {
   uint64_t q_rows;
   uint32_t S, KV, S_pad, key_blocks;
 };
-__global__ void __launch_bounds__(256)
+// STEPS: rows of a lane, in a CTA of 1024 / STEPS threads. Two where all CTAs are resident at once, whose time is a lane's chain
+// (1101 tokens, 24 heads over 8: attention and operands 23.9 us with four, 23.4; 300 tokens 13.6 and 13.1), four where rows
+// are many (1101 over 24, 423 CTAs: 25.5, with two 25.9).
+template <int STEPS>
+__global__ void __launch_bounds__(1024 / STEPS)
 attention_operands_kernel(const OperandParams p) {
   const uint64_t after = grid_dependency_wait_zero();
   grid_dependents_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 7;
   // The four rows of a lane are requested before the first is worked on (behind one another, each waited for its load:
   // B2 S4608 H24 41 us against 34).
-  uint4 lows[4], highs[4];
+  uint4 lows[STEPS], highs[STEPS];
+  constexpr uint32_t kStepRows = 128u / STEPS;
   auto request = [&](int step, const uint4 *row, bool valid) {
     lows[step] = highs[step] = make_uint4(0, 0, 0, 0);
     if (valid) {
@@ -219,20 +224,23 @@ attention_operands_kernel(const OperandParams p) {
   if (blockIdx.x < p.key_blocks) {
     const uint32_t tiles = p.S_pad / kTile, tile = blockIdx.x % tiles, kvh = (blockIdx.x / tiles) % p.KV,
                    b = blockIdx.x / (tiles * p.KV);
-    auto key_of = [&](int step) { return tile * kTile + step * 32u + warp * 4u + (lane >> 3); };
+    auto key_of = [&](int step) { return tile * kTile + step * kStepRows + warp * 4u + (lane >> 3); };
     auto row_of = [&](int step) { return ((uint64_t)b * p.S + (key_of(step) < p.S ? key_of(step) : 0)) * p.KV + kvh; };
 #pragma unroll
-    for (int step = 0; step < 4; ++step)
+    for (int step = 0; step < STEPS; ++step)
       request(step, p.k + after + row_of(step) * 16, key_of(step) < p.S);
-    __shared__ uint32_t masked[4]; // whether a segment of 32 keys has masked ones
-    if (threadIdx.x < 4)
+    __shared__ uint32_t masked[4], first_valid[4]; // whether a segment of 32 keys has masked ones; whether its first key is not
+    uint32_t own_first_valid = 0; // the same as bits, where thread 0 has the four segments' first keys
+    if (threadIdx.x < 4) {
       masked[threadIdx.x] = 0u;
+      if (STEPS != 4)
+        first_valid[threadIdx.x] = 0u;
+    }
     __syncthreads();
     float *t = p.table + (((uint64_t)b * p.KV + kvh) * tiles + tile) * (2u * kTile);
     float most = 0.0f;
-    uint32_t first_valid = 0; // (thread 0) of the four segments' first keys
 #pragma unroll
-    for (int step = 0; step < 4; ++step) {
+    for (int step = 0; step < STEPS; ++step) {
       const uint32_t j = key_of(step);
       const bool exists = j < p.S;
       const uint64_t row = row_of(step);
@@ -261,31 +269,33 @@ attention_operands_kernel(const OperandParams p) {
         t[j % kTile] = k22;
         t[kTile + j % kTile] = mask;
         if (mask != 0.0f)
-          masked[step] = 1u;
-        else
-          first_valid |= 1u << step;
+          masked[STEPS == 4 ? step : j % kTile / 32u] = 1u;
+        else if (STEPS == 4)
+          own_first_valid |= 1u << step;
+        else if (j % 32u == 0u)
+          first_valid[j % kTile / 32u] = 1u;
       }
     }
-    __shared__ float warp_max[8];
+    __shared__ float warp_max[32 / STEPS];
     most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most))); // non-negative
     if (lane == 0)
       warp_max[warp] = most;
     __syncthreads();
     if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; ++w)
+      for (int w = 1; w < 32 / STEPS; ++w)
         most = fmaxf(most, warp_max[w]);
       p.tile_bound[((uint64_t)b * p.KV + kvh) * tiles + tile] = most;
-      for (int step = 0; step < 4; ++step)
-        if (masked[step] != 0u && (first_valid >> step & 1u))
-          t[kTile + 32 * step] = -0.0f;
+      for (int segment = 0; segment < 4; ++segment)
+        if (masked[segment] != 0u && (STEPS == 4 ? own_first_valid >> segment & 1u : first_valid[segment]) != 0u)
+          t[kTile + 32 * segment] = -0.0f;
     }
   } else {
-    auto row_of = [&](int step) { return (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * 32u + warp * 4u + (lane >> 3); };
+    auto row_of = [&](int step) { return (uint64_t)(blockIdx.x - p.key_blocks) * 128u + step * kStepRows + warp * 4u + (lane >> 3); };
 #pragma unroll
-    for (int step = 0; step < 4; ++step)
+    for (int step = 0; step < STEPS; ++step)
       request(step, p.q + after + (row_of(step) < p.q_rows ? row_of(step) : 0) * 16, row_of(step) < p.q_rows);
 #pragma unroll
-    for (int step = 0; step < 4; ++step) {
+    for (int step = 0; step < STEPS; ++step) {
       const uint64_t row = row_of(step);
       const bool exists = row < p.q_rows;
       uint4 codes;
@@ -1250,7 +1260,9 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     if (blocks > 0x7fffffffull)
       return fail(kUnsupported, "Attention(INT8): problem too large");
     o.key_blocks = (uint32_t)key_blocks;
-    if (int rc = launch_ahead("attention_operands_kernel launch", attention_operands_kernel, blocks, 256, 0, stream, o))
+    const bool one_round = blocks <= 2ull * (uint64_t)sm_count();
+    if (int rc = launch_ahead("attention_operands_kernel launch", one_round ? attention_operands_kernel<2> : attention_operands_kernel<4>,
+                              blocks, one_round ? 512 : 256, 0, stream, o))
       return rc;
   }
   if (!(source && source->k)) {

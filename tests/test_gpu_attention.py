@@ -483,3 +483,30 @@ def test_attention_items_of_every_batch_head_and_query_block(ops, B, Sq, Sk, H, 
     rest[0, :, :H // KV, 5] = 0.0
     assert torch.equal(ordinary, rest)
     ops.poll_status()
+
+
+@pytest.mark.parametrize("masked", ["none", "first", "segment", "others", "random"])
+def test_operands_of_few_and_of_many_rows_are_the_same(masked):
+    """The operands' kernel takes two rows per lane where all its CTAs are resident at once and four else: one batch entry against the
+    same entry four times, with masked keys on the edges of the key table's segments of 32 (its attention is not split)."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    tokens, heads = 300, 24
+    q, k, v = (torch.randn((1, tokens, heads, 128), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3))
+    valid = torch.ones((1, tokens), dtype=torch.uint8, device="cuda")
+    if masked == "first":
+        valid[:, [0, 32, 160, 256]] = 0
+    elif masked == "segment":
+        valid[:, 64:96] = 0
+    elif masked == "others":
+        valid[:, [1, 31, 63, 95, 127, 130, 299]] = 0
+    elif masked == "random":
+        valid[:, torch.rand(tokens, generator=g, device="cuda") < 0.5] = 0
+    key_valid = None if masked == "none" else valid
+    one = ops.attention(q, k, v, key_valid=key_valid)
+    four = ops.attention(*(t.repeat(4, 1, 1, 1) for t in (q, k, v)), key_valid=None if key_valid is None else valid.repeat(4, 1))
+    torch.cuda.synchronize()
+    ops.poll_status()
+    assert bool(torch.isfinite(one.float()).all())
+    assert all(torch.equal(four[i].view(torch.int16), one[0].view(torch.int16)) for i in range(4))
