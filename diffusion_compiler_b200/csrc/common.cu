@@ -179,6 +179,24 @@ DeviceStatus *device_status_words() {
   return words;
 }
 
+DeviceStatus *device_status_words(cudaStream_t stream) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess)
+    return nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    auto it = g_status_words.find(device);
+    if (it != g_status_words.end())
+      return it->second;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return capture == cudaStreamCaptureStatusNone ? device_status_words() : nullptr;
+}
+
 int poll_device_status(const char *what) {
   DeviceStatus *words = device_status_words();
   if (!words)

@@ -75,6 +75,7 @@ private:
   void *data_ = nullptr;
 };
 DeviceStatus *device_status_words();      // per-device, allocated once
+DeviceStatus *device_status_words(cudaStream_t stream); // the same; nullptr where they are not there yet and `stream` is being captured
 int poll_device_status(const char *what); // copies back, clears, maps to kExecutionError
 
 #ifdef __CUDACC__

@@ -26,6 +26,7 @@
 // 12288 x 3072 64.7 -> 56.5 (all lanes evaluate samples, in doubles only where candidates are close), with input
 // equalisation 94.2 -> 62.6 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
 // copies through shared memory instead of registers gave nothing.
+#include "ptx.cuh"
 #include "quant_common.cuh"
 
 namespace difb200 {
@@ -65,7 +66,8 @@ __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, 
   }
 }
 
-template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB>
+// AHEAD: the next row is rotated before one is finished.
+template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB, bool AHEAD>
 __global__ void __launch_bounds__(MAXT, MINB)
 convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_per_cta) {
   static_assert(EXTRA != kNorm || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
@@ -81,12 +83,24 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   const int total_warps = blockDim.x >> 5;
   const uint32_t smem_addr = smem_u32(smem);
   const uint32_t warp_addr = smem_addr + warp * kWarpBytes;
-  float *red = reinterpret_cast<float *>(smem + total_warps * (kWarpBytes / 4)); // [2][2][total_warps]
+  float *red = reinterpret_cast<float *>(smem + total_warps * (kWarpBytes / 4)); // [2][2][total_warps], AHEAD [4][total_warps]
   const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
   constexpr float kCarry = 16.0f; // the values carried through the rotation are scaled by 2^stages
   const uint32_t columns = p.columns;
   const uint32_t col_warp = (uint32_t)wrow * (NIT * 1024u);
   const uint32_t col0 = col_warp + 512u * h + 16u * a; // this thread's run in the first group of block 0
+
+  // Rows of more than 12 blocks are one CTA per SM, whose 13 to 16 warps a barrier per row would stop together. With AHEAD a warp
+  // announces its maximum (an mbarrier for each of four rows) and looks for the others' when it has rotated its block of the next row.
+  static_assert(!AHEAD || (EXTRA == kPlain && PREFETCH && !F32 && !RESIDUAL && NIT == 1), "");
+  if (AHEAD) {
+    if (threadIdx.x == 0) {
+      for (uint32_t i = 0; i < 4u; ++i)
+        ptx::mbar_init(smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u) + 8u * i, (uint32_t)total_warps);
+      ptx::fence_barrier_init();
+    }
+    __syncthreads();
+  }
 
   // Transpose: thread a writes its 16 pairs as row a and reads pair a of every row j.
   const uint32_t wr_addr = warp_addr + h * kHalfBytes + kRowPitch * a; // + 16 c
@@ -233,10 +247,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   uint4 next[4];
   if (PREFETCH)
     fetch(row, 0, next);
-  uint32_t parity = 0;
-  for (; row < p.rows; row += row_step, parity ^= 1u) {
-    uint64_t PF[F32 ? 16 : 1];        // rotated values of the fp32 variants
-    uint32_t V[F32 ? 1 : 16 * NIT];   // rotated values of the bf16 variants, as bf16 pairs
+  // This warp's part of a row rotated: PF (fp32 variants) or V (bf16 variants, as bf16 pairs), and its largest magnitude.
+  auto rotate_row = [&](uint64_t row, uint64_t(&PF)[F32 ? 16 : 1], uint32_t(&V)[F32 ? 1 : 16 * NIT]) {
     float m = 0.0f;
     float mean = 0.0f, inv = 0.0f;
     if (EXTRA == kNorm) {
@@ -436,16 +448,15 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       }
     }
 
-    // Row maximum: thread -> warp (the bits of a non-negative float order like integers) -> row.
-    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-    float *redp = red + parity * 2 * total_warps;
-    if (NIT == 1 || warps_per_row > 1) {
-      if (lane == 0)
-        redp[warp] = m;
-      row_barrier();
-      m = lane < warps_per_row ? redp[slot * warps_per_row + lane] : 0.0f;
-      m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-    }
+    // (the bits of a non-negative float order like integers)
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+  };
+  auto maximum_of = [&](const float *maxima) { // of the row's warps
+    const float m = lane < warps_per_row ? maxima[lane] : 0.0f;
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+  };
+  // Scale, codes and residual outputs of a row whose largest rotated value is m.
+  auto finish_row = [&](uint64_t row, uint64_t(&PF)[F32 ? 16 : 1], uint32_t(&V)[F32 ? 1 : 16 * NIT], float m, float *redp) {
     const float maximum = m * (1.0f / kCarry);
     float scale = row_scale(maximum, clip);
     if (searches(EXTRA)) {
@@ -695,10 +706,60 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
     }
 #undef DIFB200_STAGE_ALL
 #undef DIFB200_STAGE
+  };
+
+  if constexpr (AHEAD) {
+    const uint32_t bar = smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u);
+    uint64_t PF[1];
+    uint32_t V[2][16];
+    uint64_t before = 0; // the row that is rotated and not finished
+    uint32_t turn = 0;
+    auto step = [&](uint32_t(&mine)[16], uint32_t(&other)[16]) {
+      const bool more = row < p.rows;
+      if (more) {
+        const float m = rotate_row(row, PF, mine);
+        if (lane == 0) {
+          red[(turn & 3u) * total_warps + warp] = m;
+          ptx::mbar_arrive(bar + 8u * (turn & 3u));
+        }
+      }
+      if (turn != 0u) {
+        const uint32_t of = turn - 1u;
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(bar + 8u * (of & 3u), (of >> 2) & 1u, p.wait_ns))) {
+          if (lane == 0 && atomicExch(&p.status->flag, 1u) == 0u) {
+            p.status->kernel = 1u;
+            p.status->role = (uint32_t)warp;
+            p.status->detail = of;
+          }
+          return false;
+        }
+        finish_row(before, PF, other, maximum_of(red + (of & 3u) * total_warps), red);
+      }
+      before = row;
+      row += row_step;
+      ++turn;
+      return more;
+    };
+    while (step(V[0], V[1]) && step(V[1], V[0])) {
+    }
+    return;
+  }
+  for (uint32_t parity = 0; row < p.rows; row += row_step, parity ^= 1u) {
+    uint64_t PF[F32 ? 16 : 1];
+    uint32_t V[F32 ? 1 : 16 * NIT];
+    float m = rotate_row(row, PF, V);
+    float *redp = red + parity * 2 * total_warps;
+    if (NIT == 1 || warps_per_row > 1) {
+      if (lane == 0)
+        redp[warp] = m;
+      row_barrier();
+      m = maximum_of(redp + slot * warps_per_row);
+    }
+    finish_row(row, PF, V, m, redp);
   }
 }
 
-template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB>
+template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB, bool AHEAD = false>
 int launch_form(const QuantParams &p, cudaStream_t stream) {
   const uint32_t groups = p.columns >> 8;
   const int warps_per_row = (int)((groups + 4u * NIT - 1u) / (4u * NIT));
@@ -715,7 +776,7 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
   const int warps = warps_per_row * rows_per_cta, threads = warps * 32;
   const size_t smem = table_offset<SIGNED, EXTRA, NIT>((uint32_t)warps) +
                       (EXTRA == kPackTable ? (size_t)((p.columns + 1023u) >> 10) * kTableBlockBytes : 0);
-  auto kernel = convrot256_kernel<SIGNED, F32, RESIDUAL, EXTRA, NIT, PREFETCH, MAXT, MINB>;
+  auto kernel = convrot256_kernel<SIGNED, F32, RESIDUAL, EXTRA, NIT, PREFETCH, MAXT, MINB, AHEAD>;
   int resident = 1;
   if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), threads, smem, &resident))
     return rc;
@@ -739,6 +800,16 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
 int launch_single(const QuantParams &p, cudaStream_t stream) {
   const uint32_t blocks = ((p.columns >> 8) + 3u) / 4u;
+  // us without / with the next row rotated ahead: 4608 x 15360 55.8 / 54.2, 1000 14.4 / 13.6, 2000 x 16384 27.1 / 25.6, signed 28.8 / 27.4,
+  // 13312 24.6 / 24.6; 200 x 15360 5.5 / 5.5, but 16 rows 3.4 / 3.6. (In fp32 the registers do not hold two rows.)
+  if constexpr (EXTRA == kPlain && !RESIDUAL && !F32)
+    if (blocks > 12u && p.rows > 2ull * (uint64_t)sm_count()) {
+      QuantParams q = p;
+      q.wait_ns = wait_limit_ns();
+      q.status = device_status_words(stream);
+      if (q.status)
+        return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1, true>(q, stream);
+    }
   if (blocks > 12u)
     return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1>(p, stream);
   constexpr bool kArithmetic = EXTRA != kPlain || RESIDUAL;

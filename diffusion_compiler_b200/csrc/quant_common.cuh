@@ -34,6 +34,8 @@ struct QuantParams {
   // into one fused operation (seen as single codes off by one), and an fma with a constant -0 as well; with
   // a -0 it cannot see, the product keeps its own rounding (x + -0 = x for every x, signed zeros included).
   uint64_t minus_zero2;
+  unsigned long long wait_ns; // limit of a bounded wait, and where it is reported
+  DeviceStatus *status;
 };
 
 // The 256-wide variants (2, 3, 5, 6), with or without residual outputs, weight packing or a norm in front.

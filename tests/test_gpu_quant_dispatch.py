@@ -223,3 +223,22 @@ def test_packing_with_a_table_of_reciprocals(impl, rows, width):
         parts = [ops.quantize_weight_rows(w[i:i + 400], impl, mse_scale=True, input_scale=eq) for i in range(0, rows, 400)]
         assert torch.equal(codes, torch.cat([p[0] for p in parts]))
         assert torch.equal(scales.view(torch.int32), torch.cat([p[1] for p in parts]).view(torch.int32))
+
+
+@pytest.mark.parametrize("impl", [2, 3])
+@pytest.mark.parametrize("extra,widths", [(1, [12544]), (5, [3072, 12288]), (449, [16384])])  # rows beyond two per SM
+def test_wide_rows_rotated_one_ahead_of_their_maximum(impl, extra, widths):
+    """Rows of more than 12 blocks, more than two per SM: the next one is rotated before one is finished. Rows are independent: the same
+    as a hundred at a time, which are not taken so; magnitudes that differ from row to row, so that a row's maximum in
+    another's place would show."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    rows = 2 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    rng = np.random.default_rng(rows + impl)
+    parts = [to_torch_bf16(bf16_normal(rng, (rows, w))) * torch.exp2((torch.arange(rows, device="cuda") % 23 - 11).float()).to(torch.bfloat16)[:, None]
+             for w in widths]
+    got = ops.quantize_int8_rows(parts, impl)
+    want = [ops.quantize_int8_rows([p[i:i + 100].contiguous() for p in parts], impl) for i in range(0, rows, 100)]
+    assert torch.equal(got[0], torch.cat([w[0] for w in want]))
+    assert torch.equal(got[1].view(torch.int32), torch.cat([w[1] for w in want]).view(torch.int32))
+    ops.poll_status()
