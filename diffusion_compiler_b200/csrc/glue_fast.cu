@@ -935,13 +935,20 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
     if (int rc = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * (int)warps, warps * warp_bytes, &resident))
       return rc;
     const uint64_t blocks = std::min<uint64_t>((wanted + warps - 1) / warps, sms * resident);
-    return launch_ahead("k_row_squares", kernel, blocks, 32 * (int)warps, warps * warp_bytes, s, p);
+    if (layer || rows <= sms)
+      return launch_ahead("k_row_squares", kernel, blocks, 32 * (int)warps, warps * warp_bytes, s, p);
+    kernel<<<(unsigned)blocks, 32 * warps, warps * warp_bytes, s>>>(p);
+    return launched(cudaGetLastError(), "k_row_squares");
   };
-  // Norm and quantiser, us, sequential / in parts: RMS, 3072 columns, 1 row 12.8 / 6.3, 150 13.2 / 7.7, 1500 23.6 / 16.9, 4700 36.8 / 32.8,
-  // 8318 51.6 / 53.5; 8192 columns, 150 35.4 / 14.9, 4700 92.5 / 88.3, 8318 132 / 151; 4096 columns, 4700 47.9 / 47.5; 1024 columns,
-  // 150 7.8 / 6.8, 600 7.9 / 7.8, 1500 11.7 / 15.6. Of the layer form, whose mean stays a chain, the deviations: 3072 columns, 150
-  // 25.0 / 19.6, 1500 44.1 / 32.4, 4700 59.1 / 52.8, 8318 75.7 / 75.5; 1024 columns, 600 12.5 / 12.5.
-  const bool in_parts = cols % (8 * kSquareParts) == 0 && cols >= 1024 && cols <= 8192 && rows <= (cols >= 2048 ? 32ull : 4ull) * (uint64_t)sm_count();
+  // The statistic is launched plainly. Launched ahead, behind a kernel that lets dependents start (a quantiser, as a rule), its few CTAs
+  // gather on the SMs that have room, and what is bound by a warp's chain takes longer: norm and quantiser from a graph, 5000 x 3072
+  // 33.9 / 38.0 ahead, layer form 48.7 / 60.5, 300 x 12288 43.8 / 61.7; in parts 300 x 3072 9.0 / 12.3, 1500 14.4 / 16.8, but up to a
+  // row per SM 150 8.5 / 7.9. (The second kernel of the layer form follows one that says nothing.)
+  // Norm and quantiser from a graph, us, sequential / in parts: RMS, 3072 columns, 1 row 12.8 / 6.3, 150 14.0 / 7.9, 600 16.0 / 10.4, 1500
+  // 18.9 / 14.4, 3000 25.0 / 22.8, 4700 33.6 / 33.2; 8192 columns, 600 33.6 / 18.7, 3000 62.2 / 62.3, 4700 83.1 / 88.5; 1024 columns, 150
+  // 8.6 / 6.9, 590 8.6 / 8.0. Of the layer form, whose mean stays a chain, the deviations: 3072 columns, 150 26.0 / 19.7, 1500 31.7 / 27.4,
+  // 3000 39.1 / 36.1; 8192 columns, 3000 97.5 / 93.0, 4700 120 / 124; 1024 columns, 590 13.7 / 12.8.
+  const bool in_parts = cols % (8 * kSquareParts) == 0 && cols >= 1024 && cols <= 8192 && rows <= (cols >= 2048 ? 20ull : 4ull) * (uint64_t)sm_count();
   if (in_parts && !layer)
     return squares();
   // Eight chunks in flight where a few warps per SM have to cover the latency alone, four where the rows
@@ -958,7 +965,8 @@ int row_stats(const void *x, uint64_t rows, uint64_t cols, float eps, bool layer
   uint64_t blocks = (warps + kStatWarps - 1) / kStatWarps;
   const uint64_t cap = (uint64_t)sm_count() * resident;
   blocks = blocks > cap ? cap : blocks;
-  if (int rc = launch_ahead("k_row_stats_sequential", kernel, blocks, 32 * kStatWarps, smem, s, X, *stats, rows, (uint32_t)cols, eps))
+  kernel<<<(unsigned)blocks, 32 * kStatWarps, smem, s>>>(X, *stats, rows, (uint32_t)cols, eps);
+  if (int rc = launched(cudaGetLastError(), "k_row_stats_sequential"))
     return rc;
   return in_parts ? squares() : kOk;
 }
