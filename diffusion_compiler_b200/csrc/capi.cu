@@ -28,7 +28,8 @@ int w8a8_linear(const void *x_bf16, const int8_t *w, const float *col_scales, co
   const void *parts[1] = {x_bf16};
   const uint64_t widths[1] = {K};
   if (int rc = quantize_int8_rows(parts, widths, 1, M, implementation, clip, nullptr, codes_scratch,
-                                  scales_scratch, nullptr, nullptr, stream))
+                                  scales_scratch, nullptr, nullptr, stream, false, nullptr, nullptr,
+                                  /*linear_follows=*/true))
     return rc;
   return linear_int8_scaled(codes_scratch, w, scales_scratch, col_scales, bias_bf16, epilogue, M, N, K,
                             out_bf16, nullptr, stream, status_words, /*weights_ready=*/true);
@@ -174,7 +175,7 @@ int difb200_rms_norm_modulate_quant(const void *x, const void *weight, const voi
   const uint64_t widths[1] = {columns};
   const NormPrologue norm{weight, scale, shift, epsilon};
   return quantize_int8_rows(parts, widths, 1, rows, implementation, clip, nullptr, codes, row_scales, nullptr, nullptr,
-                            static_cast<cudaStream_t>(stream), false, nullptr, &norm);
+                            static_cast<cudaStream_t>(stream), false, nullptr, &norm, /*linear_follows=*/true);
 }
 
 int difb200_layer_norm_modulate_quant(const void *x, const void *weight, const void *bias, const void *scale,
@@ -189,7 +190,7 @@ int difb200_layer_norm_modulate_quant(const void *x, const void *weight, const v
   const uint64_t widths[1] = {columns};
   const NormPrologue norm{weight, scale, shift, epsilon, bias, rows_per_modulation};
   return quantize_int8_rows(parts, widths, 1, rows, implementation, clip, nullptr, codes, row_scales, nullptr, nullptr,
-                            static_cast<cudaStream_t>(stream), false, nullptr, &norm);
+                            static_cast<cudaStream_t>(stream), false, nullptr, &norm, /*linear_follows=*/true);
 }
 
 int difb200_quantize_weight_rows(const void *weight, const void *input_scale, uint64_t rows, uint64_t columns,

@@ -74,7 +74,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
   const uint64_t after = grid_dependency_wait_zero(); // in the address of every load
-  grid_dependents_launch();
+  if (p.linear_follows || p.rows <= (uint64_t)gridDim.x * rows_per_cta)
+    grid_dependents_launch();
   constexpr bool kEqualised = equalises(EXTRA), kTable = EXTRA == kPackTable, kFlips = SIGNED && !kTable;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = warp / warps_per_row;         // which row of this CTA's batch

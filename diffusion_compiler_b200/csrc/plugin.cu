@@ -932,7 +932,7 @@ void run_steps(Executable &exe, Overlap *overlap = nullptr) {
         require(quantize_int8_rows(&part, &width, 1, T(norm.in[0]).rows(), (int)op.u64(ir::Implementation, 1),
                                    (float)op.f64(ir::Scale, 1.0), nullptr, static_cast<int8_t *>(D(op.out[0])),
                                    static_cast<float *>(D(op.out[1])), nullptr, nullptr, s, false, nullptr,
-                                   &prologue));
+                                   &prologue, /*linear_follows=*/true));
         break;
       }
       const bool dynamic = T(op.in.back()).dtype == ir::F32;
@@ -949,7 +949,8 @@ void run_steps(Executable &exe, Overlap *overlap = nullptr) {
                                  dynamic ? static_cast<const float *>(D(op.in.back())) : nullptr,
                                  static_cast<int8_t *>(D(op.out[0])), static_cast<float *>(D(op.out[1])),
                                  residual ? static_cast<int8_t *>(D(op.out[2])) : nullptr,
-                                 residual ? static_cast<float *>(D(op.out[3])) : nullptr, s));
+                                 residual ? static_cast<float *>(D(op.out[3])) : nullptr, s, false, nullptr, nullptr,
+                                 position + 1 < exe.order.size() && exe.steps[exe.order[position + 1]].op->opcode == ir::LinearInt8Scaled));
       break;
     }
     case ir::LinearInt8Scaled: {

@@ -34,6 +34,7 @@ struct QuantParams {
   // into one fused operation (seen as single codes off by one), and an fma with a constant -0 as well; with
   // a -0 it cannot see, the product keeps its own rounding (x + -0 = x for every x, signed zeros included).
   uint64_t minus_zero2;
+  uint32_t linear_follows; // the next kernel may start at once: a GEMM, which has its set-up (and weights) to do meanwhile
   unsigned long long wait_ns; // limit of a bounded wait, and where it is reported
   DeviceStatus *status;
 };
