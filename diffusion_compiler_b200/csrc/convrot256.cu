@@ -37,9 +37,11 @@ constexpr int kWarpBytes = kWarpBytes256;
 constexpr uint32_t kCodeHalfBytes = 544, kCodeBytes = 2 * kCodeHalfBytes; // code pairs of a half-warp's two groups, of a block
 
 // kPack: weight rows with the scale search, kEqualise: with input equalisation, kPackEqualise: with both, kPackTable: with both
-// and a table of the equalisation's reciprocals.
-enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3, kPackEqualise = 4, kPackTable = 5 };
+// and a table of the equalisation's reciprocals. kNorm: RmsNormModulate in front, kLayer: LayerNormModulate (one kernel that looked
+// at its parameters for which it is took 473 us for 33272 x 8192 in the RMS form, 449 so, 8318 x 3072 49.2 and 47.2).
+enum Extra { kPlain = 0, kPack = 1, kNorm = 2, kEqualise = 3, kPackEqualise = 4, kPackTable = 5, kLayer = 6 };
 __host__ __device__ constexpr bool searches(int extra) { return extra == kPack || extra == kPackEqualise || extra == kPackTable; }
+__host__ __device__ constexpr bool norms(int extra) { return extra == kNorm || extra == kLayer; }
 __host__ __device__ constexpr bool equalises(int extra) { return extra == kEqualise || extra == kPackEqualise || extra == kPackTable; }
 
 // Shared memory of a CTA: per warp the transpose / staging area and the row maxima; for the signed variants 16 XOR masks per
@@ -70,7 +72,7 @@ __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, 
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA, int NIT, bool PREFETCH, int MAXT, int MINB, bool AHEAD>
 __global__ void __launch_bounds__(MAXT, MINB)
 convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_per_cta) {
-  static_assert(EXTRA != kNorm || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
+  static_assert(!norms(EXTRA) || NIT == 1, "the row's barrier separates reading its statistic from writing its codes");
   static_assert(!F32 || NIT == 1, "the fp32 variants keep fp32 values: one block per warp");
   extern __shared__ __align__(128) uint32_t smem[];
   const uint64_t after = grid_dependency_wait_zero(); // in the address of every load
@@ -248,11 +250,14 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   uint4 next[4];
   if (PREFETCH)
     fetch(row, 0, next);
+  auto modulation_of = [&](uint64_t row) -> uint64_t {
+    return p.norm_mod.by ? p.norm_mod.quotient((uint32_t)row) : row / p.norm_rows_per_mod;
+  };
   // This warp's part of a row rotated: PF (fp32 variants) or V (bf16 variants, as bf16 pairs), and its largest magnitude.
   auto rotate_row = [&](uint64_t row, uint64_t(&PF)[F32 ? 16 : 1], uint32_t(&V)[F32 ? 1 : 16 * NIT]) {
     float m = 0.0f;
     float mean = 0.0f, inv = 0.0f;
-    if (EXTRA == kNorm) {
+    if (norms(EXTRA)) {
       // stands where this row's codes go: written behind the barrier of the row maximum, when all its warps have read it
       const float2 st = glue::row_stat(p.norm_stats, row);
       mean = st.x;
@@ -275,12 +280,13 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
         }
         const uint32_t c = col0 + 1024u * it;
         const bool act_a = c < columns, act_b = c + 256u < columns;
-        if (EXTRA == kNorm) {
+        if (norms(EXTRA)) {
           // The norm in front (reference cpu_executor.cpp:1241-1264 RmsNormModulate, :1108-1148
           // LayerNormModulate): the words are replaced by the bf16 result the unfused op would have
           // stored, rounding for rounding, two groups per packed operation.
-          const uint64_t at = (row / p.norm_rows_per_mod) * (uint64_t)columns + c + after;
-          const bool layer = p.norm_bias != nullptr, weighted = p.norm_weight != nullptr;
+          const uint64_t at = modulation_of(row) * columns + c + after;
+          constexpr bool layer = EXTRA == kLayer;
+          const bool weighted = p.norm_weight != nullptr;
           auto product = [&](uint64_t u, uint64_t v) { return fma2(u, v, p.minus_zero2); };
           const uint64_t inv2 = pack2(inv, inv), mean2 = pack2(mean, mean), one2 = pack2(1.0f, 1.0f);
 #pragma unroll
@@ -796,7 +802,7 @@ int launch_form(const QuantParams &p, cudaStream_t stream) {
 //   fp32 106.5 / 112.1 / 111.5 (8192), but 13.0 / 13.1 / 12.3 (4159 x 3072). Three blocks per warp, which save per-row work, were
 //   the best form before the codes were converted in pairs, and are no longer (9216 x 3072 23.2, now 21.5).
 // Signed rows that are all resident at once want the shortest path (333 x 3072 4.1 / 4.4 / 4.4).
-// A norm in front needs its registers for three tensors in flight (33272 x 3072 198 / 186 / 174), residual outputs
+// A norm in front needs its registers for three tensors in flight (33272 x 3072 176 / 189 / 168), residual outputs
 // are arithmetic (4000 x 8192 46.8 / 43.0 / 41.6).
 template <bool SIGNED, bool F32, bool RESIDUAL, int EXTRA>
 int launch_single(const QuantParams &p, cudaStream_t stream) {
@@ -869,14 +875,14 @@ int launch_variant(const QuantParams &p, bool f32, cudaStream_t stream) {
     if (pack)
       return launch_single<SIGNED, true, false, kPack>(p, stream);
     if (norm)
-      return launch_single<SIGNED, true, false, kNorm>(p, stream);
+      return p.norm_bias ? launch_single<SIGNED, true, false, kLayer>(p, stream) : launch_single<SIGNED, true, false, kNorm>(p, stream);
     return p.rcodes ? launch_single<SIGNED, true, true, kPlain>(p, stream)
                     : launch_single<SIGNED, true, false, kPlain>(p, stream);
   }
   if (p.rcodes)
     return launch_single<SIGNED, false, true, kPlain>(p, stream);
   if (norm)
-    return launch_single<SIGNED, false, false, kNorm>(p, stream);
+    return p.norm_bias ? launch_single<SIGNED, false, false, kLayer>(p, stream) : launch_single<SIGNED, false, false, kNorm>(p, stream);
   if (pack)
     return three ? launch_form<SIGNED, false, false, kPack, 3, false, 256, 2>(p, stream) : launch_single<SIGNED, false, false, kPack>(p, stream);
   return launch_single<SIGNED, false, false, kPlain>(p, stream);

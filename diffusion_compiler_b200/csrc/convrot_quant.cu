@@ -421,6 +421,8 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
     p.norm_bias = static_cast<const uint16_t *>(norm->bias);
     p.minus_zero2 = 0x8000000080000000ull;
     p.norm_rows_per_mod = norm->rows_per_modulation;
+    if (rows < (1ull << 31) && norm->rows_per_modulation < (1ull << 31))
+      p.norm_mod = divisor(norm->rows_per_modulation);
   }
   if (rows == 0)
     return kOk;

@@ -29,6 +29,7 @@ struct QuantParams {
   const uint16_t *norm_shift;  // [rows, columns]
   const uint16_t *norm_bias;   // [columns]: LayerNormModulate (mean removed, weight and bias); nullptr = RMS
   uint64_t norm_rows_per_mod;  // rows that share one row of scale / shift
+  Divisor norm_mod;            // by their number, where rows and it are below 2^31 (else 0)
   glue::RowStats norm_stats;   // per row (mean, inverse deviation)
   // Two fp32 -0, added to products of the norm. The assembler contracts mul.rn.f32x2 followed by add.rn.f32x2
   // into one fused operation (seen as single codes off by one), and an fma with a constant -0 as well; with

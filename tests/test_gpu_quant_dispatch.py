@@ -176,6 +176,22 @@ def test_layer_norm_prologue_of_rows_with_a_large_mean(K, impl):
     assert torch.equal(want[1], got[1]) and torch.equal(want[0], got[0])
 
 
+@pytest.mark.parametrize("impl", [2, 3, 5])
+@pytest.mark.parametrize("rows_per_modulation", [1, 2, 3, 7, 84, 1302, 20832])
+def test_layer_norm_prologue_finds_the_modulation_of_a_row(rows_per_modulation, impl):
+    """Scale and shift that several rows share: the bits of the same ones given row by row."""
+    import torch
+    from diffusion_compiler_b200 import ops
+    rng = np.random.default_rng(rows_per_modulation + impl)
+    t = lambda *shape, std=1.0: to_torch_bf16(bf16_normal(rng, shape, std))  # noqa: E731
+    rows, K = 20832, 256
+    x, w, b = t(rows, K), t(K), t(K, std=0.1)
+    mods = [t(rows // rows_per_modulation, K, std=0.3) for _ in range(2)]
+    got = ops.layer_norm_modulate_quant(x, w, b, *mods, 1e-6, impl)
+    want = ops.layer_norm_modulate_quant(x, w, b, *[m.repeat_interleave(rows_per_modulation, 0) for m in mods], 1e-6, impl)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
 @pytest.mark.parametrize("impl", [2, 3])
 @pytest.mark.parametrize("K", [256, 3072, 9216])
 def test_quotients_out_of_the_two_part_products_range(impl, K):
