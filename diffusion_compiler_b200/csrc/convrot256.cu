@@ -22,10 +22,11 @@
 // values), half the registers of fp32. The codes of a pair are made by one conversion and leave as 16 bits; as a
 // conversion and a byte store per element they kept the quarter-rate unit busy for 256 clocks of a block, and a warp took three
 // blocks at a time to save per-row work. Before -> now, us: 33272 x 3072 83.9 -> 71.8 (4.3 TB/s), 33272 x 8192 220.6 -> 181.7,
-// 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 55.4, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
+// 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 54.2, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
 // 12288 x 3072 64.7 -> 56.5 (all lanes evaluate samples, in doubles only where candidates are close), with input
-// equalisation 94.2 -> 62.6 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 87.9 with its statistic. Staging the input with bulk
-// copies through shared memory instead of registers gave nothing.
+// equalisation 94.2 -> 62.6 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 85.3 with its
+// statistic. Staging the input with bulk copies through shared memory instead of registers gave nothing, nor (3 to 8 % slower) did
+// scale and shift of a norm's next row prefetched into L2.
 #include "ptx.cuh"
 #include "quant_common.cuh"
 

@@ -11,9 +11,9 @@
 // The smallest problems are one launch: every CTA rotates and quantises the rows itself, while its weights are on their way. It
 // is launched ahead and waits at its start: the time between two kernels, not their work, was a third of a call (2 x 3072 x 3072,
 // calls one behind the other, weights not in L2: 8.0 us launched plainly, 5.4 so).
-// That costs a CTA about 1.5 us and saves a launch, 3 us of the host. 2 x 3072 x 3072, one launch / two / the tile kernel and a
-// quantiser, us per call of calls one behind the other: weights in L2 6.7 / 8.0 / 12.3, not in L2 8.2 / 8.0 / 12.3, of these the
-// host 5.1 / 8.0 / 8.5; from a graph, not in L2, 6.2 / 5.4 / 11.0.
+// That costs a CTA about 1.5 us and saves a launch, 3 us of the host. 2 x 3072 x 3072 from a graph, weights not in L2, all launched
+// plainly, one launch / two / the tile kernel and a quantiser: 6.2 / 5.4 / 11.0 us, of the host 5.1 / 8.0 / 8.5. Launched ahead: one
+// 4.9, the two of 4 rows 4.8.
 #include "gemm_common.cuh"
 #include "ops.h"
 #include "quant_common.cuh"
