@@ -1,5 +1,5 @@
 // QuantizeInt8Rows for sm_100a: the entry point, the 4096-wide ConvRot variants and the Direct variant
-// (the 256-wide variants are in convrot256.cu). Semantics follow the reference opcode bit for bit
+// (the 256-wide variants are in convrot256.cuh). Semantics follow the reference opcode bit for bit
 // (reference src/runtime/cpu_executor.cpp:124-307; generated GPU kernel src/compiler/compiler.cpp:635-845).
 #include "glue.h"
 #include "ops.h"
@@ -37,7 +37,7 @@ convrot4096_kernel(const QuantParams p) {
   constexpr float kCarry = 64.0f; // the values carried through the rotation are scaled by 2^stages
   const uint32_t columns = p.columns, col0 = 1024u * warp + 512u * h + 16u * a;
 
-  // transpose addressing inside a group: see convrot256.cu
+  // transpose addressing inside a group: see convrot256.cuh
   const uint32_t half_addr = warp_addr + h * 2048u;
   const uint32_t wr_addr = half_addr + 128u * a + ((a & 7u) << 4);
   const uint32_t rd_addr = half_addr + ((uint32_t)(a >> 1) << 4) + 8u * (a & 1u);

@@ -42,6 +42,7 @@ struct QuantParams {
 
 // The 256-wide variants (2, 3, 5, 6), with or without residual outputs, weight packing or a norm in front.
 int launch_convrot256(const QuantParams &p, int implementation, cudaStream_t stream);
+int launch_convrot256_pack(const QuantParams &p, bool is_signed, bool f32, cudaStream_t stream);
 
 #ifdef __CUDACC__
 
@@ -268,7 +269,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   return v;
 }
 
-// ---- 256-wide rotation: a warp's 1024 columns, 16 packed pairs per thread (layout: convrot256.cu) ----
+// ---- 256-wide rotation: a warp's 1024 columns, 16 packed pairs per thread (layout: convrot256.cuh) ----
 // Shared memory per warp: 4 groups x 256 fp32, two 16x32-word transposes whose rows are padded, so that every access is
 // free of conflicts at a constant offset.
 constexpr uint32_t kRowPitch = 144;             // bytes of a row of 16 pairs in the transpose
