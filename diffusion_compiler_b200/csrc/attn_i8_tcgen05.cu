@@ -1183,7 +1183,7 @@ int attention_int8(const int8_t *q8, const float *qs, const int8_t *k8, const fl
     return fail(kUnsupported, "Attention(INT8): pointers must be 16-byte aligned");
   DeviceStatus *status = device_status_words();
   if (!status)
-    return fail(kOutOfMemory, "Attention(INT8): cannot allocate device status words");
+    return fail(kOutOfMemory, "Attention(INT8): device status words are unavailable");
   const uint32_t s_pad = (uint32_t)((S + kTile - 1) / kTile * kTile);
   const uint32_t all_tiles = s_pad / kTile;
   uint32_t begin[2] = {0, 0}, count[2] = {all_tiles, 0};

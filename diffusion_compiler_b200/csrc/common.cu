@@ -163,6 +163,12 @@ StreamScratch::~StreamScratch() {
     cudaFreeAsync(data_, stream_);
 }
 
+namespace {
+// Zero from the start, and there with the device's copy of this code: a call that first needs the words allocates nothing, waits for
+// nothing, and may stand beside a stream capture (of its own stream or of another thread).
+__device__ DeviceStatus g_status_storage;
+} // namespace
+
 DeviceStatus *device_status_words() {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess)
@@ -171,30 +177,12 @@ DeviceStatus *device_status_words() {
   auto it = g_status_words.find(device);
   if (it != g_status_words.end())
     return it->second;
-  DeviceStatus *words = nullptr;
-  if (cudaMalloc(&words, sizeof(DeviceStatus)) != cudaSuccess)
-    return nullptr;
-  cudaMemset(words, 0, sizeof(DeviceStatus));
-  g_status_words[device] = words;
-  return words;
-}
-
-DeviceStatus *device_status_words(cudaStream_t stream) {
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess)
-    return nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    auto it = g_status_words.find(device);
-    if (it != g_status_words.end())
-      return it->second;
-  }
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
-    cudaGetLastError();
+  void *words = nullptr;
+  if (cudaGetSymbolAddress(&words, g_status_storage) != cudaSuccess) {
+    cudaGetLastError(); // the caller reports it; a later launch must not
     return nullptr;
   }
-  return capture == cudaStreamCaptureStatusNone ? device_status_words() : nullptr;
+  return g_status_words[device] = static_cast<DeviceStatus *>(words);
 }
 
 int poll_device_status(const char *what) {

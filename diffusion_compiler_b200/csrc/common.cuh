@@ -74,8 +74,7 @@ private:
   cudaStream_t stream_;
   void *data_ = nullptr;
 };
-DeviceStatus *device_status_words();      // per-device, allocated once
-DeviceStatus *device_status_words(cudaStream_t stream); // the same; nullptr where they are not there yet and `stream` is being captured
+DeviceStatus *device_status_words();      // per device, part of the library's image
 int poll_device_status(const char *what); // copies back, clears, maps to kExecutionError
 
 #ifdef __CUDACC__

@@ -815,7 +815,7 @@ int launch_single(const QuantParams &p, cudaStream_t stream) {
     if (blocks > 12u && p.rows > 2ull * (uint64_t)sm_count()) {
       QuantParams q = p;
       q.wait_ns = wait_limit_ns();
-      q.status = device_status_words(stream);
+      q.status = device_status_words();
       if (q.status)
         return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1, true>(q, stream);
     }

@@ -630,7 +630,7 @@ int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales
     return fail(kUnsupported, "LinearInt8Scaled: operands must be 16-byte aligned");
   DeviceStatus *status = status_words ? status_words : device_status_words();
   if (!status)
-    return fail(kOutOfMemory, "LinearInt8Scaled: cannot allocate device status words");
+    return fail(kOutOfMemory, "LinearInt8Scaled: device status words are unavailable");
 
   GemmParams p{};
   p.row_scales = row_scales;

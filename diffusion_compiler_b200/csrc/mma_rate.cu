@@ -86,7 +86,7 @@ int run_rate(uint32_t n_mma, double *tops, double *milliseconds, cudaStream_t st
     return rc;
   DeviceStatus *status = device_status_words();
   if (!status)
-    return fail(kOutOfMemory, "cannot allocate device status words");
+    return fail(kOutOfMemory, "device status words are unavailable");
   cudaLaunchConfig_t config{};
   config.blockDim = dim3(128);
   config.dynamicSmemBytes = kRateSmem;

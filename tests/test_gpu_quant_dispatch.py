@@ -258,3 +258,55 @@ def test_wide_rows_rotated_one_ahead_of_their_maximum(impl, extra, widths):
     assert torch.equal(got[0], torch.cat([w[0] for w in want]))
     assert torch.equal(got[1].view(torch.int32), torch.cat([w[1] for w in want]).view(torch.int32))
     ops.poll_status()
+
+
+_FIRST_CALL = """
+import ctypes as C, threading
+import torch
+from diffusion_compiler_b200 import _lib, ops
+rows = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 7
+g = torch.Generator(device="cuda").manual_seed(1)
+x = torch.randn((rows, 12544), generator=g, device="cuda").to(torch.bfloat16)
+out = torch.zeros(x.shape, dtype=torch.int8, device="cuda"), torch.zeros(rows, device="cuda")
+f = torch.randn((4, 64), generator=g, device="cuda")
+gated, base = torch.zeros_like(f), torch.ones(8, device="cuda")
+side, errors = torch.cuda.Stream(), []
+torch.cuda.synchronize()
+
+def work():
+    try:
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(side):
+            ops.quantize_int8_rows([x], 2, out=out)
+        p = lambda t: C.c_void_p(t.data_ptr())  # a kernel whose launch is checked by the thread's last error
+        _lib.check(_lib.lib().difb200_residual_gate(p(f), p(f), p(f), p(gated), 1, 4, 64, 4, C.c_void_p(side.cuda_stream)))
+    except Exception as e:
+        errors.append(e)
+
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):  # (a capture in global mode: it ends where any thread allocates)
+    y = base + 1
+    thread = threading.Thread(target=work)
+    thread.start()
+    thread.join()
+    z = y * 3
+assert not errors, errors
+graph.replay()
+torch.cuda.synchronize()
+assert bool((z == 6).all()) and torch.allclose(gated, f + f * f)
+parts = [ops.quantize_int8_rows([x[i:i + 100]], 2) for i in range(0, rows, 100)]
+assert torch.equal(out[0], torch.cat([q[0] for q in parts])) and torch.equal(out[1], torch.cat([q[1] for q in parts]))
+ops.poll_status()
+print("same codes")
+"""
+
+
+def test_first_quantiser_call_of_a_process_beside_a_capture():
+    """A quantiser has no scratch: its first call on wide rows allocates nothing, so a capture on another thread stays valid, and
+    no error is left behind for the thread's next launch."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", _FIRST_CALL], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and "same codes" in run.stdout, run.stderr[-2000:]
