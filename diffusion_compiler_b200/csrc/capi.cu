@@ -29,7 +29,7 @@ int w8a8_linear(const void *x_bf16, const int8_t *w, const float *col_scales, co
   const uint64_t widths[1] = {K};
   if (int rc = quantize_int8_rows(parts, widths, 1, M, implementation, clip, nullptr, codes_scratch,
                                   scales_scratch, nullptr, nullptr, stream, false, nullptr, nullptr,
-                                  /*linear_follows=*/true))
+                                  /*linear_follows=*/true, status_words))
     return rc;
   return linear_int8_scaled(codes_scratch, w, scales_scratch, col_scales, bias_bf16, epilogue, M, N, K,
                             out_bf16, nullptr, stream, status_words, /*weights_ready=*/true);
@@ -105,6 +105,8 @@ int difb200_poll_status(void) {
 void difb200_set_wait_limit_ns(uint64_t nanoseconds) { set_wait_limit_ns(nanoseconds); }
 
 void difb200_test_withhold_gemm_load(uint32_t k_block) { withhold_next_gemm_load(k_block); }
+
+void difb200_test_withhold_row_maximum(uint64_t limit_ns) { withhold_next_row_maximum(limit_ns); }
 
 int difb200_program_check(const uint8_t *diffir, uint64_t size) {
   ir::Program program;

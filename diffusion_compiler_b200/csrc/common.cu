@@ -23,12 +23,15 @@ std::map<std::pair<const void *, int>, int> g_once_values;
 namespace {
 std::atomic<unsigned long long> g_wait_limit_ns{1500ull * 1000ull * 1000ull};
 std::atomic<uint32_t> g_withhold_kb{0xffffffffu};
+std::atomic<unsigned long long> g_withheld_maximum_ns{0};
 } // namespace
 
 unsigned long long wait_limit_ns() { return g_wait_limit_ns.load(); }
 void set_wait_limit_ns(unsigned long long ns) { g_wait_limit_ns.store(ns ? ns : 1500ull * 1000ull * 1000ull); }
 void withhold_next_gemm_load(uint32_t k_block) { g_withhold_kb.store(k_block); }
 bool gemm_load_is_withheld() { return g_withhold_kb.load() != 0xffffffffu; }
+void withhold_next_row_maximum(unsigned long long limit_ns) { g_withheld_maximum_ns.store(limit_ns); }
+unsigned long long take_withheld_row_maximum() { return g_withheld_maximum_ns.exchange(0); }
 uint32_t take_withheld_gemm_load() { return g_withhold_kb.exchange(0xffffffffu); }
 
 int per_device_once(const void *key, int device, int (*init)(void *arg, int *value), void *arg, int *value) {

@@ -57,6 +57,10 @@ void set_wait_limit_ns(unsigned long long ns); // 0 restores the default
 void withhold_next_gemm_load(uint32_t k_block);
 uint32_t take_withheld_gemm_load();
 bool gemm_load_is_withheld();
+// The same for the quantiser of rows that are rotated one ahead of their maximum: a CTA of the next such launch waits for one
+// announcement more of a row than its warps make, and the launch's waits have this limit. take_...() returns it (0 = not armed) and disarms.
+void withhold_next_row_maximum(unsigned long long limit_ns);
+unsigned long long take_withheld_row_maximum();
 // Device memory for one call: allocated and freed in the order of the call's stream, so that neither
 // another stream nor another thread can hold the same bytes meanwhile (also under stream capture, where the two become
 // nodes of the graph). It comes from a pool of this library that keeps at most 4 MB per device across

@@ -101,7 +101,8 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   if (AHEAD) {
     if (threadIdx.x == 0) {
       for (uint32_t i = 0; i < 4u; ++i)
-        ptx::mbar_init(smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u) + 8u * i, (uint32_t)total_warps);
+        ptx::mbar_init(smem_addr + (uint32_t)total_warps * (kWarpBytes + 16u) + 8u * i,
+                       (uint32_t)total_warps + (p.withhold != 0u && blockIdx.x == 0u && i == 1u ? 1u : 0u));
       ptx::fence_barrier_init();
     }
     __syncthreads();
@@ -814,8 +815,11 @@ int launch_single(const QuantParams &p, cudaStream_t stream) {
   if constexpr (EXTRA == kPlain && !RESIDUAL && !F32)
     if (blocks > 12u && p.rows > 2ull * (uint64_t)sm_count()) {
       QuantParams q = p;
-      q.wait_ns = wait_limit_ns();
-      q.status = device_status_words();
+      if (!q.status)
+        q.status = device_status_words();
+      const unsigned long long withheld = take_withheld_row_maximum();
+      q.withhold = withheld != 0 ? 1u : 0u;
+      q.wait_ns = withheld != 0 ? withheld : wait_limit_ns();
       if (q.status)
         return launch_form<SIGNED, F32, RESIDUAL, EXTRA, 1, true, 512, 1, true>(q, stream);
     }

@@ -371,7 +371,7 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
                        uint64_t rows, int implementation, float clip, const float *clip_device,
                        int8_t *codes, float *scales, int8_t *rcodes, float *rscales,
                        cudaStream_t stream, bool mse_weight_scale, const void *equalise_bf16,
-                       const NormPrologue *norm, bool linear_follows) {
+                       const NormPrologue *norm, bool linear_follows, DeviceStatus *status_words) {
   if (part_count == 0 || part_count > kMaxParts)
     return fail(kUnsupported, "QuantizeInt8Rows: 1..8 concatenated inputs are supported");
   if (!codes || !scales || (rcodes == nullptr) != (rscales == nullptr))
@@ -404,6 +404,7 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
   p.rcodes = rcodes;
   p.rscales = rscales;
   p.linear_follows = linear_follows ? 1u : 0u;
+  p.status = status_words;
   p.mse = mse_weight_scale ? 1u : 0u;
   p.equalise = static_cast<const uint16_t *>(equalise_bf16);
   if (norm) {

@@ -26,11 +26,12 @@ int quantize_int8_rows(const void *const *parts, const uint64_t *part_widths, ui
                        uint64_t rows, int implementation, float clip, const float *clip_device,
                        int8_t *codes, float *scales, int8_t *rcodes, float *rscales,
                        cudaStream_t stream, bool mse_weight_scale = false, const void *equalise_bf16 = nullptr,
-                       const NormPrologue *norm = nullptr, bool linear_follows = false);
+                       const NormPrologue *norm = nullptr, bool linear_follows = false, DeviceStatus *status_words = nullptr);
 // linear_follows: the next launch is a LinearInt8Scaled, which may start at once, as any kernel may behind a 256-wide
 // quantiser with one row (or batch of rows) per CTA. Else the next one's CTAs would be placed as SMs happen to be free
 // instead of evenly: quantisers one behind the other, from a graph, 700 x 12288 8.2 us, 9.2 so, 4159 x 3072 Direct 16.5
 // and 20.0.
+// status_words: where a wait that runs out is reported (default: the device's).
 
 int linear_int8_scaled(const int8_t *x, const int8_t *w, const float *row_scales,
                        const float *col_scales, const void *bias_bf16, uint32_t epilogue, uint64_t M,

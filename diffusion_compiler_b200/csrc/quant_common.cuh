@@ -38,6 +38,7 @@ struct QuantParams {
   uint32_t linear_follows; // the next kernel may start at once: a GEMM, which has its set-up (and weights) to do meanwhile
   unsigned long long wait_ns; // limit of a bounded wait, and where it is reported
   DeviceStatus *status;
+  uint32_t withhold; // test aid: the first CTA waits for one announcement more of its second row than its warps make
 };
 
 // The 256-wide variants (2, 3, 5, 6), with or without residual outputs, weight packing or a norm in front.

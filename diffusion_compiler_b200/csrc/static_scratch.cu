@@ -7,7 +7,7 @@
 // where an allocation would synchronise the device, or a plugin whose owner wants a hard
 // guarantee that loading a model never grows the process's footprint. For them this file keeps
 // the scratch that the two-kernel W8A8 linear needs (the INT8 activation codes, the per-row
-// scales and the status words of the GEMM's bounded waits) in a fixed array that is part of
+// scales and the status words of the kernels' bounded waits) in a fixed array that is part of
 // the library image.
 //
 // Cost and limits: every GPU on which the library's device code is loaded holds

@@ -61,6 +61,13 @@ DIFB200_EXPORT void difb200_set_wait_limit_ns(uint64_t nanoseconds);
 DIFB200_EXPORT void difb200_test_withhold_gemm_load(uint32_t k_block);
 
 /*
+ * The same for the quantiser of more than 12288 columns and two rows per SM, whose warps tell one another a row's maximum: in the
+ * next such launch one row waits for one word more than is said, and that launch's waits (no other's) give up after
+ * `limit_ns`. The codes of a few rows are undefined.
+ */
+DIFB200_EXPORT void difb200_test_withhold_row_maximum(uint64_t limit_ns);
+
+/*
  * Host-only self-check of the library's per-device bookkeeping (one-time set-up keyed by device
  * ordinal, wait-limit state). Touches no GPU; returns 0 when the invariants hold.
  */
@@ -361,7 +368,7 @@ DIFB200_EXPORT int difb200_w8a8_linear(const void *x, const int8_t *w, const flo
 /*
  * difb200_w8a8_linear with no allocation anywhere (no counterpart in the reference).
  * Same computation and arguments as difb200_w8a8_linear, but the activation codes, row scales
- * and the GEMM's status words live in a fixed 40 MiB array inside the library instead of
+ * and the kernels' status words live in a fixed 40 MiB array inside the library instead of
  * caller scratch, and neither this call nor anything it runs calls cudaMalloc/cudaFree. It is
  * for hosts that planned their device memory up front or must not trigger an allocation while
  * they run a layer. A call needs 256 + roundup(4*M, 256) + M*K bytes; larger problems are
