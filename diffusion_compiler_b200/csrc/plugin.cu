@@ -750,11 +750,12 @@ void allocate(Executable &exe) {
 // became final.
 // A last step that works on rows, its own Input and an Output of page-locked host memory: the Input comes in, the step runs and the
 // Output leaves a block of rows at a time, so that the two copy directions run side by side. (Else the whole Output follows the whole
-// Input: 14552 tokens of the video block 13.4 ms, so 12.8: it starts to leave when the step in front is done.)
+// Input: 14552 tokens of the video block 13.4 ms, so 12.8: it starts to leave when the step in front is done.) The Input comes last,
+// after Outputs of other steps may have left: not where its host array has bytes in common with an Output's.
 struct Tail {
   static constexpr uint64_t kMost = 16, kLeastBytes = 4u << 20;
   int step = -1, input = -1, output = -1; // tensors by index
-  size_t input_view = 0, output_view = 0;
+  size_t input_view = 0;
   uint64_t rows = 0, pieces = 0, row_bytes = 0;
   uint64_t first(uint64_t piece) const { return rows * piece / pieces; }
 };
@@ -777,7 +778,7 @@ bool page_locked(const void *data, uint64_t bytes) {
 }
 // ResidualGate with a gate per row, the last step that runs, whose gate is an Input of its own.
 Tail find_tail(const Executable &exe, const dif_backend_tensor_view *inputs, size_t input_count, const dif_backend_tensor_view *outputs,
-               const std::vector<int> &out_view_of) {
+               size_t output_count, const std::vector<int> &out_view_of) {
   Tail tail;
   const ir::Program &p = exe.program;
   size_t last = exe.order.size();
@@ -800,18 +801,27 @@ Tail find_tail(const Executable &exe, const dif_backend_tensor_view *inputs, siz
     if (uses > (&other == &st ? 1u : 0u) || other.bias_tensor == in || other.mask_tensor == in)
       return tail;
   }
-  size_t view = 0;
-  while (view < input_count && p.index_of(inputs[view].tensor_id) != in)
-    ++view;
+  size_t view = input_count;
+  for (size_t i = 0; i < input_count; ++i)
+    if (p.index_of(inputs[i].tensor_id) == in) {
+      if (view != input_count) // given twice: the last one counts
+        return tail;
+      view = i;
+    }
   const uint64_t pieces = std::min({Tail::kMost, (uint64_t)gate.bytes() / Tail::kLeastBytes, (uint64_t)gate.rows()});
   if (view == input_count || pieces < 2 || inputs[view].byte_count != gate.bytes() || !inputs[view].host_data ||
       !page_locked(inputs[view].host_data, gate.bytes()) || !page_locked(outputs[out_view_of[(size_t)out]].host_data, result.bytes()))
     return tail;
+  const uintptr_t from = reinterpret_cast<uintptr_t>(inputs[view].host_data);
+  for (size_t i = 0; i < output_count; ++i) {
+    const uintptr_t to = reinterpret_cast<uintptr_t>(outputs[i].host_data);
+    if (to < from + inputs[view].byte_count && from < to + outputs[i].byte_count)
+      return tail;
+  }
   tail.step = (int)exe.order[last - 1];
   tail.input = in;
   tail.output = out;
   tail.input_view = view;
-  tail.output_view = (size_t)out_view_of[(size_t)out];
   tail.rows = gate.rows();
   tail.pieces = pieces;
   tail.row_bytes = gate.bytes() / gate.rows();
@@ -1470,7 +1480,7 @@ dif_backend_status execute(dif_backend_executable executable, const dif_backend_
       }
       Overlap overlap;
       overlap.upload_pending.assign(n, 0);
-      overlap.tail = find_tail(*exe, inputs, input_count, outputs, out_view_of);
+      overlap.tail = find_tail(*exe, inputs, input_count, outputs, output_count, out_view_of);
       const Tail &tail = overlap.tail;
       while (tail.step >= 0 && exe->pieces.size() < 2 * Tail::kMost) {
         cudaEvent_t e = nullptr;
@@ -1483,8 +1493,10 @@ dif_backend_status execute(dif_backend_executable executable, const dif_backend_
       for (size_t i = 0; i < input_count; ++i) {
         const int idx = exe->program.index_of(inputs[i].tensor_id);
         const bool is_const = idx >= 0 && exe->program.tensors[(size_t)idx].has(ir::Constant);
-        if (tail.step >= 0 && i == tail.input_view)
-          continue; // last, below
+        if (tail.step >= 0 && i == tail.input_view) {
+          check_view(*exe, inputs[i], ir::Input, "execute");
+          continue; // uploaded last, below
+        }
         const int at = upload(*exe, inputs[i], is_const ? ir::Constant : ir::Input, "execute", ctx->h2d);
         if (exe->uploaded[(size_t)at]) {
           require_cuda(cudaEventRecord(exe->uploaded[(size_t)at], ctx->h2d), "cudaEventRecord(upload)");
@@ -1492,7 +1504,6 @@ dif_backend_status execute(dif_backend_executable executable, const dif_backend_
         }
       }
       if (tail.step >= 0) {
-        check_view(*exe, inputs[tail.input_view], ir::Input, "execute");
         for (uint64_t piece = 0; piece < tail.pieces; ++piece) {
           const uint64_t from = tail.first(piece) * tail.row_bytes;
           require_cuda(cudaMemcpyAsync(static_cast<unsigned char *>(exe->dev[(size_t)tail.input]) + from,

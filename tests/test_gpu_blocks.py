@@ -8,7 +8,7 @@ import pytest
 
 import oracle_bridge as ob
 from diffusion_compiler_b200 import blocks
-from helpers import cosine, rel_l2
+from helpers import bf16_normal, cosine, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -85,6 +85,40 @@ def test_video_block_with_page_locked_arrays_keeps_the_bits(tokens):
         inputs = dict(inputs)
         inputs[ids["mods"][5]] = np.ascontiguousarray(gate[::-1])
         inputs[ids["x"]] = np.ascontiguousarray(inputs[ids["x"]][::-1])
+    ex.close()
+
+
+@pytest.mark.parametrize("case", ["shifted", "earlier output"])
+def test_outputs_may_lie_on_the_last_gates_host_array(case):
+    """Page-locked arrays that an Output has in common with the last step's gate: that Input is complete on the device before an Output
+    that needs it, or an earlier one whose Inputs stand behind it in the program, overwrites it."""
+    import torch
+    from diffusion_compiler_b200 import diffir as ir
+    from diffusion_compiler_b200 import plugin
+    rows, width = 8192, 2048  # 32 MB: eight blocks of rows
+    p = ir.Program()
+    bf = ir.DType.BF16
+    gate, first, a, b = (p.add_tensor(bf, [rows, width], ir.Role.Input) for _ in range(4))
+    early, out = (p.add_tensor(bf, [rows, width], ir.Role.Output) for _ in range(2))
+    p.add_op(ir.Opcode.ResidualGate, [a, b, first], [early])
+    p.add_op(ir.Opcode.ResidualGate, [a, b, gate], [out])
+    rng = np.random.default_rng(3)
+    given = {t: bf16_normal(rng, (rows, width)) for t in (gate, first, a, b)}
+    ex = plugin.PluginExecutor(0)
+    prepared = ex.prepare(p, {})
+    want, _ = prepared.run(given)
+    host = torch.zeros((2, rows, width), dtype=torch.int16, pin_memory=True).numpy().view(np.uint16)
+    flat = host.reshape(-1, width)
+    locked = lambda x: np.ascontiguousarray(torch.from_numpy(x.view(np.int16)).pin_memory().numpy()).view(np.uint16)  # noqa: E731
+    for _ in range(3):
+        flat[:rows] = given[gate]
+        bound = {t: locked(v) for t, v in given.items()}
+        bound[gate] = flat[:rows]
+        other = torch.zeros((rows, width), dtype=torch.int16, pin_memory=True).numpy().view(np.uint16)
+        outputs = {early: other, out: flat[rows * 3 // 4:rows * 7 // 4]} if case == "shifted" else {early: flat[:rows], out: other}
+        got, _ = prepared.run(bound, outputs=outputs)
+        for t in (early, out):
+            assert np.array_equal(got[t], want[t]), t
     ex.close()
 
 
