@@ -414,9 +414,9 @@ void plan(Executable &exe) {
       (role == 0 ? exe.steps[a].q_quantised : exe.steps[a].k_quantised) = true;
     }
   }
-  // A Slice whose elements are neighbours (nothing in front of its axis is repeated) is a part of its input's buffer, where
-  // that starts as kernels expect (16 bytes). At batch 1 the modulation vectors of a block, its streams' rows of the joint
-  // sequence: MMDiT block of 256 + 77 tokens, 16 of 51 launches. (Not token-sharded: there V's buffer is placed by its chain of aliases.)
+  // A Slice whose elements are neighbours (nothing in front of its axis is repeated) may be a part of its input's buffer, where
+  // that starts as kernels expect (16 bytes); settle_slices has the last word. At batch 1 the modulation vectors of a block, its streams' rows of the joint
+  // sequence: MMDiT block of 256 + 77 tokens, 15 of 51 launches. (Not token-sharded: there V's buffer is placed by its chain of aliases.)
   for (Step &st : exe.steps) {
     if (st.op->opcode != ir::Slice || st.skip || exe.ctx->world)
       continue;
@@ -589,10 +589,16 @@ void allocate_world(Executable &exe) {
   }
 }
 
-void allocate(Executable &exe) {
+// Where the tensors stand: in device memory of their own, in a block that tensors with other lifetimes share, or nowhere.
+struct MemoryPlan {
+  static constexpr int kNone = -1, kOwn = -2;
+  std::vector<int> place; // per tensor: its block, or one of the above
+  std::vector<size_t> block_bytes;
+  uint64_t bytes = 0; // of all tensors and blocks
+};
+MemoryPlan memory_plan(const Executable &exe) {
   const ir::Program &p = exe.program;
   const size_t n = p.tensors.size();
-  exe.dev.assign(n, nullptr);
   // Outputs of aliasing steps share the buffer of their input: every tensor belongs to the group of its root
   std::vector<size_t> root(n);
   for (size_t i = 0; i < n; ++i)
@@ -658,7 +664,6 @@ void allocate(Executable &exe) {
   for (const Step &st : exe.steps)
     if (st.alias)
       aliased[(size_t)p.index_of(st.op->out[0])] = true;
-  exe.owned.assign(n, 1);
   for (const Sharded &sh : exe.sharded) // lives inside the gather buffer (allocate_world)
     if (sh.v_root >= 0)
       aliased[(size_t)sh.v_root] = true;
@@ -675,49 +680,91 @@ void allocate(Executable &exe) {
   for (size_t i = 0; i < n; ++i)
     if (p.tensors[i].has(ir::Input) || p.tensors[i].has(ir::Constant) || p.tensors[i].has(ir::Output))
       pinned[root[i]] = true;
+  MemoryPlan plan;
+  plan.place.assign(n, MemoryPlan::kNone);
   std::vector<std::vector<size_t>> born(exe.order.size()), dying(exe.order.size());
   for (size_t i = 0; i < n; ++i) {
     if (!needed[i] || aliased[i])
       continue;
-    const size_t bytes = (size_t)p.tensors[i].bytes();
     if (!reuse || pinned[i] || first[i] == never) {
-      require_cuda(cudaMalloc(&exe.dev[i], bytes ? bytes : 16), "cudaMalloc(tensor)");
-      exe.resident_bytes += bytes;
+      plan.place[i] = MemoryPlan::kOwn;
+      plan.bytes += (size_t)p.tensors[i].bytes();
     } else {
       born[first[i]].push_back(i);
       dying[last[i]].push_back(i);
     }
   }
-  struct Block {
-    void *ptr;
-    size_t bytes;
-  };
-  std::vector<Block> free_blocks;
-  std::vector<Block> block_of(n, Block{nullptr, 0});
+  std::vector<int> free_blocks;
   for (size_t k = 0; k < exe.order.size(); ++k) {
     for (size_t i : born[k]) {
       const size_t bytes = (size_t)p.tensors[i].bytes() ? (size_t)p.tensors[i].bytes() : 16;
+      auto size_of = [&](size_t b) { return plan.block_bytes[(size_t)free_blocks[b]]; };
       size_t best = free_blocks.size();
       for (size_t b = 0; b < free_blocks.size(); ++b)
-        if (free_blocks[b].bytes >= bytes && free_blocks[b].bytes <= 2 * bytes &&
-            (best == free_blocks.size() || free_blocks[b].bytes < free_blocks[best].bytes))
+        if (size_of(b) >= bytes && size_of(b) <= 2 * bytes && (best == free_blocks.size() || size_of(b) < size_of(best)))
           best = b;
       if (best < free_blocks.size()) {
-        block_of[i] = free_blocks[best];
+        plan.place[i] = free_blocks[best];
         free_blocks.erase(free_blocks.begin() + (long)best);
       } else {
-        void *ptr = nullptr;
-        require_cuda(cudaMalloc(&ptr, bytes), "cudaMalloc(tensor)");
-        exe.world_buffers.push_back(ptr); // freed with the executable
-        exe.resident_bytes += bytes;
-        block_of[i] = Block{ptr, bytes};
+        plan.place[i] = (int)plan.block_bytes.size();
+        plan.block_bytes.push_back(bytes);
+        plan.bytes += bytes;
       }
-      exe.dev[i] = block_of[i].ptr;
-      exe.owned[i] = 0;
     }
     for (size_t i : dying[k])
-      free_blocks.push_back(block_of[i]);
+      free_blocks.push_back(plan.place[i]);
   }
+  return plan;
+}
+
+// A Slice that shares its input's buffer keeps all of it for as long as it is read. Where that takes more device memory than copies
+// would, only those Slices share that do not add to it, in program order.
+void settle_slices(Executable &exe) {
+  std::vector<Step *> slices;
+  for (Step &st : exe.steps)
+    if (st.alias && st.op->opcode == ir::Slice)
+      slices.push_back(&st);
+  if (slices.empty())
+    return;
+  auto share = [](Step *st, bool on) { st->alias = st->skip = on; };
+  const uint64_t all = memory_plan(exe).bytes;
+  for (Step *st : slices)
+    share(st, false);
+  const uint64_t none = memory_plan(exe).bytes;
+  for (Step *st : slices) {
+    share(st, true);
+    if (all > none && memory_plan(exe).bytes > none)
+      share(st, false);
+  }
+}
+
+void allocate(Executable &exe) {
+  const ir::Program &p = exe.program;
+  const size_t n = p.tensors.size();
+  settle_slices(exe);
+  const MemoryPlan plan = memory_plan(exe);
+  exe.dev.assign(n, nullptr);
+  exe.owned.assign(n, 1);
+  auto device_alloc = [&](size_t bytes) {
+    void *ptr = nullptr;
+    require_cuda(cudaMalloc(&ptr, bytes ? bytes : 16), "cudaMalloc(tensor)");
+    return ptr;
+  };
+  for (size_t i = 0; i < n; ++i)
+    if (plan.place[i] == MemoryPlan::kOwn)
+      exe.dev[i] = device_alloc((size_t)p.tensors[i].bytes());
+  std::vector<void *> blocks;
+  for (size_t bytes : plan.block_bytes) {
+    blocks.push_back(device_alloc(bytes));
+    exe.world_buffers.push_back(blocks.back()); // freed with the executable
+  }
+  for (size_t i = 0; i < n; ++i)
+    if (plan.place[i] >= 0) {
+      exe.dev[i] = blocks[(size_t)plan.place[i]];
+      exe.owned[i] = 0;
+    }
+  exe.resident_bytes += plan.bytes;
   allocate_world(exe);
   for (const Step &st : exe.steps) // program order: a chain of reshapes resolves front to back
     if (st.alias) {

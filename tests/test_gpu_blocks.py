@@ -230,6 +230,46 @@ def test_mmdit_block_at_batch_one_has_the_bits_of_batch_two():
     assert not np.array_equal(results[0][0], results[1][0])
 
 
+@pytest.mark.parametrize("case", ["kept", "output"])
+def test_slices_that_share_a_buffer_take_no_more_memory(case, monkeypatch):
+    """A few rows of a large internal tensor that are read long after it ("kept") or leave the program ("output"): sharing its buffer would
+    hold all of it, a copy does not. Slices beside them that cost nothing still share. DIFB200_ROPE_FUSION=0 copies every Slice."""
+    from diffusion_compiler_b200 import diffir as ir
+    from diffusion_compiler_b200 import plugin
+    rows, width, few = 4096, 1024, 16
+    p = ir.Program()
+    bf = ir.DType.BF16
+    attrs = lambda start: [ir.Attribute.u64(ir.AttrKey.Axis, 0), ir.Attribute.u64(ir.AttrKey.Start, start)]  # noqa: E731
+    x = p.add_tensor(bf, [rows, width], ir.Role.Input)
+    large = [p.add_tensor(bf, [rows, width]) for _ in range(5)]
+    part = p.add_tensor(bf, [few, width], ir.Role.Output if case == "output" else ir.Role.Internal)
+    other, last = p.add_tensor(bf, [few, width]), p.add_tensor(bf, [few, width])
+    out = p.add_tensor(bf, [few, width], ir.Role.Output)
+    gelu = lambda a, b: p.add_op(ir.Opcode.Gelu, [a], [b], [ir.Attribute.u64(ir.AttrKey.Approximation, 1)])  # noqa: E731
+    gelu(x, large[0])
+    p.add_op(ir.Opcode.Slice, [large[0]], [part], attrs(3))
+    p.add_op(ir.Opcode.Slice, [x], [other], attrs(5))  # of an Input, whose buffer stays anyway
+    for a, b in zip(large, large[1:]):
+        gelu(a, b)
+    p.add_op(ir.Opcode.Slice, [large[-1]], [last], attrs(7))
+    p.add_op(ir.Opcode.ResidualGate, [last, other, other if case == "output" else part], [out])
+    given = {x: bf16_normal(np.random.default_rng(1), (rows, width))}
+    results = {}
+    monkeypatch.setenv("DIFB200_PROFILE", "1")
+    for shared in (True, False):
+        monkeypatch.setenv("DIFB200_ROPE_FUSION", "1" if shared else "0")
+        ex = plugin.PluginExecutor(0)
+        prepared = ex.prepare(p, {})
+        got, _ = prepared.run(given, warmups=1)
+        copies = prepared.profile().get(int(ir.Opcode.Slice), (0.0, 0))[1]
+        results[shared] = prepared.compile_telemetry.resident_bytes, copies, got
+        ex.close()
+    assert results[True][0] <= results[False][0]
+    assert (results[True][1], results[False][1]) == (1, 3)  # two share
+    for t in results[True][2]:
+        assert np.array_equal(results[True][2][t], results[False][2][t])
+
+
 @pytest.mark.parametrize("S,world", [(512, 4), (437, 4)])
 def test_token_sharded_video_block_matches_unsharded(S, world):
     """Ranks are emulated sequentially on one GPU: every rank runs its row-local part, the gather
