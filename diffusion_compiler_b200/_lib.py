@@ -35,6 +35,8 @@ def lib() -> C.CDLL:
         L.difb200_test_withhold_gemm_load.argtypes = [u32]
         L.difb200_test_withhold_row_maximum.restype = None
         L.difb200_test_withhold_row_maximum.argtypes = [u64]
+        L.difb200_test_row_statistics.restype = C.c_int
+        L.difb200_test_row_statistics.argtypes = [vp, u64, u64, f32, i32, vp, vp]
         L.difb200_selftest_host.restype = C.c_int
         L.difb200_quantize_int8_rows.restype = C.c_int
         L.difb200_quantize_int8_rows.argtypes = [C.POINTER(vp), C.POINTER(u64), u32, u64, i32, f32, vp,

@@ -108,6 +108,19 @@ void difb200_test_withhold_gemm_load(uint32_t k_block) { withhold_next_gemm_load
 
 void difb200_test_withhold_row_maximum(uint64_t limit_ns) { withhold_next_row_maximum(limit_ns); }
 
+int difb200_test_row_statistics(const void *x, uint64_t rows, uint64_t columns, float epsilon, int32_t layer, float *pairs, void *stream) {
+  if (!x || !pairs)
+    return fail(kInvalidArgument, "row statistics: null pointer");
+  StreamScratch scratch(static_cast<cudaStream_t>(stream));
+  glue::RowStats stats{};
+  if (int rc = glue::row_stats(x, rows, columns, epsilon, layer != 0, true, pairs, 2 * sizeof(float), {}, scratch, &stats,
+                               static_cast<cudaStream_t>(stream)))
+    return rc;
+  return rows == 0 || stats.at == reinterpret_cast<unsigned char *>(pairs)
+             ? kOk
+             : fail(kInvalidArgument, "row statistics: the pairs must start on 8 bytes, apart from the rows");
+}
+
 int difb200_program_check(const uint8_t *diffir, uint64_t size) {
   ir::Program program;
   std::string text;

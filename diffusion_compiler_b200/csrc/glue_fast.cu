@@ -154,7 +154,6 @@ template <int SUMS, int STAGES>
 __global__ void __launch_bounds__(32 * kStatWarps)
 k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint32_t cols, float eps) {
   extern __shared__ uint4 stat_smem[];
-  grid_dependency_wait(); // (every load is an asynchronous copy)
   auto tile = reinterpret_cast<uint4 (*)[STAGES][32 * kStatPitch]>(stat_smem); // [kStatWarps]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t cols8 = cols >> 3, chunks = cols / kStatCols;
@@ -295,8 +294,8 @@ k_row_stats_sequential(const uint4 *x, const RowStats stats, uint64_t rows, uint
 // bits and adds the distance t - r that it has from that one's start. Every lane says between which distances that holds (the
 // same binade at the start, at most one crossing, in a step whose sums on either side are further from the boundary than t and r from
 // one another); where it does not, in one row of ten as a part's numbers cross several binades at once, or where numbers are not
-// finite, the part's terms are added one by one. Compared with the sequential chain on a CPU: 60000 rows of nine kinds of
-// numbers, some of them built to meet boundaries and ties, same bits.
+// finite, the part's terms are added one by one. Compared with the sequential kernel, all bits of the statistics: 4.8e8 rows of 1024 to
+// 8192 numbers, normal ones and others built to meet boundaries, ties and many binades, the same (tests/test_gpu_norm_streams.py has a few).
 // It is bound by the operations of five chains (about 750 per row and warp at IPC 0.5), so that many rows are better off with the
 // sequential kernel, whose lanes have a row each: row_stats has the line. 32 parts per row took the same time for few rows and
 // a fifth more for many, 8 more for few; rows kept for a second pass in registers (unrolled: 168 of them) the same.
@@ -349,12 +348,14 @@ __device__ __forceinline__ void square_chain(const uint4 &v, float mean, float (
   }
 }
 
-// A lane per part, two rows per warp at a time. GROUPS: p.groups as a constant, or 0.
+// A lane per part, two rows per warp at a time. GROUPS: p.groups as a constant, or 0. The constant of 3072 columns makes the copies'
+// addresses and the layout of shared memory known: norm and quantiser from a graph, us, constant / general: RMS, 1 row 6.1 / 6.3, 77
+// 6.7 / 7.0, 300 8.5 / 8.9, 1500 13.5 / 13.7, 2900 21.2 / 21.4; layer form, 77 18.5 / 18.6, 600 21.7 / 21.7, 2900 34.9 / 34.7.
 template <bool LAYER, int GROUPS>
 __global__ void __launch_bounds__(32 * kSquareWarps)
 k_row_squares(const SquareParams p) {
   extern __shared__ uint4 square_smem[];
-  const uint64_t after = grid_dependency_wait_zero();
+  grid_dependency_wait(); // (what it reads comes by asynchronous copies and, the mean, by plain loads: both stay behind)
   constexpr uint32_t kParts = kSquareParts, kRows = 32 / kParts;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, part = lane % kParts, groups = GROUPS ? GROUPS : p.groups;
   const uint32_t pitch = square_pitch(groups), cols8 = groups * kParts;

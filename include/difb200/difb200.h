@@ -68,6 +68,13 @@ DIFB200_EXPORT void difb200_test_withhold_gemm_load(uint32_t k_block);
 DIFB200_EXPORT void difb200_test_withhold_row_maximum(uint64_t limit_ns);
 
 /*
+ * Test aid: the row statistics in front of the norms by themselves, a pair of fp32 per row of bf16 [rows, columns]: 0 and
+ * 1 / sqrt(sum of squares / columns + epsilon), or with `layer` the mean and the same of the deviations.
+ */
+DIFB200_EXPORT int difb200_test_row_statistics(const void *x, uint64_t rows, uint64_t columns, float epsilon, int32_t layer,
+                                               float *pairs, void *stream);
+
+/*
  * Host-only self-check of the library's per-device bookkeeping (one-time set-up keyed by device
  * ordinal, wait-limit state). Touches no GPU; returns 0 when the invariants hold.
  */

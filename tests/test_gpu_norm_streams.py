@@ -116,6 +116,20 @@ def test_norm_ops_in_place(K, over):
         assert torch.equal(want.view(torch.int16), got.view(torch.int16)), layer
 
 
+def _rows_of_all_kinds(rows, cols, g):
+    """Outliers, equal numbers (ties in every step), rows whose sums meet powers of two, zeros, steps over many binades, infinities, NaN."""
+    import torch
+    x = torch.randn((rows, cols), generator=g, device="cuda")
+    x[:, :: cols // 32] *= 16.0  # (and so that single parts cross several binades)
+    x[100:400] = x[100:400].round()
+    x[400:500] = torch.exp2(torch.arange(100, device="cuda").remainder(12).float() - 6.0)[:, None]
+    x[500:600] *= torch.exp(4.0 * torch.randn((100, cols), generator=g, device="cuda"))
+    x[600:650, : cols // 2] = 0.0
+    x[650], x[651, 7], x[652, 9], x[653] = 0.0, float("inf"), float("nan"), x[653] * 2.0**-40
+    x[654:700] *= 2.0 ** torch.arange(-23, 23, device="cuda").float()[:, None]
+    return x.to(torch.bfloat16)
+
+
 @pytest.mark.parametrize("layer", [False, True])
 @pytest.mark.parametrize("cols", [1024, 2048, 2816, 3072, 8192])
 def test_statistics_of_few_rows_are_those_of_many(layer, cols):
@@ -127,15 +141,7 @@ def test_statistics_of_few_rows_are_those_of_many(layer, cols):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     rows = 20 * sms + 5
     g = torch.Generator(device="cuda").manual_seed(cols)
-    x = torch.randn((rows, cols), generator=g, device="cuda")
-    x[:, :: cols // 32] *= 16.0  # (and so that single parts cross several binades)
-    x[100:400] = x[100:400].round()
-    x[400:500] = torch.exp2(torch.arange(100, device="cuda").remainder(12).float() - 6.0)[:, None]
-    x[500:600] *= torch.exp(4.0 * torch.randn((100, cols), generator=g, device="cuda"))
-    x[600:650, : cols // 2] = 0.0
-    x[650], x[651, 7], x[652, 9], x[653] = 0.0, float("inf"), float("nan"), x[653] * 2.0**-40
-    x[654:700] *= 2.0 ** torch.arange(-23, 23, device="cuda").float()[:, None]
-    x = x.to(torch.bfloat16)
+    x = _rows_of_all_kinds(rows, cols, g)
     normal = lambda *s: (0.1 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)  # noqa: E731
     w, b, s, h = normal(cols) + 1, normal(cols), normal(rows, cols), normal(rows, cols)
     want = _call(ops, layer, x, w, b, s, h)
@@ -143,3 +149,31 @@ def test_statistics_of_few_rows_are_those_of_many(layer, cols):
         at = slice(first, first + count)
         got = _call(ops, layer, x[at].contiguous(), w, b, s[at].contiguous(), h[at].contiguous())
         assert torch.equal(got[0], want[0][at]) and torch.equal(got[1].view(torch.int32), want[1][at].view(torch.int32)), (first, count)
+
+
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("cols", [1024, 1152, 2048, 2816, 3072, 4992, 8192])
+def test_sums_in_parts_are_the_chains(layer, cols):
+    """The statistics themselves, all bits: a tensor of more rows than are cut in parts has them from the chain, its slices from the parts. A
+    wrong last bit shows here; behind a norm and a quantiser it hardly would."""
+    import ctypes as C
+
+    import torch
+    from diffusion_compiler_b200 import _lib
+    lib = _lib.lib()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    line = (20 if cols >= 2048 else 4) * sms  # the most rows that are cut in parts
+
+    def statistics(x):
+        pairs = torch.empty((x.shape[0], 2), device="cuda")
+        _lib.check(lib.difb200_test_row_statistics(C.c_void_p(x.data_ptr()), x.shape[0], cols, 1e-5, int(layer), C.c_void_p(pairs.data_ptr()),
+                                                   C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        return pairs.view(torch.int32)
+
+    for seed in range(6):
+        x = _rows_of_all_kinds(20 * sms + 700, cols, torch.Generator(device="cuda").manual_seed(100 * cols + seed))
+        want = statistics(x)
+        starts = list(range(0, x.shape[0], line - seed))
+        for first, count in [(0, 1), (101, sms + seed), (400, 333)] + [(i, line - seed) for i in starts]:
+            got = statistics(x[first:first + count].contiguous())
+            assert torch.equal(got, want[first:first + count]), (seed, first)
