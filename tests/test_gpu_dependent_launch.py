@@ -172,8 +172,9 @@ def test_gemm_directly_behind_an_attention(tokens):
 
 @pytest.mark.parametrize("rows,K", [(1, 256), (2, 3072), (8, 1024)])  # with the quantiser in the same launch: at most 8 blocks of 1024 columns
 def test_linears_of_few_rows_one_behind_the_other(rows, K):
-    """Single-call linears in one launch each, which starts while the one in front of it still runs: every one reads what the
-    last one wrote and writes the buffer that the last one read, on the stream and from a graph."""
+    """Single-call linears in one launch each, which starts as the CTAs of the one in front end: every one reads what the
+    last one wrote and writes the buffer that the last one read, on the stream and from a graph. (Behind a kernel that lets it start
+    earlier: "linear" of 4 rows below.)"""
     import torch
     from diffusion_compiler_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(rows * K)
@@ -209,8 +210,8 @@ def test_linears_of_few_rows_one_behind_the_other(rows, K):
         assert torch.equal(_bits(o), _bits(want)), i
 
 
-def _readers():
-    """name -> a call that reads bf16 rows [rows, 1024] (8 heads of 128) first of all."""
+def _readers(rows):
+    """name -> a call whose first kernel, with nothing else in front of it, reads bf16 rows [rows, 1024] (8 heads of 128)."""
     import ctypes as C
 
     import torch
@@ -218,18 +219,19 @@ def _readers():
     g = torch.Generator(device="cuda").manual_seed(7)
     normal = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
     K = 1024
-    vector, table = normal(K), normal(1200, 96)
+    vector, table, equalisation = normal(K), normal(1200, 96), normal(K).abs().clamp(0.5, 2.0)
     w8, ws = ops.quantize_weight_rows(normal(1536, K), 2)
     ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
     stream = lambda: C.c_void_p(torch.cuda.current_stream().cuda_stream)  # noqa: E731
 
-    def glue(name, x, columns, *args):
-        o = torch.zeros((x.shape[0], columns), dtype=torch.bfloat16, device="cuda")
-        _lib.check(getattr(_lib.lib(), name)(*(ptr(a) if torch.is_tensor(a) else ptr(o) if a is None else a for a in args), stream()))
+    gated, halves = (torch.zeros((rows, columns), dtype=torch.bfloat16, device="cuda") for columns in (K, K // 2))
+    codes, scales = torch.zeros((rows, K), dtype=torch.int8, device="cuda"), torch.zeros(8 * rows, device="cuda")
+
+    def glue(name, o, *args):
+        _lib.check(getattr(_lib.lib(), name)(*(ptr(a) if torch.is_tensor(a) else a for a in args), stream()))
         return o
 
     def rope(x):
-        codes, scales = torch.zeros_like(x, dtype=torch.int8), torch.zeros(8 * x.shape[0], device="cuda")
         _lib.check(_lib.lib().difb200_qk_norm_rope_quant(ptr(x), ptr(vector), ptr(table), ptr(table), None, ptr(codes), ptr(scales), 2,
                                                          x.shape[0], 8, 96, 96, x.shape[0], 1200, 0, 1e-5, 0, stream()))
         return codes, scales
@@ -240,13 +242,13 @@ def _readers():
         "residual": lambda x: ops.quantize_int8_rows([x], 3, residual=True),
         "two inputs": lambda x: ops.quantize_int8_rows([x, x], 2),
         "direct heads": lambda x: ops.quantize_int8_rows([x.view(-1, 128)], 1),
-        "packing": lambda x: ops.quantize_weight_rows(x, 2, mse_scale=True, input_scale=x[0].clamp(0.5, 2.0)),
+        "packing": lambda x: ops.quantize_weight_rows(x, 2, mse_scale=True, input_scale=equalisation),
         "rms norm": lambda x: ops.rms_norm_modulate_quant(x, vector, x, x),
         "layer norm": lambda x: ops.layer_norm_modulate_quant(x, vector, vector, x, x),
         "linear": lambda x: ops.w8a8_linear(x, w8, ws),
         "attention": lambda x: ops.attention(heads(x), heads(x), heads(x)),
-        "gate": lambda x: glue("difb200_residual_gate", x, K, x, x, x, None, 2, x.shape[0], K, x.shape[0]),
-        "swiglu": lambda x: glue("difb200_swiglu", x, K // 2, x, None, 2, x.shape[0], K // 2, K, 0, 0),
+        "gate": lambda x: glue("difb200_residual_gate", gated, x, x, x, gated, 2, rows, K, rows),
+        "swiglu": lambda x: glue("difb200_swiglu", halves, x, halves, 2, rows, K // 2, K, 0, 0),
         "rope": rope,
     })
     return calls
@@ -254,20 +256,28 @@ def _readers():
 
 @pytest.mark.parametrize("rows", [4, 332, 1200])
 def test_kernels_launched_ahead_read_what_the_kernel_in_front_writes(rows):
-    """Every kernel that is launched ahead, behind a quantiser that lets it start at once and whose codes (as the bits of bf16
-    numbers) are what it reads: the buffer holds other numbers until that quantiser is done."""
+    """Every kernel that is launched ahead, behind a quantiser that lets it start at once (a 256-wide one, all of whose rows are in one
+    batch per CTA: its CTAs say so when they start) and whose codes (as the bits of bf16 numbers) are what it reads: the
+    buffer holds other numbers until that quantiser is done. A delay in front lets the host enqueue both before the first starts."""
     import torch
     from diffusion_compiler_b200 import ops
+    # four rows of 2048 columns per CTA, three CTAs on an SM
+    assert rows <= 3 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    unit = ops.quantize_int8_rows([torch.eye(256, device="cuda").to(torch.bfloat16)], 5)[0].float()
+    assert bool((unit.abs() == 127).all())  # the rotation is orthogonal, all its entries +-1/16
     g = torch.Generator(device="cuda").manual_seed(rows)
     sources = [0.55 + 0.2 * torch.rand((rows, 2048), generator=g, device="cuda") for _ in range(2)]
     for s in sources:
-        s[:, 5] = 1.0  # the largest of a row: its code with clip 2 is 64, the others' are 35 to 48
-    sources = [s.to(torch.bfloat16) for s in sources]
+        s[:, 5] = 1.0  # the largest of a row: its code with clip 2 is 64, the others' are 34 to 49
+    sources = [(s.view(rows, 8, 256) @ (unit.T / (127 * 16))).view(rows, 2048).to(torch.bfloat16) for s in sources]
     codes, scales = torch.zeros((rows, 2048), dtype=torch.int8, device="cuda"), torch.zeros(rows, device="cuda")
     x = codes.view(torch.bfloat16)
-    write = lambda i: ops.quantize_int8_rows([sources[i]], 1, clip=2.0, out=(codes, scales))  # noqa: E731
+    write = lambda i: ops.quantize_int8_rows([sources[i]], 2, clip=2.0, out=(codes, scales))  # noqa: E731
+    for i in range(2):
+        write(i)
+        assert 32 <= int(codes.min()) and int(codes.max()) <= 66, "the codes are not the numbers that were rotated back"
     tensors = lambda r: [r] if torch.is_tensor(r) else list(r)  # noqa: E731
-    for name, call in _readers().items():
+    for name, call in _readers(rows).items():
         want = []
         for i in range(2):
             write(i)
@@ -276,6 +286,7 @@ def test_kernels_launched_ahead_read_what_the_kernel_in_front_writes(rows):
             torch.cuda.synchronize()
         assert any(not torch.equal(a, b) for a, b in zip(*want)), name
         for i in range(6):
+            torch.cuda._sleep(400_000)  # clocks, about 0.2 ms
             write(i % 2)
             got = tensors(call(x))
             torch.cuda.synchronize()
