@@ -215,19 +215,23 @@ def test_quotients_out_of_the_two_part_products_range(impl, K):
 
 
 @pytest.mark.parametrize("impl", [2, 3, 5, 6])
-@pytest.mark.parametrize("rows,width", [
-    (10656, 256),   # one warp per row: as many rows as the table of reciprocals is made for
-    (3553, 3072),   # three blocks per warp, a last round of one row
-    (4000, 2816),   # the same with a partial third block
-    (5400, 1280),   # two blocks, the second of one group
-    (1340, 8192),   # eight blocks
-    (900, 12288),   # twelve
+@pytest.mark.parametrize("more,width", [
+    (0, 256),      # one warp per row: as many rows as the table of reciprocals is made for
+    (1, 3072),     # three blocks per warp, a last round of one row
+    (448, 2816),   # the same with a partial third block
+    (72, 1280),    # two blocks, the second of one group
+    (8, 8192),     # eight blocks
+    (12, 12288),   # twelve
+    (0, 14592),    # fifteen, the last of one group: the largest table
+    (2, 15360),    # fifteen
 ])
-def test_packing_with_a_table_of_reciprocals(impl, rows, width):
+def test_packing_with_a_table_of_reciprocals(impl, more, width):
     """Rows are packed one by one: all at once, where a CTA's rows share a table of the equalisation's reciprocals, and a few hundred
     at a time, where every row makes its own. Entries beyond the table's range, infinities and NaN among them."""
     import torch
     from diffusion_compiler_b200 import ops
+    blocks = (width + 1023) // 1024
+    rows = -(-72 * torch.cuda.get_device_properties(0).multi_processor_count // blocks) + more  # the least that share a table, and more
     rng = np.random.default_rng(rows + impl)
     w = to_torch_bf16(bf16_normal(rng, (rows, width), std=0.02))
     eq = to_torch_bf16(ob.f32_to_bf16(np.exp(0.7 * rng.standard_normal(width)).astype(np.float32)))
