@@ -141,7 +141,7 @@ key_table_kernel(const int8_t *k8, const float *ks, const uint8_t *key_valid, fl
     int n2 = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const uint4 w = __ldg(row + c);
+      const uint4 w = load_global(row + c);
       n2 = __dp4a((int)w.x, (int)w.x, n2);
       n2 = __dp4a((int)w.y, (int)w.y, n2);
       n2 = __dp4a((int)w.z, (int)w.z, n2);
@@ -198,8 +198,8 @@ attention_operands_kernel(const OperandParams p) {
   auto request = [&](int step, const uint4 *row, bool valid) {
     lows[step] = highs[step] = make_uint4(0, 0, 0, 0);
     if (valid) {
-      lows[step] = __ldg(row + 2 * part);
-      highs[step] = __ldg(row + 2 * part + 1);
+      lows[step] = load_global(row + 2 * part);
+      highs[step] = load_global(row + 2 * part + 1);
     }
   };
   // codes of this lane's 16 elements of a row and the row's scale (in every lane)
@@ -653,9 +653,9 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // two, and the running form simply goes on from the carried m.
       float m_prev = -INFINITY;
       if (p.carry_in && row_ok) {
-        const float2 ml = __ldg(p.ml_state + state_row());
+        const float2 ml = load_global(p.ml_state + state_row());
         m_prev = ml.x;
-        l = hf == 0u ? ml.y : __ldg(p.l2_state + state_row());
+        l = hf == 0u ? ml.y : load_global(p.l2_state + state_row());
       }
       const float m_both = fmaxf(m_prev, m_fixed);
       // (a bound far above what the carried state holds would push that state towards underflow)
@@ -671,7 +671,7 @@ attn_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           uint32_t o[32];
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
-            const float4 x = row_ok ? __ldg(src + (8 * c + v) * pitch) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 x = row_ok ? load_global(src + (8 * c + v) * pitch) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             o[4 * v] = __float_as_uint(x.x * factor);
             o[4 * v + 1] = __float_as_uint(x.y * factor);
             o[4 * v + 2] = __float_as_uint(x.z * factor);

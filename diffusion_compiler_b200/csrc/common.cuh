@@ -103,7 +103,8 @@ inline Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
 // all CTAs of that one have called grid_dependents_launch() (or ended) and there is room. Its set-up runs then; what
 // the kernel in front wrote is read behind grid_dependency_wait(), which every thread passes that touches global
 // memory, and through loads that the compiler cannot move up: load_produced, TMA, or addresses that the wait is a part of
-// (grid_dependency_wait_zero). A kernel that lets dependents start waits first: when a kernel starts, the one two in front
+// (grid_dependency_wait_zero). None of them is non-coherent (__ldg): that path is for memory that nobody writes while the
+// kernel lives, and this one lives while the one in front writes. A kernel that lets dependents start waits first: when a kernel starts, the one two in front
 // is complete.
 // Two reads are not behind such a wait. Both are of what a kernel further in front wrote, and both hold only because
 // the kernel in between waited before it let anything start (then that kernel is complete):
@@ -114,7 +115,7 @@ inline Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
 // other: 8.2 us, 5.9, and 5.8 where it says so at its start or its end). So it says so only where the next one has work to do
 // meanwhile: CTAs that only wait would gather on the SMs that happen to be free.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The wait and a zero behind it: addresses of loads that could otherwise be moved in front of the wait (__ldg) contain it.
+// The wait and a zero behind it: addresses of loads that could otherwise be moved in front of the wait (load_global) contain it.
 __device__ __forceinline__ uint64_t grid_dependency_wait_zero() {
   uint64_t zero;
   asm volatile("griddepcontrol.wait;\nmov.u64 %0, 0;" : "=l"(zero)::"memory");
@@ -131,12 +132,44 @@ __device__ __forceinline__ uint32_t load_produced(const uint16_t *p) {
   asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
+// What __ldg is to the compiler, a value that depends on the address alone, by the coherent path. Like __ldg it is not for memory that
+// this kernel writes before.
+__device__ __forceinline__ uint4 load_global(const uint4 *p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_global(const float4 *p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 load_global(const float2 *p) {
+  float2 v;
+  asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_global(const float *p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_global(const uint16_t *p) {
+  uint16_t v;
+  asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint4 load_produced(const uint4 *p) {
   uint4 v;
   asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-// 16 bytes that are read once and were not written by a kernel that may still run.
+// 16 bytes that are read once. The second form is for what no kernel that may still run has written.
+__device__ __forceinline__ uint4 load_produced_once(const void *p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint4 load_streamed(const void *p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

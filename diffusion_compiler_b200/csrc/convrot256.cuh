@@ -61,12 +61,12 @@ constexpr uint32_t kTableBlockBytes = 8192; // of 1024 columns: [16][32 lanes] x
 // 32 bytes of one thread: one 256-bit load where every run starts on 32 bytes, else two of 128 bits.
 __device__ __forceinline__ void load_run(const uint4 *src, bool wide, uint4 &a, uint4 &b) {
   if (wide) {
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                  : "l"(src));
   } else {
-    a = __ldg(src);
-    b = __ldg(src + 1);
+    a = load_global(src);
+    b = load_global(src + 1);
   }
 }
 
@@ -89,7 +89,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   const uint32_t smem_addr = smem_u32(smem);
   const uint32_t warp_addr = smem_addr + warp * kWarpBytes;
   float *red = reinterpret_cast<float *>(smem + total_warps * (kWarpBytes / 4)); // [2][2][total_warps], AHEAD [4][total_warps]
-  const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
+  const float clip = p.clip_device ? load_global(p.clip_device + after) : p.clip;
   constexpr float kCarry = 16.0f; // the values carried through the rotation are scaled by 2^stages
   const uint32_t columns = p.columns;
   const uint32_t col_warp = (uint32_t)wrow * (NIT * 1024u);
@@ -147,7 +147,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       for (int half = 0; half < 2; ++half) {
         const uint4 one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
         const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c) + half;
-        const uint4 ea4 = c < columns ? __ldg(ep) : one, eb4 = c + 256u < columns ? __ldg(ep + 32) : one;
+        const uint4 ea4 = c < columns ? load_global(ep) : one, eb4 = c + 256u < columns ? load_global(ep + 32) : one;
         const uint32_t ea[4] = {ea4.x, ea4.y, ea4.z, ea4.w}, eb[4] = {eb4.x, eb4.y, eb4.z, eb4.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -184,7 +184,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
       const uint32_t c = col0 + (uint32_t)(q >> 1) * 1024u + (uint32_t)(q & 1) * 256u;
       if (c < columns) {
         const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
-        const uint4 e0 = __ldg(ep), e1 = __ldg(ep + 1);
+        const uint4 e0 = load_global(ep), e1 = load_global(ep + 1);
         const uint32_t w[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -296,7 +296,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
           for (int half = 0; half < 2; ++half) {
             const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
             auto pick = [&](const uint16_t *base, uint64_t index, bool active, const uint4 &other) {
-              return active ? __ldg(reinterpret_cast<const uint4 *>(base + index) + half) : other;
+              return active ? load_global(reinterpret_cast<const uint4 *>(base + index) + half) : other;
             };
             const uint4 sa4 = pick(p.norm_scale, at, act_a, zero), sb4 = pick(p.norm_scale, at + 256u, act_b, zero);
             const uint4 ha4 = pick(p.norm_shift, at, act_a, zero), hb4 = pick(p.norm_shift, at + 256u, act_b, zero);
@@ -379,7 +379,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
             auto entries = [&](uint32_t(&ea)[8], uint32_t(&eb)[8]) {
               const uint4 z = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u); // bf16 ones
               const uint4 *ep = reinterpret_cast<const uint4 *>(p.equalise + after + c);
-              const uint4 e4[4] = {act_a ? __ldg(ep) : z, act_a ? __ldg(ep + 1) : z, act_b ? __ldg(ep + 32) : z, act_b ? __ldg(ep + 33) : z};
+              const uint4 e4[4] = {act_a ? load_global(ep) : z, act_a ? load_global(ep + 1) : z, act_b ? load_global(ep + 32) : z, act_b ? load_global(ep + 33) : z};
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const uint4 &va = e4[i >> 2], &vb = e4[2 + (i >> 2)];

@@ -276,7 +276,7 @@ __device__ __forceinline__ float load_logical(const QuantParams &p, uint64_t aft
   uint32_t c = column;
   for (uint32_t i = 0; i < p.part_count; ++i) {
     if (c < p.width[i])
-      return bf16_bits_to_f32(__ldg(p.part[i] + after + row * p.width[i] + c));
+      return bf16_bits_to_f32(load_global(p.part[i] + after + row * p.width[i] + c));
     c -= p.width[i];
   }
   return 0.0f;
@@ -291,14 +291,14 @@ direct_quant_kernel(const QuantParams p) {
   const int lane = threadIdx.x & 31;
   const uint64_t warp_global = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint64_t warp_count = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const float clip = p.clip_device ? __ldg(p.clip_device + after) : p.clip;
+  const float clip = p.clip_device ? load_global(p.clip_device + after) : p.clip;
   const uint32_t K = p.columns;
   for (uint64_t row = warp_global; row < p.rows; row += warp_count) {
     float m = 0.0f;
     if (VEC8) { // single part, width % 8 == 0, 16-byte aligned rows
       const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + after + row * K);
       for (uint32_t c = lane; c < (K >> 3); c += 32) {
-        const uint4 v = __ldg(src + c);
+        const uint4 v = load_global(src + c);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -322,7 +322,7 @@ direct_quant_kernel(const QuantParams p) {
       const uint4 *src = reinterpret_cast<const uint4 *>(p.part[0] + after + row * K);
       uint2 *dst = reinterpret_cast<uint2 *>(p.codes + row * K);
       for (uint32_t c = lane; c < (K >> 3); c += 32) {
-        const uint4 v = __ldg(src + c);
+        const uint4 v = load_global(src + c);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
         uint32_t out[2] = {0, 0};
 #pragma unroll

@@ -56,9 +56,9 @@ k_residual_gate_bf16(const uint4 *res, const uint4 *branch, const uint4 *gate, u
   GRID_STRIDE(i, groups) {
     const uint64_t row = i / width8, col = i - row * width8;
     float r[8], b[8], g[8], y[8];
-    unpack8(__ldg(res + i), r);
-    unpack8(__ldg(branch + i), b);
-    unpack8(__ldg(gate + (row / rows_per_gate) * width8 + col), g);
+    unpack8(load_global(res + i), r);
+    unpack8(load_global(branch + i), b);
+    unpack8(load_global(gate + (row / rows_per_gate) * width8 + col), g);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
       y[e] = __fadd_rn(r[e], __fmul_rn(g[e], b[e]));
@@ -82,8 +82,8 @@ k_swiglu_bf16(const uint4 *x, uint4 *o, uint64_t groups, const D width, uint64_t
   GRID_STRIDE(i, groups) {
     const uint64_t row = width.quotient(i), col = i - row * width8, base = row * in_width8 + start8 + col;
     float value[8], gate[8], y[8];
-    unpack8(__ldg(x + base + (gate_first ? width8 : 0)), value);
-    unpack8(__ldg(x + base + (gate_first ? 0 : width8)), gate);
+    unpack8(load_global(x + base + (gate_first ? width8 : 0)), value);
+    unpack8(load_global(x + base + (gate_first ? 0 : width8)), gate);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
       y[e] = __fmul_rn(value[e], __fdiv_rn(gate[e], __fadd_rn(1.0f, expf(-gate[e]))));
@@ -491,7 +491,7 @@ k_row_stats_parallel(const uint4 *x, const RowStats stats, uint64_t rows, uint32
     if (layer) {
       for (uint32_t c = lane; c < cols8; c += 32) {
         float f[8];
-        unpack8(__ldg(x + r * cols8 + c), f);
+        unpack8(load_global(x + r * cols8 + c), f);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
           mean += f[e];
@@ -500,7 +500,7 @@ k_row_stats_parallel(const uint4 *x, const RowStats stats, uint64_t rows, uint32
     }
     for (uint32_t c = lane; c < cols8; c += 32) {
       float f[8];
-      unpack8(__ldg(x + r * cols8 + c), f);
+      unpack8(load_global(x + r * cols8 + c), f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float d = __fsub_rn(f[e], mean);
@@ -516,7 +516,8 @@ k_row_stats_parallel(const uint4 *x, const RowStats stats, uint64_t rows, uint32
 
 // ---- RmsNormModulate, explicit scale / shift (cpu_executor.cpp:1241-1264) ----
 // One warp per row; lane l owns the 8-element groups l, l + 32, ... CHUNKS > 0: the row has
-// CHUNKS * 256 columns and stays in registers; CHUNKS == 0: any multiple of 256, read twice.
+// CHUNKS * 256 columns and stays in registers; CHUNKS == 0: any multiple of 256, read twice. Stores hold back the loads behind them, so
+// scale, shift and weight of a row in registers are all requested first: 16384 x 3072 158 us a chunk at a time, 84 so.
 template <int CHUNKS>
 __global__ void __launch_bounds__(256)
 k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const uint4 *b, uint4 *o, uint64_t rows,
@@ -536,7 +537,7 @@ k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const u
     float sum = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
-      const uint4 v = __ldg(xr + lane + 32u * k);
+      const uint4 v = load_global(xr + lane + 32u * k);
       if (CHUNKS > 0)
         kept[CHUNKS > 0 ? k : 0] = v;
       float f[8];
@@ -551,21 +552,34 @@ k_rms_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *a, const u
     const float inv = stats.at ? row_stat(stats, r).y
                                : __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(sum, (float)cols), eps)));
     __syncwarp(); // every lane has its copy: the row may be written
+    constexpr uint32_t kBatch = CHUNKS > 0 ? CHUNKS : 1; // chunks whose loads go out before the first is stored
 #pragma unroll
-    for (uint32_t k = 0; k < chunks; ++k) {
-      const uint32_t c = lane + 32u * k;
-      float f[8], wv[8], av[8], bv[8], y[8];
-      unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k : 0] : __ldg(xr + c), f);
-      unpack8(__ldg(a + r * cols8 + c), av);
-      unpack8(__ldg(b + r * cols8 + c), bv);
-      if (w)
-        unpack8(__ldg(w + c), wv);
+    for (uint32_t k0 = 0; k0 < chunks; k0 += kBatch) {
+      uint4 as[kBatch], bs[kBatch], ws[kBatch];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float normalized = __fmul_rn(__fmul_rn(f[e], inv), w ? wv[e] : 1.0f);
-        y[e] = __fadd_rn(__fmul_rn(normalized, __fadd_rn(1.0f, av[e])), bv[e]);
+      for (uint32_t j = 0; j < kBatch; ++j) {
+        const uint32_t c = lane + 32u * (k0 + j);
+        as[j] = load_global(a + r * cols8 + c);
+        bs[j] = load_global(b + r * cols8 + c);
+        if (w)
+          ws[j] = load_global(w + c);
       }
-      o[r * cols8 + c] = pack8(y);
+#pragma unroll
+      for (uint32_t j = 0; j < kBatch; ++j) {
+        const uint32_t c = lane + 32u * (k0 + j);
+        float f[8], wv[8], av[8], bv[8], y[8];
+        unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k0 + j : 0] : load_global(xr + c), f);
+        unpack8(as[j], av);
+        unpack8(bs[j], bv);
+        if (w)
+          unpack8(ws[j], wv);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float normalized = __fmul_rn(__fmul_rn(f[e], inv), w ? wv[e] : 1.0f);
+          y[e] = __fadd_rn(__fmul_rn(normalized, __fadd_rn(1.0f, av[e])), bv[e]);
+        }
+        o[r * cols8 + c] = pack8(y);
+      }
     }
   }
 }
@@ -593,7 +607,7 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
     float mean = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
-      const uint4 v = __ldg(xr + lane + 32u * k);
+      const uint4 v = load_global(xr + lane + 32u * k);
       if (CHUNKS > 0)
         kept[CHUNKS > 0 ? k : 0] = v;
       float f[8];
@@ -609,7 +623,7 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
 #pragma unroll
     for (uint32_t k = 0; k < chunks; ++k) {
       float f[8];
-      unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k : 0] : __ldg(xr + lane + 32u * k), f);
+      unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k : 0] : load_global(xr + lane + 32u * k), f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float d = __fsub_rn(f[e], mean);
@@ -623,11 +637,11 @@ k_layer_norm_modulate_bf16(const uint4 *x, const uint4 *w, const uint4 *b, const
     for (uint32_t k = 0; k < chunks; ++k) {
       const uint32_t c = lane + 32u * k;
       float f[8], wv[8], bv[8], sc[8], sh[8], y[8];
-      unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k : 0] : __ldg(xr + c), f);
-      unpack8(__ldg(w + c), wv);
-      unpack8(__ldg(b + c), bv);
-      unpack8(__ldg(scale + mrow + c), sc);
-      unpack8(__ldg(shift + mrow + c), sh);
+      unpack8(CHUNKS > 0 ? kept[CHUNKS > 0 ? k : 0] : load_global(xr + c), f);
+      unpack8(load_global(w + c), wv);
+      unpack8(load_global(b + c), bv);
+      unpack8(load_global(scale + mrow + c), sc);
+      unpack8(load_global(shift + mrow + c), sh);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float normalized =
@@ -667,10 +681,10 @@ struct RowRopeParams {
 __device__ __forceinline__ void load_table8(const void *table, uint32_t f32, uint64_t index, float (&v)[8]) {
   if (f32) {
     const float4 *p = reinterpret_cast<const float4 *>(static_cast<const float *>(table) + index);
-    const float4 lo = __ldg(p), hi = __ldg(p + 1);
+    const float4 lo = load_global(p), hi = load_global(p + 1);
     v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
   } else {
-    unpack8(__ldg(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(table) + index)), v);
+    unpack8(load_global(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(table) + index)), v);
   }
 }
 constexpr int kRopePitch = 17;  // uint4 per row in shared memory (16 + 1 pad)
@@ -706,7 +720,7 @@ k_qk_norm_rope_row128(const RowRopeParams p) {
   const int c1 = V2 || !rotates ? c0 + 1 : j + kRun / 2;
   uint64_t w[8];
   {
-    const uint4 a = __ldg(p.w + after + c0), b = __ldg(p.w + after + c1);
+    const uint4 a = load_global(p.w + after + c0), b = load_global(p.w + after + c1);
     const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -831,7 +845,7 @@ k_direct_quant_row128(const uint4 *x, int8_t *codes, float *scales, uint64_t row
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
     float f[8];
-    unpack8(__ldg(x + row * 16 + c), f);
+    unpack8(load_global(x + row * 16 + c), f);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       n[8 * c + e] = f[e];

@@ -80,7 +80,7 @@ struct Weights {
   uint4 low[kFewBatch], high[kFewBatch];
   template <bool READY>
   __device__ __forceinline__ void load(const Columns &columns, uint32_t K, uint32_t first) {
-    auto from = [](const int8_t *at) { return READY ? load_streamed(at) : load_produced(reinterpret_cast<const uint4 *>(at)); };
+    auto from = [](const int8_t *at) { return READY ? load_streamed(at) : load_produced_once(at); };
 #pragma unroll
     for (int u = 0; u < kFewBatch; ++u) {
       const uint32_t k = k_of(first, u);
@@ -103,8 +103,8 @@ struct Weights {
 };
 
 // GROUPS: of 8 rows. READY: no kernel that may still run writes the weights (GemmParams::weights_first). Otherwise they are
-// read like everything that the kernel in front produces: the non-coherent path is for what nobody writes meanwhile. (It is
-// the faster one: 8 x 12288 x 3072, weights not in L2, 11.0 us against 11.2.)
+// read like everything that the kernel in front produces: the non-coherent path is for what nobody writes meanwhile. (With
+// the same hint, no line in L1, they take the same time: 2 x 3072 x 12288, weights not in L2, 10.3 us both ways, with .cg 10.6.)
 template <int GROUPS, bool READY>
 __global__ void __launch_bounds__(32 * kFewWarps, 2)
 gemm_i8_few_rows_kernel(const FewParams f) {
@@ -178,7 +178,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t K = p.K, tiles = (p.N + 15u) / 16u, chunks = (K + 63u) / 64u, pitch = K + 16u;
   Weights w;
-  w.load<true>(Columns(f.w, blockIdx.x * 16u, p.N, K), K, 0); // (the grid has no more CTAs than tiles)
+  w.load<false>(Columns(f.w, blockIdx.x * 16u, p.N, K), K, 0); // (the grid has no more CTAs than tiles)
 
   uint8_t *codes = few_smem + kFewWarps * kWarpBytes256;
   float *maxima = reinterpret_cast<float *>(codes + p.M * pitch), *scales = maxima + kFusedBlocks;
@@ -191,8 +191,8 @@ w8a8_few_rows_kernel(const FusedParams f) {
     {
       const uint4 zero = make_uint4(0, 0, 0, 0);
       const uint4 *src = reinterpret_cast<const uint4 *>(f.x + after + (size_t)row * K + column + 16u * a);
-      const uint4 v[4] = {act_a ? __ldg(src) : zero, act_a ? __ldg(src + 1) : zero, act_b ? __ldg(src + 32) : zero,
-                          act_b ? __ldg(src + 33) : zero};
+      const uint4 v[4] = {act_a ? load_global(src) : zero, act_a ? load_global(src + 1) : zero, act_b ? load_global(src + 32) : zero,
+                          act_b ? load_global(src + 33) : zero};
       const uint32_t wa[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
       const uint32_t wb[8] = {v[2].x, v[2].y, v[2].z, v[2].w, v[3].x, v[3].y, v[3].z, v[3].w};
       uint64_t P[16];
@@ -254,7 +254,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
     int32_t c[4] = {};
     for (uint32_t first = 0; first < chunks; first += kFewWarps * kFewBatch) {
       if (first != 0u)
-        w.load<true>(Columns(f.w, tile * 16u, p.N, K), K, first);
+        w.load<false>(Columns(f.w, tile * 16u, p.N, K), K, first);
       uint4 x[kFewBatch];
 #pragma unroll
       for (int u = 0; u < kFewBatch; ++u) {
@@ -264,7 +264,7 @@ w8a8_few_rows_kernel(const FusedParams f) {
       w.multiply(c, x);
     }
     if (tile + gridDim.x < tiles)
-      w.load<true>(Columns(f.w, (tile + gridDim.x) * 16u, p.N, K), K, 0);
+      w.load<false>(Columns(f.w, (tile + gridDim.x) * 16u, p.N, K), K, 0);
     store_sums(sums + warp * 128, c);
     __syncthreads();
     const uint32_t row = threadIdx.x >> 4, n = tile * 16u + (threadIdx.x & 15u);

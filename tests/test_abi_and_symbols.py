@@ -151,3 +151,20 @@ def test_binding_is_built_again_for_another_torch_or_python(monkeypatch, tmp_pat
     assert not build._calls_stale([])
     monkeypatch.setattr(build.importlib.metadata, "version", lambda name: "0.1")
     assert build._calls_stale([])
+
+
+def test_kernels_launched_ahead_read_coherently():
+    """Non-coherent loads are for memory that nobody writes while the kernel lives. A kernel that is launched ahead lives while the one in front
+    writes what it will read: sources that launch kernels so, and the headers they share, have no such load but load_streamed, which is for
+    what was written further in front."""
+    csrc = os.path.join(ROOT, "diffusion_compiler_b200", "csrc")
+    found, ahead = {}, 0
+    for fn in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, fn)).read())
+        launches = fn.endswith((".cuh", ".h")) or "launch_ahead(" in text or "dependent_launch(" in text
+        ahead += launches and fn.endswith(".cu")
+        loads = len(re.findall(r"__ldg\s*\(|ld\.global\.nc|ld\.global(?:\.\w+)*\.nc", text))
+        if launches and loads:
+            found[fn] = loads
+    assert ahead >= 5 and found == {"common.cuh": 1}, found
+    assert open(os.path.join(csrc, "linear_few_rows.cu")).read().count("load_streamed(") == 1  # behind READY
