@@ -103,9 +103,9 @@ inline Divisor divisor(uint64_t by) { // 1 .. 2^31 - 1
 // all CTAs of that one have called grid_dependents_launch() (or ended) and there is room. Its set-up runs then; what
 // the kernel in front wrote is read behind grid_dependency_wait(), which every thread passes that touches global
 // memory, and through loads that the compiler cannot move up: load_produced, TMA, or addresses that the wait is a part of
-// (grid_dependency_wait_zero). None of them is non-coherent (__ldg): that path is for memory that nobody writes while the
-// kernel lives, and this one lives while the one in front writes. A kernel that lets dependents start waits first: when a kernel starts, the one two in front
-// is complete.
+// (grid_dependency_wait_zero; the assembler keeps coherent loads behind the wait by itself). None of them is non-coherent
+// (__ldg): that path is for memory that nobody writes while the kernel lives, and this one lives while the one in front
+// writes. A kernel that lets dependents start waits first: when a kernel starts, the one two in front is complete.
 // Two reads are not behind such a wait. Both are of what a kernel further in front wrote, and both hold only because
 // the kernel in between waited before it let anything start (then that kernel is complete):
 // * the first weights of a GEMM, requested ahead in w8a8_linear, whose quantiser is the kernel in between;

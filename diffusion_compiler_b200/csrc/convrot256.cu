@@ -6,13 +6,9 @@ namespace {
 
 template <bool SIGNED, bool F32>
 int launch_variant(const QuantParams &p, cudaStream_t stream) {
-  const bool norm = p.norm_scale != nullptr;
-  if (norm && p.rcodes)
-    return fail(kUnsupported, "QuantizeInt8Rows: weight packing (MSE scale, input equalisation) exists for "
-                              "the 256-wide variants without residual outputs");
   if (p.rcodes)
     return launch_single<SIGNED, F32, true, kPlain>(p, stream);
-  if (norm)
+  if (p.norm_scale)
     return p.norm_bias ? launch_single<SIGNED, F32, false, kLayer>(p, stream) : launch_single<SIGNED, F32, false, kNorm>(p, stream);
   return launch_single<SIGNED, F32, false, kPlain>(p, stream);
 }

@@ -24,7 +24,7 @@
 // blocks at a time to save per-row work. Before -> now, us: 33272 x 3072 83.9 -> 71.8 (4.3 TB/s), 33272 x 8192 220.6 -> 181.7,
 // 9216 x 12288 100.4 -> 78.8, 4608 x (3072 + 12288) 70.0 -> 54.2, 2 x 3072 2.8 -> 2.6, the scale search of the weight form
 // 12288 x 3072 64.7 -> 56.5 (all lanes evaluate samples, in doubles only where candidates are close), with input
-// equalisation 94.2 -> 62.6 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 85.3 with its
+// equalisation 94.2 -> 63.1 (a table of reciprocals, packed sums), RmsNormModulate in front of 16384 x 3072 92.0 -> 85.3 with its
 // statistic. Staging the input with bulk copies through shared memory instead of registers gave nothing, nor (3 to 8 % slower) did
 // scale and shift of a norm's next row prefetched into L2.
 #pragma once
@@ -137,7 +137,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   // Input equalisation divides every row by the same vector e: the CTA's rows share a table of 1 / e as the sum of two fp32 numbers,
   // good to 2^-48, so that w / e is a product and a fused sum. (The quotient of two 8-bit significands is never within 2^-33 of a
   // rounding boundary of fp32.) Reciprocal, residual and correction in every row: packing 12288 x 3072 with
-  // the search 71.6 us, with the table and the prefetch that its registers allow 65.2 (16384 rows, seven full rounds, 94.8 and 79.0).
+  // the search 70.0 us, with the table and the prefetch that its registers allow 63.1 (16384 rows, seven full rounds, 91.0 and 77.4).
   const uint32_t table_addr = smem_addr + table_offset<SIGNED, EXTRA, NIT>((uint32_t)total_warps);
   bool equalise_fast = true; // this warp's entries are of ordinary magnitude
   if (kTable) {
@@ -247,7 +247,7 @@ convrot256_kernel(const QuantParams p, const int warps_per_row, const int rows_p
   };
 
   const uint64_t row_step = (uint64_t)gridDim.x * rows_per_cta;
-  // Where a CTA has all rows of an SM, those of a last round are spread over the SMs (12288 x 3072 with the table 71.0 -> 67.0 us);
+  // Where a CTA has all rows of an SM, those of a last round are spread over the SMs (12288 x 3072 with the table 66.5 -> 63.1 us);
   // of smaller CTAs every SM gets its share of a last round anyway.
   uint64_t row = kTable ? (uint64_t)slot * gridDim.x + blockIdx.x : (uint64_t)blockIdx.x * rows_per_cta + slot;
   uint4 next[4];

@@ -20,10 +20,10 @@ int launch_pack(const QuantParams &p, bool f32, cudaStream_t stream) {
   const bool three = blocks % 3u == 0u && p.rows * blocks > (uint64_t)sm_count() * 24u;
   if (p.equalise) {
     // With input equalisation one CTA per SM, whose rows share the table: 16 warps of three blocks with a prefetch, or 24 of one. The
-    // table takes 1.5 us, so from three rounds of 24 warps per SM on, and not where rows of more than 8 blocks leave warps idle. Every
-    // row its own reciprocals / table: 16384 x 3072 94.8 / 79.0, 12288 x 3072 71.6 / 65.2, 3072 x 12288 72.6 / 69.2, 3072 x 8192
-    // 53.9 / 52.1, fp32 112.3 / 94.5, 86.0 / 74.2, 88.7 / 84.3, 58.2 / 54.5; but 1500 x 10240 39.4 / 41.6, 3000 x 2304 25.8 / 26.9,
-    // 3000 x 512 12.3 / 13.9.
+    // table takes 1.5 us, so from three rounds of 24 warps per SM on, and not where rows of more than 8 blocks leave warps idle. From a
+    // graph, every row its own reciprocals / table: 16384 x 3072 91.0 / 77.4, 12288 x 3072 70.0 / 63.1, 3072 x 12288 70.4 / 67.7, 3072 x
+    // 8192 51.2 / 52.2, fp32 107.5 / 93.4, 80.3 / 73.1, 86.9 / 84.1, 55.6 / 54.3; but 1500 x 10240 34.9 / 39.2, 3000 x 2304 20.4 / 21.9,
+    // 3000 x 512 9.0 / 10.7.
     if (p.rows * blocks >= (uint64_t)sm_count() * 72u && (blocks % 3u == 0u || blocks <= 8u))
       return f32     ? launch_form<SIGNED, true, false, kPackTable, 1, false, 768, 1>(p, stream)
              : three ? launch_form<SIGNED, false, false, kPackTable, 3, true, 512, 1>(p, stream)
