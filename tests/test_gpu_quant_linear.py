@@ -285,9 +285,12 @@ def test_linear_of_few_rows_directly_behind_the_kernel_that_writes_its_weights(o
     """The weights' codes are written into the same buffer again and again, by kernels that let the linear start early, with no
     synchronisation in between: every linear reads the codes written directly in front of it."""
     import torch
+    # a 256-wide quantiser with one batch of four rows per CTA, three CTAs on an SM, lets the next kernel start when it starts itself
+    N = 1200
+    assert N <= 3 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
     g = torch.Generator(device="cuda").manual_seed(rows)
-    weights = [torch.randn((3000, 2048), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
-    codes, scales = torch.empty((3000, 2048), dtype=torch.int8, device="cuda"), torch.empty(3000, device="cuda")
+    weights = [torch.randn((N, 2048), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    codes, scales = torch.empty((N, 2048), dtype=torch.int8, device="cuda"), torch.empty(N, device="cuda")
     x8 = torch.randint(-127, 128, (rows, 2048), generator=g, device="cuda", dtype=torch.int8)
     xs = torch.rand(rows, generator=g, device="cuda")
     from diffusion_compiler_b200 import _lib
@@ -296,7 +299,7 @@ def test_linear_of_few_rows_directly_behind_the_kernel_that_writes_its_weights(o
         if packer == "quantize":
             ops.quantize_int8_rows([w], 2, out=(codes, scales))
         else:
-            ops._call(_lib.lib().difb200_quantize_weight_rows, 0, w.data_ptr(), None, 3000, 2048, 2, 0, codes.data_ptr(),
+            ops._call(_lib.lib().difb200_quantize_weight_rows, 0, w.data_ptr(), None, N, 2048, 2, 0, codes.data_ptr(),
                       scales.data_ptr())
 
     want = []
@@ -308,6 +311,7 @@ def test_linear_of_few_rows_directly_behind_the_kernel_that_writes_its_weights(o
     got = []
     for _ in range(4):
         for w in weights:
+            torch.cuda._sleep(400_000)  # clocks: the host enqueues both meanwhile
             write(w)
             got.append(ops.linear_int8_scaled(x8, codes, xs, scales))
     for i, out in enumerate(got):
