@@ -416,7 +416,7 @@ void plan(Executable &exe) {
   }
   // A Slice whose elements are neighbours (nothing in front of its axis is repeated) may be a part of its input's buffer, where
   // that starts as kernels expect (16 bytes); settle_slices has the last word. At batch 1 the modulation vectors of a block, its streams' rows of the joint
-  // sequence: MMDiT block of 256 + 77 tokens, 15 of 51 launches. (Not token-sharded: there V's buffer is placed by its chain of aliases.)
+  // sequence: MMDiT block of 256 + 77 tokens, 16 of 51 launches. (Not token-sharded: there V's buffer is placed by its chain of aliases.)
   for (Step &st : exe.steps) {
     if (st.op->opcode != ir::Slice || st.skip || exe.ctx->world)
       continue;
